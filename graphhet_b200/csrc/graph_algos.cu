@@ -45,7 +45,7 @@ int cdlp_run(ghb_workspace* ws, int32_t n, const int32_t* rp, const int32_t* col
 int tc_run(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int32_t* col, int64_t* counts64,
            int32_t* counts32, int64_t* total);
 int tc_run_cached(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int32_t* col, int64_t* counts64,
-                  int32_t* counts32, int64_t* total, std::atomic<int32_t>* flags_cache);
+                  int32_t* counts32, int64_t* total, std::atomic<int32_t>* flags_cache, bool ranked);
 int pagerank_run(ghb_workspace* ws, int32_t n, const int32_t* in_rp, const int32_t* in_col, const int32_t* out_rp,
                  const ghb_pr_options* o, double* rank, int32_t* iters_run);
 int msbfs_batch(ghb_workspace* ws, int32_t n, int32_t n_active, const int32_t* out_rp, const int32_t* out_col,
@@ -378,7 +378,7 @@ int ghb_graph_tc(ghb_workspace* ws, const ghb_graph* g, int64_t* counts64, int32
     GRAPH_PRELUDE();
     GHB_TRY(ws_reserve_stage(ws, sizeof(int64_t) * (size_t)g->n));
     int64_t* cnew = static_cast<int64_t*>(ws->stage);
-    GHB_TRY(tc_run_cached(ws, g->n, g->rowptr, g->col, cnew, nullptr, total, &g->tc_flags));
+    GHB_TRY(tc_run_cached(ws, g->n, g->rowptr, g->col, cnew, nullptr, total, &g->tc_flags, true));
     return launch(ws, tc_map_kernel, dim3(grid_for(g->n, 256, ws->num_sms * 8)), dim3(256), 0, g->n,
                   (const int32_t*)g->perm, (const int64_t*)cnew, counts64, counts32);
 }

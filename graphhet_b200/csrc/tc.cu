@@ -16,6 +16,7 @@
 //
 // Any other input takes the generic path: the reference's merge over every
 // entry, kept for exact parity on directed or unusual inputs.
+#include <algorithm>
 #include <atomic>
 
 #include "common.cuh"
@@ -193,8 +194,10 @@ __global__ void __launch_bounds__(1024) orient_fill_long_kernel(const int32_t* _
     }
 }
 
+// Oriented rows N+(v) = ocol[rb[v] .. re[v]).
 struct OrientedVisitor {
-    const int32_t* orp;
+    const int32_t* rb;
+    const int32_t* re;
     const int32_t* ocol;
     unsigned long long* cnt;
     __device__ bool want_row(int32_t) const { return true; }
@@ -206,8 +209,8 @@ struct OrientedVisitor {
         // way round.  (Swapping whenever N+(v) is longer measured 4 % slower
         // on 2,000 small ER graphs and 10 % slower on RMAT scale 24; plain
         // binary searches from the last hit 1.46x slower on RMAT scale 24.)
-        int32_t sb = orp[v], se = orp[v + 1];
-        int32_t lb = orp[u], le = orp[u + 1];
+        int32_t sb = rb[v], se = re[v];
+        int32_t lb = rb[u], le = re[u];
         if (se - sb > 64 && se - sb > 4 * (le - lb)) {
             const int32_t tb = sb, te = se;
             sb = lb;
@@ -283,7 +286,8 @@ __device__ __forceinline__ bool tc_probe(const int32_t* keys, uint32_t mask, int
 // Adds w's hits to cnt, b's to bc[(index in N+(a)) - bc_off]; returns a's
 // hits (lane 0 holds those of whole-warp lists, every lane those it probed
 // itself).
-__device__ __forceinline__ unsigned long long tc_row_share(const int32_t* __restrict__ orp,
+__device__ __forceinline__ unsigned long long tc_row_share(const int32_t* __restrict__ rb,
+                                                           const int32_t* __restrict__ re,
                                                            const int32_t* __restrict__ ocol, int32_t ab, int32_t k,
                                                            int32_t g0, int32_t g_end, int32_t stride,
                                                            const int32_t* keys, uint32_t mask, int shift, int32_t* bc,
@@ -296,8 +300,8 @@ __device__ __forceinline__ unsigned long long tc_row_share(const int32_t* __rest
         int32_t lb = 0, le = 0;
         if (i < g_end) {
             const int32_t b = ocol[ab + i];
-            lb = orp[b];
-            le = orp[b + 1];
+            lb = rb[b];
+            le = re[b];
             // Only N+(b)'s entries inside [min N+(a), max N+(a)] can be in
             // N+(a) (both rows ascending): lists over trim_min entries are
             // cut to that range first (two binary searches, a chain of
@@ -386,7 +390,9 @@ __device__ __forceinline__ unsigned long long tc_row_share(const int32_t* __rest
 // tails: [0], [1], [2] the three item counts, [3] the huge rows.
 // (Eight blocks per SM, 32 registers: 774-787 ms for RMAT-24 TC against
 // 789-797 ms at six blocks.)
-__global__ void __launch_bounds__(kTcWarpBlock, 8) tc_hash_warp_kernel(int32_t n, const int32_t* __restrict__ orp,
+__global__ void __launch_bounds__(kTcWarpBlock, 8) tc_hash_warp_kernel(int32_t first, int32_t n,
+                                                                    const int32_t* __restrict__ rb,
+                                                                    const int32_t* __restrict__ re,
                                                                     const int32_t* __restrict__ ocol,
                                                                     unsigned long long* cnt, int2* items,
                                                                     int64_t item_cap, int32_t* huge, int32_t* tails,
@@ -398,8 +404,8 @@ __global__ void __launch_bounds__(kTcWarpBlock, 8) tc_hash_warp_kernel(int32_t n
     int32_t* bc = s_bc[threadIdx.x >> 5];
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t a = warp; a < n; a += nwarps) {
-        const int32_t ab = orp[a], k = orp[a + 1] - ab;
+    for (int64_t a = (int64_t)first + warp; a < n; a += nwarps) {
+        const int32_t ab = rb[a], k = re[a] - ab;
         if (k == 0) continue;
         if (k > kTcWarpRow) {
             if (k <= block_row) {
@@ -422,7 +428,7 @@ __global__ void __launch_bounds__(kTcWarpBlock, 8) tc_hash_warp_kernel(int32_t n
         for (int32_t i = lane; i < k; i += 32) tc_insert(keys, kTcWarpSlots - 1, shift, ocol[ab + i]);
         __syncwarp();
         unsigned long long a_hits =
-            tc_row_share(orp, ocol, ab, k, 0, k, 32, keys, kTcWarpSlots - 1, shift, bc, 0, cnt, trim_min);
+            tc_row_share(rb, re, ocol, ab, k, 0, k, 32, keys, kTcWarpSlots - 1, shift, bc, 0, cnt, trim_min);
         __syncwarp();
         a_hits = warp_sum(a_hits);
         if (lane == 0 && a_hits) atomicAdd(cnt + a, a_hits);
@@ -439,7 +445,8 @@ __global__ void __launch_bounds__(kTcWarpBlock, 8) tc_hash_warp_kernel(int32_t n
 // keep many rows in flight per SM; slices spread the longest rows over
 // many blocks.  DYN: the hash lives in dynamic shared memory.
 template <int CAP_LOG2, bool DYN>
-__global__ void __launch_bounds__(kTcBlockThreads) tc_hash_slice_kernel(const int32_t* __restrict__ orp,
+__global__ void __launch_bounds__(kTcBlockThreads) tc_hash_slice_kernel(const int32_t* __restrict__ rb,
+                                                                        const int32_t* __restrict__ re,
                                                                         const int32_t* __restrict__ ocol,
                                                                         unsigned long long* cnt, const int2* items,
                                                                         const int32_t* count, int32_t trim_min) {
@@ -453,7 +460,7 @@ __global__ void __launch_bounds__(kTcBlockThreads) tc_hash_slice_kernel(const in
     for (int32_t r = blockIdx.x; r < nitems; r += gridDim.x) {
         const int2 it = items[r];
         const int32_t a = it.x, gs = it.y;
-        const int32_t ab = orp[a], k = orp[a + 1] - ab;
+        const int32_t ab = rb[a], k = re[a] - ab;
         const int32_t ge = min(k, gs + kTcSlice);
         int log2cap = 1;
         while ((1 << log2cap) < 2 * k) ++log2cap;
@@ -465,7 +472,7 @@ __global__ void __launch_bounds__(kTcBlockThreads) tc_hash_slice_kernel(const in
         const int shift = 32 - log2cap;
         for (int32_t i = threadIdx.x; i < k; i += blockDim.x) tc_insert(keys, cap - 1, shift, ocol[ab + i]);
         __syncthreads();
-        unsigned long long a_hits = tc_row_share(orp, ocol, ab, k, gs + warp_in_block * 32, ge, warps * 32, keys,
+        unsigned long long a_hits = tc_row_share(rb, re, ocol, ab, k, gs + warp_in_block * 32, ge, warps * 32, keys,
                                                  cap - 1, shift, s_bc, gs, cnt, trim_min);
         a_hits = warp_sum(a_hits);
         if (lane_id() == 0 && a_hits) atomicAdd(&s_hits, a_hits);
@@ -500,23 +507,26 @@ size_t tc_lists_ints(int32_t n, int64_t m) { return (size_t)(6 * tc_item_cap(n, 
 
 namespace {
 
-int tc_count_oriented(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* orp, const int32_t* ocol,
-                      unsigned long long* cnt, const WalkBuffers& wb, int32_t* lists) {
+// Rows first .. n - 1 of the oriented CSR N+(v) = ocol[rb[v] .. re[v]) (the
+// rows below `first` are empty).
+int tc_count_oriented(ghb_workspace* ws, int32_t first, int32_t n, int64_t m, const int32_t* rb, const int32_t* re,
+                      const int32_t* ocol, unsigned long long* cnt, const WalkBuffers& wb, int32_t* lists) {
+    const OrientedVisitor gallop{rb, re, ocol, cnt};
     if (!ws->tune.tc_hash)
-        return walk(ws, orp, ocol, (const int32_t*)nullptr, (const int32_t*)nullptr, (int64_t)n, (int64_t)n, wb,
-                    OrientedVisitor{orp, ocol, cnt});
+        return walk_range(ws, rb, re, ocol, (const int32_t*)nullptr, (const int32_t*)nullptr, (int64_t)n, (int64_t)n,
+                          wb, gallop);
     const int64_t item_cap = tc_item_cap(n, m);
     int2* items = reinterpret_cast<int2*>(lists);
     int32_t* huge = lists + 6 * item_cap;
     int32_t* tails = huge + n;
     GHB_CUDA_TRY(cudaMemsetAsync(tails, 0, 4 * sizeof(int32_t), ws->stream));
-    GHB_TRY(launch(ws, tc_hash_warp_kernel, dim3(grid_for((int64_t)n * 32, kTcWarpBlock, ws->num_sms * 8)),
-                   dim3(kTcWarpBlock), 0, n, orp, ocol, cnt, items, item_cap, huge, tails,
+    GHB_TRY(launch(ws, tc_hash_warp_kernel, dim3(grid_for((int64_t)(n - first) * 32, kTcWarpBlock, ws->num_sms * 8)),
+                   dim3(kTcWarpBlock), 0, first, n, rb, re, ocol, cnt, items, item_cap, huge, tails,
                    std::min<int32_t>(std::max<int32_t>(ws->tune.tc_block_row, kTcWarpRow), kTcBlockRow),
                    ws->tune.tc_trim_min));
     GHB_TRY(launch(ws, tc_hash_slice_kernel<kTcMidLog2, false>, dim3(ws->num_sms * ws->tune.tc_slice_blocks),
-                   dim3(kTcBlockThreads), 0,
-                   orp, ocol, cnt, (const int2*)items, (const int32_t*)tails, ws->tune.tc_trim_min));
+                   dim3(kTcBlockThreads), 0, rb, re, ocol, cnt, (const int2*)items, (const int32_t*)tails,
+                   ws->tune.tc_trim_min));
     const size_t smem = sizeof(int32_t) << kTcBigLog2;
     static bool attr_set[64] = {false};
     if (ws->device >= 0 && ws->device < 64 && !attr_set[ws->device]) {
@@ -524,15 +534,346 @@ int tc_count_oriented(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* or
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr_set[ws->device] = true;
     }
-    GHB_TRY(launch(ws, tc_hash_slice_kernel<kTcMid2Log2, false>, dim3(ws->num_sms * 6), dim3(kTcBlockThreads), 0,
-                   orp, ocol, cnt, (const int2*)(items + item_cap), (const int32_t*)(tails + 1),
+    GHB_TRY(launch(ws, tc_hash_slice_kernel<kTcMid2Log2, false>, dim3(ws->num_sms * 6), dim3(kTcBlockThreads), 0, rb,
+                   re, ocol, cnt, (const int2*)(items + item_cap), (const int32_t*)(tails + 1),
                    ws->tune.tc_trim_min));
-    GHB_TRY(launch(ws, tc_hash_slice_kernel<kTcBigLog2, true>, dim3(ws->num_sms * 3), dim3(kTcBlockThreads), smem,
-                   orp, ocol, cnt, (const int2*)(items + 2 * item_cap), (const int32_t*)(tails + 2),
+    GHB_TRY(launch(ws, tc_hash_slice_kernel<kTcBigLog2, true>, dim3(ws->num_sms * 3), dim3(kTcBlockThreads), smem, rb,
+                   re, ocol, cnt, (const int2*)(items + 2 * item_cap), (const int32_t*)(tails + 2),
                    ws->tune.tc_trim_min));
     // Rows over the block path's length: the galloping walk.
-    return walk(ws, orp, ocol, (const int32_t*)huge, (const int32_t*)(tails + 3), (int64_t)0,
-                (int64_t)ws->num_sms * 64, wb, OrientedVisitor{orp, ocol, cnt});
+    return walk_range(ws, rb, re, ocol, (const int32_t*)huge, (const int32_t*)(tails + 3), (int64_t)0,
+                      (int64_t)ws->num_sms * 64, wb, gallop);
+}
+
+// ---- hub bitmaps: triangles whose lowest id is a hub, on rank-ordered CSRs
+//
+// In a resident graph ids are ranks by degree, so N+(v) = {w in row(v): w < v}
+// is a prefix of the sorted row (no oriented copy is made), and most of it
+// lies among the first kTcHubs ids: on RMAT, 98 % of all probes at scale 18.
+// There a vertex's hub neighbours are one kTcHubs-bit row, 16 bytes per lane of a
+// warp, and |N+(a) and N+(b) and hubs| is an AND and a popcount of it: about
+// 27 instructions for 4,096 ids, where probing b's list costs about 15 for 32
+// entries.  The triangle's third count, w's, comes from the AND's bits: each
+// lane adds the words of successive b into bit-sliced counters (Harley-Seal
+// carry-save adders, 3.3 LOP3 per word and b), so a row ends with one atomic
+// per hub neighbour instead of one per triangle.
+//
+// Triangles without a hub lie in the rows' tails [he, oe) and go to the hash
+// kernels.  b below kTcBitMin hub neighbours, or of an id past the bitmap
+// table, has its hub neighbours probed one by one in a's bitmap.
+constexpr int32_t kTcHubs = 4096;
+constexpr int32_t kTcHubWords = kTcHubs / 32;
+constexpr int32_t kTcBitRows = 1 << 18;  // ids that may have a bitmap (512 bytes each, 128 MB)
+constexpr int32_t kTcBitMin = 32;        // hub neighbours from which a vertex has one
+constexpr int32_t kTcHubDirect = 8;      // rows over this many entries are listed as items
+constexpr int32_t kTcHubSlice = 128;     // entries of N+(a) per item: counts fit eight bit slices
+constexpr int kTcHubThreads = 128;
+constexpr int kTcHubBlocks = 4;  // per SM: 120 registers a thread
+constexpr int kTcSlices = 8;
+
+// oe[u]: end of N+(u); he[u]: end of its hub part.
+__global__ void tc_rank_ends_kernel(int32_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ col,
+                                    int32_t* he, int32_t* oe) {
+    for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t b = rp[u], e = rp[u + 1];
+        const int32_t o = b < e ? upper_bound_pos(col, b, e, (int32_t)u - 1) : b;
+        oe[u] = o;
+        he[u] = u <= kTcHubs ? o : (b < o ? upper_bound_pos(col, b, o, kTcHubs - 1) : b);
+    }
+}
+
+// Warp w's kTcHubWords shared words: the hub bits of entries [b, e).
+__device__ __forceinline__ uint4 tc_hub_bits(const int32_t* __restrict__ col, int32_t b, int32_t e, uint32_t* words) {
+    const int lane = lane_id();
+    reinterpret_cast<uint4*>(words)[lane] = make_uint4(0, 0, 0, 0);
+    __syncwarp();
+    for (int32_t j = b + lane; j < e; j += 32) {
+        const int32_t w = col[j];
+        atomicOr(words + (w >> 5), 1u << (w & 31));
+    }
+    __syncwarp();
+    return reinterpret_cast<const uint4*>(words)[lane];
+}
+
+__global__ void __launch_bounds__(256) tc_hub_bitmap_kernel(int32_t rows, const int32_t* __restrict__ rp,
+                                                            const int32_t* __restrict__ he,
+                                                            const int32_t* __restrict__ col, uint4* bits) {
+    __shared__ __align__(16) uint32_t s_words[8][kTcHubWords];
+    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t u = warp; u < rows; u += nwarps) {
+        const int32_t b = rp[u], e = he[u];
+        if (e - b < kTcBitMin) continue;
+        bits[u * 32 + lane_id()] = tc_hub_bits(col, b, e, s_words[threadIdx.x >> 5]);
+        __syncwarp();
+    }
+}
+
+// s, c = sum and carry of three bits per position.
+__device__ __forceinline__ void csa(uint32_t& s, uint32_t& c, uint32_t x, uint32_t y) {
+    const uint32_t t = s;
+    s = t ^ x ^ y;
+    c = (t & x) | (t & y) | (x & y);
+}
+
+// Counts of a block: hubs in shared memory (the top hubs' counts change with
+// nearly every entry, and reductions to one line of L2 are served one after
+// another: RMAT-20 took 2.8 ms with every count in global memory), others in
+// global memory.  A vertex is in fewer triangles than the graph has edges, so
+// 32 bits hold a hub's.
+struct TcCounts {
+    uint32_t* hub;
+    unsigned long long* cnt;
+    __device__ __forceinline__ void add(int32_t v, uint32_t x) const {
+        if (v < kTcHubs) atomicAdd(hub + v, x);
+        else atomicAdd(cnt + v, (unsigned long long)x);
+    }
+    __device__ __forceinline__ void clear() const {
+        for (int i = threadIdx.x; i < kTcHubs; i += blockDim.x) hub[i] = 0;
+        __syncthreads();
+    }
+    __device__ __forceinline__ void flush() const {
+        __syncthreads();
+        for (int i = threadIdx.x; i < kTcHubs; i += blockDim.x)
+            if (hub[i]) atomicAdd(cnt + i, (unsigned long long)hub[i]);
+    }
+};
+
+// Entries [g0, g1) of N+(a) against N+(a)'s hub part: adds every triangle
+// (a, b, w), w a hub, to its three counts.
+__device__ __forceinline__ void tc_hub_row(int32_t a, int32_t g0, int32_t g1, const int32_t* __restrict__ rp,
+                                           const int32_t* __restrict__ he, const int32_t* __restrict__ col,
+                                           const uint4* __restrict__ bits, int32_t bit_rows, const TcCounts& cnt,
+                                           uint32_t* words) {
+    const int lane = lane_id();
+    const int32_t ab = rp[a], ah = he[a];
+    __syncwarp();
+    uint32_t A[4];
+    {
+        uint4 x;
+        if (a < bit_rows && ah - ab >= kTcBitMin) {
+            x = bits[(int64_t)a * 32 + lane];
+            reinterpret_cast<uint4*>(words)[lane] = x;
+            __syncwarp();
+        } else {
+            x = tc_hub_bits(col, ab, ah, words);
+        }
+        A[0] = x.x, A[1] = x.y, A[2] = x.z, A[3] = x.w;
+    }
+    uint32_t S[kTcSlices][4];
+#pragma unroll
+    for (int s = 0; s < kTcSlices; ++s)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) S[s][i] = 0;
+    uint32_t a_hits = 0;
+    for (int32_t g = g0; g < g1; g += 32) {
+        const int32_t i = g + lane;
+        int32_t b = -1, lb = 0, d = 0;
+        if (i < g1) {
+            b = col[ab + i];
+            lb = rp[b];
+            d = he[b] - lb;
+        }
+        const bool dense = b >= 0 && b < bit_rows && d >= kTcBitMin;
+        unsigned mask = __ballot_sync(0xffffffffu, dense);
+        while (mask) {
+            uint4 x[8];
+            int32_t mine = 0;  // lane q < 8 keeps the q-th b of this group
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int32_t bq = __shfl_sync(0xffffffffu, b, mask ? __ffs(mask) - 1 : 0);
+                x[q] = make_uint4(0, 0, 0, 0);
+                if (mask && lane * 128 < bq) x[q] = __ldg(bits + (int64_t)bq * 32 + lane);  // N+(b) < b
+                if (lane == q) mine = mask ? bq : -1;
+                mask &= mask - 1;
+            }
+            uint32_t sum = 0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                x[q].x &= A[0];
+                x[q].y &= A[1];
+                x[q].z &= A[2];
+                x[q].w &= A[3];
+                const uint32_t p = __popc(x[q].x) + __popc(x[q].y) + __popc(x[q].z) + __popc(x[q].w);
+                a_hits += p;
+                const uint32_t all = __reduce_add_sync(0xffffffffu, p);
+                if (lane == q) sum = all;
+            }
+            if (sum) cnt.add(mine, sum);
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                uint32_t v[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    v[q] = w == 0 ? x[q].x : w == 1 ? x[q].y : w == 2 ? x[q].z : x[q].w;
+                uint32_t t0, t1, f0, f1, c;
+                csa(S[0][w], t0, v[0], v[1]);
+                csa(S[0][w], t1, v[2], v[3]);
+                csa(S[1][w], f0, t0, t1);
+                csa(S[0][w], t0, v[4], v[5]);
+                csa(S[0][w], t1, v[6], v[7]);
+                csa(S[1][w], f1, t0, t1);
+                csa(S[2][w], c, f0, f1);
+#pragma unroll
+                for (int s = 3; s < kTcSlices; ++s) {
+                    const uint32_t t = S[s][w] & c;
+                    S[s][w] ^= c;
+                    c = t;
+                }
+            }
+        }
+        // The other b: their hub neighbours packed warp-wide over a scan of
+        // the counts, each probed in a's bitmap.
+        if (dense) d = 0;
+        if (__any_sync(0xffffffffu, d > 0)) {
+            int32_t incl = d;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += x;
+            }
+            const int32_t excl = incl - d;
+            const int32_t total = __shfl_sync(0xffffffffu, incl, 31);
+            for (int32_t k0 = 0; k0 < total; k0 += 32) {
+                const int32_t k = k0 + lane;
+                int owner = 0;
+#pragma unroll
+                for (int s = 16; s >= 1; s >>= 1) {
+                    const int32_t ev = __shfl_sync(0xffffffffu, excl, owner + s);
+                    if (ev <= k) owner += s;
+                }
+                const int32_t ob = __shfl_sync(0xffffffffu, lb, owner);
+                const int32_t oe = __shfl_sync(0xffffffffu, excl, owner);
+                const int32_t bo = __shfl_sync(0xffffffffu, b, owner);
+                if (k < total) {
+                    const int32_t w = col[ob + (k - oe)];
+                    if ((words[w >> 5] >> (w & 31)) & 1u) {
+                        cnt.add(bo, 1);
+                        cnt.add(w, 1);
+                        ++a_hits;
+                    }
+                }
+            }
+        }
+    }
+    a_hits = __reduce_add_sync(0xffffffffu, a_hits);
+    if (a_hits == 0) return;
+    if (lane == 0) cnt.add(a, a_hits);
+    // The slices back to counts, a lane per hub neighbour of a.  (A lane per
+    // word, walking its own set bits, took longer than the loop above: the
+    // lowest ids' words are full and the others nearly empty.)
+    __syncwarp();
+    uint4* slices = reinterpret_cast<uint4*>(words);
+#pragma unroll
+    for (int s = 0; s < kTcSlices; ++s) slices[s * 32 + lane] = make_uint4(S[s][0], S[s][1], S[s][2], S[s][3]);
+    __syncwarp();
+    for (int32_t j = ab + lane; j < ah; j += 32) {
+        const int32_t w = col[j];
+        uint32_t c = 0;
+#pragma unroll
+        for (int s = 0; s < kTcSlices; ++s) c |= ((words[s * kTcHubWords + (w >> 5)] >> (w & 31)) & 1u) << s;
+        if (c) cnt.add(w, c);
+    }
+}
+
+// Rows with a hub neighbour and two entries or more, 32 rows per warp's step
+// (their bounds in one load each); rows over kTcHubDirect entries are listed
+// as slices for tc_hub_items_kernel.
+__global__ void __launch_bounds__(kTcHubThreads, kTcHubBlocks) tc_hub_rows_kernel(
+    int32_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ he, const int32_t* __restrict__ oe,
+    const int32_t* __restrict__ col, const uint4* __restrict__ bits, int32_t bit_rows, unsigned long long* cnt,
+    int2* items, int32_t* tail, int32_t* next) {
+    __shared__ __align__(16) uint32_t s_words[kTcHubThreads / 32][kTcSlices * kTcHubWords];
+    __shared__ uint32_t s_hub[kTcHubs];
+    const TcCounts counts{s_hub, cnt};
+    counts.clear();
+    uint32_t* words = s_words[threadIdx.x >> 5];
+    const int lane = lane_id();
+    while (true) {
+        // Rows differ by orders of magnitude: each warp draws its next 32.
+        int32_t base = 0;
+        if (lane == 0) base = atomicAdd(next, 1);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if ((int64_t)base * 32 >= n) break;
+        const int64_t u = (int64_t)base * 32 + lane;
+        int32_t k = 0;
+        if (u < n) {
+            const int32_t b = rp[u];
+            k = he[u] > b ? oe[u] - b : 0;
+        }
+        if (k > kTcHubDirect) {
+            const int32_t ns = (k + kTcHubSlice - 1) / kTcHubSlice;
+            const int32_t pos = atomicAdd(tail, ns);
+            for (int32_t s = 0; s < ns; ++s) items[pos + s] = make_int2((int32_t)u, s * kTcHubSlice);
+            k = 0;
+        }
+        unsigned rows = __ballot_sync(0xffffffffu, k >= 2);
+        while (rows) {
+            const int l = __ffs(rows) - 1;
+            rows &= rows - 1;
+            const int32_t kl = __shfl_sync(0xffffffffu, k, l);
+            tc_hub_row(base * 32 + l, 0, kl, rp, he, col, bits, bit_rows, counts, words);
+        }
+    }
+    counts.flush();
+}
+
+__global__ void __launch_bounds__(kTcHubThreads, kTcHubBlocks) tc_hub_items_kernel(
+    const int32_t* __restrict__ rp, const int32_t* __restrict__ he, const int32_t* __restrict__ oe,
+    const int32_t* __restrict__ col, const uint4* __restrict__ bits, int32_t bit_rows, unsigned long long* cnt,
+    const int2* items, const int32_t* tail, int32_t* next) {
+    __shared__ __align__(16) uint32_t s_words[kTcHubThreads / 32][kTcSlices * kTcHubWords];
+    __shared__ uint32_t s_hub[kTcHubs];
+    const TcCounts counts{s_hub, cnt};
+    counts.clear();
+    const int32_t count = *tail;
+    while (true) {
+        int32_t r = 0;
+        if (lane_id() == 0) r = atomicAdd(next, 1);
+        r = __shfl_sync(0xffffffffu, r, 0);
+        if (r >= count) break;
+        const int2 it = items[r];
+        tc_hub_row(it.x, it.y, min(it.y + kTcHubSlice, oe[it.x] - rp[it.x]), rp, he, col, bits, bit_rows, counts,
+                   s_words[threadIdx.x >> 5]);
+    }
+    counts.flush();
+}
+
+// Scratch of the rank-ordered path.
+struct TcRanked {
+    int32_t *he, *oe, *tails;  // tails: [0] listed slices, [1] rows drawn, [2] slices drawn
+    uint4* bits;
+    int32_t bit_rows;
+    static TcRanked carve(Carver& c, int32_t n) {
+        TcRanked r;
+        r.bit_rows = std::min(n, kTcBitRows);
+        r.he = c.take<int32_t>(n);
+        r.oe = c.take<int32_t>(n);
+        r.tails = c.take<int32_t>(8);
+        r.bits = c.take<uint4>((size_t)r.bit_rows * 32);
+        return r;
+    }
+};
+
+// Triangles of a symmetric, loop-free CSR with strictly increasing rows whose
+// ids are ranks (hubs first), into cnt (zeroed by the caller).
+int tc_count_ranked(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* rp, const int32_t* col,
+                    unsigned long long* cnt, const WalkBuffers& wb, int32_t* lists, const TcRanked& r) {
+    GHB_TRY(launch(ws, tc_rank_ends_kernel, dim3(grid_for(n, 256, ws->num_sms * 8)), dim3(256), 0, n, rp, col, r.he,
+                   r.oe));
+    if (!ws->tune.tc_hash) return tc_count_oriented(ws, 0, n, m, rp, (const int32_t*)r.oe, col, cnt, wb, lists);
+    GHB_CUDA_TRY(cudaMemsetAsync(r.tails, 0, 3 * sizeof(int32_t), ws->stream));
+    GHB_TRY(launch(ws, tc_hub_bitmap_kernel, dim3(grid_for((int64_t)r.bit_rows * 32, 256, ws->num_sms * 8)), dim3(256),
+                   0, r.bit_rows, rp, (const int32_t*)r.he, col, r.bits));
+    int2* items = reinterpret_cast<int2*>(lists);  // fewer than n + m / 256, free again before the hash kernels
+    GHB_TRY(launch(ws, tc_hub_rows_kernel, dim3(grid_for(n, kTcHubThreads, ws->num_sms * kTcHubBlocks)), dim3(kTcHubThreads), 0, n,
+                   rp, (const int32_t*)r.he, (const int32_t*)r.oe, col, (const uint4*)r.bits, r.bit_rows, cnt, items,
+                   r.tails, r.tails + 1));
+    GHB_TRY(launch(ws, tc_hub_items_kernel, dim3(ws->num_sms * kTcHubBlocks), dim3(kTcHubThreads), 0, rp, (const int32_t*)r.he,
+                   (const int32_t*)r.oe, col, (const uint4*)r.bits, r.bit_rows, cnt, (const int2*)items,
+                   (const int32_t*)r.tails, r.tails + 2));
+    if (n <= kTcHubs) return GHB_OK;  // every id is a hub
+    return tc_count_oriented(ws, kTcHubs, n, m, (const int32_t*)r.he, (const int32_t*)r.oe, col, cnt, wb, lists);
 }
 
 // The reference's merge over every entry (any CSR).
@@ -627,7 +968,8 @@ int tc_oriented_core(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* row
                  KeepCountVisitor{rowptr, keep}));
     GHB_TRY(scan_exclusive_i32(ws, keep, orp, n, bsums));
     GHB_TRY(orient_fill(ws, n, rowptr, col, orp, ocol, lists));
-    GHB_TRY(tc_count_oriented(ws, n, m, orp, ocol, cnt, wb, lists));
+    GHB_TRY(tc_count_oriented(ws, 0, n, m, (const int32_t*)orp, (const int32_t*)orp + 1, (const int32_t*)ocol, cnt, wb,
+                              lists));
     if (counts64)
         GHB_TRY(launch(ws, tc_finish_kernel, dim3(grid_for(n, 256, ws->num_sms * 8)), dim3(256), 0, n,
                        (const unsigned long long*)cnt, 6, counts64, (int32_t*)nullptr,
@@ -636,36 +978,41 @@ int tc_oriented_core(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* row
 }
 
 // flags_cache (may be NULL): the input check's flags for this CSR, -1 when
-// not yet known; a known value skips the check.
+// not yet known; a known value skips the check.  ranked: ids are ranks by
+// degree, hubs first (a resident graph's).
 int tc_run_cached(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int32_t* col, int64_t* counts64,
-                  int32_t* counts32, int64_t* total, std::atomic<int32_t>* flags_cache) {
+                  int32_t* counts32, int64_t* total, std::atomic<int32_t>* flags_cache, bool ranked) {
     cudaStream_t st = ws->stream;
     int32_t* hp = reinterpret_cast<int32_t*>(ws->host_pinned);
     GHB_CUDA_TRY(cudaMemcpyAsync(hp, rowptr + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     GHB_CUDA_TRY(cudaStreamSynchronize(st));
     const int64_t m = hp[0];
 
+    WalkBuffers wb;
+    TcRanked rk = {};
+    int32_t *flags, *keep = nullptr, *orp = nullptr, *ocol = nullptr, *lists;
+    unsigned long long *cnt, *tot;
+    int64_t* bsums = nullptr;
+    auto carve = [&](Carver& c) {
+        wb = WalkBuffers::carve(c, n);
+        flags = c.take<int32_t>(8);
+        cnt = c.take<unsigned long long>(n);
+        tot = c.take<unsigned long long>(1);
+        lists = c.take<int32_t>(tc_lists_ints(n, m));
+        if (ranked) {
+            rk = TcRanked::carve(c, n);
+            return;
+        }
+        keep = c.take<int32_t>((size_t)n + 1);
+        orp = c.take<int32_t>((size_t)n + 1);
+        bsums = c.take<int64_t>(scan_scratch_words(n));
+        ocol = c.take<int32_t>(m > 0 ? m : 1);
+    };
     Carver sizing(nullptr);
-    WalkBuffers::carve(sizing, n);
-    sizing.take<int32_t>(8);
-    sizing.take<unsigned long long>(n);
-    sizing.take<unsigned long long>(1);
-    sizing.take<int32_t>((size_t)n + 1);
-    sizing.take<int32_t>((size_t)n + 1);
-    sizing.take<int64_t>(scan_scratch_words(n));
-    sizing.take<int32_t>(m > 0 ? m : 1);
-    sizing.take<int32_t>(tc_lists_ints(n, m));
+    carve(sizing);
     GHB_TRY(ws_reserve(ws, sizing.off));
     Carver c(ws->scratch);
-    WalkBuffers wb = WalkBuffers::carve(c, n);
-    int32_t* flags = c.take<int32_t>(8);
-    unsigned long long* cnt = c.take<unsigned long long>(n);
-    unsigned long long* tot = c.take<unsigned long long>(1);
-    int32_t* keep = c.take<int32_t>((size_t)n + 1);
-    int32_t* orp = c.take<int32_t>((size_t)n + 1);
-    int64_t* bsums = c.take<int64_t>(scan_scratch_words(n));
-    int32_t* ocol = c.take<int32_t>(m > 0 ? m : 1);
-    int32_t* lists = c.take<int32_t>(tc_lists_ints(n, m));
+    carve(c);
 
     GHB_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * n, st));
     GHB_CUDA_TRY(cudaMemsetAsync(tot, 0, sizeof(unsigned long long), st));
@@ -680,13 +1027,16 @@ int tc_run_cached(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int
         if (flags_cache) flags_cache->store(check, std::memory_order_relaxed);
     }
     const bool oriented = check == 0;
-    if (oriented) {
+    if (oriented && ranked) {
+        GHB_TRY(tc_count_ranked(ws, n, m, rowptr, col, cnt, wb, lists, rk));
+    } else if (oriented) {
         GHB_CUDA_TRY(cudaMemsetAsync(keep, 0, sizeof(int32_t) * n, st));
         GHB_TRY(walk(ws, rowptr, col, (const int32_t*)nullptr, (const int32_t*)nullptr, (int64_t)n, (int64_t)n,
                      wb, KeepCountVisitor{rowptr, keep}));
         GHB_TRY(scan_exclusive_i32(ws, keep, orp, n, bsums));
         GHB_TRY(orient_fill(ws, n, rowptr, col, orp, ocol, lists));
-        GHB_TRY(tc_count_oriented(ws, n, m, orp, ocol, cnt, wb, lists));
+        GHB_TRY(tc_count_oriented(ws, 0, n, m, (const int32_t*)orp, (const int32_t*)orp + 1, (const int32_t*)ocol, cnt,
+                                  wb, lists));
     } else {
         GHB_TRY(walk(ws, rowptr, col, (const int32_t*)nullptr, (const int32_t*)nullptr, (int64_t)n, (int64_t)n, wb,
                      MergeVisitor{rowptr, col, cnt}));
@@ -705,7 +1055,7 @@ int tc_run_cached(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int
 
 int tc_run(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int32_t* col, int64_t* counts64,
            int32_t* counts32, int64_t* total) {
-    return tc_run_cached(ws, n, rowptr, col, counts64, counts32, total, nullptr);
+    return tc_run_cached(ws, n, rowptr, col, counts64, counts32, total, nullptr, false);
 }
 
 }  // namespace ghb
