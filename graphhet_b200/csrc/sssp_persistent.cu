@@ -4,8 +4,9 @@
 // several launches per relaxation round, like the reference's
 // frontier loop (GPU_SSSP_csr.cuh:286-307, a device-to-host copy of the
 // queue length per iteration).  Here every round runs inside one launch and
-// the grid meets at a bounded barrier between passes; the last block to
-// arrive decides the next pass:
+// the grid meets at a bounded barrier between passes; every block then
+// derives the next pass from the same counters.  Passes over small queues run
+// on block 0 alone, the others waiting at one barrier:
 //
 //   LIGHT  relax the light range (entries with w < delta of the weight-sorted
 //          rows; the whole row when there is no split) of every near-queue
@@ -42,9 +43,70 @@ namespace ghb {
 constexpr int32_t kSpDirect = 64;
 constexpr int32_t kSpChunk = 256;
 constexpr int kSsspThreads = 512;
+// Passes over small queues run on block 0 alone (see sssp_persistent_kernel):
+// its queues' first kSoloQueue entries lie in shared memory, and it hands back
+// to the grid after kSoloTurns passes at the latest.
+constexpr int32_t kSoloQueue = 2048;
+constexpr int32_t kSoloChunks = 32;
+// A queue is small up to kSoloEntries entries of mean degree.  1501 x 1999
+// grid: 30.8 ms with 3072, 35.8 with 6144 and 40.3 with 12288 (one block then
+// takes several turns of 512 rows per pass), 59.7 with every pass on the grid
+// and its decision read back through L2 (300 x 300: 3.3 ms against 9.0).
+constexpr int64_t kSoloEntries = 3072;
+constexpr int kSoloTurns = 1 << 14;
 constexpr unsigned long long kSsspTimeBudgetNs = 120ull * 1000000000ull;  // two minutes
 
 enum SsspMode : int32_t { kLight = 0, kHeavy = 1, kSplit = 2, kDone = 3, kChunk = 4 };
+
+// What a pass appends to.  Three slots by pass number: pass p fills slot
+// p % 3, every block reads it after the pass's barrier, and block 0 clears
+// slot (p + 1) % 3 during pass p (all blocks read it last before the barrier
+// of pass p - 1).
+struct SpSlot {
+    int32_t q_tail;       // the next near queue
+    int32_t c_tail;       // chunks
+    int32_t r_add;        // additions to R
+    int32_t far_add;      // additions to the far list
+    unsigned long long fmin;  // smallest far distance added (bits)
+    unsigned long long examined;
+    int32_t stop;         // the time budget ran out
+    int32_t pad[23];
+};
+static_assert(sizeof(SpSlot) == 128, "a slot is one cache line");
+
+// Where the traversal stands: every block holds it in shared memory and
+// derives the next pass from it and the slot just filled, so no block waits
+// for another's decision to be written and read back.
+struct SpState {
+    int32_t mode;         // SsspMode of the current pass
+    int32_t solo;         // 1: block 0 runs it alone
+    int32_t round;        // stamp of the near queue being filled
+    int32_t phase;        // stamp of the far list being filled
+    int32_t epoch;        // stamp of R (bumped after every HEAVY pass)
+    int32_t nq;           // items of the current queue (near queue, R in HEAVY, far list in SPLIT)
+    int32_t nc;           // chunk items of the current (CHUNK) pass
+    int32_t qsel;         // near queue buffer read by the current pass
+    int32_t chunk_of;     // the pass (LIGHT or HEAVY) whose rows a CHUNK pass finishes
+    int32_t fsel;         // far buffer filled (a SPLIT reads the other)
+    int32_t q_next;       // near-queue entries filled by a pass whose chunks are still to come
+    int32_t r_count, far_count;  // R's and the far list's entries
+    int32_t failed;       // a budget ran out
+    double thr;           // end of the current bucket
+    double new_thr;       // end of the next bucket (SPLIT)
+    // Bucket width: the light/heavy split stays at delta; the width of the
+    // buckets may move within [width_min, width_max] from one bucket to the
+    // next (equal to delta when the width does not adapt).
+    double width, width_min, width_max;
+    unsigned long long fmin;  // smallest pending far distance (bits; an upper bound on stale entries)
+    unsigned long long examined;
+    long long passes, light_passes, heavy_passes, splits, chunk_passes;
+    long long pass_budget;
+    long long lp_mark;              // LIGHT passes before the current bucket
+    unsigned long long ex_mark;     // entries examined before the current bucket
+    unsigned long long adapt_work;  // a bucket examining fewer entries is small
+    int32_t solo_max;               // queues up to this many vertices run on block 0 alone
+    int32_t pad;
+};
 
 struct SsspRunState {
     unsigned bar_count;  // barrier arrivals (own cache line)
@@ -52,39 +114,11 @@ struct SsspRunState {
     unsigned bar_release;  // barrier epochs (own cache line)
     unsigned pad_b[31];
     int32_t status;
-    int32_t mode;         // SsspMode of the current pass
-    int32_t round;        // stamp of the near queue being filled
-    int32_t phase;        // stamp of the far list being filled
-    int32_t epoch;        // stamp of R (bumped after every HEAVY pass)
-    int32_t nq;           // items of the current queue (near queue, or R in HEAVY)
-    int32_t nc;           // chunk items of the current (CHUNK) pass
-    int32_t qsel;         // near queue buffer read by the current pass
-    int32_t chunk_of;     // the pass (LIGHT or HEAVY) whose rows a CHUNK pass finishes
-    int32_t fsel;         // far buffer filled by relaxations
-    int32_t q_tail;       // appends to the next near queue
-    int32_t c_tail;       // chunks appended by the current pass
-    int32_t r_tail;       // appends to R
-    int32_t far_tail;     // entries of the far list being filled
-    int32_t kept_tail;    // entries kept by a SPLIT pass
-    int32_t pad0;
-    double thr;           // end of the current bucket
-    double new_thr;       // end of the next bucket (SPLIT)
-    double delta;
-    unsigned long long fmin;  // smallest pending far distance (bits; an upper bound on stale entries)
-    unsigned long long examined;
-    long long passes, light_passes, heavy_passes, splits, chunk_passes;
-    long long pass_budget;            // passes allowed (set by the host)
-    unsigned long long t_start;       // global timer at the start
-    unsigned long long bar_limit_ns;
     unsigned bar_extra;
-    unsigned pad1;
-    // Bucket width: the light/heavy split stays at delta; the width of the
-    // buckets may move within [width_min, width_max] from one bucket to the
-    // next (equal to delta when the width does not adapt).
-    double width, width_min, width_max;
-    long long lp_mark;              // LIGHT passes before the current bucket
-    unsigned long long ex_mark;     // entries examined before the current bucket
-    unsigned long long adapt_work;  // a bucket examining fewer entries is small
+    unsigned long long bar_limit_ns;
+    unsigned pad_c[28];
+    SpSlot slot[3];
+    SpState s;  // set by the host; block 0's after a solo run and at the end
 };
 
 namespace {
@@ -92,6 +126,18 @@ namespace {
 __device__ __forceinline__ double sp_dist(const unsigned long long* d, int32_t v) {
     return __longlong_as_double((long long)__ldcg(d + v));
 }
+
+// A queue whose first `cap` entries may lie in shared memory (solo runs).
+struct SpQueue {
+    int32_t* fast;
+    int32_t* mem;
+    int32_t cap;
+    __device__ __forceinline__ int32_t get(int32_t i) const { return i < cap ? fast[i] : __ldcg(mem + i); }
+    __device__ __forceinline__ void put(int32_t i, int32_t v) const {
+        if (i < cap) fast[i] = v;
+        else mem[i] = v;
+    }
+};
 
 struct SpCtx {
     const int32_t* __restrict__ rp;
@@ -103,12 +149,13 @@ struct SpCtx {
     int32_t* far_stamp;
     int32_t* r_stamp;
     int32_t* R;
-    int32_t* q_next;
+    SpQueue q_next;
     int32_t* far_cur;
     int4* chunks;
-    SsspRunState* st;
+    SpSlot* slot;
     double thr;
     int32_t round, phase, epoch;
+    int32_t q_base, r_base, far_base;  // entries that were there before the pass
 };
 
 // Entries a lane relaxes per step: their column, weight and distance loads
@@ -116,29 +163,24 @@ struct SpCtx {
 // flight instead of one dependent chain.
 constexpr int kSpBatch = 4;
 
-// The compare-and-update part of relaxing an entry u -> v, nd = d[u] + w,
-// cur = the distance of v read before.
-__device__ __forceinline__ void sp_update(const SpCtx& c, int32_t v, double nd, double cur,
-                                          unsigned long long* s_fmin) {
-    if (nd < cur) {
-        const unsigned long long nb = (unsigned long long)__double_as_longlong(nd);
-        const unsigned long long old = atomicMin(c.dist + v, nb);
-        if (nb < old) {
-            if (nd < c.thr) {
-                if (atomicExch(c.near_stamp + v, c.round) != c.round) c.q_next[warp_append_active(&c.st->q_tail)] = v;
-            } else {
-                if (atomicExch(c.far_stamp + v, c.phase) != c.phase)
-                    c.far_cur[warp_append_active(&c.st->far_tail)] = v;
-                atomicMin(s_fmin, nb);
-            }
-        }
-    }
-}
+// What a thread has found in a pass: entries relaxed (a pass relaxes fewer
+// than 2^31) and its smallest far distance (bits).
+struct SpFound {
+    unsigned exam = 0;
+    unsigned long long fmin = ~0ull;
+};
 
 // Relax entries j[q] (those with ok[q]) of rows whose source distances are
-// du[q].
+// du[q]; every lane of the warp calls it.  Each step's accesses are issued for
+// all kSpBatch entries before any answer is used: a small pass is a chain of
+// round trips to L2, and this is four of them (columns and weights, distances,
+// stamps, queue tails).  The stamp is taken without waiting for the minimum:
+// whoever stamps v first queues it, and the distance in memory is then at most
+// nd, its own or a smaller one.  (When the smaller one came in an earlier
+// round the entry is spare; one per vertex and round at most, so the queues
+// hold.)
 __device__ __forceinline__ void sp_relax_batch(const SpCtx& c, const double* du, const int32_t* j, const bool* ok,
-                                               unsigned long long& exam, unsigned long long* s_fmin) {
+                                               SpFound& found) {
     int32_t v[kSpBatch];
     double w[kSpBatch], cur[kSpBatch];
 #pragma unroll
@@ -148,29 +190,63 @@ __device__ __forceinline__ void sp_relax_batch(const SpCtx& c, const double* du,
     }
 #pragma unroll
     for (int q = 0; q < kSpBatch; ++q) cur[q] = ok[q] ? sp_dist(c.dist, v[q]) : 0.0;
+    int32_t old[kSpBatch], tag[kSpBatch];
 #pragma unroll
-    for (int q = 0; q < kSpBatch; ++q)
+    for (int q = 0; q < kSpBatch; ++q) {
+        old[q] = tag[q] = 0;
         if (ok[q]) {
-            ++exam;
-            sp_update(c, v[q], du[q] + w[q], cur[q], s_fmin);
+            ++found.exam;
+            const double nd = du[q] + w[q];
+            if (nd < cur[q]) {
+                const unsigned long long nb = (unsigned long long)__double_as_longlong(nd);
+                atomicMin(c.dist + v[q], nb);
+                const bool near = nd < c.thr;
+                // Rounds and phases start at 1 and 0; far tags are kept apart by their sign.
+                tag[q] = near ? c.round : ~c.phase;
+                old[q] = atomicExch((near ? c.near_stamp : c.far_stamp) + v[q], tag[q]);
+                if (!near && nb < found.fmin) found.fmin = nb;
+            }
         }
+    }
+    unsigned near_m[kSpBatch], far_m[kSpBatch];
+    int32_t nnear = 0, nfar = 0;
+#pragma unroll
+    for (int q = 0; q < kSpBatch; ++q) {
+        near_m[q] = __ballot_sync(0xffffffffu, old[q] != tag[q] && tag[q] > 0);
+        far_m[q] = __ballot_sync(0xffffffffu, old[q] != tag[q] && tag[q] < 0);
+        nnear += __popc(near_m[q]);
+        nfar += __popc(far_m[q]);
+    }
+    if (nnear + nfar == 0) return;
+    const int lane = lane_id();
+    int32_t base = 0;
+    if (lane == 0 && nnear) base = c.q_base + atomicAdd(&c.slot->q_tail, nnear);
+    if (lane == 1 && nfar) base = c.far_base + atomicAdd(&c.slot->far_add, nfar);
+    int32_t near_at = __shfl_sync(0xffffffffu, base, 0), far_at = __shfl_sync(0xffffffffu, base, 1);
+    const unsigned below = (1u << lane) - 1u;
+#pragma unroll
+    for (int q = 0; q < kSpBatch; ++q) {
+        if ((near_m[q] >> lane) & 1u) c.q_next.put(near_at + __popc(near_m[q] & below), v[q]);
+        if ((far_m[q] >> lane) & 1u) c.far_cur[far_at + __popc(far_m[q] & below)] = v[q];
+        near_at += __popc(near_m[q]);
+        far_at += __popc(far_m[q]);
+    }
 }
 
 // Relax [jb, je) of one row (distance du) with the whole warp.
-__device__ __forceinline__ void sp_warp_range(const SpCtx& c, double du, int32_t jb, int32_t je,
-                                              unsigned long long& exam, unsigned long long* s_fmin) {
-    const int lane = lane_id();
-    for (int32_t j0 = jb + lane; j0 < je; j0 += 32 * kSpBatch) {
+__device__ __forceinline__ void sp_warp_range(const SpCtx& c, double du, int32_t jb, int32_t je, SpFound& found) {
+    for (int64_t j0 = jb; j0 < je; j0 += 32 * kSpBatch) {
         int32_t jj[kSpBatch];
         bool ok[kSpBatch];
         double dd[kSpBatch];
 #pragma unroll
         for (int q = 0; q < kSpBatch; ++q) {
-            jj[q] = j0 + 32 * q;
-            ok[q] = jj[q] < je;
+            const int64_t j = j0 + lane_id() + 32 * q;
+            ok[q] = j < je;
+            jj[q] = (int32_t)j;
             dd[q] = du;
         }
-        sp_relax_batch(c, dd, jj, ok, exam, s_fmin);
+        sp_relax_batch(c, dd, jj, ok, found);
     }
 }
 
@@ -178,11 +254,11 @@ __device__ __forceinline__ void sp_warp_range(const SpCtx& c, double du, int32_t
 // longer than kSpDirect are appended, whole, to the chunk list of the CHUNK
 // pass that follows.
 __device__ __forceinline__ void sp_rows(const SpCtx& c, int32_t u, int32_t b, int32_t e, double du,
-                                        unsigned long long& exam, unsigned long long* s_fmin) {
+                                        SpFound& found) {
     const int lane = lane_id();
     if (e - b > kSpDirect) {
         const int32_t nch = (e - b + kSpChunk - 1) / kSpChunk;
-        const int32_t pos = atomicAdd(&c.st->c_tail, nch);
+        const int32_t pos = atomicAdd(&c.slot->c_tail, nch);
         for (int32_t k = 0; k < nch; ++k) {
             const int32_t cb = b + k * kSpChunk;
             c.chunks[pos + k] = make_int4(u, cb, min(e, cb + kSpChunk), 0);
@@ -197,11 +273,25 @@ __device__ __forceinline__ void sp_rows(const SpCtx& c, int32_t u, int32_t b, in
         const int32_t lb = __shfl_sync(0xffffffffu, b, leader);
         const int32_t lend = __shfl_sync(0xffffffffu, e, leader);
         const double ld = __shfl_sync(0xffffffffu, du, leader);
-        sp_warp_range(c, ld, lb, lend, exam, s_fmin);
+        sp_warp_range(c, ld, lb, lend, found);
     }
     if (e - b >= 32) e = b;
-    // Shorter rows: gathered warp-wide over a scan of their lengths.
     const int32_t d = e - b;
+    // Rows of a mesh: each lane its own, without the scan below.
+    if (__reduce_max_sync(0xffffffffu, (unsigned)d) <= (unsigned)kSpBatch) {
+        int32_t jj[kSpBatch];
+        bool ok[kSpBatch];
+        double dd[kSpBatch];
+#pragma unroll
+        for (int q = 0; q < kSpBatch; ++q) {
+            jj[q] = b + q;
+            ok[q] = q < d;
+            dd[q] = du;
+        }
+        sp_relax_batch(c, dd, jj, ok, found);
+        return;
+    }
+    // Shorter rows: gathered warp-wide over a scan of their lengths.
     int32_t incl = d;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -230,18 +320,12 @@ __device__ __forceinline__ void sp_rows(const SpCtx& c, int32_t u, int32_t b, in
             ok[q] = k < total;
             jj[q] = ob + (k - oe);
         }
-        sp_relax_batch(c, dd, jj, ok, exam, s_fmin);
+        sp_relax_batch(c, dd, jj, ok, found);
     }
 }
 
-__device__ __forceinline__ bool sp_barrier(SsspRunState* st) {
-    return grid_sync_leader(&st->bar_count, &st->bar_release, &st->status, NoLeader(), st->bar_limit_ns,
-                            st->bar_extra);
-}
-template <class F>
-__device__ __forceinline__ bool sp_barrier(SsspRunState* st, const F& leader) {
-    return grid_sync_leader(&st->bar_count, &st->bar_release, &st->status, leader, st->bar_limit_ns,
-                            st->bar_extra);
+__device__ __forceinline__ bool sp_barrier(SsspRunState* st, unsigned long long limit_ns, unsigned extra) {
+    return grid_sync_leader(&st->bar_count, &st->bar_release, &st->status, NoLeader(), limit_ns, extra);
 }
 
 // Bucket-width adaptation: more LIGHT passes than this in a bucket halve
@@ -257,7 +341,164 @@ __device__ __forceinline__ double sp_next_thr(double thr, double delta, double m
     return nthr;
 }
 
+// The next pass, from the state and what the pass just finished appended.
+__device__ __forceinline__ void sp_decide(SpState& s, const SpSlot& c) {
+    const int32_t md0 = s.mode;
+    ++s.passes;
+    s.examined += c.examined;
+    s.r_count += c.r_add;
+    s.far_count += c.far_add;
+    s.q_next += c.q_tail;
+    if (c.fmin < s.fmin) s.fmin = c.fmin;
+    if ((md0 == kLight || md0 == kHeavy) && c.c_tail > 0) {
+        // Long rows were cut into chunks: a CHUNK pass finishes them in the
+        // same round (same stamps, same next queue).
+        s.nc = c.c_tail;
+        s.chunk_of = md0;
+        s.mode = kChunk;
+        s.solo = s.nc <= kSoloChunks && s.solo_max > 0;
+        return;
+    }
+    if (md0 == kChunk) ++s.chunk_passes;
+    const int32_t md = md0 == kChunk ? s.chunk_of : md0;
+    s.qsel ^= 1;
+    s.nq = s.q_next;
+    s.q_next = 0;
+    s.nc = 0;
+    if (md == kSplit) {
+        s.thr = s.new_thr;
+        ++s.splits;
+    } else if (md == kHeavy) {
+        s.r_count = 0;
+        ++s.epoch;
+        ++s.heavy_passes;
+    } else {
+        ++s.light_passes;
+    }
+    int32_t next = kDone;
+    int32_t solo_max = s.solo_max;
+    if (s.nq > 0) {
+        next = kLight;
+    } else if (md == kLight && s.r_count > 0) {
+        next = kHeavy;
+        s.nq = s.r_count;
+    } else if (s.far_count > 0) {
+        // Next bucket: the one holding the smallest pending far distance (its
+        // recorded minimum can be low when an entry settled later; a SPLIT
+        // that queues nothing then repeats with the exact minimum of the
+        // entries it kept).
+        //
+        // Its width: halved after a bucket that took more than kSpAdaptLight
+        // LIGHT passes (its vertices were relaxed again and again), doubled
+        // after one that took at most two and examined little (passes with
+        // too little work for the grid).  Exact distances do not depend on
+        // it: the passes form a label-correcting loop in which a HEAVY pass
+        // that lowers a distance inside the bucket sends it back to a LIGHT
+        // pass, and R is refilled after every HEAVY pass.
+        const long long lp = s.light_passes - s.lp_mark;
+        const unsigned long long ex = s.examined - s.ex_mark;
+        if (lp > kSpAdaptLight) s.width = fmax(s.width * 0.5, s.width_min);
+        else if (lp <= 2 && ex < s.adapt_work) s.width = fmin(s.width * 2.0, s.width_max);
+        s.lp_mark = s.light_passes;
+        s.ex_mark = s.examined;
+        const double mn = s.fmin == ~0ull ? s.thr : __longlong_as_double((long long)s.fmin);
+        s.new_thr = sp_next_thr(s.thr, s.width, mn);
+        s.fmin = ~0ull;
+        s.nq = s.far_count;
+        s.far_count = 0;
+        s.fsel ^= 1;
+        ++s.phase;
+        next = kSplit;
+        solo_max *= 4;  // one distance per entry, no row
+    }
+    ++s.round;
+    // Budgets: a correct run needs far fewer passes and far less time; past
+    // either, stop with an error status.
+    if (next != kDone && (s.passes > s.pass_budget || c.stop)) {
+        s.failed = 1;
+        next = kDone;
+    }
+    s.mode = next;
+    s.solo = next != kDone && s.nq <= solo_max;
+}
+
 }  // namespace
+
+// A warp's findings into its block's totals.
+__device__ __forceinline__ void sp_total(const SpFound& found, unsigned long long* examined,
+                                         unsigned long long* fmin) {
+    const unsigned exam = __reduce_add_sync(0xffffffffu, found.exam);
+    if (lane_id() == 0 && exam) atomicAdd(examined, (unsigned long long)exam);
+    if (__any_sync(0xffffffffu, found.fmin != ~0ull)) {
+        unsigned long long m = found.fmin;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = min(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (lane_id() == 0) atomicMin(fmin, m);
+    }
+}
+
+// One pass's share of warp `warp` of `nwarps` (thread `tid` of `nt`).
+__device__ __forceinline__ void sp_pass(const SpState& s, SpCtx& c, const SpQueue& q_cur, int32_t* fa, int32_t* fb,
+                                        int64_t tid, int64_t nt, SpFound& found) {
+    const int lane = lane_id();
+    const int64_t warp = tid >> 5, nwarps = nt >> 5;
+    const bool split = c.le != nullptr;
+    if (s.mode == kChunk) {
+        // The long rows of the pass just finished, a chunk per warp.
+        for (int64_t i = warp; i < s.nc; i += nwarps) {
+            const int4 ch = __ldcg(c.chunks + i);
+            const double du = sp_dist(c.dist, ch.x);
+            sp_warp_range(c, du, ch.y, ch.z, found);
+        }
+    } else if (s.mode == kSplit) {
+        const int32_t* far = s.fsel ? fa : fb;
+        const double old_thr = s.thr, nthr = s.new_thr;
+        for (int64_t i = tid; i < s.nq; i += nt) {
+            const int32_t v = __ldcg(far + i);
+            const double d = sp_dist(c.dist, v);
+            if (d < old_thr) continue;  // settled in an earlier bucket
+            if (d < nthr) {
+                if (atomicExch(c.near_stamp + v, c.round) != c.round)
+                    c.q_next.put(c.q_base + warp_append_active(&c.slot->q_tail), v);
+            } else {
+                if (atomicExch(c.far_stamp + v, ~c.phase) != ~c.phase)
+                    c.far_cur[c.far_base + warp_append_active(&c.slot->far_add)] = v;
+                const unsigned long long db = (unsigned long long)__double_as_longlong(d);
+                if (db < found.fmin) found.fmin = db;
+            }
+        }
+    } else {
+        // Queue rows, 32 per warp; on small queues fewer, so that their rows
+        // spread over every warp instead of queueing behind each other.
+        int64_t per = 32;
+        while (per > 1 && nwarps * (per >> 1) >= s.nq) per >>= 1;
+        for (int64_t base = warp * per; base < s.nq; base += nwarps * per) {
+            const int64_t i = base + lane;
+            int32_t u = -1, b = 0, e = 0;
+            double du = 0.0;
+            bool settled = false;  // joins R
+            if (lane < per && i < s.nq) {
+                if (s.mode == kLight) {
+                    u = q_cur.get((int32_t)i);
+                    b = c.rp[u];
+                    e = split ? c.le[u] : c.rp[u + 1];
+                    du = sp_dist(c.dist, u);
+                    if (split) settled = atomicExch(c.r_stamp + u, c.epoch) != c.epoch;
+                } else {
+                    u = __ldcg(c.R + i);
+                    b = c.le[u];
+                    e = c.rp[u + 1];
+                    du = sp_dist(c.dist, u);
+                }
+            }
+            sp_rows(c, u, b, e, du, found);
+            if (split && s.mode == kLight) {
+                const int32_t at = warp_append(&c.slot->r_add, settled);
+                if (settled) c.R[c.r_base + at] = u;
+            }
+        }
+    }
+}
 
 __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent_kernel(
     int32_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ le, const int32_t* __restrict__ col,
@@ -267,211 +508,160 @@ __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent_kernel(
     unsigned long long* dist = reinterpret_cast<unsigned long long*>(dist_d);
     const int64_t gtid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t gsize = (int64_t)gridDim.x * blockDim.x;
-    const int64_t warp = gtid >> 5;
-    const int64_t nwarps = gsize >> 5;
-    const int lane = lane_id();
     const bool split = le != nullptr;
+    __shared__ SpState s;
+    __shared__ SpSlot own;  // the slot of a solo pass
+    __shared__ unsigned long long s_fmin, s_exam, s_t0;
+    __shared__ int32_t s_fast[2][kSoloQueue];
+    const unsigned long long limit_ns = st->bar_limit_ns;
+    const unsigned extra = st->bar_extra;
 
     // ---- init
     const unsigned long long ib = (unsigned long long)__double_as_longlong(inf);
     for (int64_t v = gtid; v < n; v += gsize) {
         dist[v] = (v == src) ? 0ull : ib;
         near_stamp[v] = -1;
-        far_stamp[v] = -1;
+        far_stamp[v] = 0;
         if (split) r_stamp[v] = -1;
+    }
+    if (threadIdx.x == 0) {
+        s = st->s;
+        s_fmin = ~0ull;
+        s_exam = 0;
+        s_t0 = global_timer_ns();
     }
     if (gtid == 0) {
         qa[0] = src;
-        st->nq = 1;
-        st->mode = kLight;
-        st->round = 1;
-        st->fmin = ~0ull;
-        st->t_start = global_timer_ns();
+        for (int k = 0; k < 3; ++k) st->slot[k].fmin = ~0ull;
     }
-    if (!sp_barrier(st)) return;
+    if (!sp_barrier(st, limit_ns, extra)) return;
 
-    __shared__ unsigned long long s_fmin, s_exam;
-    __shared__ int32_t s_state[9];
-    __shared__ double s_thr, s_new_thr;
-    volatile SsspRunState* vs = st;
-    while (true) {
-        if (threadIdx.x == 0) {
-            s_state[0] = vs->mode;
-            s_state[1] = vs->nq;
-            s_state[2] = vs->nc;
-            s_state[3] = vs->qsel;
-            s_state[4] = vs->chunk_of;
-            s_state[5] = vs->fsel;
-            s_state[6] = vs->round;
-            s_state[7] = vs->phase;
-            s_state[8] = vs->epoch;
-            s_thr = vs->thr;
-            s_new_thr = vs->new_thr;
-            s_fmin = ~0ull;
-            s_exam = 0;
-        }
-        __syncthreads();
-        const int32_t mode = s_state[0];
-        if (mode == kDone) break;
-        const int32_t nq = s_state[1], nc = s_state[2];
-        const int32_t qsel = s_state[3], fsel = s_state[5];
-        SpCtx c;
-        c.rp = rp;
-        c.le = le;
-        c.col = col;
-        c.wt = wt;
-        c.dist = dist;
-        c.near_stamp = near_stamp;
-        c.far_stamp = far_stamp;
-        c.r_stamp = r_stamp;
-        c.R = R;
-        c.q_next = qsel ? qa : qb;
-        c.far_cur = fsel ? fb : fa;
-        c.chunks = chunks;
-        c.st = st;
-        c.thr = s_thr;
-        c.round = s_state[6];
-        c.phase = s_state[7];
-        c.epoch = s_state[8];
-        unsigned long long exam = 0;
-
-        if (mode == kChunk) {
-            // The long rows of the pass just finished, a chunk per warp.
-            for (int64_t i = warp; i < nc; i += nwarps) {
-                const int4 ch = __ldcg(chunks + i);
-                const double du = sp_dist(dist, ch.x);
-                sp_warp_range(c, du, ch.y, ch.z, exam, &s_fmin);
-            }
-        } else if (mode == kLight || mode == kHeavy) {
-            const int32_t* q = mode == kHeavy ? R : (qsel ? qb : qa);
-            // Queue rows, 32 per warp.
-            for (int64_t base = warp * 32; base < nq; base += nwarps * 32) {
-                const int64_t i = base + lane;
-                int32_t u = -1, b = 0, e = 0;
-                double du = 0.0;
-                if (i < nq) {
-                    u = q[i];
-                    du = sp_dist(dist, u);
-                    if (mode == kLight) {
-                        b = rp[u];
-                        e = split ? le[u] : rp[u + 1];
-                        if (split && atomicExch(r_stamp + u, c.epoch) != c.epoch)
-                            R[warp_append_active(&st->r_tail)] = u;
-                    } else {
-                        b = le[u];
-                        e = rp[u + 1];
+    SpCtx c;
+    c.rp = rp;
+    c.le = le;
+    c.col = col;
+    c.wt = wt;
+    c.dist = dist;
+    c.near_stamp = near_stamp;
+    c.far_stamp = far_stamp;
+    c.r_stamp = r_stamp;
+    c.R = R;
+    c.chunks = chunks;
+    unsigned turn = 0;  // the grid's passes: which slot is filled
+    while (s.mode != kDone) {
+        auto context = [&](int32_t cap) {
+            c.q_next = SpQueue{s_fast[s.qsel ^ 1], s.qsel ? qa : qb, cap};
+            c.far_cur = s.fsel ? fb : fa;
+            c.thr = s.thr;
+            c.round = s.round;
+            c.phase = s.phase;
+            c.epoch = s.epoch;
+            c.q_base = s.q_next;
+            c.r_base = s.r_count;
+            c.far_base = s.far_count;
+        };
+        if (s.solo) {
+            // ---- a run of small passes on block 0, the others at the barrier
+            // below: a pass then costs its own chain of loads and a block
+            // barrier, not a grid barrier and a state read through L2.
+            if (blockIdx.x == 0) {
+                // The queue's first entries move to shared memory for the run.
+                const int32_t held = s.mode == kLight ? min(s.nq, kSoloQueue) : 0;
+                for (int32_t i = threadIdx.x; i < held; i += blockDim.x)
+                    s_fast[s.qsel][i] = __ldcg((s.qsel ? qb : qa) + i);
+                // Entries that an unfinished round (its chunks come next) has
+                // queued move as well.
+                const int32_t held_next = min(s.q_next, kSoloQueue);
+                for (int32_t i = threadIdx.x; i < held_next; i += blockDim.x)
+                    s_fast[s.qsel ^ 1][i] = __ldcg((s.qsel ? qa : qb) + i);
+                const unsigned long long t_run = global_timer_ns();
+                if (threadIdx.x == 0) {
+                    own.q_tail = own.c_tail = own.r_add = own.far_add = own.stop = 0;
+                    own.fmin = ~0ull;
+                    own.examined = 0;
+                }
+                __syncthreads();
+                c.slot = &own;
+                for (int turns = 0; s.solo && turns < kSoloTurns; ++turns) {
+                    context(kSoloQueue);
+                    const SpQueue q_cur{s_fast[s.qsel], s.qsel ? qb : qa, kSoloQueue};
+                    SpFound found;
+                    sp_pass(s, c, q_cur, fa, fb, threadIdx.x, blockDim.x, found);
+                    sp_total(found, &own.examined, &own.fmin);
+                    __syncthreads();
+                    if (threadIdx.x == 0) {
+                        const bool look = (turns & 15) == 15;
+                        const unsigned long long now = look ? global_timer_ns() : 0;
+                        own.stop = look && now - s_t0 > kSsspTimeBudgetNs;
+                        sp_decide(s, own);
+                        own.q_tail = own.c_tail = own.r_add = own.far_add = 0;
+                        own.fmin = ~0ull;
+                        own.examined = 0;
+                        // The others' wait is bounded: hand back well before it ends.
+                        if (look && now - t_run > limit_ns / 8) s.solo = 0;
                     }
+                    __syncthreads();
                 }
-                sp_rows(c, u, b, e, du, exam, &s_fmin);
-            }
-        } else {  // kSplit
-            const int32_t* far = fsel ? fb : fa;
-            int32_t* kept = fsel ? fa : fb;
-            const double old_thr = s_thr, nthr = s_new_thr;
-            const int32_t next_phase = c.phase;  // already advanced by the leader
-            for (int64_t i = gtid; i < nq; i += gsize) {
-                const int32_t v = far[i];
-                const double d = sp_dist(dist, v);
-                if (d < old_thr) continue;  // settled in an earlier bucket
-                if (d < nthr) {
-                    if (atomicExch(near_stamp + v, c.round) != c.round) c.q_next[warp_append_active(&st->q_tail)] = v;
-                } else {
-                    if (atomicExch(far_stamp + v, next_phase) != next_phase)
-                        kept[warp_append_active(&st->kept_tail)] = v;
-                    atomicMin(&s_fmin, (unsigned long long)__double_as_longlong(d));
+                // Back to global memory: the queue that the next pass reads,
+                // and the one that an unfinished round fills.
+                const int32_t back = s.mode == kLight ? min(s.nq, kSoloQueue) : 0;
+                for (int32_t i = threadIdx.x; i < back; i += blockDim.x)
+                    (s.qsel ? qb : qa)[i] = s_fast[s.qsel][i];
+                const int32_t back_next = min(s.q_next, kSoloQueue);
+                for (int32_t i = threadIdx.x; i < back_next; i += blockDim.x)
+                    (s.qsel ? qa : qb)[i] = s_fast[s.qsel ^ 1][i];
+                // One pass of the whole grid follows even where the next is
+                // small: the run above ended by its own limits then.
+                if (threadIdx.x == 0) {
+                    s.solo = 0;
+                    st->s = s;
                 }
             }
+            if (!sp_barrier(st, limit_ns, extra)) return;
+            if (blockIdx.x != 0 && threadIdx.x < sizeof(SpState) / 4)
+                reinterpret_cast<int32_t*>(&s)[threadIdx.x] =
+                    __ldcg(reinterpret_cast<const int32_t*>(&st->s) + threadIdx.x);
+            __syncthreads();
+            continue;
         }
-        // Block totals, then the barrier whose last arrival decides.
-        exam = warp_sum(exam);
-        if (lane == 0 && exam) atomicAdd(&s_exam, exam);
+        SpSlot* slot = &st->slot[turn % 3];
+        context(0);
+        c.slot = slot;
+        const SpQueue q_cur{nullptr, s.qsel ? qb : qa, 0};
+        SpFound found;
+        sp_pass(s, c, q_cur, fa, fb, gtid, gsize, found);
+        // Block totals, then the barrier.
+        sp_total(found, &s_exam, &s_fmin);
         __syncthreads();
         if (threadIdx.x == 0) {
-            if (s_exam) atomicAdd(&st->examined, s_exam);
-            if (s_fmin != ~0ull) atomicMin(&st->fmin, s_fmin);
+            if (s_exam) atomicAdd(&slot->examined, s_exam);
+            if (s_fmin != ~0ull) atomicMin(&slot->fmin, s_fmin);
+            s_exam = 0;
+            s_fmin = ~0ull;
+            if (blockIdx.x == 0) {
+                SpSlot* clear = &st->slot[(turn + 1) % 3];
+                clear->q_tail = clear->c_tail = clear->r_add = clear->far_add = clear->stop = 0;
+                clear->fmin = ~0ull;
+                clear->examined = 0;
+                if (global_timer_ns() - s_t0 > kSsspTimeBudgetNs) slot->stop = 1;
+            }
         }
-        const bool ok = sp_barrier(st, [&]() {
-            SsspRunState* s = st;
-            volatile SsspRunState* v = st;
-            const int32_t md0 = v->mode;
-            s->passes = v->passes + 1;
-            if ((md0 == kLight || md0 == kHeavy) && v->c_tail > 0) {
-                // Long rows were cut into chunks: a CHUNK pass finishes them
-                // in the same round (same stamps, same next queue).
-                s->nc = v->c_tail;
-                s->c_tail = 0;
-                s->chunk_of = md0;
-                s->mode = kChunk;
-                return;
-            }
-            if (md0 == kChunk) s->chunk_passes = v->chunk_passes + 1;
-            const int32_t md = md0 == kChunk ? v->chunk_of : md0;
-            const int32_t nq_next = v->q_tail;
-            s->q_tail = 0;
-            s->c_tail = 0;
-            s->qsel = v->qsel ^ 1;
-            s->nq = nq_next;
-            s->nc = 0;
-            if (md == kSplit) {
-                s->far_tail = v->kept_tail;
-                s->kept_tail = 0;
-                s->fsel = v->fsel ^ 1;
-                s->thr = v->new_thr;
-                s->splits = v->splits + 1;
-            } else if (md == kHeavy) {
-                s->r_tail = 0;
-                s->epoch = v->epoch + 1;
-                s->heavy_passes = v->heavy_passes + 1;
-            } else {
-                s->light_passes = v->light_passes + 1;
-            }
-            int32_t next = kDone;
-            if (nq_next > 0) {
-                next = kLight;
-            } else if (md == kLight && v->r_tail > 0) {
-                next = kHeavy;
-                s->nq = v->r_tail;
-            } else if (v->far_tail > 0) {
-                // Next bucket: the one holding the smallest pending far
-                // distance (its recorded minimum can be low when an entry
-                // settled later; a SPLIT that queues nothing then repeats
-                // with the exact minimum of the entries it kept).
-                const unsigned long long fb_ = v->fmin;
-                const double thr = v->thr;
-                // The next bucket's width: halved after a bucket that took
-                // more than kSpAdaptLight LIGHT passes (its vertices were
-                // relaxed again and again), doubled after one that took at
-                // most two and examined little (passes with too little work
-                // for the grid).  Exact distances do not depend on it: the
-                // passes form a label-correcting loop in which a HEAVY pass
-                // that lowers a distance inside the bucket sends it back to
-                // a LIGHT pass, and R is refilled after every HEAVY pass.
-                double width = v->width;
-                const long long lp = v->light_passes - v->lp_mark;
-                const unsigned long long ex = v->examined - v->ex_mark;
-                if (lp > kSpAdaptLight) width = fmax(width * 0.5, v->width_min);
-                else if (lp <= 2 && ex < v->adapt_work) width = fmin(width * 2.0, v->width_max);
-                s->width = width;
-                s->lp_mark = v->light_passes;
-                s->ex_mark = v->examined;
-                const double mn = fb_ == ~0ull ? thr : __longlong_as_double((long long)fb_);
-                s->new_thr = sp_next_thr(thr, width, mn);
-                s->fmin = ~0ull;
-                s->nq = v->far_tail;
-                s->phase = v->phase + 1;
-                next = kSplit;
-            }
-            s->round = v->round + 1;
-            // Budgets: a correct run needs far fewer passes and far less
-            // time; past either, stop with an error status.
-            if (next != kDone &&
-                (v->passes > v->pass_budget || global_timer_ns() - v->t_start > kSsspTimeBudgetNs)) {
-                s->status = kDevOverflow;
-                next = kDone;
-            }
-            s->mode = next;
-        });
-        if (!ok) return;
+        if (!sp_barrier(st, limit_ns, extra)) return;
+        if (threadIdx.x == 0) {
+            SpSlot f;
+            const int4 a = __ldcg(reinterpret_cast<const int4*>(slot));
+            const ulonglong2 b = __ldcg(reinterpret_cast<const ulonglong2*>(slot) + 1);
+            f.stop = __ldcg(&slot->stop);
+            f.q_tail = a.x, f.c_tail = a.y, f.r_add = a.z, f.far_add = a.w;
+            f.fmin = b.x, f.examined = b.y;
+            sp_decide(s, f);
+        }
+        ++turn;
+        __syncthreads();
+    }
+    if (gtid == 0) {
+        st->s = s;
+        if (s.failed) st->status = kDevOverflow;
     }
 
     // ---- results in the caller's ids
@@ -591,28 +781,32 @@ int sssp_persistent_run(ghb_workspace* ws, int32_t n, const int32_t* rp, const i
     Carver c(ws->scratch);
     carve(c, &qa, &qb, &ch, &fa, &fb, &ns, &fs, &rs, &R, &rstate);
 
-    GHB_CUDA_TRY(cudaMemsetAsync(rstate, 0, sizeof(SsspRunState), st));
-    {
-        // thr, delta, then the barrier limit and test knob (pageable
-        // sources: the copies stage them before returning).
-        const double td[2] = {delta, delta};
-        GHB_CUDA_TRY(cudaMemcpyAsync(&rstate->thr, td, sizeof(double), cudaMemcpyHostToDevice, st));
-        GHB_CUDA_TRY(cudaMemcpyAsync(&rstate->delta, td + 1, sizeof(double), cudaMemcpyHostToDevice, st));
-        const unsigned long long bar[2] = {(unsigned long long)ws->tune.barrier_limit_us * 1000ull,
-                                           (unsigned long long)ws->tune.barrier_extra};
-        GHB_CUDA_TRY(cudaMemcpyAsync(&rstate->bar_limit_ns, bar, sizeof(bar), cudaMemcpyHostToDevice, st));
-        // Every productive pass lowers some distance: 64 passes per vertex
-        // bound any correct run, as in the host-driven loop.
-        const long long budget = 64ll * n + 1024;
-        GHB_CUDA_TRY(cudaMemcpyAsync(&rstate->pass_budget, &budget, sizeof(budget), cudaMemcpyHostToDevice, st));
-        // Bucket widths: delta, or from delta / 64 to delta * 64 when they
-        // adapt; a bucket is small below eight entries per thread.
-        const bool adapt = ws->tune.sssp_adapt != 0;
-        const double wd[3] = {delta, adapt ? delta / 64.0 : delta, adapt ? delta * 64.0 : delta};
-        GHB_CUDA_TRY(cudaMemcpyAsync(&rstate->width, wd, sizeof(wd), cudaMemcpyHostToDevice, st));
-        const unsigned long long work = 8ull * (unsigned long long)blocks * kSsspThreads;
-        GHB_CUDA_TRY(cudaMemcpyAsync(&rstate->adapt_work, &work, sizeof(work), cudaMemcpyHostToDevice, st));
-    }
+    // The start state, in one copy from pinned memory (its words are not
+    // written again before this call's read-back).
+    SsspRunState* h0 = reinterpret_cast<SsspRunState*>(ws->host_pinned);
+    static_assert(sizeof(SsspRunState) <= sizeof(int64_t) * kHostPinnedWords, "the run state fits the pinned words");
+    std::memset(static_cast<void*>(h0), 0, sizeof(SsspRunState));
+    h0->bar_limit_ns = (unsigned long long)ws->tune.barrier_limit_us * 1000ull;
+    h0->bar_extra = (unsigned)ws->tune.barrier_extra;
+    h0->s.mode = kLight;
+    h0->s.round = 1;
+    h0->s.nq = 1;
+    h0->s.fmin = ~0ull;
+    h0->s.thr = delta;
+    // Every productive pass lowers some distance: 64 passes per vertex bound
+    // any correct run, as in the host-driven loop.
+    h0->s.pass_budget = 64ll * n + 1024;
+    // Bucket widths: delta, or from delta / 64 to delta * 64 when they adapt;
+    // a bucket is small below eight entries per thread.
+    const bool adapt = ws->tune.sssp_adapt != 0;
+    h0->s.width = delta;
+    h0->s.width_min = adapt ? delta / 64.0 : delta;
+    h0->s.width_max = adapt ? delta * 64.0 : delta;
+    h0->s.adapt_work = 8ull * (unsigned long long)blocks * kSsspThreads;
+    // Small passes: a few entries per thread of one block.
+    h0->s.solo_max = (int32_t)std::min<int64_t>(kSoloQueue, std::max<int64_t>(16, kSoloEntries * (int64_t)n / std::max<int64_t>(m, 1)));
+    h0->s.solo = 1;
+    GHB_CUDA_TRY(cudaMemcpyAsync(rstate, h0, sizeof(SsspRunState), cudaMemcpyHostToDevice, st));
     if (stats) GHB_CUDA_TRY(cudaEventRecord(ws->ev_start, st));
     GHB_TRY(launch_coop(ws, sssp_persistent_kernel, dim3(blocks), dim3(kSsspThreads), 0, n, rp, le, col, wt, src, inf,
                         dist, qa, qb, ch, fa, fb, ns, fs, rs, R, rstate, perm, out));
@@ -640,11 +834,11 @@ int sssp_persistent_run(ghb_workspace* ws, int32_t n, const int32_t* rp, const i
         float ms = 0.f;
         GHB_CUDA_TRY(cudaEventElapsedTime(&ms, ws->ev_start, ws->ev_stop));
         const unsigned long long* ha = reinterpret_cast<const unsigned long long*>(ws->host_pinned);
-        stats->levels = (int32_t)(h.light_passes + h.heavy_passes + h.chunk_passes);
-        stats->pull_levels = (int32_t)h.splits;
+        stats->levels = (int32_t)(h.s.light_passes + h.s.heavy_passes + h.s.chunk_passes);
+        stats->pull_levels = (int32_t)h.s.splits;
         stats->edges_reached = (int64_t)ha[0];
         stats->reached = (int64_t)ha[1];
-        stats->edges_examined = (int64_t)h.examined;
+        stats->edges_examined = (int64_t)h.s.examined;
         stats->device_ms = ms;
     }
     return GHB_OK;
