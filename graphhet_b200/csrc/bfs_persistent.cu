@@ -33,6 +33,22 @@ namespace ghb {
 constexpr int32_t kBigChunkRows = 2047;  // 4 per thread of a 512-thread block, plus the total
 constexpr int32_t kBigChunk = 256;
 
+// Runs of small top-down levels on a squad, the grid's first blocks (see
+// bfs_squad_run): frontiers of up to kSquadRows vertices and kSquadEntries
+// out-entries in all, each block's share in its shared memory.  2999 x 2001
+// grid: 18.0 ms with 32 blocks, 19.5 with 16, 20.5 with 8, 27 on one block as
+// far as its frontiers fit, 28-29.6 with every level on the grid (300 x 300:
+// 1.4 ms against 3.3).  Loading the claimed rows' first columns ahead changed
+// nothing.
+constexpr int kSquadBlocks = 32;
+constexpr int32_t kSquadShare = 1024;    // vertices a block can hold
+constexpr int32_t kSquadLean = 640;      // a block with more asks for the frontier to be dealt out again
+constexpr int32_t kSquadOne = 192;       // a frontier up to this size starts on one block
+constexpr int kSquadLevel = 12;          // levels before the first run
+constexpr int32_t kSquadRows = kSquadBlocks * 320;
+constexpr unsigned long long kSquadEntries = 4 * kSquadRows;
+constexpr int32_t kSquadWords = 1 << 17;  // bitmap words that a squad clears in passing
+
 struct BfsRunState {
     unsigned bar_count;            // barrier arrivals (own cache line)
     unsigned pad_a[31];
@@ -63,6 +79,17 @@ struct BfsRunState {
     unsigned long long bar_limit_ns; // grid-barrier wait limit (set by the host before the launch)
     unsigned bar_extra;              // arrivals beyond the grid every barrier waits for (0; tests: 1)
     unsigned pad3;
+    // Squad runs: the levels' barrier words by level % 3 (own cache lines;
+    // zero between runs) and what a run hands back.
+    struct {
+        unsigned long long word;
+        unsigned long long pad[15];
+    } squad[3];
+    int32_t squad_queue;             // vertices handed back in the queue
+    int32_t squad_level;             // the level they are the frontier of
+    unsigned long long squad_mf;     // their out-entries
+    unsigned long long squad_mr;     // out-entries of all the vertices reached in the run
+    unsigned long long squad_reached;
 };
 
 namespace {
@@ -141,6 +168,7 @@ constexpr unsigned long long kPlDir = 1ull << 33;      // bottom-up
 constexpr unsigned long long kPlAppend = 1ull << 34;   // top-down level appends to the queue
 constexpr unsigned long long kPlQueueOk = 1ull << 35;  // the queue holds the frontier
 constexpr unsigned long long kPlBig = 1ull << 36;      // long rows deferred: no decision yet
+constexpr unsigned long long kPlSquad = 1ull << 37;    // the squad runs the next levels
 
 __device__ __forceinline__ unsigned long long p_payload(int32_t nf, bool done, int dir, bool append, bool queue_ok) {
     return ((unsigned long long)nf & kPlNf) | (done ? kPlDone : 0ull) | (dir ? kPlDir : 0ull) |
@@ -214,6 +242,273 @@ __device__ __forceinline__ int32_t p_append(int nd, int fmt, unsigned long long 
     return (nd == 0 && (fmt == 1 || (fmt == 0 && mf < (unsigned long long)kAppendMaxEdges))) ? 1 : 0;
 }
 
+// A squad run.  A level on the grid is a grid barrier (2.4 us) and a chain of
+// dependent accesses through L2: queue, row bounds, columns, claim, queue
+// slot.  On the squad each block expands the vertices it claimed itself: they
+// wait in its shared memory with their row bounds, which were read while the
+// claim was in flight, so a level is columns, claim and one round trip to the
+// level's barrier word, which carries the totals that every block decides from.
+struct SquadShared {
+    int32_t v[2][kSquadShare];  // the block's frontier by parity
+    int2 row[2][kSquadShare];   // and its row bounds
+    int32_t count[2];           // its vertices
+    unsigned long long mf;      // out-entries of the claims of the level being expanded
+    unsigned long long total;   // the level's barrier word
+    int ok;
+};
+// Barrier word of a level: claims, their out-entries (each block's capped),
+// blocks that ask for an end of the run, arrivals.
+constexpr unsigned long long kSqNf = 1ull, kSqMf = 1ull << 24, kSqEnd = 1ull << 48, kSqArrive = 1ull << 56;
+constexpr unsigned long long kSqField = (1ull << 24) - 1;
+constexpr unsigned long long kSqMfCap = kSqField / kSquadBlocks;
+
+// Claims the entries j[q] (those with ok[q]) for the next level; every lane of
+// the warp calls it.  The claims of a batch are issued together, with the row
+// bounds of the vertices claimed.  Claims past the block's share go to the
+// grid's queue.
+constexpr int kSquadBatch = 4;
+struct SquadCtx {  // the traversal's arrays (in shared memory, not on the callers' stacks)
+    const int32_t* rp;
+    const int32_t* col;
+    uint32_t* visited;
+    int32_t* depth;
+    int32_t* queue[3];
+    uint32_t* f[3];
+    BfsRunState* st;
+    int32_t max_depth;
+};
+__device__ __forceinline__ void squad_visit(const SquadCtx& c, SquadShared& sh, const int32_t* j, const bool* ok,
+                                            int32_t next_depth, int par, unsigned& mf) {
+    int32_t v[kSquadBatch], b[kSquadBatch], e[kSquadBatch];
+    uint32_t was[kSquadBatch];
+#pragma unroll
+    for (int q = 0; q < kSquadBatch; ++q) v[q] = ok[q] ? c.col[j[q]] : -1;
+#pragma unroll
+    for (int q = 0; q < kSquadBatch; ++q) {
+        was[q] = 0xffffffffu;
+        b[q] = e[q] = 0;
+        if (v[q] >= 0) {
+            was[q] = atomicOr(c.visited + (v[q] >> 5), 1u << (v[q] & 31));
+            b[q] = c.rp[v[q]];
+            e[q] = c.rp[v[q] + 1];
+        }
+    }
+    unsigned m[kSquadBatch];
+    int32_t total = 0;
+#pragma unroll
+    for (int q = 0; q < kSquadBatch; ++q) {
+        m[q] = __ballot_sync(0xffffffffu, v[q] >= 0 && !((was[q] >> (v[q] & 31)) & 1u));
+        total += __popc(m[q]);
+    }
+    if (total == 0) return;
+    const int lane = lane_id();
+    int32_t at = 0;
+    if (lane == 0) at = atomicAdd(&sh.count[par], total);
+    at = __shfl_sync(0xffffffffu, at, 0);
+#pragma unroll
+    for (int q = 0; q < kSquadBatch; ++q) {
+        if ((m[q] >> lane) & 1u) {
+            const int32_t p = at + __popc(m[q] & ((1u << lane) - 1u));
+            if (p < kSquadShare) {
+                sh.v[par][p] = v[q];
+                sh.row[par][p] = make_int2(b[q], e[q]);
+            } else {
+                c.queue[next_depth % 3][atomicAdd(&c.st->squad_queue, 1)] = v[q];
+            }
+            c.depth[v[q]] = next_depth;
+            mf += (unsigned)(e[q] - b[q]);  // claims are distinct: a sum of rows stays below 2^31
+        }
+        at += __popc(m[q]);
+    }
+}
+
+// The block expands its frontier (parity par, n_f vertices): rows of 32
+// entries or more a warp each, shorter ones packed warp-wide over a scan of
+// their lengths, rows of up to kSquadBatch entries one per lane.
+__device__ __forceinline__ void squad_expand(const SquadCtx& c, SquadShared& sh, int32_t n_f, int32_t next_depth,
+                                             int par, unsigned& mf) {
+    const int lane = lane_id(), wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    int32_t per = 32;
+    while (per > 1 && nw * (per >> 1) >= n_f) per >>= 1;
+    for (int32_t base = wid * per; base < n_f; base += nw * per) {
+        int32_t b = 0, e = 0;
+        if (lane < per && base + lane < n_f) {
+            const int2 r = sh.row[par][base + lane];
+            b = r.x;
+            e = r.y;
+        }
+        int32_t j[kSquadBatch];
+        bool ok[kSquadBatch];
+        unsigned med = __ballot_sync(0xffffffffu, e - b >= 32);
+        while (med) {
+            const int l = __ffs(med) - 1;
+            med &= med - 1;
+            const int32_t lb = __shfl_sync(0xffffffffu, b, l), le = __shfl_sync(0xffffffffu, e, l);
+            for (int32_t j0 = lb;; j0 += 32 * kSquadBatch) {
+#pragma unroll
+                for (int q = 0; q < kSquadBatch; ++q) {
+                    j[q] = j0 + lane + 32 * q;
+                    ok[q] = le - j0 > lane + 32 * q;
+                }
+                squad_visit(c, sh, j, ok, next_depth, par ^ 1, mf);
+                if (le - j0 <= 32 * kSquadBatch) break;
+            }
+        }
+        const int32_t d = e - b >= 32 ? 0 : e - b;
+        if (__reduce_max_sync(0xffffffffu, (unsigned)d) <= (unsigned)kSquadBatch) {
+#pragma unroll
+            for (int q = 0; q < kSquadBatch; ++q) {
+                j[q] = b + q;
+                ok[q] = q < d;
+            }
+            squad_visit(c, sh, j, ok, next_depth, par ^ 1, mf);
+            continue;
+        }
+        int32_t incl = d;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += x;
+        }
+        const int32_t excl = incl - d;
+        const int32_t total = __shfl_sync(0xffffffffu, incl, 31);
+        for (int32_t k0 = 0; k0 < total; k0 += 32 * kSquadBatch) {
+#pragma unroll
+            for (int q = 0; q < kSquadBatch; ++q) {
+                const int32_t k = k0 + 32 * q + lane;
+                int owner = 0;
+#pragma unroll
+                for (int sft = 16; sft >= 1; sft >>= 1) {
+                    const int32_t ev = __shfl_sync(0xffffffffu, excl, owner + sft);
+                    if (ev <= k) owner += sft;
+                }
+                const int32_t ob = __shfl_sync(0xffffffffu, b, owner);
+                const int32_t oe = __shfl_sync(0xffffffffu, excl, owner);
+                ok[q] = k < total;
+                j[q] = ob + (k - oe);
+            }
+            squad_visit(c, sh, j, ok, next_depth, par ^ 1, mf);
+        }
+    }
+}
+
+// The squad's blocks run levels from L (its frontier: n_f vertices in the
+// queue and their bits in its bitmap) while the frontiers stay small.  The bits
+// of frontier L - 1 are cleared too, through its clear_nf vertices or word by
+// word.  At the end the next frontier is in the queue, without bits, and the
+// run's totals are in st->squad_*.  False when a wait gave
+// up.  Out of line: its registers do not weigh on the loops of the levels that
+// the whole grid runs.
+__device__ __noinline__ bool bfs_squad_run(const SquadCtx& c, SquadShared& sh, int32_t L, int32_t n_f,
+                                           int32_t clear_nf, int64_t clear_words) {
+    BfsRunState* st = c.st;
+    uint32_t* f_cur = c.f[L % 3];
+    uint32_t* f_clear = c.f[(L + 2) % 3];
+    const int32_t* q_clear = c.queue[(L + 2) % 3];
+    const int squad = n_f <= kSquadOne ? 1 : min(kSquadBlocks, (int)gridDim.x);
+    const int me = blockIdx.x, lane = lane_id();
+    if (me >= squad) return true;
+    const int tid = me * blockDim.x + threadIdx.x, nt = squad * blockDim.x;
+    // Neighbouring vertices of the queue stay together.
+    const int32_t i0 = (int32_t)((int64_t)n_f * me / squad), i1 = (int32_t)((int64_t)n_f * (me + 1) / squad);
+    const int32_t* q = c.queue[L % 3];
+    for (int32_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+        const int32_t u = __ldcg(q + i);
+        sh.v[0][i - i0] = u;
+        sh.row[0][i - i0] = make_int2(c.rp[u], c.rp[u + 1]);
+        f_cur[u >> 5] = 0u;
+    }
+    for (int32_t i = tid; i < clear_nf; i += nt) f_clear[__ldcg(q_clear + i) >> 5] = 0u;
+    for (int64_t w = tid; w < clear_words; w += nt) f_clear[w] = 0u;
+    if (threadIdx.x == 0) {
+        sh.count[1] = 0;
+        sh.mf = 0;
+    }
+    __syncthreads();
+    const unsigned long long limit = st->bar_limit_ns, t_run = global_timer_ns();
+    unsigned long long mr = 0, got = 0, last_mf = 0;  // thread 0: this block's totals
+    int32_t count = i1 - i0;
+    int par = 0;
+    bool again = true;
+    int32_t lev = L;
+    while (again) {
+        unsigned mf = 0;
+        // The next level's word: every block has read it (two levels ago), and
+        // adds to it only after this level's barrier.
+        unsigned long long cleared = 0;
+        if (me == 0 && threadIdx.x == 0 && squad > 1) cleared = atomicExch(&st->squad[(lev + 1) % 3].word, 0ull);
+        squad_expand(c, sh, count, lev + 1, par, mf);
+        mf = __reduce_add_sync(0xffffffffu, mf);
+        if (lane == 0 && mf) atomicAdd(&sh.mf, (unsigned long long)mf);
+        __syncthreads();
+        count = sh.count[par ^ 1];
+        if (threadIdx.x == 0) {
+            last_mf = sh.mf;
+            mr += last_mf;
+            got += (unsigned)count;
+            sh.count[par] = 0;  // the next level's claims
+            sh.mf = 0;
+            // One block asks for the end when its share is lopsided, the
+            // first also in time for the other blocks' wait, which is bounded.
+            const bool end = count > kSquadLean ||
+                             (me == 0 && (lev & 15) == 15 && global_timer_ns() - t_run > limit / 8);
+            unsigned long long* word = &st->squad[lev % 3].word;
+            const unsigned long long mine = kSqArrive + kSqNf * (unsigned)min(count, (int32_t)kSqMfCap) +
+                                            kSqMf * min(last_mf, kSqMfCap) + (end ? kSqEnd : 0ull);
+            // Relaxed: the blocks share nothing within a run but the visited
+            // bits, whose claims have all been answered, and this word.  (The
+            // word cleared at the level's start has been answered too.)
+            unsigned long long seen = mine;
+            if (squad > 1 && cleared != ~0ull) seen += atomicAdd(word, mine);
+            unsigned spins = 0;
+            uint64_t t0 = 0;
+            int ok = 1;
+            while ((int)(seen >> 56) < squad) {
+                seen = *(volatile unsigned long long*)word;
+                if ((++spins & 127u) == 0) {
+                    if (*(volatile int32_t*)&st->status != 0) {
+                        ok = 0;
+                        break;
+                    }
+                    const uint64_t t = global_timer_ns();
+                    if (t0 == 0) t0 = t;
+                    else if (t - t0 > limit) {
+                        atomicExch(&st->status, (int32_t)kDevBarrierTimeout);
+                        ok = 0;
+                        break;
+                    }
+                }
+            }
+            sh.total = seen;
+            sh.ok = ok;
+        }
+        __syncthreads();
+        if (!sh.ok) return false;
+        const unsigned long long t = sh.total;
+        const int32_t nf_all = (int32_t)(t & kSqField);
+        const unsigned long long mf_all = (t >> 24) & kSqField;
+        ++lev;
+        par ^= 1;
+        again = nf_all > 0 && nf_all <= kSquadRows && mf_all <= kSquadEntries && lev < c.max_depth &&
+                ((t >> 48) & 0xffull) == 0;
+    }
+    // The frontier back to the queue.
+    const int32_t held = min(count, kSquadShare);
+    __shared__ int32_t s_at;
+    if (threadIdx.x == 0) {
+        s_at = held ? atomicAdd(&st->squad_queue, held) : 0;
+        if (last_mf) atomicAdd(&st->squad_mf, last_mf);
+        if (mr) atomicAdd(&st->squad_mr, mr);
+        if (got) atomicAdd(&st->squad_reached, got);
+        if (me == 0) st->squad_level = lev;
+    }
+    __syncthreads();
+    const int32_t at = s_at;
+    int32_t* q_out = c.queue[lev % 3];
+    for (int32_t i = threadIdx.x; i < held; i += blockDim.x) q_out[at + i] = sh.v[par][i];
+    return true;
+}
+
 }  // namespace
 
 // The learned policy's part of a level decision, kept out of line so that
@@ -230,6 +525,10 @@ __device__ __noinline__ void level_eval(const float* pol, const float* feat, flo
     if (margin < band) policy_eval_block(pol, feat, h1, h2, logit);
 }
 
+// kSquad: with squad runs (graphs of low mean degree).  A variant of its own:
+// the runs' shared memory and registers cost a graph whose levels are few and
+// wide about a tenth (RMAT-24: 0.59 ms instead of 0.52).
+template <bool kSquad>
 __global__ void __launch_bounds__(512, 2) bfs_persistent_kernel(
     int32_t n, int32_t n_active, const int32_t* __restrict__ out_rp, const int32_t* __restrict__ out_col,
     const int32_t* __restrict__ in_rp, const int32_t* __restrict__ in_col, int32_t src, int32_t max_depth,
@@ -260,6 +559,31 @@ __global__ void __launch_bounds__(512, 2) bfs_persistent_kernel(
     // stays in L2, and no block pays to stage it in shared memory.
     const bool net = pol != nullptr;
     const bool can_pull = in_rp != nullptr;
+    // Small levels run on the squad where nothing asks for a level's timing,
+    // features or a given schedule.  They stay top-down whatever the direction
+    // rule says: so few entries cost less than a bottom-up level's barrier.
+    const bool squad_ok = kSquad && !trace && !net && (policy == GHB_POLICY_HEURISTIC || policy == GHB_POLICY_PUSH);
+    auto squad_fits = [&](int32_t rows, unsigned long long entries) {
+        return squad_ok && rows <= kSquadRows && entries <= kSquadEntries;
+    };
+    SquadShared* s_squad = nullptr;
+    SquadCtx* s_ctx = nullptr;
+    if constexpr (kSquad) {
+        __shared__ SquadShared squad_shared;
+        __shared__ SquadCtx squad_ctx;
+        s_squad = &squad_shared;
+        s_ctx = &squad_ctx;
+    }
+    if (kSquad && threadIdx.x == 0) {
+        s_ctx->rp = out_rp;
+        s_ctx->col = out_col;
+        s_ctx->visited = visited;
+        s_ctx->depth = depth;
+        s_ctx->queue[0] = qa, s_ctx->queue[1] = qb, s_ctx->queue[2] = qc;
+        s_ctx->f[0] = f0, s_ctx->f[1] = f1, s_ctx->f[2] = f2;
+        s_ctx->st = st;
+        s_ctx->max_depth = max_depth;
+    }
     // The first level's state, worked out by every block (s_pl: the state
     // payload each barrier hands on; see p_sync).
     __shared__ unsigned long long s_pl;
@@ -325,6 +649,70 @@ __global__ void __launch_bounds__(512, 2) bfs_persistent_kernel(
         const int32_t* q_clear = cslot == 0 ? qa : (cslot == 1 ? qb : qc);
         const int32_t clear_nf = last_nf;
         const bool clear_sparse = last_top && (int64_t)clear_nf * 4 < words;
+        if (kSquad && (pl & kPlSquad)) {
+            // ---- the squad runs this level and the small ones after it; the
+            // other blocks wait at the barrier below.
+            if ((int)blockIdx.x < kSquadBlocks) {
+                if (!bfs_squad_run(*s_ctx, *s_squad, L, n_f, clear_sparse ? clear_nf : 0, clear_sparse ? 0 : words))
+                    return;
+            }
+            // Whichever block closes the barrier sets the handed-back
+            // frontier's bits and decides by the rule of any level.
+            if (!p_sync(st, [&]() {
+                    const int32_t nf = vs->squad_queue, lev = vs->squad_level;
+                    const int fs = lev % 3;
+                    uint32_t* f_out = fs == 0 ? f0 : (fs == 1 ? f1 : f2);
+                    const int32_t* q_out = fs == 0 ? qa : (fs == 1 ? qb : qc);
+                    for (int32_t i = threadIdx.x; i < nf; i += blockDim.x) {
+                        const int32_t u = __ldcg(q_out + i);
+                        atomicOr(f_out + (u >> 5), 1u << (u & 31));
+                    }
+                    if (threadIdx.x == 0) {
+                        const unsigned long long mf = vs->squad_mf, mr = vs->squad_mr, m_r = vs->m_r + mr;
+                        // The run expanded its first frontier and all that it
+                        // reached but the last.
+                        const unsigned long long ex = vs->examined + vs->mf[slot] + mr - mf;
+                        const bool done = nf == 0 || lev >= max_depth;
+                        const double m_u = (double)(m_total - (long long)m_r);
+                        const bool again = !done && squad_fits(nf, mf);
+                        const int nd = policy != GHB_POLICY_PUSH && can_pull && !again && (double)mf > m_u / alpha &&
+                                               (double)mf > (double)m_total / gamma
+                                           ? 1
+                                           : 0;
+                        s_pl = p_payload(nf, done, nd, p_append(nd, 0, mf) != 0, true) | (again ? kPlSquad : 0ull);
+                        st->examined = ex;
+                        st->ex_prev = ex;
+                        st->m_r = m_r;
+                        st->reached = vs->reached + (long long)vs->squad_reached;
+                        st->levels = lev;
+                        st->level = lev;
+                        st->t_prev = global_timer_ns();
+                        st->dir = nd;
+                        st->append = p_append(nd, 0, mf);
+                        st->queue_ok = 1;
+                        st->done = done ? 1 : 0;
+                        for (int k = 0; k < 3; ++k) {
+                            st->nf[k] = 0;
+                            st->mf[k] = 0;
+                            st->d2[k] = 0;
+                            st->dmax[k] = 0;
+                            st->big[k] = 0;
+                            st->squad[k].word = 0;
+                        }
+                        st->mf[fs] = mf;  // a run that follows starts from it
+                        st->squad_queue = 0;
+                        st->squad_mf = 0;
+                        st->squad_mr = 0;
+                        st->squad_reached = 0;
+                    }
+                }, &s_pl))
+                return;
+            if (s_pl & kPlDone) break;
+            L = vs->level - 1;  // the run's last level: its bits are cleared already
+            last_nf = 0;
+            last_top = true;
+            continue;
+        }
         last_nf = n_f;
         last_top = dir == 0;
         auto clear_frontier_bitmap = [&]() {
@@ -429,6 +817,13 @@ __global__ void __launch_bounds__(512, 2) bfs_persistent_kernel(
                 const bool done = nf_next == 0 || L + 1 >= max_depth;
                 st->done = done ? 1 : 0;
                 s_pl = p_payload(nf_next, done, nd, p_append(nd, fmt, mf_next) != 0, dir == 0 && append);
+                // A small frontier in the queue goes to the squad, if it can
+                // also clear this level's bits: a traversal that is still
+                // narrow after kSquadLevel levels repays the hand-over (about
+                // two levels' time each way).
+                if (kSquad && !done && L >= kSquadLevel && dir == 0 && append && squad_fits(nf_next, mf_next) &&
+                    ((int64_t)n_f * 4 < words ? n_f <= 4 * kSquadRows : words <= kSquadWords))
+                    s_pl |= kPlSquad;
                 st->nf[cslot] = 0;
                 st->mf[cslot] = 0;
                 st->d2[cslot] = 0;
@@ -725,7 +1120,7 @@ bool bfs_persistent_available(ghb_workspace* ws, int* blocks) {
     if (!known[dev]) {
         int coop = 0, per_sm = 0;
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-        if (coop && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bfs_persistent_kernel, 512, 0) ==
+        if (coop && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bfs_persistent_kernel<true>, 512, 0) ==
                         cudaSuccess)
             cached[dev] = std::min(per_sm, 2);
         known[dev] = true;
@@ -803,7 +1198,11 @@ int bfs_persistent_run(ghb_workspace* ws, int32_t n, int32_t n_active, const int
     GHB_CUDA_TRY(cudaStreamSynchronize(st));
     const int64_t m_total = hp[0];
     if (stats) GHB_CUDA_TRY(cudaEventRecord(ws->ev_start, st));
-    GHB_TRY(launch_coop(ws, bfs_persistent_kernel, dim3(blocks), dim3(512), 0, n,
+    // Meshes, road networks, paths: up to 4.5 entries per vertex.  (A random
+    // graph with six has ten levels, and the larger kernel cost it 5 %.)
+    const bool low_degree = 2 * m_total <= 9 * (int64_t)n;
+    GHB_TRY(launch_coop(ws, low_degree ? bfs_persistent_kernel<true> : bfs_persistent_kernel<false>, dim3(blocks),
+                        dim3(512), 0, n,
                         n_active, out_rp, out_col, in_rp, in_col, src, max_depth, depth, vis, f0, f1, f2, qa, qb, qc, big,
                         policy, alpha, beta, gamma, (float)ws->tune.pol_band, m_total,
                         (const int8_t*)(sched_len ? sched : nullptr), sched_len,
