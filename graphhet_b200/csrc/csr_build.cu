@@ -8,10 +8,11 @@
 // keep the last entry of every equal-key run, and derive rowptr from the run
 // boundaries without atomics.
 #include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_scan.cuh>
 
 #include "common.cuh"
 #include "ghb_gen.h"
+#include "scan.cuh"
+#include "sorted_rows.cuh"
 
 namespace ghb {
 namespace {
@@ -50,38 +51,123 @@ __global__ void make_keys_kernel(const int32_t* __restrict__ src, const int32_t*
     }
 }
 
-// keep[i] = 1 when entry i is the last of its equal-key run and not a sentinel.
-__global__ void mark_last_kernel(const uint64_t* __restrict__ keys, int64_t count, uint64_t sentinel,
-                                 int32_t* __restrict__ keep) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        uint64_t k = keys[i];
-        bool last = (i + 1 == count) || keys[i + 1] != k;
-        keep[i] = (last && k != sentinel) ? 1 : 0;
+// Compaction of the sorted keys by tiles of kTile: an entry stays when it is
+// the last of its equal-key run and not a sentinel.  The flags come from
+// comparing neighbours in registers, twice (once to count per tile, once to
+// write), so no flag or position array goes through memory; the row offsets
+// are written at the runs' first entries, so the kept keys need no copy.
+constexpr int kTileThreads = 256, kTileItems = 8;
+constexpr int64_t kTile = kTileThreads * kTileItems;
+
+// Keys of the tile's items (consecutive per thread) with the key before and
+// after them; `none` (no key has that value) beyond the ends.
+constexpr uint64_t kNoKey = ~0ull;
+struct TileKeys {
+    uint64_t k[kTileItems + 2];
+    __device__ __forceinline__ void load(const uint64_t* __restrict__ keys, int64_t first, int64_t count) {
+        k[0] = first > 0 && first <= count ? keys[first - 1] : kNoKey;
+#pragma unroll
+        for (int q = 0; q <= kTileItems; ++q) k[q + 1] = first + q < count ? keys[first + q] : kNoKey;
     }
+    __device__ __forceinline__ bool first_of_run(int q) const { return k[q + 1] != k[q]; }
+    __device__ __forceinline__ bool kept(int q, uint64_t sentinel) const {
+        return k[q + 1] != k[q + 2] && k[q + 1] < sentinel;
+    }
+};
+
+__global__ void __launch_bounds__(kTileThreads) count_kept_kernel(const uint64_t* __restrict__ keys, int64_t count,
+                                                                  uint64_t sentinel, int32_t* tile_kept) {
+    __shared__ int32_t s_sum;
+    if (threadIdx.x == 0) s_sum = 0;
+    __syncthreads();
+    // Neighbouring threads read neighbouring keys: a count needs no order.
+    const int64_t base = blockIdx.x * kTile;
+    int32_t c = 0;
+#pragma unroll
+    for (int q = 0; q < kTileItems; ++q) {
+        const int64_t i = base + q * kTileThreads + threadIdx.x;
+        const uint64_t k = i < count ? keys[i] : kNoKey;
+        const uint64_t next = i + 1 < count ? keys[i + 1] : kNoKey;
+        c += k < sentinel && k != next ? 1 : 0;
+    }
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane_id() == 0 && c) atomicAdd(&s_sum, c);
+    __syncthreads();
+    if (threadIdx.x == 0) tile_kept[blockIdx.x] = s_sum;
 }
 
-__global__ void compact_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ vals,
-                               const int32_t* __restrict__ keep, const int32_t* __restrict__ pos,
-                               int64_t count, int bits, const double* __restrict__ w_in,
-                               int weight_mode, uint64_t wstream, int transposed,
-                               uint64_t* __restrict__ out_keys, int32_t* __restrict__ col,
-                               double* __restrict__ w) {
+__global__ void __launch_bounds__(kTileThreads) compact_kernel(const uint64_t* __restrict__ keys,
+                                                               const uint32_t* __restrict__ vals,
+                                                               const int32_t* __restrict__ tile_pos, int64_t count,
+                                                               int32_t n, int bits, uint64_t sentinel,
+                                                               const double* __restrict__ w_in, int weight_mode,
+                                                               uint64_t wstream, int transposed,
+                                                               int32_t* __restrict__ rowptr, int32_t* __restrict__ col,
+                                                               double* __restrict__ w) {
+    __shared__ int32_t s_warp[kTileThreads / 32];
+    __shared__ uint64_t s_out[kTile];    // kept keys, in order
+    __shared__ uint32_t s_val[kTile];
+    __shared__ RowGaps gaps;
     const uint64_t mask = (1ull << bits) - 1;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        if (!keep[i]) continue;
-        uint64_t k = keys[i];
-        int32_t p = pos[i];
-        uint32_t r = (uint32_t)(k >> bits), c = (uint32_t)(k & mask);
-        out_keys[p] = k;
-        col[p] = (int32_t)c;
-        if (w) {
-            if (w_in) {
-                w[p] = w_in[vals[i]];
-            } else {
-                uint32_t a = transposed ? c : r, b = transposed ? r : c;
-                w[p] = ghb_pair_weight(wstream, a, b, weight_mode);
+    const int lane = lane_id(), wid = threadIdx.x >> 5;
+    if (threadIdx.x == 0) gaps.count = 0;
+    const int64_t first = blockIdx.x * kTile + (int64_t)threadIdx.x * kTileItems;
+    TileKeys t;
+    t.load(keys, first, count);
+    uint32_t v[kTileItems];
+#pragma unroll
+    for (int q = 0; q < kTileItems; ++q) v[q] = vals && first + q < count ? vals[first + q] : 0u;
+    int32_t mine = 0;
+#pragma unroll
+    for (int q = 0; q < kTileItems; ++q) mine += t.kept(q, sentinel) ? 1 : 0;
+    int32_t incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += x;
+    }
+    if (lane == 31) s_warp[wid] = incl;
+    __syncthreads();
+    int32_t before = 0, all = 0;
+#pragma unroll
+    for (int i = 0; i < kTileThreads / 32; ++i) {
+        if (i < wid) before += s_warp[i];
+        all += s_warp[i];
+    }
+    const int32_t p0 = tile_pos[blockIdx.x];
+    int32_t p = before + incl - mine;  // kept entries of the tile before this item
+#pragma unroll
+    for (int q = 0; q < kTileItems; ++q) {
+        // Rows (previous key's, this key's] start here; sentinels and the end
+        // close the last row.
+        if (first + q <= count && (t.first_of_run(q) || first + q == count)) {
+            const int64_t prev = t.k[q] == kNoKey ? -1 : (int64_t)min(t.k[q] >> bits, (uint64_t)n);
+            const int64_t cur = t.k[q + 1] >= sentinel ? (int64_t)n : (int64_t)(t.k[q + 1] >> bits);
+            if (t.k[q] == kNoKey || t.k[q] < sentinel) fill_rows(gaps, rowptr, prev + 1, cur, p0 + p);
+        }
+        if (t.kept(q, sentinel)) {
+            s_out[p] = t.k[q + 1];
+            s_val[p] = v[q];
+            ++p;
+        }
+    }
+    __syncthreads();
+    fill_long_rows(gaps, rowptr);
+    // Coalesced writes; a thread's weight gathers are independent.
+#pragma unroll
+    for (int q = 0; q < kTileItems; ++q) {
+        const int32_t i = q * kTileThreads + threadIdx.x;
+        if (i < all) {
+            const uint64_t k = s_out[i];
+            const uint32_t r = (uint32_t)(k >> bits), c = (uint32_t)(k & mask);
+            col[p0 + i] = (int32_t)c;
+            if (w) {
+                if (w_in) {
+                    w[p0 + i] = __ldg(w_in + s_val[i]);
+                } else {
+                    const uint32_t a = transposed ? c : r, b = transposed ? r : c;
+                    w[p0 + i] = ghb_pair_weight(wstream, a, b, weight_mode);
+                }
             }
         }
     }
@@ -90,13 +176,18 @@ __global__ void compact_kernel(const uint64_t* __restrict__ keys, const uint32_t
 // rowptr from sorted row ids: rowptr[r] = number of entries with row < r.
 __global__ void rowptr_from_sorted_kernel(const uint64_t* __restrict__ keys, int64_t m, int bits,
                                           int32_t n, int32_t* __restrict__ rowptr) {
+    __shared__ RowGaps gaps;
+    if (threadIdx.x == 0) gaps.count = 0;
+    __syncthreads();
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p <= m;
          p += (int64_t)gridDim.x * blockDim.x) {
         // Boundary between entry p-1 and entry p: rows (prev, cur] start at p.
         int64_t prev = (p == 0) ? -1 : (int64_t)(keys[p - 1] >> bits);
         int64_t cur = (p == m) ? (int64_t)n : (int64_t)(keys[p] >> bits);
-        for (int64_t r = prev + 1; r <= cur; ++r) rowptr[r] = (int32_t)p;
+        if (cur > prev) fill_rows(gaps, rowptr, prev + 1, cur, (int32_t)p);
     }
+    __syncthreads();
+    fill_long_rows(gaps, rowptr);
 }
 
 __global__ void transpose_keys_kernel(const int32_t* __restrict__ rowptr,
@@ -180,8 +271,9 @@ int ghb_csr_build(ghb_workspace* ws, int32_t n, const int32_t* src, const int32_
     const uint64_t sentinel = 1ull << (2 * bits);
     const bool want_vals = (w_in != nullptr) && (w != nullptr);
 
-    // Scratch: keys x2, vals x2, keep, pos, compacted keys, CUB temp.
-    size_t sort_tmp = 0, scan_tmp = 0;
+    // Scratch: keys x2, vals x2, counts and positions by tile, CUB temp.
+    size_t sort_tmp = 0;
+    const int64_t tiles = count / kTile + 1;  // the end of the entries lies in a tile
     {
         cub::DoubleBuffer<uint64_t> dk(nullptr, nullptr);
         cub::DoubleBuffer<uint32_t> dv(nullptr, nullptr);
@@ -189,29 +281,29 @@ int ghb_csr_build(ghb_workspace* ws, int32_t n, const int32_t* src, const int32_
             cub::DeviceRadixSort::SortPairs(nullptr, sort_tmp, dk, dv, (int64_t)count, 0, end_bit);
         else
             cub::DeviceRadixSort::SortKeys(nullptr, sort_tmp, dk, (int64_t)count, 0, end_bit);
-        cub::DeviceScan::ExclusiveSum(nullptr, scan_tmp, (int32_t*)nullptr, (int32_t*)nullptr,
-                                      (int64_t)count);
     }
     auto carve = [&](Carver& c, uint64_t** k0, uint64_t** k1, uint32_t** v0, uint32_t** v1,
-                     int32_t** keep, int32_t** pos, void** tmp, int32_t** bad) {
+                     int32_t** kept, int32_t** pos, int64_t** sums, void** tmp, int32_t** bad) {
         *k0 = c.take<uint64_t>(count + 1);
         *k1 = c.take<uint64_t>(count + 1);
         *v0 = want_vals ? c.take<uint32_t>(count + 1) : nullptr;
         *v1 = want_vals ? c.take<uint32_t>(count + 1) : nullptr;
-        *keep = c.take<int32_t>(count + 1);
-        *pos = c.take<int32_t>(count + 1);
-        *tmp = c.take<char>(sort_tmp > scan_tmp ? sort_tmp : scan_tmp);
+        *kept = c.take<int32_t>(tiles);
+        *pos = c.take<int32_t>(tiles + 1);
+        *sums = c.take<int64_t>(scan_scratch_words(tiles));
+        *tmp = c.take<char>(sort_tmp);
         *bad = c.take<int32_t>(4);
     };
     uint64_t *k0, *k1;
     uint32_t *v0, *v1;
-    int32_t *keep, *pos, *bad;
+    int32_t *kept, *pos, *bad;
+    int64_t* sums;
     void* tmp;
     Carver sizing(nullptr);
-    carve(sizing, &k0, &k1, &v0, &v1, &keep, &pos, &tmp, &bad);
+    carve(sizing, &k0, &k1, &v0, &v1, &kept, &pos, &sums, &tmp, &bad);
     GHB_TRY(ws_reserve(ws, sizing.off));
     Carver c(ws->scratch);
-    carve(c, &k0, &k1, &v0, &v1, &keep, &pos, &tmp, &bad);
+    carve(c, &k0, &k1, &v0, &v1, &kept, &pos, &sums, &tmp, &bad);
 
     GHB_CUDA_TRY(cudaMemsetAsync(bad, 0, sizeof(int32_t), ws->stream));
     const unsigned g = ws->num_sms * 8;
@@ -230,17 +322,10 @@ int ghb_csr_build(ghb_workspace* ws, int32_t n, const int32_t* src, const int32_
         ws->launches++;
         uint64_t* keys = dk.Current();
         uint32_t* vals = want_vals ? dv.Current() : nullptr;
-        uint64_t* other = dk.Alternate();
-        GHB_TRY(launch(ws, mark_last_kernel, dim3(g), dim3(256), 0, (const uint64_t*)keys, count,
-                       sentinel, keep));
-        size_t sb = scan_tmp;
-        GHB_CUDA_TRY(cub::DeviceScan::ExclusiveSum(tmp, sb, keep, pos, (int64_t)count, ws->stream));
-        ws->launches++;
-        // m = pos[count-1] + keep[count-1]
-        GHB_CUDA_TRY(cudaMemcpyAsync(ws->host_pinned, pos + count - 1, sizeof(int32_t),
-                                     cudaMemcpyDeviceToHost, ws->stream));
-        GHB_CUDA_TRY(cudaMemcpyAsync(reinterpret_cast<int32_t*>(ws->host_pinned) + 1, keep + count - 1,
-                                     sizeof(int32_t), cudaMemcpyDeviceToHost, ws->stream));
+        GHB_TRY(launch(ws, count_kept_kernel, dim3((unsigned)tiles), dim3(kTileThreads), 0, (const uint64_t*)keys, count,
+                       sentinel, kept));
+        GHB_TRY(scan_exclusive_i32(ws, kept, pos, tiles, sums));
+        GHB_CUDA_TRY(cudaMemcpyAsync(ws->host_pinned, pos + tiles, sizeof(int32_t), cudaMemcpyDeviceToHost, ws->stream));
         GHB_CUDA_TRY(cudaMemcpyAsync(reinterpret_cast<int32_t*>(ws->host_pinned) + 2, bad,
                                      sizeof(int32_t), cudaMemcpyDeviceToHost, ws->stream));
         GHB_CUDA_TRY(cudaStreamSynchronize(ws->stream));
@@ -249,15 +334,12 @@ int ghb_csr_build(ghb_workspace* ws, int32_t n, const int32_t* src, const int32_
             set_error("invalid argument: edge endpoint outside [0, n)");
             return GHB_ERR_INVALID_ARGUMENT;
         }
-        const int64_t m = (int64_t)hp[0] + hp[1];
-        GHB_TRY(launch(ws, compact_kernel, dim3(g), dim3(256), 0, (const uint64_t*)keys,
-                       (const uint32_t*)vals, (const int32_t*)keep, (const int32_t*)pos, count,
-                       bits, w_in, (int)(w_in ? 0 : weight_mode),
-                       ghb_stream(weight_seed, GHB_PURPOSE_WEIGHT),
-                       (int)((flags & GHB_BUILD_TRANSPOSE) != 0), other, col,
+        const int64_t m = hp[0];
+        GHB_TRY(launch(ws, compact_kernel, dim3((unsigned)tiles), dim3(kTileThreads), 0, (const uint64_t*)keys,
+                       (const uint32_t*)vals, (const int32_t*)pos, count, n, bits, sentinel, w_in,
+                       (int)(w_in ? 0 : weight_mode), ghb_stream(weight_seed, GHB_PURPOSE_WEIGHT),
+                       (int)((flags & GHB_BUILD_TRANSPOSE) != 0), rowptr, col,
                        (weight_mode != 0 || w_in) ? w : (double*)nullptr));
-        GHB_TRY(launch(ws, rowptr_from_sorted_kernel, dim3(grid_for(m + 1, 256, g)), dim3(256), 0,
-                       (const uint64_t*)other, m, bits, n, rowptr));
         *m_out = m;
     } else {
         GHB_CUDA_TRY(cudaMemsetAsync(rowptr, 0, sizeof(int32_t) * ((size_t)n + 1), ws->stream));

@@ -13,10 +13,13 @@
 // GPU_csr.hpp:282-339); results are mapped back to the caller's ids.
 #include <cub/device/device_radix_sort.cuh>
 
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
 #include "graph.cuh"
+#include "scan.cuh"
+#include "sorted_rows.cuh"
 
 namespace ghb {
 namespace {
@@ -112,22 +115,48 @@ __global__ void relabel_keys_kernel(int32_t n, const int32_t* __restrict__ rp, c
     }
 }
 
-__global__ void relabel_out_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ vals, int64_t m,
-                                   int bits, const double* __restrict__ w, int32_t* col, double* w_out) {
+// Columns, weights and row offsets of the sorted keys in one pass over them;
+// *repeat is set when a row holds an entry twice.
+__global__ void __launch_bounds__(256) relabel_out_kernel(const uint64_t* __restrict__ keys,
+                                                          const uint32_t* __restrict__ vals, int64_t m, int32_t n,
+                                                          int bits, const double* __restrict__ w, int32_t* col,
+                                                          double* w_out, int32_t* __restrict__ rowptr,
+                                                          int32_t* repeat) {
+    constexpr int kItems = 4;  // weight gathers in flight per thread
+    __shared__ RowGaps gaps;
+    if (threadIdx.x == 0) gaps.count = 0;
+    __syncthreads();
     const uint64_t mask = (1ull << bits) - 1;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
-        col[i] = (int32_t)(keys[i] & mask);
-        if (w_out) w_out[i] = w[vals[i]];
+    bool twice = false;
+    for (int64_t i0 = blockIdx.x * (int64_t)(256 * kItems) + threadIdx.x; i0 <= m;
+         i0 += (int64_t)gridDim.x * (256 * kItems)) {
+        uint32_t v[kItems];
+#pragma unroll
+        for (int q = 0; q < kItems; ++q) {
+            const int64_t i = i0 + q * 256;
+            v[q] = w_out && i < m ? vals[i] : 0u;
+        }
+        double x[kItems];
+#pragma unroll
+        for (int q = 0; q < kItems; ++q) x[q] = w_out && i0 + q * 256 < m ? w[v[q]] : 0.0;
+#pragma unroll
+        for (int q = 0; q < kItems; ++q) {
+            const int64_t i = i0 + q * 256;
+            if (i > m) break;
+            const uint64_t k = i < m ? keys[i] : (uint64_t)n << bits;
+            const uint64_t kp = i > 0 ? keys[i - 1] : 0;
+            const int64_t prev = i > 0 ? (int64_t)(kp >> bits) : -1, cur = (int64_t)(k >> bits);
+            if (cur > prev) fill_rows(gaps, rowptr, prev + 1, cur, (int32_t)i);
+            if (i < m) {
+                col[i] = (int32_t)(k & mask);
+                if (w_out) w_out[i] = x[q];
+                twice |= i > 0 && k == kp;
+            }
+        }
     }
-}
-
-__global__ void rowptr_from_keys_kernel(const uint64_t* __restrict__ keys, int64_t m, int bits, int32_t n,
-                                        int32_t* __restrict__ rowptr) {
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p <= m; p += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t prev = (p == 0) ? -1 : (int64_t)(keys[p - 1] >> bits);
-        const int64_t cur = (p == m) ? (int64_t)n : (int64_t)(keys[p] >> bits);
-        for (int64_t r = prev + 1; r <= cur; ++r) rowptr[r] = (int32_t)p;
-    }
+    if (twice) *repeat = 1;
+    __syncthreads();
+    fill_long_rows(gaps, rowptr);
 }
 
 __global__ void outdeg_kernel(int32_t n, const int32_t* __restrict__ rp, int32_t* outdeg) {
@@ -147,29 +176,10 @@ int bits_for_n(int32_t n) {
     return bits;
 }
 
-template <class T>
-int dalloc(T** p, size_t count, int64_t* total) {
-    GHB_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(p), sizeof(T) * (count ? count : 1)));
-    *total += (int64_t)(sizeof(T) * (count ? count : 1));
-    return GHB_OK;
-}
-
 // Relabel one CSR (rows and columns through perm), rows sorted, weights
-// carried along.
-// Sets *flag when a sorted row holds an entry twice (warp per row).
-__global__ void repeat_check_kernel(int32_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ col,
-                                    int32_t* flag) {
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t v = warp; v < n; v += nwarps) {
-        const int32_t b = rp[v], e = rp[v + 1];
-        for (int32_t j = b + 1 + lane_id(); j < e; j += 32)
-            if (col[j] == col[j - 1]) *flag = 1;
-    }
-}
-
+// carried along; *repeat (device) is set when a row holds an entry twice.
 int relabel_csr(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* rp, const int32_t* col, const double* w,
-                const int32_t* perm, int32_t* rp_out, int32_t* col_out, double* w_out) {
+                const int32_t* perm, int32_t* rp_out, int32_t* col_out, double* w_out, int32_t* repeat) {
     if (m == 0) {
         GHB_CUDA_TRY(cudaMemsetAsync(rp_out, 0, sizeof(int32_t) * ((size_t)n + 1), ws->stream));
         return GHB_OK;
@@ -206,12 +216,9 @@ int relabel_csr(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* rp, cons
     if (want_vals) GHB_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tb, dk, dv, m, 0, 2 * bits, ws->stream));
     else GHB_CUDA_TRY(cub::DeviceRadixSort::SortKeys(tmp, tb, dk, m, 0, 2 * bits, ws->stream));
     ws->launches++;
-    GHB_TRY(launch(ws, relabel_out_kernel, dim3(g), dim3(256), 0, (const uint64_t*)dk.Current(),
-                   (const uint32_t*)(want_vals ? dv.Current() : nullptr), m, bits, w, col_out,
-                   want_vals ? w_out : (double*)nullptr));
-    GHB_TRY(launch(ws, rowptr_from_keys_kernel, dim3(grid_for(m + 1, 256, g)), dim3(256), 0,
-                   (const uint64_t*)dk.Current(), m, bits, n, rp_out));
-    return GHB_OK;
+    return launch(ws, relabel_out_kernel, dim3(grid_for(m + 1, 256 * 4, g)), dim3(256), 0, (const uint64_t*)dk.Current(),
+                  (const uint32_t*)(want_vals ? dv.Current() : nullptr), m, n, bits, w, col_out,
+                  want_vals ? w_out : (double*)nullptr, rp_out, repeat);
 }
 
 }  // namespace
@@ -240,22 +247,10 @@ int ghb_graph_destroy(ghb_graph* g) {
     int cur = 0;
     cudaGetDevice(&cur);
     cudaSetDevice(g->device);
-    cudaFree(g->perm);
-    cudaFree(g->iperm);
-    cudaFree(g->rowptr);
-    cudaFree(g->col);
-    cudaFree(g->w);
-    cudaFree(g->outdeg);
+    cudaFree(g->slab);
     cudaFree(g->sw_col);
     cudaFree(g->sw_w);
     cudaFree(g->sw_le);
-    if (g->directed) {
-        cudaFree(g->in_rowptr);
-        cudaFree(g->in_col);
-        cudaFree(g->in_w);
-        cudaFree(g->all_rowptr);
-        cudaFree(g->all_col);
-    }
     cudaSetDevice(cur);
     delete g;
     return GHB_OK;
@@ -294,17 +289,37 @@ int ghb_graph_create(ghb_workspace* ws, int32_t n, const int32_t* out_rowptr, co
         s = (x);                  \
         if (s != GHB_OK) return fail(s); \
     } while (0)
-    GG_TRY(dalloc(&g->perm, n, &g->device_bytes));
-    GG_TRY(dalloc(&g->iperm, n, &g->device_bytes));
-    GG_TRY(dalloc(&g->rowptr, (size_t)n + 1, &g->device_bytes));
-    GG_TRY(dalloc(&g->col, (size_t)g->m, &g->device_bytes));
-    if (g->weighted) GG_TRY(dalloc(&g->w, (size_t)g->m, &g->device_bytes));
-    GG_TRY(dalloc(&g->outdeg, n, &g->device_bytes));
-    if (directed) {
-        GG_TRY(dalloc(&g->in_rowptr, (size_t)n + 1, &g->device_bytes));
-        GG_TRY(dalloc(&g->in_col, (size_t)g->m_in, &g->device_bytes));
-        if (in_w) GG_TRY(dalloc(&g->in_w, (size_t)g->m_in, &g->device_bytes));
-    } else {
+    // One allocation for all of the handle's arrays (an allocation and its
+    // release each cost hundreds of microseconds at these sizes).
+    auto carve = [&](Carver& c) {
+        g->perm = c.take<int32_t>(n);
+        g->iperm = c.take<int32_t>(n);
+        g->rowptr = c.take<int32_t>((size_t)n + 1);
+        g->col = c.take<int32_t>(std::max<int64_t>(g->m, 1));
+        if (g->weighted) g->w = c.take<double>(std::max<int64_t>(g->m, 1));
+        g->outdeg = c.take<int32_t>(n);
+        if (directed) {
+            g->in_rowptr = c.take<int32_t>((size_t)n + 1);
+            g->in_col = c.take<int32_t>(std::max<int64_t>(g->m_in, 1));
+            if (in_w) g->in_w = c.take<double>(std::max<int64_t>(g->m_in, 1));
+            g->all_rowptr = c.take<int32_t>((size_t)n + 1);
+            g->all_col = c.take<int32_t>(std::max<int64_t>(g->m + g->m_in, 1));
+        }
+    };
+    Carver need(nullptr);
+    carve(need);
+    {
+        const cudaError_t e = cudaMalloc(&g->slab, need.off);
+        if (e != cudaSuccess) {
+            set_error(std::string("resident graph: ") + cudaGetErrorString(e));
+            g->slab = nullptr;
+            return fail(e == cudaErrorMemoryAllocation ? GHB_ERR_OUT_OF_MEMORY : GHB_ERR_CUDA);
+        }
+    }
+    g->device_bytes = (int64_t)need.off;
+    Carver slab(g->slab);
+    carve(slab);
+    if (!directed) {
         g->in_rowptr = g->rowptr;
         g->in_col = g->col;
         g->in_w = g->w;
@@ -315,7 +330,8 @@ int ghb_graph_create(ghb_workspace* ws, int32_t n, const int32_t* out_rowptr, co
     {
         size_t sort_tmp = 0;
         cub::DoubleBuffer<uint64_t> dk0(nullptr, nullptr);
-        cub::DeviceRadixSort::SortKeys(nullptr, sort_tmp, dk0, (int64_t)n, 0, 64);
+        // Ids enter in order and the sort is stable: only the degrees are sorted.
+        cub::DeviceRadixSort::SortKeys(nullptr, sort_tmp, dk0, (int64_t)n, 32, 64);
         Carver sizing(nullptr);
         sizing.take<uint64_t>(n);
         sizing.take<uint64_t>(n);
@@ -332,7 +348,7 @@ int ghb_graph_create(ghb_workspace* ws, int32_t n, const int32_t* out_rowptr, co
                       directed ? in_rowptr : (const int32_t*)nullptr, k0));
         cub::DoubleBuffer<uint64_t> dk(k0, k1);
         size_t tb = sort_tmp;
-        cudaError_t e = cub::DeviceRadixSort::SortKeys(tmp, tb, dk, (int64_t)n, 0, 64, st);
+        cudaError_t e = cub::DeviceRadixSort::SortKeys(tmp, tb, dk, (int64_t)n, 32, 64, st);
         if (e != cudaSuccess) {
             set_error(std::string("degree sort: ") + cudaGetErrorString(e));
             return fail(GHB_ERR_CUDA);
@@ -349,25 +365,18 @@ int ghb_graph_create(ghb_workspace* ws, int32_t n, const int32_t* out_rowptr, co
         g->n_active = hp[0];
     }
     // 2. relabelled CSRs
-    GG_TRY(relabel_csr(ws, n, g->m, out_rowptr, out_col, out_w, g->perm, g->rowptr, g->col, g->w));
-    if (directed) GG_TRY(relabel_csr(ws, n, g->m_in, in_rowptr, in_col, in_w, g->perm, g->in_rowptr, g->in_col, g->in_w));
+    int32_t* repeat = reinterpret_cast<int32_t*>(ws->dev_small);  // [0] out-rows, [1] in-rows (not used)
+    GG_TRY(cudaMemsetAsync(repeat, 0, 2 * sizeof(int32_t), st) == cudaSuccess ? GHB_OK : GHB_ERR_CUDA);
+    GG_TRY(relabel_csr(ws, n, g->m, out_rowptr, out_col, out_w, g->perm, g->rowptr, g->col, g->w, repeat));
+    if (directed)
+        GG_TRY(relabel_csr(ws, n, g->m_in, in_rowptr, in_col, in_w, g->perm, g->in_rowptr, g->in_col, g->in_w,
+                           repeat + 1));
     GG_TRY(launch(ws, outdeg_kernel, dim3(grid_for(n, 256, ws->num_sms * 8)), dim3(256), 0, n,
                   (const int32_t*)g->rowptr, g->outdeg));
-    {
-        int32_t* flag = reinterpret_cast<int32_t*>(ws->dev_small);
-        GG_TRY(cudaMemsetAsync(flag, 0, sizeof(int32_t), st) == cudaSuccess ? GHB_OK : GHB_ERR_CUDA);
-        GG_TRY(launch(ws, repeat_check_kernel, dim3(grid_for((int64_t)n * 32, 256, ws->num_sms * 8)), dim3(256), 0, n,
-                      (const int32_t*)g->rowptr, (const int32_t*)g->col, flag));
-        GG_TRY(cudaMemcpyAsync(hp + 2, flag, sizeof(int32_t), cudaMemcpyDeviceToHost, st) == cudaSuccess ? GHB_OK
-                                                                                                      : GHB_ERR_CUDA);
-        GG_TRY(cudaStreamSynchronize(st) == cudaSuccess ? GHB_OK : GHB_ERR_CUDA);
-        g->repeats = hp[2] != 0;
-    }
-    if (directed) {
-        GG_TRY(dalloc(&g->all_rowptr, (size_t)n + 1, &g->device_bytes));
-        GG_TRY(dalloc(&g->all_col, (size_t)(g->m + g->m_in), &g->device_bytes));
+    if (directed)
         GG_TRY(ghb_csr_merge_in_out(ws, n, g->in_rowptr, g->in_col, g->rowptr, g->col, g->all_rowptr, g->all_col));
-    }
+    GG_TRY(cudaMemcpyAsync(hp + 2, repeat, sizeof(int32_t), cudaMemcpyDeviceToHost, st) == cudaSuccess ? GHB_OK
+                                                                                                     : GHB_ERR_CUDA);
     g->perm_host.resize(n);
     GG_TRY(cudaMemcpyAsync(g->perm_host.data(), g->perm, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st) == cudaSuccess
                ? GHB_OK
@@ -375,6 +384,7 @@ int ghb_graph_create(ghb_workspace* ws, int32_t n, const int32_t* out_rowptr, co
 #undef GG_TRY
     GHB_CUDA_TRY(cudaEventRecord(ws->ev_b, st));
     GHB_CUDA_TRY(cudaEventSynchronize(ws->ev_b));
+    g->repeats = hp[2] != 0;
     cudaEventElapsedTime(&g->build_ms, ws->ev_a, ws->ev_b);
     *out = g;
     return GHB_OK;

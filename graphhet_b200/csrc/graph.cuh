@@ -16,6 +16,7 @@ struct ghb_graph {
     bool weighted = false;
     bool repeats = false;    // some out-row holds an entry twice
     int device = 0;
+    void* slab = nullptr;  // the allocation that holds perm .. outdeg
     // perm[old] = new, iperm[new] = old.  New ids are ranked by total degree,
     // descending, ties by old id.
     int32_t* perm = nullptr;
