@@ -16,7 +16,7 @@
 //          buckets);
 //   round  every queued vertex relaxes its out-edges for its active sources:
 //          a warp per vertex (rows up to kMsspWarpRow entries) or per
-//          256-entry chunk of a longer row (chunk table built per round);
+//          chunk of a longer row (chunk table built per round);
 //          lanes run over the sources when at least 4 are active (all 32
 //          lanes of the warp relax one edge for 32 sources), over the edges
 //          otherwise.  An improved distance below hi activates the target
@@ -37,8 +37,12 @@
 namespace ghb {
 namespace {
 
-constexpr int32_t kMsspWarpRow = 1024;
-constexpr int32_t kMsspChunk = 256;
+// Rows over kMsspWarpRow entries are cut into chunks that a warp each relaxes
+// in the same round: a round ends with its longest chain of steps.  64 sources
+// on RMAT-18: 9.6 ms with 32, 10.2 with 64, 10.8 with 128; 34 ms with rows of up
+// to 1,024 entries on one warp, an entry at a time.
+constexpr int32_t kMsspWarpRow = 32;
+constexpr int32_t kMsspChunk = 32;
 constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;  // +infinity
 
 struct MsspCounters {
@@ -102,61 +106,149 @@ __global__ void __launch_bounds__(256) mssp_scan_kernel(int32_t n_scan, int32_t 
     mssp_scan_body(n_scan, ks, words, lo, hi, d, act, queue, cnt);
 }
 
-// Relax entries [eb, ee) of v's row for v's active sources.
-__device__ __forceinline__ void mssp_relax_range(int32_t v, int32_t eb, int32_t ee, int32_t ks, int32_t words,
-                                                 double hi, const int32_t* __restrict__ col,
-                                                 const double* __restrict__ wt, unsigned long long* d,
-                                                 const unsigned long long* act_cur,
-                                                 unsigned long long* act_next, int32_t* inq_next,
-                                                 int32_t* queue_next, MsspCounters* cnt,
-                                                 unsigned long long& examined) {
+// Queues the vertices u of the lanes with `want` for the next round (once each).
+__device__ __forceinline__ void mssp_queue(bool want, int32_t u, int32_t* inq_next, int32_t* queue_next,
+                                           MsspCounters* cnt) {
+    const bool first = want && atomicExch(inq_next + u, 1) == 0;
+    const int32_t at = warp_append(&cnt->queued, first);
+    if (first) queue_next[at] = u;
+}
+
+// Relax entries [eb, ee) of v's row for v's active sources.  A row is a chain
+// of round trips (column, distance, minimum, queue), so a warp issues those of
+// several entries together: the columns and weights of 32 entries in one load,
+// the distances of kFlight / groups entries at a time.  A distance read above
+// the new one is lowered without waiting for the answer; whoever else lowers it
+// meanwhile marks the same target, so nothing is lost.
+constexpr int kMsspFlight = 8;  // distance loads in flight per lane
+struct MsspArrays {
+    const int32_t* __restrict__ col;
+    const double* __restrict__ wt;
+    unsigned long long* d;
+    const unsigned long long* act_cur;
+    unsigned long long* act_next;
+    int32_t* inq_next;
+    int32_t* queue_next;
+    MsspCounters* cnt;
+    int32_t ks, words;
+    double hi;
+};
+// Lanes over sources: lane handles s = lane + 32 (g0 + t), t < GROUPS.
+template <int GROUPS>
+__device__ __forceinline__ void mssp_relax_wide(const MsspArrays& a, int32_t v, int32_t eb, int32_t ee, int g0) {
+    constexpr int kB = kMsspFlight / GROUPS;  // entries per step
     const int lane = lane_id();
-    int nact = 0;
-    for (int w = 0; w < words; ++w) nact += __popcll(__ldcg(act_cur + (int64_t)v * words + w));
-    auto relax_one = [&](int32_t u, int s, double nd) {
-        unsigned long long* p = d + (int64_t)u * ks + s;
-        const unsigned long long nb = (unsigned long long)__double_as_longlong(nd);
-        if (nb < __ldcg(p)) {
-            const unsigned long long old = atomicMin(p, nb);
-            if (nb < old && nd < hi) {
-                atomicOr(act_next + (int64_t)u * words + (s >> 6), 1ull << (s & 63));
-                if (atomicExch(inq_next + u, 1) == 0) queue_next[warp_append_active(&cnt->queued)] = u;
+    double dv[GROUPS];
+    unsigned on = 0;
+#pragma unroll
+    for (int t = 0; t < GROUPS; ++t) {
+        const int s = lane + 32 * (g0 + t);
+        const bool live = (__ldcg(a.act_cur + (int64_t)v * a.words + (s >> 6)) >> (s & 63)) & 1ull;
+        dv[t] = live ? __longlong_as_double((long long)__ldcg(a.d + (int64_t)v * a.ks + s)) : 0.0;
+        on |= live ? 1u << t : 0u;
+    }
+    if (!__any_sync(0xffffffffu, on != 0)) return;
+    for (int32_t j0 = eb; j0 < ee; j0 += 32) {
+        const int32_t left = ee - j0 < 32 ? ee - j0 : 32;
+        const int32_t uj = lane < left ? a.col[j0 + lane] : 0;
+        const double wj = lane < left ? a.wt[j0 + lane] : 0.0;
+        for (int32_t k0 = 0; k0 < left; k0 += kB) {
+            int32_t u[kB];
+            double nd[kB][GROUPS], cur[kB][GROUPS];
+#pragma unroll
+            for (int q = 0; q < kB; ++q) {
+                u[q] = __shfl_sync(0xffffffffu, uj, (k0 + q) & 31);
+                const double w = __shfl_sync(0xffffffffu, wj, (k0 + q) & 31);
+#pragma unroll
+                for (int t = 0; t < GROUPS; ++t) {
+                    nd[q][t] = dv[t] + w;
+                    cur[q][t] = 0.0;
+                    if (k0 + q < left && ((on >> t) & 1u))
+                        cur[q][t] = __longlong_as_double((long long)__ldcg(a.d + (int64_t)u[q] * a.ks + lane + 32 * (g0 + t)));
+                }
             }
-        }
-    };
-    if (nact >= 4) {
-        // Lanes over sources: lane handles s = lane + 32 t, t < ks / 32; the
-        // row's entries are read once and relaxed for every group.
-        const int groups = ks >> 5;
-        double dv[8];
-        bool a[8];
+            unsigned hit = 0;  // entries of the step with a target below hi
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            const int s = lane + 32 * t;
-            a[t] = t < groups && ((__ldcg(act_cur + (int64_t)v * words + (s >> 6)) >> (s & 63)) & 1ull);
-            dv[t] = a[t] ? __longlong_as_double((long long)__ldcg(d + (int64_t)v * ks + s)) : 0.0;
-        }
-        for (int32_t j = eb; j < ee; ++j) {
-            const int32_t u = col[j];
-            const double w = wt[j];
+            for (int q = 0; q < kB; ++q)
 #pragma unroll
-            for (int t = 0; t < 8; ++t)
-                if (a[t]) relax_one(u, lane + 32 * t, dv[t] + w);
-        }
-        if (lane == 0) examined += (unsigned long long)(ee - eb) * (unsigned long long)nact;
-    } else {
-        // Lanes over entries, the few active sources one after another.
-        for (int w = 0; w < words; ++w) {
-            unsigned long long bits = __ldcg(act_cur + (int64_t)v * words + w);
-            while (bits) {
-                const int s = w * 64 + __ffsll((long long)bits) - 1;
-                bits &= bits - 1;
-                const double dv = __longlong_as_double((long long)__ldcg(d + (int64_t)v * ks + s));
-                for (int32_t j = eb + lane; j < ee; j += 32) relax_one(col[j], s, dv + wt[j]);
-                if (lane == 0) examined += (unsigned long long)(ee - eb);
+                for (int t = 0; t < GROUPS; ++t) {
+                    const bool low = nd[q][t] < cur[q][t];
+                    if (low)
+                        atomicMin(a.d + (int64_t)u[q] * a.ks + lane + 32 * (g0 + t),
+                                  (unsigned long long)__double_as_longlong(nd[q][t]));
+                    const unsigned m = __ballot_sync(0xffffffffu, low && nd[q][t] < a.hi);
+                    if (m) {
+                        // The group's 32 sources: half a word.
+                        if (lane == 0)
+                            atomicOr(reinterpret_cast<unsigned*>(a.act_next + (int64_t)u[q] * a.words) + g0 + t, m);
+                        hit |= 1u << q;
+                    }
+                }
+            if (hit) {
+                int32_t mine = 0;
+#pragma unroll
+                for (int q = 0; q < kB; ++q) mine = lane == q ? u[q] : mine;
+                mssp_queue((hit >> lane) & 1u, mine, a.inq_next, a.queue_next, a.cnt);
             }
         }
     }
+}
+// Lanes over entries, the few active sources one after another.
+__device__ __forceinline__ void mssp_relax_narrow(const MsspArrays& a, int32_t v, int32_t eb, int32_t ee) {
+    constexpr int kB = 4;
+    const int lane = lane_id();
+    for (int w = 0; w < a.words; ++w) {
+        unsigned long long bits = __ldcg(a.act_cur + (int64_t)v * a.words + w);
+        while (bits) {
+            const int b = __ffsll((long long)bits) - 1;
+            const int s = w * 64 + b;
+            bits &= bits - 1;
+            const double dv = __longlong_as_double((long long)__ldcg(a.d + (int64_t)v * a.ks + s));
+            for (int64_t j0 = eb; j0 < ee; j0 += 32 * kB) {
+                int32_t u[kB];
+                double nd[kB], cur[kB];
+#pragma unroll
+                for (int q = 0; q < kB; ++q) {
+                    const int64_t j = j0 + 32 * q + lane;
+                    u[q] = j < ee ? a.col[j] : -1;
+                    nd[q] = j < ee ? dv + a.wt[j] : 0.0;
+                }
+#pragma unroll
+                for (int q = 0; q < kB; ++q)
+                    cur[q] = u[q] >= 0 ? __longlong_as_double((long long)__ldcg(a.d + (int64_t)u[q] * a.ks + s)) : 0.0;
+                unsigned near = 0;
+#pragma unroll
+                for (int q = 0; q < kB; ++q)
+                    if (u[q] >= 0 && nd[q] < cur[q]) {
+                        atomicMin(a.d + (int64_t)u[q] * a.ks + s, (unsigned long long)__double_as_longlong(nd[q]));
+                        if (nd[q] < a.hi) {
+                            atomicOr(a.act_next + (int64_t)u[q] * a.words + w, 1ull << b);
+                            near |= 1u << q;
+                        }
+                    }
+                if (!__any_sync(0xffffffffu, near != 0)) continue;
+#pragma unroll
+                for (int q = 0; q < kB; ++q)
+                    mssp_queue((near >> q) & 1u, u[q], a.inq_next, a.queue_next, a.cnt);
+            }
+        }
+    }
+}
+__device__ __forceinline__ void mssp_relax_range(int32_t v, int32_t eb, int32_t ee, const MsspArrays& a,
+                                                 unsigned long long& examined) {
+    int nact = 0;
+    for (int w = 0; w < a.words; ++w) nact += __popcll(__ldcg(a.act_cur + (int64_t)v * a.words + w));
+    if (nact >= 4) {
+        // 64 sources at a time: the row's entries come from L1 after the first
+        // walk, and are few bytes beside the distances.
+        const int groups = a.ks >> 5;
+        int g = 0;
+        for (; g + 2 <= groups; g += 2) mssp_relax_wide<2>(a, v, eb, ee, g);
+        if (g < groups) mssp_relax_wide<1>(a, v, eb, ee, g);
+    } else {
+        mssp_relax_narrow(a, v, eb, ee);
+    }
+    if (lane_id() == 0) examined += (unsigned long long)(ee - eb) * (unsigned long long)nact;
 }
 
 // A warp per queued vertex; rows longer than kMsspWarpRow go to `big`.
@@ -172,6 +264,7 @@ __global__ void __launch_bounds__(256) mssp_relax_kernel(int32_t q, const int32_
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     unsigned long long examined = 0;
+    const MsspArrays arrays{col, wt, d, act_cur, act_next, inq_next, queue_next, cnt, ks, words, hi};
     for (int64_t i = warp; i < q; i += nwarps) {
         const int32_t v = queue[i];
         const int32_t eb = rp[v], ee = rp[v + 1];
@@ -179,8 +272,7 @@ __global__ void __launch_bounds__(256) mssp_relax_kernel(int32_t q, const int32_
             if (lane_id() == 0) big[atomicAdd(&cnt_cur->big, 1)] = v;
             continue;
         }
-        mssp_relax_range(v, eb, ee, ks, words, hi, col, wt, d, act_cur, act_next, inq_next, queue_next, cnt,
-                         examined);
+        mssp_relax_range(v, eb, ee, arrays, examined);
     }
     if (lane_id() == 0 && examined) atomicAdd(&cnt->examined, examined);
 }
@@ -195,7 +287,7 @@ __global__ void mssp_big_chunks_kernel(const int32_t* __restrict__ big, const Ms
     }
 }
 
-// A warp per 256-entry chunk of the long rows (row by binary search).
+// A warp per chunk of the long rows (row by binary search).
 __global__ void __launch_bounds__(256) mssp_relax_big_kernel(const int32_t* __restrict__ big,
                                                              const int32_t* __restrict__ cpre,
                                                              const MsspCounters* cnt_cur,
@@ -212,6 +304,7 @@ __global__ void __launch_bounds__(256) mssp_relax_big_kernel(const int32_t* __re
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     unsigned long long examined = 0;
+    const MsspArrays arrays{col, wt, d, act_cur, act_next, inq_next, queue_next, cnt, ks, words, hi};
     for (int64_t c = warp; c < total; c += nwarps) {
         int32_t lo = 0, hi_i = nb - 1;
         while (lo < hi_i) {
@@ -222,8 +315,7 @@ __global__ void __launch_bounds__(256) mssp_relax_big_kernel(const int32_t* __re
         const int32_t v = big[lo];
         const int32_t eb = rp[v] + (int32_t)(c - cpre[lo]) * kMsspChunk;
         const int32_t ee = min(rp[v + 1], eb + kMsspChunk);
-        mssp_relax_range(v, eb, ee, ks, words, hi, col, wt, d, act_cur, act_next, inq_next, queue_next, cnt,
-                         examined);
+        mssp_relax_range(v, eb, ee, arrays, examined);
     }
     if (lane_id() == 0 && examined) atomicAdd(&cnt->examined, examined);
 }
@@ -240,7 +332,7 @@ __global__ void mssp_clear_kernel(int32_t q, const int32_t* __restrict__ queue, 
 
 // ---------------------------------------------------------------------------
 // The whole pass in one cooperative launch: set-up, every bucket scan and
-// relaxation round (long rows as 256-entry chunks in a CHUNK phase of the
+// relaxation round (long rows as chunks in a CHUNK phase of the
 // same round, then the clear of the processed vertices' act words), the
 // output, separated by the bounded grid barrier; the last block to arrive
 // decides the next phase (the host-driven pass's rules: rounds until the
@@ -248,6 +340,7 @@ __global__ void mssp_clear_kernel(int32_t q, const int32_t* __restrict__ queue, 
 // smallest pending distance).  No host round trip inside a pass.
 
 constexpr int kMsspThreads = 256;
+constexpr int kMsspBlocks = 4;
 enum MsspPhase : int32_t { kMpScan = 0, kMpRelax = 1, kMpChunks = 2, kMpClear = 3, kMpDone = 4 };
 
 struct MsspRunState {
@@ -273,12 +366,11 @@ __device__ __forceinline__ double mp_pmin(const MsspCounters* c) {
     return b == kInfBits ? INFINITY : __longlong_as_double((long long)b);
 }
 
-// Eight blocks per SM, every thread slot of the SM (32 registers, a
-// 148-byte spill): 256 sources on RMAT-22 in 1.08 s, against 1.30-1.34 s at
-// six blocks per SM (40 registers) and 1.66 s at four (64 registers).  The
-// pass waits on its gathers and atomics, so resident warps pay for the
-// spill.
-__global__ void __launch_bounds__(kMsspThreads, 8) mssp_pass_kernel(
+// Four blocks per SM (64 registers, a small spill): with eight distance loads
+// in flight per lane, 64 sources on RMAT-18 take 10.2 ms, against 11.0 at three
+// blocks, 10.4 at five and 11.6 at six; half the loads in flight take 10.8 ms.
+// The pass waits on its gathers and atomics.
+__global__ void __launch_bounds__(kMsspThreads, kMsspBlocks) mssp_pass_kernel(
     int32_t n, int32_t n_active, int32_t k, int32_t ks, int32_t words, const int32_t* __restrict__ rp,
     const int32_t* __restrict__ col, const double* __restrict__ wt, const int32_t* srcs, const int32_t* __restrict__ perm,
     double inf, double* dist_out, unsigned long long* d, unsigned long long* act_a, unsigned long long* act_b,
@@ -335,6 +427,7 @@ __global__ void __launch_bounds__(kMsspThreads, 8) mssp_pass_kernel(
         int32_t* q_next = sel ? q_a : q_b;
         MsspCounters* cn = cnt;  // the round being filled
         const double lo = s_lo, hi = lo + st->delta;
+        const MsspArrays arrays{col, wt, d, act_cur, act_next, inq_next, q_next, cn, ks, words, hi};
         unsigned long long examined = 0;
         if (phase == kMpScan) {
             mssp_scan_body(n_active, ks, words, lo, hi, d, act_cur, q_cur, cn);
@@ -351,14 +444,12 @@ __global__ void __launch_bounds__(kMsspThreads, 8) mssp_pass_kernel(
                         chunks[pos + c] = make_int4(v, eb + c * kMsspChunk, min(ee, eb + (c + 1) * kMsspChunk), 0);
                     continue;
                 }
-                mssp_relax_range(v, eb, ee, ks, words, hi, col, wt, d, act_cur, act_next, inq_next, q_next, cn,
-                                 examined);
+                mssp_relax_range(v, eb, ee, arrays, examined);
             }
         } else if (phase == kMpChunks) {
             for (int64_t i = warp; i < nch; i += nwarps) {
                 const int4 ch = __ldcg(chunks + i);
-                mssp_relax_range(ch.x, ch.y, ch.z, ks, words, hi, col, wt, d, act_cur, act_next, inq_next, q_next,
-                                 cn, examined);
+                mssp_relax_range(ch.x, ch.y, ch.z, arrays, examined);
             }
         } else {  // kMpClear: the processed vertices' act words and queue flags
             for (int64_t i = gtid; i < q; i += gsize) {
@@ -463,7 +554,7 @@ static int mssp_pass_blocks(ghb_workspace* ws) {
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
         if (coop && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mssp_pass_kernel, kMsspThreads, 0) ==
                         cudaSuccess)
-            cached[dev] = std::max(0, std::min(per_sm, 8)) * ws->num_sms;
+            cached[dev] = std::max(0, std::min(per_sm, kMsspBlocks)) * ws->num_sms;
         if (!cached[dev]) cached[dev] = -1;
     }
     return cached[dev] > 0 ? cached[dev] : 0;
@@ -486,7 +577,7 @@ int mssssp_pass_one_launch(ghb_workspace* ws, int32_t n, int32_t n_active, int64
     cudaStream_t st = ws->stream;
     const int32_t ks = (k + 31) & ~31;
     const int32_t words = (ks + 63) / 64;
-    // Chunks of one round: rows over kMsspWarpRow entries, ceil(len / 256) each.
+    // Chunks of one round: rows over kMsspWarpRow entries, ceil(len / kMsspChunk) each.
     const int64_t chunk_cap = m / kMsspChunk + m / kMsspWarpRow + 64;
     auto carve = [&](Carver& c, unsigned long long** d, unsigned long long** aa, unsigned long long** ab,
                      int32_t** ia, int32_t** ib, int32_t** qa, int32_t** qb, int4** ch, MsspCounters** cnt,
