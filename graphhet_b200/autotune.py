@@ -19,11 +19,9 @@ from typing import Callable, Dict, List, Optional, Sequence, Tuple
 
 SPACES: Dict[str, Dict[str, List[int]]] = {
     "pagerank": {
-        "pr_cache_kb": [0, 48, 96, 144, 192, 200],
+        "pr_cache_kb": [0, 32, 64, 80, 96, 112],
         "pr_threads": [256, 512, 1024],
         "pr_blocks_per_sm": [1, 2, 4],
-        "pr_short": [8, 16, 32, 64],
-        "pr_chunk": [128, 256, 512, 1024],
     },
     "msbfs": {
         "ms_warp_rest": [64, 128, 256, 512, 2048],

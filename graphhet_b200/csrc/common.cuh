@@ -61,11 +61,11 @@ enum DeviceStatus : int32_t {
 // for PageRank, scales 22 and 24 for the multi-source BFS); ghb_tune_set
 // changes them for other graphs.
 struct Tuning {
-    int32_t pr_cache_kb = 144;     // PageRank hub cache: shared memory per block (KB)
+    int32_t pr_cache_kb = 80;     // PageRank hub cache: shared memory per block (KB)
     int32_t pr_threads = 1024;     // threads of the persistent PageRank blocks
     int32_t pr_blocks_per_sm = 1;  // persistent PageRank blocks per SM
-    int32_t pr_short = 64;         // rows up to this many entries: one thread per row
-    int32_t pr_chunk = 1024;       // longer rows: chunks of this many entries, warp per chunk
+    int32_t pr_short = 64;         // accepted, without effect: every warp takes a tile of entries
+    int32_t pr_chunk = 1024;       // accepted, without effect
     int32_t ms_warp_rest = 512;    // multi-source pull: longer rest of a row -> a block
     int32_t ms_pull_div = 16;      // multi-source: pull when frontier entries > m / ms_pull_div
     int32_t pol_band = 1;          // learned policy: the network picks a level's direction and format only
@@ -80,7 +80,7 @@ struct Tuning {
     int32_t ms_persistent = 1;     // multi-source BFS: 1 = one cooperative launch per pass, 0 = host-driven levels
     int32_t ms_learned = 0;        // multi-source BFS pass: 1 = the installed direction model decides each level
     int32_t bfs_blocks_per_sm = 2; // whole-traversal BFS: 512-thread blocks per SM (1 or 2)
-    int32_t pr_gathers = 4;        // PageRank long rows: contribution gathers in flight per lane (4 or 8)
+    int32_t pr_gathers = 4;        // accepted, without effect: eight gathers are in flight per lane
     int32_t mssp_persistent = 1;   // multi-source SSSP: 1 = one cooperative launch per pass, 0 = host-driven
     int32_t tc_slice_blocks = 16;  // triangle counting: blocks per SM of the 2,048-slot slice kernel
     int32_t tc_trim_min = 0;       // triangle counting: lists N+(b) over this many entries are range-trimmed

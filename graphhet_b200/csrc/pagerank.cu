@@ -10,10 +10,9 @@
 // partials of the next S and of the L1 change; a one-block kernel reduces the
 // partials in a fixed order (deterministic S and norm, FP64 in both modes).
 //
-// Rows of up to 32 entries are summed by one thread each; longer rows are
-// cut into 256-entry chunks summed by one warp each and combined per row in
-// chunk order.  Both kernels serve the hubs' contributions from a shared-
-// memory cache (a degree-relabelled graph puts the hubs first).
+// The non-empty rows' entries are cut into tiles of 256, a warp each; rows that
+// cross tiles are combined in tile order.  The hubs' contributions come from a
+// shared-memory cache (a degree-relabelled graph puts the hubs first).
 //
 // FP32 mode: ranks and contributions are stored as float (half the gather
 // footprint: 64 MiB at n = 2^24, resident in the 126 MB L2); each lane keeps
@@ -87,7 +86,7 @@ struct PrScalars {
 template <class T>
 __global__ void __launch_bounds__(kPrThreads) pr_init_kernel(int32_t n, const int32_t* __restrict__ out_rp,
                                                              int32_t* __restrict__ outdeg, T* rank,
-                                                             T* contrib, double* part_sink) {
+                                                             T* contrib, T* contrib_next, double* part_sink) {
     __shared__ double red[kPrThreads / 32];
     double sink = 0.0;
     const double r0 = 1.0 / (double)n;
@@ -97,6 +96,7 @@ __global__ void __launch_bounds__(kPrThreads) pr_init_kernel(int32_t n, const in
         outdeg[v] = d;
         rank[v] = (T)r0;
         contrib[v] = d > 0 ? (T)(r0 / (double)d) : (T)0;
+        contrib_next[v] = (T)0;  // an isolated vertex's is not written again
         if (d == 0) sink += (double)(T)r0;
     }
     sink = warp_sum(sink);
@@ -110,13 +110,11 @@ __global__ void __launch_bounds__(kPrThreads) pr_init_kernel(int32_t n, const in
 }
 
 template <class T>
-__device__ __forceinline__ void pr_finish_row(int64_t v, double sum, const PrScalars* sc, double damping,
-                                              const int32_t* __restrict__ outdeg, const T* rank_old,
-                                              T* rank_new, T* contrib_new, int track_l1, double& sink,
-                                              double& l1) {
-    const double r = sc->base + damping * sum;
+__device__ __forceinline__ void pr_finish_row(int64_t v, int32_t d, double sum, double base, double damping,
+                                              const T* rank_old, T* rank_new, T* contrib_new, int track_l1,
+                                              double& sink, double& l1) {
+    const double r = base + damping * sum;
     const T rt = (T)r;
-    const int32_t d = outdeg[v];
     rank_new[v] = rt;
     contrib_new[v] = d > 0 ? (T)(r / (double)d) : (T)0;
     if (d == 0) sink += (double)rt;
@@ -146,12 +144,11 @@ __device__ __forceinline__ void block_partials(double sink, double l1, double* p
 }
 
 // Shared-memory cache of the first K contributions (K from the workspace's
-// pr_cache_kb, 192 KB by default).
-// On a degree-relabelled graph these are the hubs' (the top 32K vertices of
-// an RMAT scale-22 graph hold half of all entries), so about half of the
-// gathers are served from shared memory instead of L2 sectors.  The kernels
-// that use it run persistent blocks (pr_threads x pr_blocks_per_sm per SM,
-// 1024 x 1 by default), so each block fills the cache once per launch.
+// pr_cache_kb).  On a degree-relabelled graph these are the hubs' (the top 10 K
+// vertices of an RMAT scale-22 graph hold a third of all entries), so their
+// gathers take no L2 sector.  The kernel runs persistent blocks (pr_threads x
+// pr_blocks_per_sm per SM, 1024 x 1 by default), so each fills the cache once
+// per launch.
 constexpr int kPrPersistThreads = 1024;
 
 template <class T>
@@ -169,137 +166,14 @@ __device__ __forceinline__ T gather(const T* cache, int32_t K, const T* __restri
     return u < K ? cache[u] : load_contrib<T>(contrib_old + u, pol);
 }
 
-// Rows of up to `short_max` entries: one thread per row, gathers four at a time
-// (independent loads), Kahan-summed in row order.  Longer rows are skipped
-// here (chunk path).
-template <class T>
-__global__ void __launch_bounds__(kPrPersistThreads) pr_rows_short_kernel(
-    int32_t n, const int32_t* __restrict__ in_rp, const int32_t* __restrict__ in_col,
-    const int32_t* __restrict__ outdeg, const T* __restrict__ contrib_old, const T* rank_old,
-    T* rank_new, T* contrib_new, const PrScalars* sc, double damping, int track_l1, double* part_sink,
-    double* part_l1, int32_t short_max, int32_t cache_elems) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* cache = reinterpret_cast<T*>(smem_raw);
-    const int32_t K = fill_hub_cache<T>(cache, contrib_old, n, cache_elems);
-    const uint64_t pol_stream = policy_evict_first();
-    const uint64_t pol_keep = policy_evict_last();
-    double sink = 0.0, l1 = 0.0;
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t b = in_rp[r], e = in_rp[r + 1];
-        if (e - b > short_max) continue;
-        KSum<T> acc;
-        for (int32_t j = b; j < e; j += 4) {
-            int32_t u[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) u[k] = (j + k < e) ? ld_stream(in_col + j + k, pol_stream) : -1;
-            T x[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) x[k] = u[k] >= 0 ? gather<T>(cache, K, contrib_old, u[k], pol_keep) : (T)0;
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (u[k] >= 0) acc.add(x[k]);
-        }
-        pr_finish_row<T>(r, acc.value(), sc, damping, outdeg, rank_old, rank_new, contrib_new, track_l1, sink, l1);
-    }
-    block_partials<T>(sink, l1, part_sink, part_l1, blockIdx.x);
-}
-
-__global__ void pr_long_flags_kernel(int32_t n, const int32_t* __restrict__ in_rp, int32_t* flag, int32_t short_max) {
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
-        flag[v] = (in_rp[v + 1] - in_rp[v]) > short_max ? 1 : 0;
-}
-
-// Long rows in ascending order, and their chunk counts.
-__global__ void pr_long_compact_kernel(int32_t n, const int32_t* __restrict__ in_rp, const int32_t* __restrict__ flag,
-                                       const int32_t* __restrict__ pos, int32_t* long_rows, int32_t* nchunks,
-                                       int32_t chunk) {
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
-        if (!flag[v]) continue;
-        const int32_t i = pos[v];
-        long_rows[i] = (int32_t)v;
-        nchunks[i] = (in_rp[v + 1] - in_rp[v] + chunk - 1) / chunk;
-    }
-}
-
-// chunk_row[c] = index (in long_rows) of the row chunk c belongs to.
-__global__ void pr_chunk_rows_kernel(int32_t nlong, const int32_t* __restrict__ chunk_prefix, int32_t* chunk_row) {
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t i = warp; i < nlong; i += nwarps)
-        for (int32_t c = chunk_prefix[i] + lane_id(); c < chunk_prefix[i + 1]; c += 32) chunk_row[c] = (int32_t)i;
-}
-
-// One warp per chunk of `chunk` entries: a partial sum, G independent
-// 32-wide loads in flight per lane (4 or 8: the workspace's pr_gathers),
-// hub contributions from shared memory.
-template <class T, int G>
-__global__ void __launch_bounds__(kPrPersistThreads) pr_chunk_kernel(
-    int32_t n, const int32_t* __restrict__ in_rp, const int32_t* __restrict__ in_col,
-    const int32_t* __restrict__ long_rows, const int32_t* __restrict__ chunk_prefix,
-    const int32_t* __restrict__ chunk_row, int32_t nchunks, const T* __restrict__ contrib_old, double* chunk_sum,
-    int32_t chunk, int32_t cache_elems) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* cache = reinterpret_cast<T*>(smem_raw);
-    const int32_t K = fill_hub_cache<T>(cache, contrib_old, n, cache_elems);
-    const uint64_t pol_stream = policy_evict_first();
-    const uint64_t pol_keep = policy_evict_last();
-    const int lane = lane_id();
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t ch = warp; ch < nchunks; ch += nwarps) {
-        const int32_t i = chunk_row[ch];
-        const int32_t u = long_rows[i];
-        const int32_t rb = in_rp[u], re = in_rp[u + 1];
-        const int32_t b = rb + (int32_t)(ch - chunk_prefix[i]) * chunk;
-        const int32_t e = min(re, b + chunk);
-        KSum<T> acc;
-        for (int32_t j0 = b; j0 < e; j0 += 32 * G) {
-            int32_t x[G];
-#pragma unroll
-            for (int k = 0; k < G; ++k) {
-                const int32_t j = j0 + lane + 32 * k;
-                x[k] = j < e ? ld_stream(in_col + j, pol_stream) : -1;
-            }
-            T y[G];
-#pragma unroll
-            for (int k = 0; k < G; ++k) y[k] = x[k] >= 0 ? gather<T>(cache, K, contrib_old, x[k], pol_keep) : (T)0;
-#pragma unroll
-            for (int k = 0; k < G; ++k)
-                if (x[k] >= 0) acc.add(y[k]);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc.merge_from_lane(o, 32);
-        if (lane == 0) chunk_sum[ch] = acc.value();
-    }
-}
-
-// Long rows: the chunk partials summed in chunk order, then the row update.
-template <class T>
-__global__ void __launch_bounds__(kPrThreads) pr_long_finish_kernel(
-    int32_t nlong, const int32_t* __restrict__ long_rows, const int32_t* __restrict__ chunk_prefix,
-    const double* __restrict__ chunk_sum, const int32_t* __restrict__ outdeg, const T* rank_old, T* rank_new,
-    T* contrib_new, const PrScalars* sc, double damping, int track_l1, double* part_sink, double* part_l1,
-    int slot0) {
-    double sink = 0.0, l1 = 0.0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nlong;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (int32_t c = chunk_prefix[i]; c < chunk_prefix[i + 1]; ++c) s += chunk_sum[c];
-        pr_finish_row<T>(long_rows[i], s, sc, damping, outdeg, rank_old, rank_new, contrib_new, track_l1, sink, l1);
-    }
-    block_partials<T>(sink, l1, part_sink, part_l1, slot0 + blockIdx.x);
-}
-
 // One block: S and L1 from the partials (fixed order), next base.
-__global__ void __launch_bounds__(1024) pr_reduce_kernel(const double* part_sink, const double* part_l1,
-                                                         int nparts, int32_t n, double damping,
-                                                         PrScalars* sc, double* l1_hist, int iter,
-                                                         int has_l1) {
-    __shared__ double rs[1024], rl[1024];
+__device__ __forceinline__ void pr_reduce(const double* part_sink, const double* part_l1, int nparts, int32_t n,
+                                          double damping, PrScalars* sc, double* l1_hist, int iter, int has_l1) {
+    __shared__ double rs[kPrThreads], rl[kPrThreads];
     double s = 0.0, l = 0.0;
     for (int i = threadIdx.x; i < nparts; i += blockDim.x) {
-        s += part_sink[i];
-        if (has_l1) l += part_l1[i];
+        s += __ldcg(part_sink + i);
+        if (has_l1) l += __ldcg(part_l1 + i);
     }
     rs[threadIdx.x] = s;
     rl[threadIdx.x] = l;
@@ -321,6 +195,287 @@ __global__ void __launch_bounds__(1024) pr_reduce_kernel(const double* part_sink
         }
     }
 }
+__global__ void __launch_bounds__(kPrThreads) pr_reduce_kernel(const double* part_sink, const double* part_l1,
+                                                               int nparts, int32_t n, double damping, PrScalars* sc) {
+    pr_reduce(part_sink, part_l1, nparts, n, damping, sc, nullptr, 0, 0);
+}
+
+// ---- tiles
+//
+// The entries of the non-empty rows, taken in order, are cut into tiles of
+// kPrTile; a warp takes a tile, whatever rows it holds.  So every warp has the
+// same number of gathers, all of them in flight at once, where a thread per
+// short row left a third of the lanes idle and its blocks uneven, and rows cut
+// into chunks needed kernels of their own.  A tile inside one row is summed in
+// registers; in a mixed one the values go through the warp's shared memory and
+// each row's are summed by a lane (by the warp from 32 values on).  A row that
+// crosses tiles leaves a partial sum per tile: tail[t] in the tile where it
+// begins, head[t] in those that it continues into; pr_finish_kernel adds them in
+// tile order, so results do not depend on timing.
+constexpr int kPrPerLane = 8;
+constexpr int32_t kPrTile = 32 * kPrPerLane;
+
+// Non-empty rows in ascending order: row ids and their first entries.
+struct PrRows {
+    const int32_t* __restrict__ id;     // id[i]
+    const int32_t* __restrict__ begin;  // begin[i], begin[k] = m
+    const int32_t* __restrict__ deg;    // out-degrees
+    const int32_t* __restrict__ tile;   // tile[t]: the row (index) that holds entry t * kPrTile
+    int32_t k;
+    int32_t m;
+    int32_t tiles;
+};
+
+__global__ void pr_row_flags_kernel(int32_t n, const int32_t* __restrict__ in_rp, int32_t* flag) {
+    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
+        flag[v] = in_rp[v + 1] > in_rp[v] ? 1 : 0;
+}
+
+// pos = exclusive scan of the flags: the non-empty rows' ids, offsets and
+// out-degrees in order.  Rows without entries go to `bare`, those with
+// out-entries from the front, isolated ones from the back; count[0], count[1].
+__global__ void __launch_bounds__(256) pr_row_lists_kernel(int32_t n, const int32_t* __restrict__ in_rp,
+                                                           const int32_t* __restrict__ pos,
+                                                           const int32_t* __restrict__ outdeg, int32_t* id,
+                                                           int32_t* begin, int32_t* deg, int32_t* bare,
+                                                           int32_t* count) {
+    __shared__ int32_t s_n[2], s_at[2];
+    for (int64_t v0 = blockIdx.x * (int64_t)blockDim.x; v0 < n; v0 += (int64_t)gridDim.x * blockDim.x) {
+        if (threadIdx.x < 2) s_n[threadIdx.x] = 0;
+        __syncthreads();
+        const int64_t v = v0 + threadIdx.x;
+        int kind = -1;
+        int32_t at = 0;
+        if (v < n) {
+            const int32_t b = in_rp[v], d = outdeg[v];
+            if (in_rp[v + 1] > b) {
+                const int32_t i = pos[v];
+                id[i] = (int32_t)v;
+                begin[i] = b;
+                deg[i] = d;
+            } else {
+                kind = d > 0 ? 0 : 1;
+                at = atomicAdd(&s_n[kind], 1);
+            }
+            if (v == n - 1) begin[pos[n]] = in_rp[n];
+        }
+        __syncthreads();
+        if (threadIdx.x < 2 && s_n[threadIdx.x]) s_at[threadIdx.x] = atomicAdd(count + threadIdx.x, s_n[threadIdx.x]);
+        __syncthreads();
+        if (kind == 0) bare[s_at[0] + at] = (int32_t)v;
+        if (kind == 1) bare[n - 1 - (s_at[1] + at)] = (int32_t)v;
+        __syncthreads();
+    }
+}
+
+__global__ void pr_tile_rows_kernel(int32_t k, const int32_t* __restrict__ begin, int32_t tiles, int32_t* tile) {
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < tiles; t += (int64_t)gridDim.x * blockDim.x) {
+        int32_t lo = 0, hi = k - 1;  // the last row that begins at or before the entry
+        while (lo < hi) {
+            const int32_t mid = (int32_t)(((int64_t)lo + hi + 1) >> 1);
+            if ((int64_t)begin[mid] <= t * kPrTile) lo = mid;
+            else hi = mid - 1;
+        }
+        tile[t] = lo;
+    }
+}
+
+template <class T>
+__device__ __forceinline__ double warp_total(KSum<T> acc) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc.merge_from_lane(o, 32);
+    return __shfl_sync(0xffffffffu, acc.value(), 0);
+}
+
+// Bound by the gathers: each takes a 32-byte sector of L2 or its own pass of
+// the L1 pipe.  12 M vertices, 160 M entries, FP64: 0.66 ms an iteration (240 G
+// gathers/s), where a thread per short row and a warp per chunk of a longer one
+// took 0.35 + 0.49 ms; straight on the caller's ids ten iterations take 9.5 ms,
+// 19.1 before.
+template <class T>
+__global__ void __launch_bounds__(kPrPersistThreads) pr_tile_kernel(
+    PrRows R, int32_t n, const int32_t* __restrict__ in_col, const T* __restrict__ contrib_old, const T* rank_old,
+    T* rank_new, T* contrib_new, const PrScalars* sc, double damping, int track_l1, double* head, double* tail, double* part_sink, double* part_l1,
+    int32_t cache_elems) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T* cache = reinterpret_cast<T*>(smem_raw);
+    T* vals = cache + ((cache_elems + 3) & ~3) + (threadIdx.x >> 5) * kPrTile;
+    const int32_t K = fill_hub_cache<T>(cache, contrib_old, n, cache_elems);
+    const uint64_t pol_stream = policy_evict_first();
+    const uint64_t pol_keep = policy_evict_last();
+    const int lane = lane_id();
+    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    double sink = 0.0, l1 = 0.0;
+    const double base = sc->base;
+    auto finish = [&](int32_t row, int32_t d, double sum) {
+        pr_finish_row<T>(row, d, sum, base, damping, rank_old, rank_new, contrib_new, track_l1, sink, l1);
+    };
+    // A tile is a chain of columns, gathers and writes; the next tile's columns
+    // and this tile's row data are loaded under the gathers.
+    auto load_cols = [&](int64_t t, int32_t (&u)[kPrPerLane]) {
+        const int64_t t0 = t * kPrTile;
+#pragma unroll
+        for (int q = 0; q < kPrPerLane; ++q)
+            u[q] = t0 + q * 32 + lane < R.m ? ld_stream(in_col + t0 + q * 32 + lane, pol_stream) : -1;
+    };
+    int32_t ahead[kPrPerLane];
+    int32_t ahead0 = 0, ahead1 = 0;
+    if (warp < R.tiles) {
+        load_cols(warp, ahead);
+        ahead0 = R.tile[warp];
+        ahead1 = warp + 1 < R.tiles ? R.tile[warp + 1] : R.k - 1;
+    }
+    for (int64_t t = warp; t < R.tiles; t += nwarps) {
+        const int64_t t0 = t * kPrTile, t1 = min(t0 + kPrTile, (int64_t)R.m);
+        T x[kPrPerLane];
+        unsigned ok = 0;
+#pragma unroll
+        for (int q = 0; q < kPrPerLane; ++q) {
+            x[q] = ahead[q] >= 0 ? gather<T>(cache, K, contrib_old, ahead[q], pol_keep) : (T)0;
+            ok |= ahead[q] >= 0 ? 1u << q : 0u;
+        }
+        const int32_t i0 = ahead0, i1 = ahead1;
+        int32_t i = i0 + lane, b = 0, e = 0, id = 0, deg = 0;
+        auto load_row = [&]() {
+            b = e = 0;
+            if (i <= i1) {
+                b = R.begin[i];
+                e = R.begin[i + 1];
+                id = R.id[i];
+                deg = R.deg[i];
+            }
+        };
+        load_row();
+        if (t + nwarps < R.tiles) {
+            load_cols(t + nwarps, ahead);
+            ahead0 = R.tile[t + nwarps];
+            ahead1 = t + nwarps + 1 < R.tiles ? R.tile[t + nwarps + 1] : R.k - 1;
+        }
+        if (__shfl_sync(0xffffffffu, e, 0) >= t1) {  // one row
+            KSum<T> acc;
+#pragma unroll
+            for (int q = 0; q < kPrPerLane; ++q)
+                if ((ok >> q) & 1u) acc.add(x[q]);
+            const double v = warp_total(acc);
+            if (lane == 0) {
+                if (b < t0) head[t] = v;
+                else if (e > t1) tail[t] = v;
+                else finish(id, deg, v);
+            }
+            continue;
+        }
+#pragma unroll
+        for (int q = 0; q < kPrPerLane; ++q) vals[q * 32 + lane] = x[q];
+        __syncwarp();
+        while (true) {
+            const int32_t s = (int32_t)(max((int64_t)b, t0) - t0);
+            const int32_t len = i <= i1 ? (int32_t)(min((int64_t)e, t1) - t0) - s : 0;  // 0 or less: the next tile's row
+            double v = 0.0;
+            if (len > 0 && len < 32) {
+                KSum<T> acc;
+                for (int32_t j = s; j < s + len; ++j) acc.add(vals[j]);
+                v = acc.value();
+            }
+            unsigned longer = __ballot_sync(0xffffffffu, len >= 32);
+            while (longer) {
+                const int l = __ffs(longer) - 1;
+                longer &= longer - 1;
+                const int32_t ls = __shfl_sync(0xffffffffu, s, l), ll = __shfl_sync(0xffffffffu, len, l);
+                KSum<T> acc;
+                for (int32_t j = lane; j < ll; j += 32) acc.add(vals[ls + j]);
+                const double w = warp_total(acc);
+                if (lane == l) v = w;
+            }
+            if (len > 0) {
+                if (b < t0) head[t] = v;
+                else if (e > t1) tail[t] = v;
+                else finish(id, deg, v);
+            }
+            i += 32;
+            if (__shfl_sync(0xffffffffu, i, 0) > i1) break;
+            load_row();
+        }
+        __syncwarp();
+    }
+    block_partials<T>(sink, l1, part_sink, part_l1, blockIdx.x);
+}
+
+// The rows that cross tiles (a thread per tile in which one begins; the warp
+// together where it spans more than kPrSpan) and the rows without entries, whose
+// rank is the base: isolated ones pass nothing on, so until the last iteration
+// only their share of S is counted (all: every row, when the change is tracked
+// or ranks are due).  Then, in the
+// block that ends last, S and L1 from all blocks' partials in a fixed order and
+// the next base.
+constexpr int64_t kPrSpan = 16;
+template <class T>
+__global__ void __launch_bounds__(kPrThreads) pr_finish_kernel(
+    PrRows R, int32_t n, const int32_t* __restrict__ bare, const int32_t* __restrict__ bare_count, int all,
+    const double* __restrict__ head,
+    const double* __restrict__ tail, const int32_t* __restrict__ outdeg, const T* rank_old, T* rank_new,
+    T* contrib_new, PrScalars* sc, double damping, int track_l1, double* part_sink, double* part_l1, int slot0,
+    int nparts, double* l1_hist, int iter, int32_t* done) {
+    const int lane = lane_id();
+    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t nt = (int64_t)gridDim.x * blockDim.x;
+    const double base = sc->base;
+    double sink = 0.0, l1 = 0.0;
+    for (int64_t tb = tid - lane; tb < R.tiles; tb += nt) {
+        const int64_t t = tb + lane;
+        int32_t row = -1, deg = 0;
+        int64_t last = 0;
+        if (t < R.tiles) {
+            // The tile's last row crosses its end when it holds the next tile's
+            // first entry as well, and begins here unless it began before.
+            const int32_t i = t + 1 < R.tiles ? R.tile[t + 1] : R.k - 1;
+            const int64_t b = R.begin[i], e = R.begin[i + 1];
+            if (b >= t * kPrTile && b < (t + 1) * kPrTile && e > (t + 1) * kPrTile) {
+                row = R.id[i];
+                deg = R.deg[i];
+                last = (e - 1) / kPrTile;
+            }
+        }
+        double sum = 0.0;
+        if (row >= 0 && last - t <= kPrSpan) {
+            sum = tail[t];
+            for (int64_t x = t + 1; x <= last; ++x) sum += head[x];
+        }
+        unsigned wide = __ballot_sync(0xffffffffu, row >= 0 && last - t > kPrSpan);
+        while (wide) {
+            const int l = __ffs(wide) - 1;
+            wide &= wide - 1;
+            const int64_t t2 = tb + l, last2 = __shfl_sync(0xffffffffu, last, l);
+            double s = lane == 0 ? tail[t2] : 0.0;
+            for (int64_t x = t2 + 1 + lane; x <= last2; x += 32) s += head[x];
+            s = warp_sum(s);
+            if (lane == l) sum = s;
+        }
+        if (row >= 0)
+            pr_finish_row<T>(row, deg, sum, base, damping, rank_old, rank_new, contrib_new, track_l1, sink, l1);
+    }
+    const int32_t with_out = bare_count[0], isolated = bare_count[1];
+    for (int64_t i = tid; i < with_out; i += nt)
+        pr_finish_row<T>(bare[i], outdeg[bare[i]], 0.0, base, damping, rank_old, rank_new, contrib_new, track_l1, sink,
+                         l1);
+    if (all) {
+        for (int64_t i = tid; i < isolated; i += nt)
+            pr_finish_row<T>(bare[n - 1 - i], 0, 0.0, base, damping, rank_old, rank_new, contrib_new, track_l1, sink, l1);
+    } else if (tid == 0) {
+        sink += (double)(T)base * (double)isolated;
+    }
+    block_partials<T>(sink, l1, part_sink, part_l1, slot0 + blockIdx.x);
+    __shared__ int s_last;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(done, 1) == (int32_t)gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!s_last) return;
+    if (threadIdx.x == 0) *done = 0;
+    pr_reduce(part_sink, part_l1, nparts, n, damping, sc, l1_hist, iter, track_l1);
+}
 
 template <class T>
 __global__ void pr_to_f64_kernel(const T* src, double* dst, int32_t n) {
@@ -331,107 +486,97 @@ __global__ void pr_to_f64_kernel(const T* src, double* dst, int32_t n) {
 
 template <class T>
 int pagerank_impl(ghb_workspace* ws, int32_t n, const int32_t* in_rp, const int32_t* in_col,
-                  const int32_t* out_rp, const ghb_pr_options* o, double* rank_out, int32_t* iters_run) {
+                  const int32_t* out_rp, const ghb_pr_options* o, double* rank_out, int32_t* iters_run, bool ranked) {
     cudaStream_t st = ws->stream;
     const Tuning& tu = ws->tune;
-    const int32_t short_max = tu.pr_short, chunk = tu.pr_chunk;
     const int pthreads = tu.pr_threads;
-    const size_t cache_bytes = (size_t)tu.pr_cache_kb * 1024;
+    const unsigned max_rows = ws->num_sms * tu.pr_blocks_per_sm;  // persistent blocks
+    // Hub cache and the warps' tiles share a block's shared memory.
+    const size_t tile_bytes = (size_t)(pthreads / 32) * kPrTile * sizeof(T);
+    const size_t block_smem = (size_t)(227 * 1024) / tu.pr_blocks_per_sm - (tu.pr_blocks_per_sm > 1 ? 1024 : 0);
+    // Shared memory taken from L1 costs more than it gives past some 96 KB (160 M
+    // entries, FP64, ten iterations: 8.3 ms without a cache, 7.8 with 64 to 96 KB,
+    // 8.4 with 112, 13.1 with 144), and where the first ids are not the hubs
+    // nothing is gained from 32 KB on (9.7 ms with 0 or 32 KB, 10.8 with 64).
+    const int32_t cache_kb = ranked ? tu.pr_cache_kb : std::min(tu.pr_cache_kb, 32);
+    const size_t cache_bytes = std::min((size_t)cache_kb * 1024,
+                                        block_smem > tile_bytes + 1024 ? (block_smem - tile_bytes - 1024) & ~(size_t)255 : 0);
     const int32_t cache_elems = (int32_t)(cache_bytes / sizeof(T));
-    const unsigned grid_rows = ws->num_sms * tu.pr_blocks_per_sm;  // persistent blocks
-    const unsigned grid_long = ws->num_sms * 2;
-    const int nparts = grid_rows + grid_long;
+    const size_t smem = (size_t)((cache_elems + 3) & ~3) * sizeof(T) + tile_bytes;
     int32_t* hp = reinterpret_cast<int32_t*>(ws->host_pinned);
     GHB_CUDA_TRY(cudaMemcpyAsync(hp, in_rp + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     GHB_CUDA_TRY(cudaStreamSynchronize(st));
     const int64_t m = hp[0];
-    // Upper bounds: long rows <= min(n, m / (short_max + 1)), chunks <= m / chunk + long rows.
-    const int64_t max_long = std::min<int64_t>(n, m / (short_max + 1) + 1);
-    const int64_t max_chunks = m / chunk + max_long + 1;
-    auto carve = [&](Carver& c, T** ra, T** rb, T** ca, T** cb, int32_t** outdeg, int32_t** flag, int32_t** pos,
-                     int32_t** long_rows, int32_t** nch, int32_t** cpre, int32_t** crow, double** csum, int64_t** bs,
-                     double** ps, double** pl, PrScalars** sc, double** hist) {
-        *ra = c.take<T>(n);
-        *rb = c.take<T>(n);
-        *ca = c.take<T>(n);
-        *cb = c.take<T>(n);
-        *outdeg = c.take<int32_t>(n);
-        *flag = c.take<int32_t>(n);
-        *pos = c.take<int32_t>((size_t)n + 1);
-        *long_rows = c.take<int32_t>(max_long);
-        *nch = c.take<int32_t>(max_long);
-        *cpre = c.take<int32_t>(max_long + 1);
-        *crow = c.take<int32_t>(max_chunks);
-        *csum = c.take<double>(max_chunks);
-        *bs = c.take<int64_t>(scan_scratch_words(n > max_long ? n : max_long));
-        *ps = c.take<double>(nparts);
-        *pl = c.take<double>(nparts);
-        *sc = c.take<PrScalars>(1);
-        *hist = c.take<double>(o->iterations > 0 ? o->iterations : 1);
-    };
+    const int32_t tiles = (int32_t)((m + kPrTile - 1) / kPrTile);
+    const unsigned grid_rows = tiles ? grid_for((int64_t)tiles * 32, pthreads, max_rows) : 0;
+    const unsigned grid_fin = grid_for(std::max<int64_t>(tiles, n / 8), kPrThreads, ws->num_sms * 8);
+    const int nparts = (int)(grid_rows + grid_fin);
+    const unsigned g = ws->num_sms * 8;
+    const unsigned grid_init = grid_for(n, kPrThreads, nparts);  // one partial slot per block
     T *ra, *rb, *ca, *cb;
-    int32_t *outdeg, *flag, *pos, *long_rows, *nch, *cpre, *crow;
-    double *csum, *ps, *pl, *hist;
+    int32_t *outdeg, *flag, *pos, *row_id, *row_begin, *row_deg, *bare, *bare_count, *tile, *done;
+    double *head, *tail, *ps, *pl, *hist;
     int64_t* bs;
     PrScalars* sc;
+    auto carve = [&](Carver& c) {
+        ra = c.take<T>(n);
+        rb = c.take<T>(n);
+        ca = c.take<T>(n);
+        cb = c.take<T>(n);
+        outdeg = c.take<int32_t>(n);
+        flag = c.take<int32_t>(n);
+        pos = c.take<int32_t>((size_t)n + 1);
+        row_id = c.take<int32_t>(n);
+        row_begin = c.take<int32_t>((size_t)n + 1);
+        row_deg = c.take<int32_t>(n);
+        bare = c.take<int32_t>(n);
+        tile = c.take<int32_t>((size_t)tiles + 1);
+        head = c.take<double>((size_t)tiles + 1);
+        tail = c.take<double>((size_t)tiles + 1);
+        bs = c.take<int64_t>(scan_scratch_words(n));
+        ps = c.take<double>(nparts);
+        pl = c.take<double>(nparts);
+        sc = c.take<PrScalars>(1);
+        bare_count = c.take<int32_t>(2);
+        done = c.take<int32_t>(1);
+        hist = c.take<double>(o->iterations > 0 ? o->iterations : 1);
+    };
     Carver sizing(nullptr);
-    carve(sizing, &ra, &rb, &ca, &cb, &outdeg, &flag, &pos, &long_rows, &nch, &cpre, &crow, &csum, &bs, &ps, &pl, &sc,
-          &hist);
+    carve(sizing);
     GHB_TRY(ws_reserve(ws, sizing.off));
     Carver c(ws->scratch);
-    carve(c, &ra, &rb, &ca, &cb, &outdeg, &flag, &pos, &long_rows, &nch, &cpre, &crow, &csum, &bs, &ps, &pl, &sc,
-          &hist);
+    carve(c);
 
     const double d = o->damping;
-    const unsigned g = ws->num_sms * 8;
-    GHB_CUDA_TRY(cudaFuncSetAttribute(pr_rows_short_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)cache_bytes));
-    GHB_CUDA_TRY(cudaFuncSetAttribute(pr_chunk_kernel<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)cache_bytes));
-    GHB_CUDA_TRY(cudaFuncSetAttribute(pr_chunk_kernel<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)cache_bytes));
-    GHB_CUDA_TRY(cudaMemsetAsync(ps, 0, sizeof(double) * nparts, st));
-    GHB_CUDA_TRY(cudaMemsetAsync(pl, 0, sizeof(double) * nparts, st));
-    GHB_TRY(launch(ws, pr_init_kernel<T>, dim3(grid_rows), dim3(kPrThreads), 0, n, out_rp, outdeg, ra, ca, ps));
-    GHB_TRY(launch(ws, pr_reduce_kernel, dim3(1), dim3(1024), 0, (const double*)ps, (const double*)pl, nparts, n, d,
-                   sc, (double*)nullptr, 0, 0));
-    // Long-row list (ascending) and its chunks.
-    GHB_TRY(launch(ws, pr_long_flags_kernel, dim3(grid_for(n, 256, g)), dim3(256), 0, n, in_rp, flag, short_max));
+    GHB_CUDA_TRY(cudaFuncSetAttribute(pr_tile_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // ps, pl, sc, bare_count and done lie behind one another.
+    GHB_CUDA_TRY(cudaMemsetAsync(ps, 0, (size_t)(reinterpret_cast<char*>(done + 1) - reinterpret_cast<char*>(ps)), st));
+    GHB_TRY(launch(ws, pr_init_kernel<T>, dim3(grid_init), dim3(kPrThreads), 0, n, out_rp, outdeg, ra, ca, cb, ps));
+    GHB_TRY(launch(ws, pr_reduce_kernel, dim3(1), dim3(kPrThreads), 0, (const double*)ps, (const double*)pl, nparts, n, d,
+                   sc));
+    // The non-empty rows, the empty ones, and each tile's first row.
+    GHB_TRY(launch(ws, pr_row_flags_kernel, dim3(grid_for(n, 256, g)), dim3(256), 0, n, in_rp, flag));
     GHB_TRY(scan_exclusive_i32(ws, flag, pos, n, bs));
     GHB_CUDA_TRY(cudaMemcpyAsync(hp, pos + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    GHB_TRY(launch(ws, pr_row_lists_kernel, dim3(grid_for(n, 256, g)), dim3(256), 0, n, in_rp, (const int32_t*)pos,
+                   (const int32_t*)outdeg, row_id, row_begin, row_deg, bare, bare_count));
     GHB_CUDA_TRY(cudaStreamSynchronize(st));
-    const int32_t nlong = hp[0];
-    int32_t nchunks = 0;
-    if (nlong > 0) {
-        GHB_TRY(launch(ws, pr_long_compact_kernel, dim3(grid_for(n, 256, g)), dim3(256), 0, n, in_rp,
-                       (const int32_t*)flag, (const int32_t*)pos, long_rows, nch, chunk));
-        GHB_TRY(scan_exclusive_i32(ws, nch, cpre, nlong, bs));
-        GHB_CUDA_TRY(cudaMemcpyAsync(hp, cpre + nlong, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-        GHB_CUDA_TRY(cudaStreamSynchronize(st));
-        nchunks = hp[0];
-        GHB_TRY(launch(ws, pr_chunk_rows_kernel, dim3(grid_for((int64_t)nlong * 32, 256, g)), dim3(256), 0, nlong,
-                       (const int32_t*)cpre, crow));
-    }
+    const PrRows rows{row_id, row_begin, row_deg, tile, hp[0], (int32_t)m, tiles};
+    if (tiles)
+        GHB_TRY(launch(ws, pr_tile_rows_kernel, dim3(grid_for(tiles, 256, g)), dim3(256), 0, rows.k,
+                       (const int32_t*)row_begin, tiles, tile));
 
     T *r_cur = ra, *r_nxt = rb, *c_cur = ca, *c_nxt = cb;
     const bool track = o->tolerance > 0 || o->l1_history != nullptr;
     int it = 0;
     for (; it < o->iterations; ++it) {
-        GHB_TRY(launch(ws, pr_rows_short_kernel<T>, dim3(grid_rows), dim3(pthreads), cache_bytes, n, in_rp, in_col,
-                       (const int32_t*)outdeg, (const T*)c_cur, (const T*)r_cur, r_nxt, c_nxt, (const PrScalars*)sc, d,
-                       track ? 1 : 0, ps, pl, short_max, cache_elems));
-        if (nlong > 0) {
-            GHB_TRY(launch(ws, ws->tune.pr_gathers == 8 ? pr_chunk_kernel<T, 8> : pr_chunk_kernel<T, 4>,
-                           dim3(grid_rows), dim3(pthreads), cache_bytes, n, in_rp, in_col,
-                           (const int32_t*)long_rows, (const int32_t*)cpre, (const int32_t*)crow, nchunks,
-                           (const T*)c_cur, csum, chunk, cache_elems));
-        }
-        GHB_TRY(launch(ws, pr_long_finish_kernel<T>, dim3(grid_long), dim3(kPrThreads), 0, nlong,
-                       (const int32_t*)long_rows, (const int32_t*)cpre, (const double*)csum, (const int32_t*)outdeg,
-                       (const T*)r_cur, r_nxt, c_nxt, (const PrScalars*)sc, d, track ? 1 : 0, ps, pl,
-                       (int)grid_rows));
-        GHB_TRY(launch(ws, pr_reduce_kernel, dim3(1), dim3(1024), 0, (const double*)ps, (const double*)pl, nparts, n,
-                       d, sc, hist, it, track ? 1 : 0));
+        if (tiles)
+            GHB_TRY(launch(ws, pr_tile_kernel<T>, dim3(grid_rows), dim3(pthreads), smem, rows, n, in_col,
+                           (const T*)c_cur, (const T*)r_cur, r_nxt, c_nxt, (const PrScalars*)sc,
+                           d, track ? 1 : 0, head, tail, ps, pl, cache_elems));
+        GHB_TRY(launch(ws, pr_finish_kernel<T>, dim3(grid_fin), dim3(kPrThreads), 0, rows, n, (const int32_t*)bare,
+                       (const int32_t*)bare_count, track || it + 1 == o->iterations ? 1 : 0, (const double*)head, (const double*)tail, (const int32_t*)outdeg, (const T*)r_cur, r_nxt, c_nxt,
+                       sc, d, track ? 1 : 0, ps, pl, (int)grid_rows, nparts, hist, it, done));
         std::swap(r_cur, r_nxt);
         std::swap(c_cur, c_nxt);
         if (o->tolerance > 0) {
@@ -458,8 +603,8 @@ int pagerank_impl(ghb_workspace* ws, int32_t n, const int32_t* in_rp, const int3
 
 int pagerank_run(ghb_workspace* ws, int32_t n, const int32_t* in_rp, const int32_t* in_col, const int32_t* out_rp,
                  const ghb_pr_options* o, double* rank, int32_t* iters_run) {
-    if (o->precision == GHB_PR_FP64) return pagerank_impl<double>(ws, n, in_rp, in_col, out_rp, o, rank, iters_run);
-    return pagerank_impl<float>(ws, n, in_rp, in_col, out_rp, o, rank, iters_run);
+    if (o->precision == GHB_PR_FP64) return pagerank_impl<double>(ws, n, in_rp, in_col, out_rp, o, rank, iters_run, true);
+    return pagerank_impl<float>(ws, n, in_rp, in_col, out_rp, o, rank, iters_run, true);
 }
 
 }  // namespace ghb
@@ -477,6 +622,6 @@ extern "C" int ghb_pagerank(ghb_workspace* ws, int32_t n, const int32_t* in_rowp
     GHB_REQUIRE(options->precision == GHB_PR_FP64 || options->precision == GHB_PR_FP32_KAHAN,
                 "bad precision");
     if (options->precision == GHB_PR_FP64)
-        return pagerank_impl<double>(ws, n, in_rowptr, in_col, out_rowptr, options, rank, iterations_run);
-    return pagerank_impl<float>(ws, n, in_rowptr, in_col, out_rowptr, options, rank, iterations_run);
+        return pagerank_impl<double>(ws, n, in_rowptr, in_col, out_rowptr, options, rank, iterations_run, false);
+    return pagerank_impl<float>(ws, n, in_rowptr, in_col, out_rowptr, options, rank, iterations_run, false);
 }

@@ -63,9 +63,9 @@ int ghb_workspace_counters(ghb_workspace* ws, int64_t* kernel_launches, int64_t*
 /* Process-wide workspace on the current device (used by the C++ wrappers). */
 ghb_workspace* ghb_default_workspace(void);
 /* Launch shapes and thresholds of this workspace (no counterpart in the
- * reference): "pr_cache_kb" PageRank hub cache in shared memory, "pr_threads"
- * and "pr_blocks_per_sm" its persistent blocks, "pr_short" / "pr_chunk" its
- * row split, "ms_warp_rest" / "ms_pull_div" the multi-source BFS's block-row
+ * reference): "pr_cache_kb" PageRank hub cache in shared memory (as much of it
+ * as the block shape leaves room for), "pr_threads" and "pr_blocks_per_sm" its
+ * persistent blocks, "pr_short" / "pr_chunk" accepted without effect, "ms_warp_rest" / "ms_pull_div" the multi-source BFS's block-row
  * threshold and direction switch, "pol_band" (0-64) the band, in log2
  * units around the direction rule's threshold, inside which the learned
  * policy's network chooses a BFS level's direction and output format (0:
@@ -79,8 +79,8 @@ ghb_workspace* ghb_default_workspace(void);
  * oriented row the hash path takes (longer rows gallop), "ms_persistent" (0
  * or 1; default 1) whether a multi-source BFS pass is one cooperative launch
  * or host-driven levels, "bfs_blocks_per_sm" (1 or 2; default 2) the blocks
- * per SM of the whole-traversal BFS launch, "pr_gathers" (4 or 8) the
- * contribution gathers PageRank keeps in flight per lane on long rows,
+ * per SM of the whole-traversal BFS launch, "pr_gathers" (4 or 8)
+ * accepted without effect,
  * "mssp_persistent" (0 or 1; default 1) whether a multi-source SSSP pass is
  * one cooperative launch or host-driven rounds, "mssp_width_log2" (-10 -
  * 10; default 2) the multi-source bucket width as the single-source weight
