@@ -176,6 +176,45 @@ int bits_for_n(int32_t n) {
     return bits;
 }
 
+}  // namespace
+
+// perm / iperm of the degree ranking (total degree with in_rp, descending, ties
+// by id); *n_active (device, preset to n) gets the first id without entries.
+int rank_by_degree(ghb_workspace* ws, int32_t n, const int32_t* out_rp, const int32_t* in_rp, int32_t* perm,
+                   int32_t* iperm, int32_t** n_active) {
+    // Ids enter in order and the sort is stable: only the degrees are sorted.
+    size_t sort_tmp = 0;
+    {
+        cub::DoubleBuffer<uint64_t> dk(nullptr, nullptr);
+        cub::DeviceRadixSort::SortKeys(nullptr, sort_tmp, dk, (int64_t)n, 32, 64);
+    }
+    uint64_t *k0, *k1;
+    void* tmp;
+    int32_t* nact;
+    auto carve = [&](Carver& c) {
+        k0 = c.take<uint64_t>(n);
+        k1 = c.take<uint64_t>(n);
+        nact = c.take<int32_t>(8);
+        tmp = c.take<char>(sort_tmp);
+    };
+    Carver sizing(nullptr);
+    carve(sizing);
+    GHB_TRY(ws_reserve(ws, sizing.off));
+    Carver c(ws->scratch);
+    carve(c);
+    const unsigned gr = grid_for(n, 256, ws->num_sms * 8);
+    GHB_TRY(launch(ws, degree_key_kernel, dim3(gr), dim3(256), 0, n, out_rp, in_rp, k0));
+    cub::DoubleBuffer<uint64_t> dk(k0, k1);
+    size_t tb = sort_tmp;
+    GHB_CUDA_TRY(cub::DeviceRadixSort::SortKeys(tmp, tb, dk, (int64_t)n, 32, 64, ws->stream));
+    ws->launches++;
+    const int32_t nn = n;
+    GHB_CUDA_TRY(cudaMemcpyAsync(nact, &nn, sizeof(int32_t), cudaMemcpyHostToDevice, ws->stream));
+    GHB_TRY(launch(ws, perm_from_keys_kernel, dim3(gr), dim3(256), 0, n, (const uint64_t*)dk.Current(), perm, iperm, nact));
+    *n_active = nact;
+    return GHB_OK;
+}
+
 // Relabel one CSR (rows and columns through perm), rows sorted, weights
 // carried along; *repeat (device) is set when a row holds an entry twice.
 int relabel_csr(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* rp, const int32_t* col, const double* w,
@@ -220,8 +259,6 @@ int relabel_csr(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* rp, cons
                   (const uint32_t*)(want_vals ? dv.Current() : nullptr), m, n, bits, w, col_out,
                   want_vals ? w_out : (double*)nullptr, rp_out, repeat);
 }
-
-}  // namespace
 
 int map_back_i32(ghb_workspace* ws, const ghb_graph* g, const int32_t* src_new, int32_t* dst_old) {
     return launch(ws, map_back_kernel<int32_t>, dim3(grid_for(g->n, 256, ws->num_sms * 8)), dim3(256), 0, g->n,
@@ -328,38 +365,9 @@ int ghb_graph_create(ghb_workspace* ws, int32_t n, const int32_t* out_rowptr, co
     }
     // 1. degree ranking -> perm / iperm / n_active
     {
-        size_t sort_tmp = 0;
-        cub::DoubleBuffer<uint64_t> dk0(nullptr, nullptr);
-        // Ids enter in order and the sort is stable: only the degrees are sorted.
-        cub::DeviceRadixSort::SortKeys(nullptr, sort_tmp, dk0, (int64_t)n, 32, 64);
-        Carver sizing(nullptr);
-        sizing.take<uint64_t>(n);
-        sizing.take<uint64_t>(n);
-        sizing.take<int32_t>(8);
-        sizing.take<char>(sort_tmp);
-        GG_TRY(ws_reserve(ws, sizing.off));
-        Carver c(ws->scratch);
-        uint64_t* k0 = c.take<uint64_t>(n);
-        uint64_t* k1 = c.take<uint64_t>(n);
-        int32_t* nact = c.take<int32_t>(8);
-        void* tmp = c.take<char>(sort_tmp);
-        const unsigned gr = grid_for(n, 256, ws->num_sms * 8);
-        GG_TRY(launch(ws, degree_key_kernel, dim3(gr), dim3(256), 0, n, out_rowptr,
-                      directed ? in_rowptr : (const int32_t*)nullptr, k0));
-        cub::DoubleBuffer<uint64_t> dk(k0, k1);
-        size_t tb = sort_tmp;
-        cudaError_t e = cub::DeviceRadixSort::SortKeys(tmp, tb, dk, (int64_t)n, 32, 64, st);
-        if (e != cudaSuccess) {
-            set_error(std::string("degree sort: ") + cudaGetErrorString(e));
-            return fail(GHB_ERR_CUDA);
-        }
-        ws->launches++;
-        int32_t nn = n;
-        e = cudaMemcpyAsync(nact, &nn, sizeof(int32_t), cudaMemcpyHostToDevice, st);
-        if (e != cudaSuccess) return fail(GHB_ERR_CUDA);
-        GG_TRY(launch(ws, perm_from_keys_kernel, dim3(gr), dim3(256), 0, n, (const uint64_t*)dk.Current(), g->perm,
-                      g->iperm, nact));
-        e = cudaMemcpyAsync(hp, nact, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
+        int32_t* nact = nullptr;
+        GG_TRY(rank_by_degree(ws, n, out_rowptr, directed ? in_rowptr : (const int32_t*)nullptr, g->perm, g->iperm, &nact));
+        cudaError_t e = cudaMemcpyAsync(hp, nact, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return fail(GHB_ERR_CUDA);
         g->n_active = hp[0];

@@ -50,6 +50,13 @@ struct ghb_graph {
 
 namespace ghb {
 
+// The degree ranking and the relabelling behind ghb_graph_create (they use the
+// workspace's scratch; see graph.cu).
+int rank_by_degree(ghb_workspace* ws, int32_t n, const int32_t* out_rp, const int32_t* in_rp, int32_t* perm,
+                   int32_t* iperm, int32_t** n_active);
+int relabel_csr(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* rp, const int32_t* col, const double* w,
+                const int32_t* perm, int32_t* rp_out, int32_t* col_out, double* w_out, int32_t* repeat);
+
 // Result mapping kernels (new-id array -> caller's ids).
 int map_back_i32(ghb_workspace* ws, const ghb_graph* g, const int32_t* src_new, int32_t* dst_old);
 int map_back_f64(ghb_workspace* ws, const ghb_graph* g, const double* src_new, double* dst_old);

@@ -21,12 +21,20 @@
 
 #include "common.cuh"
 #include "edge_walk.cuh"
+#include "graph.cuh"
 #include "scan.cuh"
 
 namespace ghb {
 namespace {
 
 constexpr int32_t kTcFlagLoop = 1, kTcFlagUnsorted = 2, kTcFlagAsym = 4;
+constexpr int32_t kTcFlags = 7;
+// Above the flags, the lengths that the rows have: a bit per class of them, so
+// that a count launches only the kernels whose rows exist.
+constexpr int32_t kTcLen32 = 8, kTcLen128 = 16, kTcLen1024 = 32, kTcLen4096 = 64, kTcLenMore = 128;
+__device__ __forceinline__ int32_t tc_length_bit(int32_t d) {
+    return d <= 32 ? kTcLen32 : d <= 128 ? kTcLen128 : d <= 1024 ? kTcLen1024 : d <= 4096 ? kTcLen4096 : kTcLenMore;
+}
 
 // First position in [b, e) of a sorted row whose entry is >= x (e if none):
 // a galloping search (probes b, b+1, b+3, b+7, ... then a binary search in the
@@ -79,7 +87,8 @@ struct CheckVisitor {
         if (u == v) f |= kTcFlagLoop;
         if (j + 1 < rowptr[u + 1] && col[j + 1] <= v) f |= kTcFlagUnsorted;
         if (!row_contains(col, rowptr[v], rowptr[v + 1], u)) f |= kTcFlagAsym;
-        if (f) atomicOr(flags, f);
+        if (j == rowptr[u]) f |= tc_length_bit(rowptr[u + 1] - j);
+        if (f & ~*(volatile const int32_t*)flags) atomicOr(flags, f);
     }
     __device__ void finish() const {}
 };
@@ -508,9 +517,11 @@ size_t tc_lists_ints(int32_t n, int64_t m) { return (size_t)(6 * tc_item_cap(n, 
 namespace {
 
 // Rows first .. n - 1 of the oriented CSR N+(v) = ocol[rb[v] .. re[v]) (the
-// rows below `first` are empty).
+// rows below `first` are empty).  lengths: the kTcLen bits that the rows may
+// have.
 int tc_count_oriented(ghb_workspace* ws, int32_t first, int32_t n, int64_t m, const int32_t* rb, const int32_t* re,
-                      const int32_t* ocol, unsigned long long* cnt, const WalkBuffers& wb, int32_t* lists) {
+                      const int32_t* ocol, unsigned long long* cnt, const WalkBuffers& wb, int32_t* lists,
+                      int32_t lengths) {
     const OrientedVisitor gallop{rb, re, ocol, cnt};
     if (!ws->tune.tc_hash)
         return walk_range(ws, rb, re, ocol, (const int32_t*)nullptr, (const int32_t*)nullptr, (int64_t)n, (int64_t)n,
@@ -524,9 +535,13 @@ int tc_count_oriented(ghb_workspace* ws, int32_t first, int32_t n, int64_t m, co
                    dim3(kTcWarpBlock), 0, first, n, rb, re, ocol, cnt, items, item_cap, huge, tails,
                    std::min<int32_t>(std::max<int32_t>(ws->tune.tc_block_row, kTcWarpRow), kTcBlockRow),
                    ws->tune.tc_trim_min));
+    if (lengths < kTcLen1024) return GHB_OK;
     GHB_TRY(launch(ws, tc_hash_slice_kernel<kTcMidLog2, false>, dim3(ws->num_sms * ws->tune.tc_slice_blocks),
                    dim3(kTcBlockThreads), 0, rb, re, ocol, cnt, (const int2*)items, (const int32_t*)tails,
                    ws->tune.tc_trim_min));
+    // A lower tc_block_row sends shorter rows to the galloping walk.
+    const bool gallops = lengths >= kTcLenMore || ws->tune.tc_block_row < kTcBlockRow;
+    if (lengths < kTcLen4096 && !gallops) return GHB_OK;
     const size_t smem = sizeof(int32_t) << kTcBigLog2;
     static bool attr_set[64] = {false};
     if (ws->device >= 0 && ws->device < 64 && !attr_set[ws->device]) {
@@ -537,6 +552,7 @@ int tc_count_oriented(ghb_workspace* ws, int32_t first, int32_t n, int64_t m, co
     GHB_TRY(launch(ws, tc_hash_slice_kernel<kTcMid2Log2, false>, dim3(ws->num_sms * 6), dim3(kTcBlockThreads), 0, rb,
                    re, ocol, cnt, (const int2*)(items + item_cap), (const int32_t*)(tails + 1),
                    ws->tune.tc_trim_min));
+    if (!gallops) return GHB_OK;
     GHB_TRY(launch(ws, tc_hash_slice_kernel<kTcBigLog2, true>, dim3(ws->num_sms * 3), dim3(kTcBlockThreads), smem, rb,
                    re, ocol, cnt, (const int2*)(items + 2 * item_cap), (const int32_t*)(tails + 2),
                    ws->tune.tc_trim_min));
@@ -839,6 +855,8 @@ __global__ void __launch_bounds__(kTcHubThreads, kTcHubBlocks) tc_hub_items_kern
     counts.flush();
 }
 
+constexpr int64_t kTcRankEntries = 1 << 20;  // entries from which raw rows may be relabelled for the count
+
 // Scratch of the rank-ordered path.
 struct TcRanked {
     int32_t *he, *oe, *tails;  // tails: [0] listed slices, [1] rows drawn, [2] slices drawn
@@ -858,10 +876,10 @@ struct TcRanked {
 // Triangles of a symmetric, loop-free CSR with strictly increasing rows whose
 // ids are ranks (hubs first), into cnt (zeroed by the caller).
 int tc_count_ranked(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* rp, const int32_t* col,
-                    unsigned long long* cnt, const WalkBuffers& wb, int32_t* lists, const TcRanked& r) {
+                    unsigned long long* cnt, const WalkBuffers& wb, int32_t* lists, const TcRanked& r, int32_t lengths) {
     GHB_TRY(launch(ws, tc_rank_ends_kernel, dim3(grid_for(n, 256, ws->num_sms * 8)), dim3(256), 0, n, rp, col, r.he,
                    r.oe));
-    if (!ws->tune.tc_hash) return tc_count_oriented(ws, 0, n, m, rp, (const int32_t*)r.oe, col, cnt, wb, lists);
+    if (!ws->tune.tc_hash) return tc_count_oriented(ws, 0, n, m, rp, (const int32_t*)r.oe, col, cnt, wb, lists, lengths);
     GHB_CUDA_TRY(cudaMemsetAsync(r.tails, 0, 3 * sizeof(int32_t), ws->stream));
     GHB_TRY(launch(ws, tc_hub_bitmap_kernel, dim3(grid_for((int64_t)r.bit_rows * 32, 256, ws->num_sms * 8)), dim3(256),
                    0, r.bit_rows, rp, (const int32_t*)r.he, col, r.bits));
@@ -873,7 +891,7 @@ int tc_count_ranked(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* rp, 
                    (const int32_t*)r.oe, col, (const uint4*)r.bits, r.bit_rows, cnt, (const int2*)items,
                    (const int32_t*)r.tails, r.tails + 2));
     if (n <= kTcHubs) return GHB_OK;  // every id is a hub
-    return tc_count_oriented(ws, kTcHubs, n, m, (const int32_t*)r.he, (const int32_t*)r.oe, col, cnt, wb, lists);
+    return tc_count_oriented(ws, kTcHubs, n, m, (const int32_t*)r.he, (const int32_t*)r.oe, col, cnt, wb, lists, lengths);
 }
 
 // The reference's merge over every entry (any CSR).
@@ -906,6 +924,16 @@ struct MergeVisitor {
     }
     __device__ void finish() const {}
 };
+
+// Counts by rank to the caller's ids.
+__global__ void tc_unrank_kernel(int32_t n, const int32_t* __restrict__ perm, const int64_t* __restrict__ by_rank,
+                                 int64_t* counts64, int32_t* counts32) {
+    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t c = by_rank[perm[v]];
+        if (counts64) counts64[v] = c;
+        if (counts32) counts32[v] = (int32_t)(uint32_t)(uint64_t)c;
+    }
+}
 
 __global__ void tc_finish_kernel(int32_t n, const unsigned long long* __restrict__ cnt, int scale,
                                  int64_t* counts64, int32_t* counts32, unsigned long long* total) {
@@ -969,7 +997,7 @@ int tc_oriented_core(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* row
     GHB_TRY(scan_exclusive_i32(ws, keep, orp, n, bsums));
     GHB_TRY(orient_fill(ws, n, rowptr, col, orp, ocol, lists));
     GHB_TRY(tc_count_oriented(ws, 0, n, m, (const int32_t*)orp, (const int32_t*)orp + 1, (const int32_t*)ocol, cnt, wb,
-                              lists));
+                              lists, INT32_MAX));
     if (counts64)
         GHB_TRY(launch(ws, tc_finish_kernel, dim3(grid_for(n, 256, ws->num_sms * 8)), dim3(256), 0, n,
                        (const unsigned long long*)cnt, 6, counts64, (int32_t*)nullptr,
@@ -1026,9 +1054,39 @@ int tc_run_cached(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int
         check = hp[0];
         if (flags_cache) flags_cache->store(check, std::memory_order_relaxed);
     }
-    const bool oriented = check == 0;
+    const bool oriented = (check & kTcFlags) == 0;
+    if (oriented && !ranked && ws->tune.tc_hash && check >= kTcLen1024 && m >= kTcRankEntries) {
+        // Rows over 128 entries in a graph that is not small: ranks by degree,
+        // and the hub bitmaps, repay a relabelled copy of the rows (RMAT-19 on
+        // the caller's ids: 9.9 ms by the hash kernels, 3.7 this way).  Without
+        // long rows the copy costs more than the count (an ER graph of as many
+        // entries counts in 1.2 ms), and so it does on a small graph (RMAT,
+        // 1,000 vertices: 0.18 ms against 0.31).
+        GHB_CUDA_TRY(cudaStreamSynchronize(st));
+        int32_t *perm, *iperm, *rp, *rcol, *repeat, *nact;
+        int64_t* by_rank;
+        auto stage = [&](Carver& k) {
+            perm = k.take<int32_t>(n);
+            iperm = k.take<int32_t>(n);
+            rp = k.take<int32_t>((size_t)n + 1);
+            rcol = k.take<int32_t>(m);
+            repeat = k.take<int32_t>(1);
+            by_rank = k.take<int64_t>(n);
+        };
+        Carver need(nullptr);
+        stage(need);
+        GHB_TRY(ws_reserve_stage(ws, need.off));
+        Carver k(ws->stage);
+        stage(k);
+        GHB_TRY(rank_by_degree(ws, n, rowptr, nullptr, perm, iperm, &nact));
+        GHB_TRY(relabel_csr(ws, n, m, rowptr, col, nullptr, perm, rp, rcol, nullptr, repeat));
+        std::atomic<int32_t> known{check};
+        GHB_TRY(tc_run_cached(ws, n, rp, rcol, by_rank, nullptr, total, &known, true));
+        return launch(ws, tc_unrank_kernel, dim3(grid_for(n, 256, ws->num_sms * 8)), dim3(256), 0, n, (const int32_t*)perm,
+                      (const int64_t*)by_rank, counts64, counts32);
+    }
     if (oriented && ranked) {
-        GHB_TRY(tc_count_ranked(ws, n, m, rowptr, col, cnt, wb, lists, rk));
+        GHB_TRY(tc_count_ranked(ws, n, m, rowptr, col, cnt, wb, lists, rk, check));
     } else if (oriented) {
         GHB_CUDA_TRY(cudaMemsetAsync(keep, 0, sizeof(int32_t) * n, st));
         GHB_TRY(walk(ws, rowptr, col, (const int32_t*)nullptr, (const int32_t*)nullptr, (int64_t)n, (int64_t)n,
@@ -1036,7 +1094,14 @@ int tc_run_cached(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int
         GHB_TRY(scan_exclusive_i32(ws, keep, orp, n, bsums));
         GHB_TRY(orient_fill(ws, n, rowptr, col, orp, ocol, lists));
         GHB_TRY(tc_count_oriented(ws, 0, n, m, (const int32_t*)orp, (const int32_t*)orp + 1, (const int32_t*)ocol, cnt,
-                                  wb, lists));
+                                  wb, lists, check));
+    } else if (!(check & kTcFlagUnsorted) && ws->tune.tc_hash && check >= kTcLen128) {
+        // Directed rows, loops: on strictly increasing rows the reference's
+        // merge is an intersection, which the hash kernels count for every
+        // entry of the rows themselves (directed RMAT-19 in a resident graph:
+        // 2.4 s by one lane's merge per entry, 59 ms by the kernels).  Rows of
+        // up to 32 entries merge in fewer launches.
+        GHB_TRY(tc_count_oriented(ws, 0, n, m, rowptr, rowptr + 1, col, cnt, wb, lists, check));
     } else {
         GHB_TRY(walk(ws, rowptr, col, (const int32_t*)nullptr, (const int32_t*)nullptr, (int64_t)n, (int64_t)n, wb,
                      MergeVisitor{rowptr, col, cnt}));

@@ -54,3 +54,38 @@ def test_past_the_bitmap_table(G):
     src = np.concatenate([low, np.arange(hubs, n - 1)]).astype(np.int32)
     dst = np.concatenate([rng.integers(0, hubs, low.size), np.arange(hubs + 1, n)]).astype(np.int32)
     check(G, O.make_graph(n, src, dst, False, weight_mode=0))
+
+
+@pytest.mark.parametrize("longest", [20, 32, 33, 128, 129, 1024, 1025, 4097])
+@pytest.mark.parametrize("loops", [False, True])
+def test_directed_rows(G, longest, loops):
+    """Directed rows of every length class of the hash kernels, with and
+    without self-loops, against the reference's merge over every entry."""
+    rng = np.random.default_rng(longest)
+    n = 6000
+    hub = np.arange(40)
+    src = np.concatenate([np.repeat(hub, longest), rng.integers(0, n, 3 * n), np.arange(0, n, 7) if loops else hub[:0]])
+    dst = np.concatenate([np.concatenate([rng.choice(n, longest, replace=False) for _ in hub]),
+                          np.concatenate([rng.integers(0, 200, n), rng.integers(0, n, 2 * n)]),
+                          np.arange(0, n, 7) if loops else hub[:0]])
+    rp, col, _ = O.build_csr(n, src.astype(np.int32), dst.astype(np.int32), drop_self_loops=not loops, weight_mode=0)
+    irp, icol, _ = O.build_csr(n, dst.astype(np.int32), src.astype(np.int32), drop_self_loops=not loops, weight_mode=0)
+    og = O.Graph(n=n, rowptr=rp, col=col, w=None, directed=True, in_rowptr=irp, in_col=icol, in_w=None)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    g = G.CSRGraph(n=n, rowptr=t(rp), col=t(col), directed=True)
+    g.in_rowptr, g.in_col = t(irp), t(icol)
+    ref = O.tc(og)
+    for c64, c32, _ in (G.tc(g), G.ResidentGraph(g).tc()):
+        assert np.array_equal(c32.cpu().numpy(), ref)
+        assert np.array_equal(c64.cpu().numpy().astype(np.int32), ref)
+
+
+@pytest.mark.parametrize("scale", [15, 16])  # below and above the entries from which raw rows are relabelled
+def test_raw_rows_of_a_skewed_graph(G, scale):
+    og = O.rmat_graph(scale, 16, 5, directed=False, weight_mode=0)
+    assert (og.m >= 1 << 20) == (scale == 16)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    c64, c32, total = G.tc(G.CSRGraph(n=og.n, rowptr=t(og.rowptr), col=t(og.col), directed=False))
+    ref, ref_total = O.tc_oriented(og)
+    assert np.array_equal(c64.cpu().numpy(), ref) and total == ref_total
+    assert np.array_equal(c32.cpu().numpy(), ref.astype(np.int32))
