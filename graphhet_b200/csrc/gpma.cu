@@ -77,9 +77,12 @@ constexpr int32_t kCopyChunk = 256;
 // Rows of the batch with at most row_warp_max existing entries + updates
 // are rebuilt by one warp (a launch argument: kRowWarpSmall for small
 // batches, where a long row on one warp would be the critical path,
-// kRowWarpLarge otherwise); longer rows by the grid-wide kernels.
+// kRowWarpLarge otherwise); longer rows by the grid-wide kernels.  A step of 32
+// entries is a search in the row's updates, some 2 us of dependent loads, so the
+// longest row on one warp sets the kernel's time: 100,000 updates on an RMAT-21
+// graph took 0.41 ms in it with rows of up to 4,096 entries.
 constexpr int32_t kRowWarpSmall = 256;
-constexpr int32_t kRowWarpLarge = 4096;
+constexpr int32_t kRowWarpLarge = 512;
 // The grid-wide kernels give each warp a chunk of this many entries of a
 // long row (one search for the chunk's row, 8 entries per lane).
 constexpr int32_t kBigChunk = 256;
@@ -247,12 +250,12 @@ __device__ __forceinline__ int64_t seg_of(const T* __restrict__ X, int64_t len, 
 
 // Rank of an existing entry (column c at index j of row k) in the rebuilt
 // row: j + (inserts before c) - (deletes before c); -1 when it is deleted.
-// Updates of row k are skey[a, z), sorted.
+// Row k's updates begin at a; those of columns near c are skey[lo, hi), sorted.
 __device__ __forceinline__ int32_t old_rank(const uint64_t* __restrict__ skey, const int8_t* __restrict__ typ,
                                             const int32_t* __restrict__ insX, const int32_t* __restrict__ delX,
-                                            int32_t a, int32_t z, uint32_t r, int32_t c, int32_t j) {
+                                            int32_t a, int32_t lo, int32_t hi, uint32_t r, int32_t c, int32_t j) {
     const uint64_t key = ((uint64_t)r << 32) | (uint32_t)c;
-    int32_t lo = a, hi = z;
+    const int32_t z = hi;
     while (lo < hi) {
         const int32_t mid = (lo + hi) >> 1;
         if (skey[mid] < key) lo = mid + 1;
@@ -264,6 +267,60 @@ __device__ __forceinline__ int32_t old_rank(const uint64_t* __restrict__ skey, c
         if (typ[q] == kDel) return -1;
     }
     return j + (insX[lo] - insX[a]) - (delX[lo] - delX[a]);
+}
+
+// Entries [j0, j0 + len), len <= kBigChunk, of an existing row (slots from s) to
+// their ranks in the rebuilt one (from o, d2 entries; updates skey[a, z)), by a
+// warp: all loads issued together, then one search for the updates that fall
+// between the chunk's first and last column.  Most chunks hold none (100,000
+// updates meet one entry in 450 of the rows they touch): their entries keep
+// their order at one common offset.  Returns the ranks outside the row.
+__device__ __forceinline__ unsigned scatter_old_chunk(const uint64_t* __restrict__ skey, const int8_t* __restrict__ typ,
+                                                      const int32_t* __restrict__ insX, const int32_t* __restrict__ delX,
+                                                      int32_t a, int32_t z, uint32_t r, const int32_t* __restrict__ col,
+                                                      const double* __restrict__ val, int64_t s, int32_t j0, int32_t len,
+                                                      int32_t* __restrict__ scol, double* __restrict__ sval, int64_t o,
+                                                      int32_t d2) {
+    const int lane = lane_id();
+    constexpr int kPer = kBigChunk / 32;
+    int32_t c[kPer];
+    double w[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        const int32_t j = u * 32 + lane;
+        c[u] = j < len ? col[s + j0 + j] : 0;
+        w[u] = j < len ? val[s + j0 + j] : 0.0;
+    }
+    // Lane 0: the first update at or past the first column; lane 1: the first
+    // one past the last column.
+    int32_t lo = a, hi = z;
+    if (lane < 2) {
+        const uint32_t edge = (uint32_t)col[s + j0 + (lane == 0 ? 0 : len - 1)];
+        const uint64_t key = (((uint64_t)r << 32) | edge) + (uint64_t)lane;
+        while (lo < hi) {
+            const int32_t mid = (lo + hi) >> 1;
+            if (skey[mid] < key) lo = mid + 1;
+            else hi = mid;
+        }
+    }
+    const int32_t u0 = __shfl_sync(0xffffffffu, lo, 0), u1 = __shfl_sync(0xffffffffu, lo, 1);
+    unsigned bad = 0;
+    const int32_t off = (insX[u0] - insX[a]) - (delX[u0] - delX[a]);
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        const int32_t j = u * 32 + lane;
+        if (j >= len) break;
+        int32_t rk = j0 + j + off;
+        if (u0 != u1) rk = old_rank(skey, typ, insX, delX, a, u0, u1, r, c[u], j0 + j);
+        if (rk < 0 && u0 != u1) continue;
+        if (rk < 0 || rk >= d2) {
+            ++bad;
+            continue;
+        }
+        scol[o + rk] = c[u];
+        sval[o + rk] = w[u];
+    }
+    return bad;
 }
 
 // Rank of insert i (its row's updates start at a): insertion point - deletes
@@ -321,17 +378,9 @@ __global__ void upd_rows_warp_kernel(const int32_t* __restrict__ row_id, const i
         const int64_t s = start[r];
         const int64_t o = dst_start ? dst_start[r] : (int64_t)scrX[k];
         unsigned long long bad = 0;
-        for (int32_t j = lane; j < d; j += 32) {
-            const int32_t c = col[s + j];
-            const int32_t rk = old_rank(skey, typ, insX, delX, a, z, (uint32_t)r, c, j);
-            if (rk < 0) continue;
-            if (rk >= d2) {
-                ++bad;
-                continue;
-            }
-            scol[o + rk] = c;
-            sval[o + rk] = val[s + j];
-        }
+        for (int32_t j0 = 0; j0 < d; j0 += kBigChunk)
+            bad += scatter_old_chunk(skey, typ, insX, delX, a, z, (uint32_t)r, col, val, s, j0, min(kBigChunk, d - j0),
+                                     scol, sval, o, d2);
         for (int32_t i = a + lane; i < z; i += 32) {
             if (typ[i] != kIns) continue;
             const int32_t rk = new_rank(pos, insX, delX, a, i);
@@ -440,22 +489,9 @@ __global__ void big_scatter_old_kernel(const int32_t* __restrict__ big, const in
         const int64_t s = start[r];
         const int64_t o = dst_start ? dst_start[r] : (int64_t)scrX[k];
         const int32_t j0 = (int32_t)(ch - bex[i]) * kBigChunk;
-        unsigned long long bad = 0;
-#pragma unroll 2
-        for (int u = 0; u < kBigChunk / 32; ++u) {
-            const int32_t j = j0 + u * 32 + lane;
-            if (j >= d) break;
-            const int32_t c = col[s + j];
-            const int32_t rk = old_rank(skey, typ, insX, delX, a, z, (uint32_t)r, c, j);
-            if (rk < 0) continue;
-            if (rk >= d2) {
-                ++bad;
-                continue;
-            }
-            scol[o + rk] = c;
-            sval[o + rk] = val[s + j];
-        }
-        if (bad) atomicAdd(bad_rank, bad);
+        const unsigned bad = scatter_old_chunk(skey, typ, insX, delX, a, z, (uint32_t)r, col, val, s, j0,
+                                               min(kBigChunk, d - j0), scol, sval, o, d2);
+        if (bad) atomicAdd(bad_rank, (unsigned long long)bad);
     }
 }
 
@@ -1269,6 +1305,26 @@ int apply_pass(ghb_workspace* ws, ghb_gpma* g, const uint64_t* keys, const doubl
     return GHB_OK;
 }
 
+// The compact CSR of the current rows into the given arrays (val may be NULL).
+int compact_rows(ghb_workspace* ws, ghb_gpma* g, int32_t* rowptr, int32_t* col, double* val) {
+    const int32_t n = g->n;
+    int64_t* block_sums;
+    int32_t *cc, *coff, *chunk_row;
+    auto carve = [&](Carver& c) {
+        block_sums = c.take<int64_t>(scan_scratch_words((int64_t)n));
+        cc = c.take<int32_t>((int64_t)n + 1);
+        coff = c.take<int32_t>((int64_t)n + 1);
+        chunk_row = c.take<int32_t>(copy_chunk_slots(g->m));
+    };
+    Carver sizing(nullptr);
+    carve(sizing);
+    GHB_TRY(ws_reserve(ws, sizing.off));
+    Carver c(ws->scratch);
+    carve(c);
+    GHB_TRY(scan_exclusive_i32(ws, g->deg, rowptr, n, block_sums));
+    return copy_rows<int32_t>(ws, n, g->start, g->deg, g->col, g->val, rowptr, col, val, cc, coff, chunk_row, block_sums);
+}
+
 int snapshot(ghb_workspace* ws, ghb_gpma* g, bool weights) {
     if (g->s_ok && (!weights || g->s_val_ok)) return GHB_OK;
     const int32_t n = g->n;
@@ -1287,20 +1343,7 @@ int snapshot(ghb_workspace* ws, ghb_gpma* g, bool weights) {
         GHB_TRY(dev_alloc(&g->s_val, c));
         g->s_val_cap = c;
     }
-    Carver sizing(nullptr);
-    sizing.take<int64_t>(scan_scratch_words((int64_t)n));
-    sizing.take<int32_t>((int64_t)n + 1);
-    sizing.take<int32_t>((int64_t)n + 1);
-    sizing.take<int32_t>(copy_chunk_slots(g->m));
-    GHB_TRY(ws_reserve(ws, sizing.off));
-    Carver c(ws->scratch);
-    int64_t* block_sums = c.take<int64_t>(scan_scratch_words((int64_t)n));
-    int32_t* cc = c.take<int32_t>((int64_t)n + 1);
-    int32_t* coff = c.take<int32_t>((int64_t)n + 1);
-    int32_t* chunk_row = c.take<int32_t>(copy_chunk_slots(g->m));
-    GHB_TRY(scan_exclusive_i32(ws, g->deg, g->s_rowptr, n, block_sums));
-    GHB_TRY(copy_rows<int32_t>(ws, n, g->start, g->deg, g->col, g->val, g->s_rowptr, g->s_col,
-                               weights ? g->s_val : nullptr, cc, coff, chunk_row, block_sums));
+    GHB_TRY(compact_rows(ws, g, g->s_rowptr, g->s_col, weights ? g->s_val : nullptr));
     g->s_ok = true;
     g->s_val_ok = weights;
     return GHB_OK;
@@ -1551,7 +1594,8 @@ int ghb_gpma_export(ghb_workspace* ws, ghb_gpma* g, int32_t* rowptr, int32_t* co
     ws = ws_resolve(ws);
     GHB_REQUIRE(ws && g, "NULL workspace / graph");
     GHB_REQUIRE(rowptr && (g->m == 0 || col), "NULL rowptr / col");
-    GHB_TRY(snapshot(ws, g, w != nullptr));
+    // Straight into the caller's arrays unless a snapshot is there to copy.
+    if (!g->s_ok || (w && !g->s_val_ok)) return compact_rows(ws, g, rowptr, col, w);
     GHB_CUDA_TRY(cudaMemcpyAsync(rowptr, g->s_rowptr, sizeof(int32_t) * ((size_t)g->n + 1),
                                  cudaMemcpyDeviceToDevice, ws->stream));
     if (g->m > 0) {
