@@ -21,7 +21,7 @@ int sssp_pred_run(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int
 int sssp_delta_run(ghb_workspace* ws, ghb_graph* g, int32_t src, double inf, double delta, double* dist_out,
                    ghb_traversal_stats* stats);
 int sssp_choose_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const double* w, int32_t src,
-                      const ghb_sssp_options* opt, double* delta);
+                      const ghb_sssp_options* opt, int64_t light_m, double* delta);
 
 // Resident SSSP: delta-stepping with the light/heavy split when the rows fit
 // the weight-sorted copy's key (n <= 2^25), else the near/far form.
@@ -29,7 +29,7 @@ static int graph_sssp_dispatch(ghb_workspace* ws, const ghb_graph* g, int32_t sr
                                const ghb_sssp_options* options, ghb_traversal_stats* stats) {
     if (g->m > 0 && g->n <= (1 << 25)) {
         double delta = 0.0;
-        GHB_TRY(sssp_choose_delta(ws, g->n, g->rowptr, g->w, src_new, options, &delta));
+        GHB_TRY(sssp_choose_delta(ws, g->n, g->rowptr, g->w, src_new, options, g->m, &delta));
         return sssp_delta_run(ws, const_cast<ghb_graph*>(g), src_new, inf, delta, dnew, stats);
     }
     return sssp_run(ws, g->n, g->rowptr, g->col, g->w, src_new, inf, dnew, options, stats);

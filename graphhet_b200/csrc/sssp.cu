@@ -331,7 +331,8 @@ __global__ void fill_i32(int32_t* p, int64_t count, int32_t value) {
 
 // Bucket width from a weight sample when the caller gives none: the mean
 // weight times 32 over the mean degree (wider buckets on sparse graphs,
-// where rounds are latency-bound).
+// where rounds are latency-bound).  The policy network's bins and the
+// multi-source pass scale this width.
 int sssp_pick_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const double* w, double* delta) {
     cudaStream_t st = ws->stream;
     int32_t* hp = reinterpret_cast<int32_t*>(ws->host_pinned);
@@ -357,13 +358,30 @@ int sssp_pick_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const d
     return GHB_OK;
 }
 
-// The width for one SSSP call: the caller's, else the weight rule above,
-// scaled by the policy network's bin when the learned policy is asked for
-// and a network is installed.  With record_trace, trace row 0 gets the
-// features, then 12 the width used, 13 -1, 14 the rule's width, 15 1 when
-// the network chose it; the caller's driver fills 13 (device ms).
+// Share of the weight rule's width that a call takes when nobody names one.
+// A narrower bucket trades entries relaxed twice for rounds: a round costs
+// its grid barriers whatever the graph, the entries it saves grow with the
+// graph.  With the light/heavy split (light_m entries, 0 without it), where
+// a settled vertex's heavy entries are read once however narrow the bucket,
+// half the width pays from 2^24 entries on (ms at the whole, half width:
+// RMAT-22 8.65, 5.96; RMAT-21 4.70, 3.65, its directed form 3.80, 2.87;
+// uniform, 2^21 vertices of degree 32 2.85, 2.36, of degree 8 2.26, 2.05;
+// 2^20 of degree 16 1.06, 0.94) and not below (2^20 of degree 10 0.94,
+// 0.95, directed of degree 8 0.77, 0.81).  Sparse graphs keep the whole
+// width: a 1501 x 1999 grid takes 41 ms with it and 48 with half.  Without
+// the split the entries saved are few (RMAT-21 raw 6.59, 6.56).
+static double sssp_default_share(int32_t n, int64_t light_m) {
+    return light_m >= (1ll << 24) && light_m >= 6ll * n ? 0.5 : 1.0;
+}
+
+// The width for one SSSP call: the caller's, else the weight rule's share
+// above, or the rule's width scaled by the policy network's bin when the
+// learned policy is asked for and a network is installed.  With
+// record_trace, trace row 0 gets the features, then 12 the width used, 13
+// -1, 14 the weight rule's width, 15 1 when the network chose it; the
+// caller's driver fills 13 (device ms).
 int sssp_choose_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const double* w, int32_t src,
-                      const ghb_sssp_options* opt, double* delta) {
+                      const ghb_sssp_options* opt, int64_t light_m, double* delta) {
     if (opt && opt->delta > 0) {
         *delta = opt->delta;
         return GHB_OK;
@@ -371,7 +389,11 @@ int sssp_choose_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const
     GHB_TRY(sssp_pick_delta(ws, n, rowptr, w, delta));
     const bool learned = opt && opt->policy == GHB_POLICY_LEARNED;
     const bool tracing = opt && opt->record_trace && opt->trace && opt->trace_cap > 0;
-    if (!learned && !tracing) return GHB_OK;
+    const double share = sssp_default_share(n, light_m);
+    if (!learned && !tracing) {
+        *delta *= share;
+        return GHB_OK;
+    }
     cudaStream_t st = ws->stream;
     int32_t* hp = reinterpret_cast<int32_t*>(ws->host_pinned);
     GHB_CUDA_TRY(cudaMemcpyAsync(hp, rowptr + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
@@ -413,6 +435,7 @@ int sssp_choose_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const
             by_net = true;
         }
     }
+    if (!by_net) *delta *= share;
     if (tracing) {
         float* row = opt->trace;
         for (int k = 0; k < GHB_TRACE_COLS; ++k) row[k] = -1.f;
@@ -435,7 +458,7 @@ int sssp_run(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int32_t*
     if (!opt) opt = &defaults;
     cudaStream_t st = ws->stream;
     double delta = 0.0;
-    GHB_TRY(sssp_choose_delta(ws, n, rowptr, w, src, opt, &delta));
+    GHB_TRY(sssp_choose_delta(ws, n, rowptr, w, src, opt, 0, &delta));
     int blocks = 0;
     if (ws->tune.sssp_persistent && sssp_persistent_available(ws, &blocks))
         return sssp_persistent_run(ws, n, rowptr, nullptr, col, w, src, inf, delta, dist_out, nullptr, nullptr,
