@@ -297,7 +297,7 @@ int ghb_bfs(ghb_workspace* ws, int32_t n, const int32_t* out_rowptr, const int32
         GHB_REQUIRE(src >= 0 && src < n, "source outside [0, n)");
         GHB_REQUIRE(max_depth >= 0, "max_depth < 0");
         const bool can_pull = in_rowptr != nullptr && in_col != nullptr;
-        return bfs_persistent_run(ws, n, n, out_rowptr, out_col, can_pull ? in_rowptr : nullptr,
+        return bfs_persistent_run(ws, n, n, -1, out_rowptr, out_col, can_pull ? in_rowptr : nullptr,
                                   can_pull ? in_col : nullptr, src, max_depth, depth, nullptr, nullptr, options, stats);
     }
     return bfs_run(ws, n, n, out_rowptr, out_col, in_rowptr, in_col, src, max_depth, depth, options,

@@ -127,8 +127,10 @@ __global__ void bfs_push_persistent_kernel(const int32_t* __restrict__ rowptr, c
 __global__ void bfs_bitmap_from_queue_kernel(const int32_t* __restrict__ q, int32_t count, uint32_t* f);
 
 bool bfs_use_persistent(ghb_workspace* ws, const ghb_bfs_options* opt);
-int bfs_persistent_run(ghb_workspace* ws, int32_t n, int32_t n_active, const int32_t* out_rp, const int32_t* out_col,
-                       const int32_t* in_rp, const int32_t* in_col, int32_t src, int32_t max_depth, int32_t* depth,
+// m: entries, or -1 to read them from out_rp (one wait).  With perm, src is
+// the caller's id and depth_out is written in the caller's ids.
+int bfs_persistent_run(ghb_workspace* ws, int32_t n, int32_t n_active, int64_t m, const int32_t* out_rp,
+                       const int32_t* out_col, const int32_t* in_rp, const int32_t* in_col, int32_t src, int32_t max_depth, int32_t* depth,
                        const int32_t* perm, int32_t* depth_out, const ghb_bfs_options* opt,
                        ghb_traversal_stats* stats);
 

@@ -20,6 +20,7 @@
 // Every grid barrier is bounded (grid_barrier): on timeout all blocks leave
 // and the host reports GHB_ERR_TIMEOUT.
 #include <algorithm>
+#include <cstring>
 #include <vector>
 
 #include "bfs_kernels.cuh"
@@ -546,6 +547,7 @@ __global__ void __launch_bounds__(512, 2) bfs_persistent_kernel(
     const int64_t words_active = ((int64_t)n_active + 31) / 32;
 
     // ---- init
+    if (perm) src = perm[src];
     for (int64_t v = gtid; v < n; v += gsize) depth[v] = (v == src) ? 0 : kInfDepth;
     for (int64_t w = gtid; w < words; w += gsize) {
         const uint32_t bit = (w == (src >> 5)) ? (1u << (src & 31)) : 0u;
@@ -1131,9 +1133,11 @@ bool bfs_persistent_available(ghb_workspace* ws, int* blocks) {
 }
 
 // One cooperative launch for the whole traversal.  depth: per-vertex output
-// in the graph's ids; with perm, depth_out[v] = depth[perm[v]] as well.
-int bfs_persistent_run(ghb_workspace* ws, int32_t n, int32_t n_active, const int32_t* out_rp, const int32_t* out_col,
-                       const int32_t* in_rp, const int32_t* in_col, int32_t src, int32_t max_depth, int32_t* depth,
+// in the graph's ids; with perm, src is the caller's id and
+// depth_out[v] = depth[perm[v]] as well.  m: the entries where the caller
+// knows them (a resident graph: no wait before the launch), else -1.
+int bfs_persistent_run(ghb_workspace* ws, int32_t n, int32_t n_active, int64_t m, const int32_t* out_rp,
+                       const int32_t* out_col, const int32_t* in_rp, const int32_t* in_col, int32_t src, int32_t max_depth, int32_t* depth,
                        const int32_t* perm, int32_t* depth_out, const ghb_bfs_options* opt,
                        ghb_traversal_stats* stats) {
     int blocks = 0;
@@ -1186,17 +1190,19 @@ int bfs_persistent_run(ghb_workspace* ws, int32_t n, int32_t n_active, const int
         pol = policy_device_params();
         if (!pol) policy = GHB_POLICY_HEURISTIC;
     }
-    int32_t* hp = reinterpret_cast<int32_t*>(ws->host_pinned);
-    GHB_CUDA_TRY(cudaMemcpyAsync(hp, out_rp + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    GHB_CUDA_TRY(cudaMemsetAsync(rs, 0, sizeof(BfsRunState), st));
-    {
-        // Barrier limit and test knob (pageable source: staged by the call).
-        const unsigned long long bar[2] = {(unsigned long long)ws->tune.barrier_limit_us * 1000ull,
-                                           (unsigned long long)ws->tune.barrier_extra};
-        GHB_CUDA_TRY(cudaMemcpyAsync(&rs->bar_limit_ns, bar, sizeof(bar), cudaMemcpyHostToDevice, st));
+    int64_t m_total = m;
+    if (m < 0) {
+        int32_t* hp = reinterpret_cast<int32_t*>(ws->host_pinned);
+        GHB_CUDA_TRY(cudaMemcpyAsync(hp, out_rp + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        GHB_CUDA_TRY(cudaStreamSynchronize(st));
+        m_total = hp[0];
     }
-    GHB_CUDA_TRY(cudaStreamSynchronize(st));
-    const int64_t m_total = hp[0];
+    // The start state (pageable source: staged by the call).
+    BfsRunState h0;
+    std::memset(static_cast<void*>(&h0), 0, sizeof(h0));
+    h0.bar_limit_ns = (unsigned long long)ws->tune.barrier_limit_us * 1000ull;
+    h0.bar_extra = (unsigned)ws->tune.barrier_extra;
+    GHB_CUDA_TRY(cudaMemcpyAsync(rs, &h0, sizeof(h0), cudaMemcpyHostToDevice, st));
     if (stats) GHB_CUDA_TRY(cudaEventRecord(ws->ev_start, st));
     // Meshes, road networks, paths: up to 4.5 entries per vertex.  (A random
     // graph with six has ten levels, and the larger kernel cost it 5 %.)

@@ -264,6 +264,14 @@ int map_back_i32(ghb_workspace* ws, const ghb_graph* g, const int32_t* src_new, 
     return launch(ws, map_back_kernel<int32_t>, dim3(grid_for(g->n, 256, ws->num_sms * 8)), dim3(256), 0, g->n,
                   (const int32_t*)g->perm, src_new, dst_old);
 }
+int map_source(ghb_workspace* ws, const ghb_graph* g, int32_t src, int32_t* src_new) {
+    int32_t* hp = reinterpret_cast<int32_t*>(ws->host_pinned);
+    GHB_CUDA_TRY(cudaMemcpyAsync(hp, g->perm + src, sizeof(int32_t), cudaMemcpyDeviceToHost, ws->stream));
+    GHB_CUDA_TRY(cudaStreamSynchronize(ws->stream));
+    *src_new = hp[0];
+    return GHB_OK;
+}
+
 int map_back_f64(ghb_workspace* ws, const ghb_graph* g, const double* src_new, double* dst_old) {
     return launch(ws, map_back_kernel<double>, dim3(grid_for(g->n, 256, ws->num_sms * 8)), dim3(256), 0, g->n,
                   (const int32_t*)g->perm, src_new, dst_old);
@@ -385,10 +393,6 @@ int ghb_graph_create(ghb_workspace* ws, int32_t n, const int32_t* out_rowptr, co
         GG_TRY(ghb_csr_merge_in_out(ws, n, g->in_rowptr, g->in_col, g->rowptr, g->col, g->all_rowptr, g->all_col));
     GG_TRY(cudaMemcpyAsync(hp + 2, repeat, sizeof(int32_t), cudaMemcpyDeviceToHost, st) == cudaSuccess ? GHB_OK
                                                                                                      : GHB_ERR_CUDA);
-    g->perm_host.resize(n);
-    GG_TRY(cudaMemcpyAsync(g->perm_host.data(), g->perm, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st) == cudaSuccess
-               ? GHB_OK
-               : GHB_ERR_CUDA);
 #undef GG_TRY
     GHB_CUDA_TRY(cudaEventRecord(ws->ev_b, st));
     GHB_CUDA_TRY(cudaEventSynchronize(ws->ev_b));

@@ -30,7 +30,6 @@ struct ghb_graph {
     int32_t* all_rowptr = nullptr;  // CDLP rows (in then out); == rowptr when undirected
     int32_t* all_col = nullptr;
     int32_t* outdeg = nullptr;       // out-degree per new id
-    std::vector<int32_t> perm_host;  // host copy of perm (maps sources without a round trip)
     // Rows of the out-CSR sorted by weight instead of by column (built on the
     // first SSSP call; same rowptr), for delta-stepping's light/heavy split.
     int32_t* sw_col = nullptr;
@@ -56,6 +55,9 @@ int rank_by_degree(ghb_workspace* ws, int32_t n, const int32_t* out_rp, const in
                    int32_t* iperm, int32_t** n_active);
 int relabel_csr(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* rp, const int32_t* col, const double* w,
                 const int32_t* perm, int32_t* rp_out, int32_t* col_out, double* w_out, int32_t* repeat);
+
+// One vertex in the graph's ids (waits for the stream; src_new may be &src).
+int map_source(ghb_workspace* ws, const ghb_graph* g, int32_t src, int32_t* src_new);
 
 // Result mapping kernels (new-id array -> caller's ids).
 int map_back_i32(ghb_workspace* ws, const ghb_graph* g, const int32_t* src_new, int32_t* dst_old);

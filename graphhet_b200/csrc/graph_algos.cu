@@ -19,20 +19,25 @@ int sssp_pred_run(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int
                   const int32_t* in_rp, const int32_t* in_col, const double* in_w, int32_t src, double inf,
                   const double* dist, int32_t* pred);
 int sssp_delta_run(ghb_workspace* ws, ghb_graph* g, int32_t src, double inf, double delta, double* dist_out,
-                   ghb_traversal_stats* stats);
+                   double* out, ghb_traversal_stats* stats);
 int sssp_choose_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const double* w, int32_t src,
-                      const ghb_sssp_options* opt, int64_t light_m, double* delta);
+                      const int32_t* perm, const ghb_sssp_options* opt, int64_t light_m, double* delta,
+                      int64_t* entries);
 
 // Resident SSSP: delta-stepping with the light/heavy split when the rows fit
-// the weight-sorted copy's key (n <= 2^25), else the near/far form.
-static int graph_sssp_dispatch(ghb_workspace* ws, const ghb_graph* g, int32_t src_new, double inf, double* dnew,
-                               const ghb_sssp_options* options, ghb_traversal_stats* stats) {
+// the weight-sorted copy's key (n <= 2^25), else the near/far form.  Distances
+// in the graph's ids (dnew) and in the caller's (dist), as src.
+static int graph_sssp_dispatch(ghb_workspace* ws, const ghb_graph* g, int32_t src, double inf, double* dnew,
+                               double* dist, const ghb_sssp_options* options, ghb_traversal_stats* stats) {
     if (g->m > 0 && g->n <= (1 << 25)) {
         double delta = 0.0;
-        GHB_TRY(sssp_choose_delta(ws, g->n, g->rowptr, g->w, src_new, options, g->m, &delta));
-        return sssp_delta_run(ws, const_cast<ghb_graph*>(g), src_new, inf, delta, dnew, stats);
+        int64_t entries = 0;
+        GHB_TRY(sssp_choose_delta(ws, g->n, g->rowptr, g->w, src, g->perm, options, g->m, &delta, &entries));
+        return sssp_delta_run(ws, const_cast<ghb_graph*>(g), src, inf, delta, dnew, dist, stats);
     }
-    return sssp_run(ws, g->n, g->rowptr, g->col, g->w, src_new, inf, dnew, options, stats);
+    GHB_TRY(map_source(ws, g, src, &src));
+    GHB_TRY(sssp_run(ws, g->n, g->rowptr, g->col, g->w, src, inf, dnew, options, stats));
+    return map_back_f64(ws, g, dnew, dist);
 }
 int wcc_run(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int32_t* col, int32_t* label);
 int wcc_afforest_run(ghb_workspace* ws, int32_t n, int32_t n_active, const int32_t* rowptr, const int32_t* col,
@@ -46,8 +51,8 @@ int tc_run(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int32_t* c
            int32_t* counts32, int64_t* total);
 int tc_run_cached(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int32_t* col, int64_t* counts64,
                   int32_t* counts32, int64_t* total, std::atomic<int32_t>* flags_cache, bool ranked);
-int pagerank_run(ghb_workspace* ws, int32_t n, const int32_t* in_rp, const int32_t* in_col, const int32_t* out_rp,
-                 const ghb_pr_options* o, double* rank, int32_t* iters_run);
+int pagerank_run(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* in_rp, const int32_t* in_col,
+                 const int32_t* out_rp, const ghb_pr_options* o, double* rank, int32_t* iters_run);
 int msbfs_batch(ghb_workspace* ws, int32_t n, int32_t n_active, const int32_t* out_rp, const int32_t* out_col,
                 const int32_t* in_rp, const int32_t* in_col, const int32_t* srcs_dev, int32_t k,
                 const int32_t* perm, int32_t* depth, int64_t* levels_out, int64_t* examined_out);
@@ -97,6 +102,11 @@ __global__ void comp_map_kernel(int32_t n, const int32_t* __restrict__ perm, con
         out[v] = cmin[label_new[perm[v]]];
 }
 
+__global__ void source_map_kernel(int32_t k, const int32_t* __restrict__ srcs, const int32_t* __restrict__ perm,
+                                  int32_t* out) {
+    for (int32_t i = threadIdx.x; i < k; i += blockDim.x) out[i] = perm[srcs[i]];
+}
+
 // pred_new holds new ids: map the row and the value.
 __global__ void pred_map_kernel(int32_t n, const int32_t* __restrict__ perm, const int32_t* __restrict__ iperm,
                                 const int32_t* __restrict__ pred_new, int32_t* out) {
@@ -138,10 +148,11 @@ int ghb_graph_bfs(ghb_workspace* ws, const ghb_graph* g, int32_t src, int32_t ma
     GHB_TRY(ws_reserve_stage(ws, sizeof(int32_t) * (size_t)g->n));
     int32_t* dnew = static_cast<int32_t*>(ws->stage);
     if (bfs_use_persistent(ws, options))
-        return bfs_persistent_run(ws, g->n, g->n_active, g->rowptr, g->col, g->in_rowptr, g->in_col,
-                                  g->perm_host[src], max_depth, dnew, g->perm, depth, options, stats);
-    GHB_TRY(bfs_run(ws, g->n, g->n_active, g->rowptr, g->col, g->in_rowptr, g->in_col, g->perm_host[src], max_depth,
-                    dnew, options, stats));
+        return bfs_persistent_run(ws, g->n, g->n_active, g->m, g->rowptr, g->col, g->in_rowptr, g->in_col, src,
+                                  max_depth, dnew, g->perm, depth, options, stats);
+    GHB_TRY(map_source(ws, g, src, &src));
+    GHB_TRY(bfs_run(ws, g->n, g->n_active, g->rowptr, g->col, g->in_rowptr, g->in_col, src, max_depth, dnew, options,
+                    stats));
     return map_back_i32(ws, g, dnew, depth);
 }
 
@@ -153,8 +164,9 @@ int ghb_graph_bfs_pred(ghb_workspace* ws, const ghb_graph* g, int32_t src, int32
     GHB_TRY(ws_reserve_stage(ws, 2 * sizeof(int32_t) * (size_t)g->n + 256));
     int32_t* dnew = static_cast<int32_t*>(ws->stage);
     int32_t* pnew = dnew + (((size_t)g->n + 63) & ~(size_t)63);
-    GHB_TRY(ghb_bfs_pred(ws, g->n, g->rowptr, g->col, g->in_rowptr, g->in_col, g->perm_host[src], max_depth, dnew,
-                         pnew, options, stats));
+    GHB_TRY(map_source(ws, g, src, &src));
+    GHB_TRY(ghb_bfs_pred(ws, g->n, g->rowptr, g->col, g->in_rowptr, g->in_col, src, max_depth, dnew, pnew, options,
+                         stats));
     GHB_TRY(map_back_i32(ws, g, dnew, depth));
     return launch(ws, pred_map_kernel, dim3(grid_for(g->n, 256, ws->num_sms * 8)), dim3(256), 0, g->n,
                   (const int32_t*)g->perm, (const int32_t*)g->iperm, (const int32_t*)pnew, pred);
@@ -170,10 +182,7 @@ int ghb_graph_msbfs(ghb_workspace* ws, const ghb_graph* g, const int32_t* srcs, 
         GHB_CUDA_TRY(cudaMemcpyAsync(hs.data(), srcs, sizeof(int32_t) * n_src, cudaMemcpyDeviceToHost, st));
         GHB_CUDA_TRY(cudaStreamSynchronize(st));
     }
-    for (int32_t i = 0; i < n_src; ++i) {
-        GHB_REQUIRE(hs[i] >= 0 && hs[i] < g->n, "source outside [0, n)");
-        hs[i] = g->perm_host[hs[i]];
-    }
+    for (int32_t i = 0; i < n_src; ++i) GHB_REQUIRE(hs[i] >= 0 && hs[i] < g->n, "source outside [0, n)");
     if (n_src > 0 && msbfs_persistent_available(ws, n_src)) {
         // One cooperative launch per pass; the kernel maps the caller's
         // sources and writes depths in the caller's ids through perm.
@@ -203,11 +212,11 @@ int ghb_graph_msbfs(ghb_workspace* ws, const ghb_graph* g, const int32_t* srcs, 
     int64_t levels = 0, examined = 0;
     for (int32_t s0 = 0; s0 < n_src; s0 += kMsPass) {
         const int32_t k = std::min<int32_t>(kMsPass, n_src - s0);
-        GHB_CUDA_TRY(cudaMemcpyAsync(snew, hs.data() + s0, sizeof(int32_t) * k, cudaMemcpyHostToDevice, st));
+        GHB_TRY(launch(ws, source_map_kernel, dim3(1), dim3(256), 0, k, srcs + s0, (const int32_t*)g->perm, snew));
         GHB_TRY(msbfs_batch(ws, g->n, g->n_active, g->rowptr, g->col, g->in_rowptr, g->in_col, snew, k,
                             (const int32_t*)g->perm, depth + (int64_t)s0 * g->n, &levels, &examined));
     }
-    GHB_CUDA_TRY(cudaStreamSynchronize(st));  // hs (host) is read by the copies above
+    GHB_CUDA_TRY(cudaStreamSynchronize(st));
     if (stats) {
         GHB_CUDA_TRY(cudaEventRecord(ws->ev_stop, st));
         GHB_CUDA_TRY(cudaEventSynchronize(ws->ev_stop));
@@ -294,10 +303,7 @@ int ghb_graph_mssssp(ghb_workspace* ws, const ghb_graph* g, const int32_t* srcs,
         GHB_CUDA_TRY(cudaMemcpyAsync(hs.data(), srcs, sizeof(int32_t) * n_src, cudaMemcpyDeviceToHost, st));
         GHB_CUDA_TRY(cudaStreamSynchronize(st));
     }
-    for (int32_t i = 0; i < n_src; ++i) {
-        GHB_REQUIRE(hs[i] >= 0 && hs[i] < g->n, "source outside [0, n)");
-        hs[i] = g->perm_host[hs[i]];
-    }
+    for (int32_t i = 0; i < n_src; ++i) GHB_REQUIRE(hs[i] >= 0 && hs[i] < g->n, "source outside [0, n)");
     if (n_src == 0) return GHB_OK;
     return mssssp_run(ws, g->n, g->n_active, g->rowptr, g->col, g->w, hs.data(), n_src, 0.0, inf,
                       (const int32_t*)g->perm, dist, stats);
@@ -311,8 +317,7 @@ int ghb_graph_sssp(ghb_workspace* ws, const ghb_graph* g, int32_t src, double in
     GHB_REQUIRE(src >= 0 && src < g->n, "source outside [0, n)");
     GHB_TRY(ws_reserve_stage(ws, sizeof(double) * (size_t)g->n));
     double* dnew = static_cast<double*>(ws->stage);
-    GHB_TRY(graph_sssp_dispatch(ws, g, g->perm_host[src], inf, dnew, options, stats));
-    return map_back_f64(ws, g, dnew, dist);
+    return graph_sssp_dispatch(ws, g, src, inf, dnew, dist, options, stats);
 }
 
 int ghb_graph_sssp_pred(ghb_workspace* ws, const ghb_graph* g, int32_t src, double inf, double* dist, int32_t* pred,
@@ -324,10 +329,9 @@ int ghb_graph_sssp_pred(ghb_workspace* ws, const ghb_graph* g, int32_t src, doub
     GHB_TRY(ws_reserve_stage(ws, (sizeof(double) + sizeof(int32_t)) * (size_t)g->n + 512));
     double* dnew = static_cast<double*>(ws->stage);
     int32_t* pnew = reinterpret_cast<int32_t*>(dnew + (((size_t)g->n + 63) & ~(size_t)63));
-    GHB_TRY(graph_sssp_dispatch(ws, g, g->perm_host[src], inf, dnew, options, stats));
-    GHB_TRY(sssp_pred_run(ws, g->n, g->rowptr, g->col, g->w, g->in_rowptr, g->in_col, g->in_w, g->perm_host[src], inf,
-                          dnew, pnew));
-    GHB_TRY(map_back_f64(ws, g, dnew, dist));
+    GHB_TRY(graph_sssp_dispatch(ws, g, src, inf, dnew, dist, options, stats));
+    GHB_TRY(map_source(ws, g, src, &src));
+    GHB_TRY(sssp_pred_run(ws, g->n, g->rowptr, g->col, g->w, g->in_rowptr, g->in_col, g->in_w, src, inf, dnew, pnew));
     return launch(ws, pred_map_kernel, dim3(grid_for(g->n, 256, ws->num_sms * 8)), dim3(256), 0, g->n,
                   (const int32_t*)g->perm, (const int32_t*)g->iperm, (const int32_t*)pnew, pred);
 }
@@ -357,7 +361,7 @@ int ghb_graph_pagerank(ghb_workspace* ws, const ghb_graph* g, const ghb_pr_optio
     GHB_REQUIRE(options->precision == GHB_PR_FP64 || options->precision == GHB_PR_FP32_KAHAN, "bad precision");
     GHB_TRY(ws_reserve_stage(ws, sizeof(double) * (size_t)g->n));
     double* rnew = static_cast<double*>(ws->stage);
-    GHB_TRY(pagerank_run(ws, g->n, g->in_rowptr, g->in_col, g->rowptr, options, rnew, iterations_run));
+    GHB_TRY(pagerank_run(ws, g->n, g->m_in, g->in_rowptr, g->in_col, g->rowptr, options, rnew, iterations_run));
     return map_back_f64(ws, g, rnew, rank);
 }
 

@@ -543,7 +543,16 @@ __global__ void __launch_bounds__(256) mssp_out_kernel(int32_t n, int32_t k, int
 // Bucket width of a pass: the caller's, else mean weight x 32 / mean degree
 // (the single-source rule) times 4 (a pass has 256 sources' work per bucket,
 // so fewer, fuller buckets pay).
-int sssp_pick_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const double* w, double* delta);
+int sssp_pick_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const double* w, double* delta,
+                    int64_t* entries);
+
+namespace {
+
+__global__ void mssp_sources_kernel(int32_t k, const int32_t* __restrict__ perm, int32_t* srcs) {
+    for (int i = threadIdx.x; i < k; i += blockDim.x) srcs[i] = perm[srcs[i]];
+}
+
+}  // namespace
 
 static int mssp_pass_blocks(ghb_workspace* ws) {
     static int cached[64] = {0};
@@ -753,21 +762,23 @@ int mssssp_pass(ghb_workspace* ws, int32_t n, int32_t n_active, const int32_t* r
     return GHB_OK;
 }
 
+// Sources and output in the caller's ids, which perm (may be NULL) maps to
+// the graph's.
 int mssssp_run(ghb_workspace* ws, int32_t n, int32_t n_active, const int32_t* rp, const int32_t* col,
                const double* wt, const int32_t* srcs_host, int32_t n_src, double delta, double inf,
                const int32_t* perm, double* dist, ghb_traversal_stats* stats) {
     cudaStream_t st = ws->stream;
+    int64_t m = -1;
     if (!(delta > 0)) {
-        GHB_TRY(sssp_pick_delta(ws, n, rp, wt, &delta));
+        GHB_TRY(sssp_pick_delta(ws, n, rp, wt, &delta, &m));
         delta = std::ldexp(delta, ws->tune.mssp_width_log2);
     }
     GHB_TRY(ws_reserve_stage(ws, sizeof(int32_t) * 256));
     int32_t* sdev = static_cast<int32_t*>(ws->stage);
     if (stats) GHB_CUDA_TRY(cudaEventRecord(ws->ev_start, st));
     int64_t rounds = 0, examined = 0;
-    int64_t m = 0;
     const bool one_launch = ws->tune.mssp_persistent && mssp_pass_blocks(ws) > 0;
-    if (one_launch) {
+    if (one_launch && m < 0) {
         int32_t* hp = reinterpret_cast<int32_t*>(ws->host_pinned);
         GHB_CUDA_TRY(cudaMemcpyAsync(hp, rp + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
         GHB_CUDA_TRY(cudaStreamSynchronize(st));
@@ -776,6 +787,7 @@ int mssssp_run(ghb_workspace* ws, int32_t n, int32_t n_active, const int32_t* rp
     for (int32_t s0 = 0; s0 < n_src; s0 += 256) {
         const int32_t k = std::min<int32_t>(256, n_src - s0);
         GHB_CUDA_TRY(cudaMemcpyAsync(sdev, srcs_host + s0, sizeof(int32_t) * k, cudaMemcpyHostToDevice, st));
+        if (perm) GHB_TRY(launch(ws, mssp_sources_kernel, dim3(1), dim3(256), 0, k, perm, sdev));
         if (one_launch)
             GHB_TRY(mssssp_pass_one_launch(ws, n, n_active, m, rp, col, wt, sdev, k, delta, inf, perm,
                                            dist + (int64_t)s0 * n, &rounds, &examined));

@@ -485,7 +485,7 @@ __global__ void pr_to_f64_kernel(const T* src, double* dst, int32_t n) {
 }
 
 template <class T>
-int pagerank_impl(ghb_workspace* ws, int32_t n, const int32_t* in_rp, const int32_t* in_col,
+int pagerank_impl(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* in_rp, const int32_t* in_col,
                   const int32_t* out_rp, const ghb_pr_options* o, double* rank_out, int32_t* iters_run, bool ranked) {
     cudaStream_t st = ws->stream;
     const Tuning& tu = ws->tune;
@@ -504,9 +504,11 @@ int pagerank_impl(ghb_workspace* ws, int32_t n, const int32_t* in_rp, const int3
     const int32_t cache_elems = (int32_t)(cache_bytes / sizeof(T));
     const size_t smem = (size_t)((cache_elems + 3) & ~3) * sizeof(T) + tile_bytes;
     int32_t* hp = reinterpret_cast<int32_t*>(ws->host_pinned);
-    GHB_CUDA_TRY(cudaMemcpyAsync(hp, in_rp + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    GHB_CUDA_TRY(cudaStreamSynchronize(st));
-    const int64_t m = hp[0];
+    if (m < 0) {
+        GHB_CUDA_TRY(cudaMemcpyAsync(hp, in_rp + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        GHB_CUDA_TRY(cudaStreamSynchronize(st));
+        m = hp[0];
+    }
     const int32_t tiles = (int32_t)((m + kPrTile - 1) / kPrTile);
     const unsigned grid_rows = tiles ? grid_for((int64_t)tiles * 32, pthreads, max_rows) : 0;
     const unsigned grid_fin = grid_for(std::max<int64_t>(tiles, n / 8), kPrThreads, ws->num_sms * 8);
@@ -601,10 +603,11 @@ int pagerank_impl(ghb_workspace* ws, int32_t n, const int32_t* in_rp, const int3
 
 }  // namespace
 
-int pagerank_run(ghb_workspace* ws, int32_t n, const int32_t* in_rp, const int32_t* in_col, const int32_t* out_rp,
-                 const ghb_pr_options* o, double* rank, int32_t* iters_run) {
-    if (o->precision == GHB_PR_FP64) return pagerank_impl<double>(ws, n, in_rp, in_col, out_rp, o, rank, iters_run, true);
-    return pagerank_impl<float>(ws, n, in_rp, in_col, out_rp, o, rank, iters_run, true);
+int pagerank_run(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* in_rp, const int32_t* in_col,
+                 const int32_t* out_rp, const ghb_pr_options* o, double* rank, int32_t* iters_run) {
+    if (o->precision == GHB_PR_FP64)
+        return pagerank_impl<double>(ws, n, m, in_rp, in_col, out_rp, o, rank, iters_run, true);
+    return pagerank_impl<float>(ws, n, m, in_rp, in_col, out_rp, o, rank, iters_run, true);
 }
 
 }  // namespace ghb
@@ -622,6 +625,6 @@ extern "C" int ghb_pagerank(ghb_workspace* ws, int32_t n, const int32_t* in_rowp
     GHB_REQUIRE(options->precision == GHB_PR_FP64 || options->precision == GHB_PR_FP32_KAHAN,
                 "bad precision");
     if (options->precision == GHB_PR_FP64)
-        return pagerank_impl<double>(ws, n, in_rowptr, in_col, out_rowptr, options, rank, iterations_run, false);
-    return pagerank_impl<float>(ws, n, in_rowptr, in_col, out_rowptr, options, rank, iterations_run, false);
+        return pagerank_impl<double>(ws, n, -1, in_rowptr, in_col, out_rowptr, options, rank, iterations_run, false);
+    return pagerank_impl<float>(ws, n, -1, in_rowptr, in_col, out_rowptr, options, rank, iterations_run, false);
 }

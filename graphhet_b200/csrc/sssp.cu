@@ -32,8 +32,8 @@ namespace ghb {
 
 bool sssp_persistent_available(ghb_workspace* ws, int* blocks);
 int sssp_persistent_run(ghb_workspace* ws, int32_t n, const int32_t* rp, const int32_t* le, const int32_t* col,
-                        const double* wt, int32_t src, double inf, double delta, double* dist, const int32_t* perm,
-                        double* out, ghb_traversal_stats* stats);
+                        const double* wt, int64_t m, int32_t src, double inf, double delta, double* dist,
+                        const int32_t* perm, double* out, ghb_traversal_stats* stats);
 int graph_light_ends(ghb_workspace* ws, ghb_graph* g, double delta, const int32_t** le);
 
 namespace {
@@ -134,9 +134,15 @@ __global__ void sssp_split_kernel(const int32_t* __restrict__ far, int32_t far_c
         atomicMin(reinterpret_cast<unsigned long long*>(min_far), (unsigned long long)__double_as_longlong(mn));
 }
 
-__global__ void mean_weight_kernel(const double* __restrict__ w, int64_t m, int64_t stride, double* out) {
+// About a million of the weights: out[0] their sum, out[1] their number,
+// out[2] the entries.
+__global__ void mean_weight_kernel(int32_t n, const int32_t* __restrict__ rowptr, const double* __restrict__ w,
+                                   double* out) {
+    const int64_t m = rowptr[n];
+    const int64_t stride = m >= (1 << 20) ? m / (1 << 20) : 1;
     double s = 0.0;
     int64_t c = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) out[2] = (double)m;
     for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * stride; i < m;
          i += (int64_t)gridDim.x * blockDim.x * stride) {
         s += w[i];
@@ -333,23 +339,22 @@ __global__ void fill_i32(int32_t* p, int64_t count, int32_t value) {
 // weight times 32 over the mean degree (wider buckets on sparse graphs,
 // where rounds are latency-bound).  The policy network's bins and the
 // multi-source pass scale this width.
-int sssp_pick_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const double* w, double* delta) {
+// *entries: the rows' entries.
+int sssp_pick_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const double* w, double* delta,
+                    int64_t* entries) {
     cudaStream_t st = ws->stream;
-    int32_t* hp = reinterpret_cast<int32_t*>(ws->host_pinned);
-    GHB_CUDA_TRY(cudaMemcpyAsync(hp, rowptr + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    double* acc = reinterpret_cast<double*>(ws->dev_small);
+    GHB_CUDA_TRY(cudaMemsetAsync(acc, 0, 3 * sizeof(double), st));
+    GHB_TRY(launch(ws, mean_weight_kernel, dim3(64), dim3(256), 0, n, rowptr, w, acc));
+    GHB_CUDA_TRY(cudaMemcpyAsync(ws->host_pinned, acc, 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
     GHB_CUDA_TRY(cudaStreamSynchronize(st));
-    const int64_t m = hp[0];
+    const double* h = reinterpret_cast<const double*>(ws->host_pinned);
+    const int64_t m = (int64_t)h[2];
+    *entries = m;
     if (m == 0) {
         *delta = 1.0;
         return GHB_OK;
     }
-    double* acc = reinterpret_cast<double*>(ws->dev_small);
-    GHB_CUDA_TRY(cudaMemsetAsync(acc, 0, 2 * sizeof(double), st));
-    const int64_t stride = std::max<int64_t>(1, m / (1 << 20));
-    GHB_TRY(launch(ws, mean_weight_kernel, dim3(64), dim3(256), 0, w, m, stride, acc));
-    GHB_CUDA_TRY(cudaMemcpyAsync(ws->host_pinned, acc, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
-    GHB_CUDA_TRY(cudaStreamSynchronize(st));
-    const double* h = reinterpret_cast<const double*>(ws->host_pinned);
     const double mean_w = h[1] > 0 ? h[0] / h[1] : 1.0;
     const double mean_d = (double)m / (double)n;
     double d = mean_w * 32.0 / std::max(1.0, mean_d);
@@ -380,13 +385,17 @@ static double sssp_default_share(int32_t n, int64_t light_m) {
 // record_trace, trace row 0 gets the features, then 12 the width used, 13
 // -1, 14 the weight rule's width, 15 1 when the network chose it; the
 // caller's driver fills 13 (device ms).
+// src is the caller's id where perm is given.  *entries: the rows' entries,
+// -1 when they were not read.
 int sssp_choose_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const double* w, int32_t src,
-                      const ghb_sssp_options* opt, int64_t light_m, double* delta) {
+                      const int32_t* perm, const ghb_sssp_options* opt, int64_t light_m, double* delta,
+                      int64_t* entries) {
+    *entries = -1;
     if (opt && opt->delta > 0) {
         *delta = opt->delta;
         return GHB_OK;
     }
-    GHB_TRY(sssp_pick_delta(ws, n, rowptr, w, delta));
+    GHB_TRY(sssp_pick_delta(ws, n, rowptr, w, delta, entries));
     const bool learned = opt && opt->policy == GHB_POLICY_LEARNED;
     const bool tracing = opt && opt->record_trace && opt->trace && opt->trace_cap > 0;
     const double share = sssp_default_share(n, light_m);
@@ -396,10 +405,14 @@ int sssp_choose_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const
     }
     cudaStream_t st = ws->stream;
     int32_t* hp = reinterpret_cast<int32_t*>(ws->host_pinned);
-    GHB_CUDA_TRY(cudaMemcpyAsync(hp, rowptr + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    if (perm) {
+        GHB_CUDA_TRY(cudaMemcpyAsync(hp, perm + src, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        GHB_CUDA_TRY(cudaStreamSynchronize(st));
+        src = hp[0];
+    }
     GHB_CUDA_TRY(cudaMemcpyAsync(hp + 1, rowptr + src, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     GHB_CUDA_TRY(cudaStreamSynchronize(st));
-    const int64_t m = hp[0];
+    const int64_t m = *entries;
     const double deg_src = (double)(hp[2] - hp[1]);
     double* acc = reinterpret_cast<double*>(ws->dev_small);
     double init[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -458,10 +471,11 @@ int sssp_run(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int32_t*
     if (!opt) opt = &defaults;
     cudaStream_t st = ws->stream;
     double delta = 0.0;
-    GHB_TRY(sssp_choose_delta(ws, n, rowptr, w, src, opt, 0, &delta));
+    int64_t m = -1;
+    GHB_TRY(sssp_choose_delta(ws, n, rowptr, w, src, nullptr, opt, 0, &delta, &m));
     int blocks = 0;
     if (ws->tune.sssp_persistent && sssp_persistent_available(ws, &blocks))
-        return sssp_persistent_run(ws, n, rowptr, nullptr, col, w, src, inf, delta, dist_out, nullptr, nullptr,
+        return sssp_persistent_run(ws, n, rowptr, nullptr, col, w, m, src, inf, delta, dist_out, nullptr, nullptr,
                                    stats);
 
     Carver sizing(nullptr);
@@ -615,8 +629,9 @@ int graph_weight_sorted(ghb_workspace* ws, ghb_graph* g) {
 // light entries (w < delta) of its near queue; once the bucket is empty the
 // heavy entries of every vertex it settled are relaxed once.  Rows are read
 // from the weight-sorted copy, so a light pass reads only a row prefix.
+// src is the caller's id; dist_out is in the graph's ids, out in the caller's.
 int sssp_delta_run(ghb_workspace* ws, ghb_graph* g, int32_t src, double inf, double delta, double* dist_out,
-                   ghb_traversal_stats* stats) {
+                   double* out, ghb_traversal_stats* stats) {
     const int32_t n = g->n;
     cudaStream_t st = ws->stream;
     GHB_TRY(graph_weight_sorted(ws, g));
@@ -633,10 +648,11 @@ int sssp_delta_run(ghb_workspace* ws, ghb_graph* g, int32_t src, double inf, dou
         if (ws->tune.sssp_persistent && sssp_persistent_available(ws, &blocks)) {
             const int32_t* le = nullptr;
             GHB_TRY(graph_light_ends(ws, g, delta, &le));
-            return sssp_persistent_run(ws, n, g->rowptr, le, g->sw_col, g->sw_w, src, inf, delta, dist_out, nullptr,
-                                       nullptr, stats);
+            return sssp_persistent_run(ws, n, g->rowptr, le, g->sw_col, g->sw_w, g->m, src, inf, delta, dist_out,
+                                       g->perm, out, stats);
         }
     }
+    GHB_TRY(map_source(ws, g, src, &src));
     auto carve = [&](Carver& c, WalkBuffers* wb, int32_t** qa, int32_t** qb, int32_t** fa, int32_t** fb, int32_t** ns,
                      int32_t** fs, int32_t** rs, int32_t** R, int32_t** le, SsspCounters** cnt, double** minfar,
                      int32_t** rtail) {
@@ -774,7 +790,7 @@ int sssp_delta_run(ghb_workspace* ws, ghb_graph* g, int32_t src, double inf, dou
         stats->edges_examined = examined;
         stats->device_ms = ms;
     }
-    return GHB_OK;
+    return map_back_f64(ws, g, dist_out, out);
 }
 
 int sssp_pred_run(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int32_t* col, const double* w,

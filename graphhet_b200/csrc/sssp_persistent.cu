@@ -517,6 +517,7 @@ __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent_kernel(
     const unsigned extra = st->bar_extra;
 
     // ---- init
+    if (perm) src = perm[src];
     const unsigned long long ib = (unsigned long long)__double_as_longlong(inf);
     for (int64_t v = gtid; v < n; v += gsize) {
         dist[v] = (v == src) ? 0ull : ib;
@@ -742,20 +743,24 @@ int graph_light_ends(ghb_workspace* ws, ghb_graph* g, double delta, const int32_
 // One cooperative launch for the whole traversal.  rp/col/wt: the rows to
 // relax (a resident graph's weight-sorted copy when le is given, whose
 // light ranges [rp[u], le[u]) hold the entries below delta).  dist: per
-// vertex in the graph's ids; with perm, out[v] = dist[perm[v]] as well.
+// vertex in the graph's ids; with perm, src is the caller's id and
+// out[v] = dist[perm[v]] as well.  m: the rows' entries where the caller
+// knows them, else -1.
 int sssp_persistent_run(ghb_workspace* ws, int32_t n, const int32_t* rp, const int32_t* le, const int32_t* col,
-                        const double* wt, int32_t src, double inf, double delta, double* dist, const int32_t* perm,
-                        double* out, ghb_traversal_stats* stats) {
+                        const double* wt, int64_t m, int32_t src, double inf, double delta, double* dist,
+                        const int32_t* perm, double* out, ghb_traversal_stats* stats) {
     int blocks = 0;
     if (!sssp_persistent_available(ws, &blocks)) {
         set_error("cooperative launch unavailable");
         return GHB_ERR_UNSUPPORTED;
     }
     cudaStream_t st = ws->stream;
-    int32_t* hp = reinterpret_cast<int32_t*>(ws->host_pinned);
-    GHB_CUDA_TRY(cudaMemcpyAsync(hp, rp + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    GHB_CUDA_TRY(cudaStreamSynchronize(st));
-    const int64_t m = hp[0];
+    if (m < 0) {
+        int32_t* hp = reinterpret_cast<int32_t*>(ws->host_pinned);
+        GHB_CUDA_TRY(cudaMemcpyAsync(hp, rp + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        GHB_CUDA_TRY(cudaStreamSynchronize(st));
+        m = hp[0];
+    }
     // Chunks of one pass: rows over kSpDirect entries, ceil(len / kSpChunk)
     // each, so fewer than m / kSpChunk + m / kSpDirect.
     const int64_t chunk_cap = m / 32 + 64;
@@ -781,10 +786,9 @@ int sssp_persistent_run(ghb_workspace* ws, int32_t n, const int32_t* rp, const i
     Carver c(ws->scratch);
     carve(c, &qa, &qb, &ch, &fa, &fb, &ns, &fs, &rs, &R, &rstate);
 
-    // The start state, in one copy from pinned memory (its words are not
-    // written again before this call's read-back).
-    SsspRunState* h0 = reinterpret_cast<SsspRunState*>(ws->host_pinned);
-    static_assert(sizeof(SsspRunState) <= sizeof(int64_t) * kHostPinnedWords, "the run state fits the pinned words");
+    // The start state (pageable source: staged by the copy).
+    SsspRunState start;
+    SsspRunState* h0 = &start;
     std::memset(static_cast<void*>(h0), 0, sizeof(SsspRunState));
     h0->bar_limit_ns = (unsigned long long)ws->tune.barrier_limit_us * 1000ull;
     h0->bar_extra = (unsigned)ws->tune.barrier_extra;
@@ -811,6 +815,18 @@ int sssp_persistent_run(ghb_workspace* ws, int32_t n, const int32_t* rp, const i
     GHB_TRY(launch_coop(ws, sssp_persistent_kernel, dim3(blocks), dim3(kSsspThreads), 0, n, rp, le, col, wt, src, inf,
                         dist, qa, qb, ch, fa, fb, ns, fs, rs, R, rstate, perm, out));
     if (stats) GHB_CUDA_TRY(cudaEventRecord(ws->ev_stop, st));
+    // The reached vertices and their entries, counted behind the traversal:
+    // one wait for both.
+    constexpr size_t kReachedWord = (sizeof(SsspRunState) + 7) / 8;
+    static_assert(kReachedWord + 2 <= (size_t)kHostPinnedWords, "the run state and two sums fit the pinned words");
+    if (stats) {
+        unsigned long long* acc = reinterpret_cast<unsigned long long*>(ws->dev_small);
+        GHB_CUDA_TRY(cudaMemsetAsync(acc, 0, 2 * sizeof(unsigned long long), st));
+        GHB_TRY(launch(ws, sp_reached_kernel, dim3(grid_for(n, 256, ws->num_sms * 8)), dim3(256), 0, n, rp,
+                       (const double*)dist, inf, acc));
+        GHB_CUDA_TRY(cudaMemcpyAsync(ws->host_pinned + kReachedWord, acc, 2 * sizeof(unsigned long long),
+                                     cudaMemcpyDeviceToHost, st));
+    }
     GHB_CUDA_TRY(cudaMemcpyAsync(ws->host_pinned, rstate, sizeof(SsspRunState), cudaMemcpyDeviceToHost, st));
     GHB_CUDA_TRY(cudaStreamSynchronize(st));
     SsspRunState h;
@@ -824,16 +840,9 @@ int sssp_persistent_run(ghb_workspace* ws, int32_t n, const int32_t* rp, const i
         return GHB_ERR_TIMEOUT;
     }
     if (stats) {
-        unsigned long long* acc = reinterpret_cast<unsigned long long*>(ws->dev_small);
-        GHB_CUDA_TRY(cudaMemsetAsync(acc, 0, 2 * sizeof(unsigned long long), st));
-        GHB_TRY(launch(ws, sp_reached_kernel, dim3(grid_for(n, 256, ws->num_sms * 8)), dim3(256), 0, n, rp,
-                       (const double*)dist, inf, acc));
-        GHB_CUDA_TRY(cudaMemcpyAsync(ws->host_pinned, acc, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                                     st));
-        GHB_CUDA_TRY(cudaStreamSynchronize(st));
         float ms = 0.f;
         GHB_CUDA_TRY(cudaEventElapsedTime(&ms, ws->ev_start, ws->ev_stop));
-        const unsigned long long* ha = reinterpret_cast<const unsigned long long*>(ws->host_pinned);
+        const int64_t* ha = ws->host_pinned + kReachedWord;
         stats->levels = (int32_t)(h.s.light_passes + h.s.heavy_passes + h.s.chunk_passes);
         stats->pull_levels = (int32_t)h.s.splits;
         stats->edges_reached = (int64_t)ha[0];
