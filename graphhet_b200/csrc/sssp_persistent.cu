@@ -20,6 +20,8 @@
 //   SPLIT  move the far list's entries below the next bucket's end into the
 //          near queue; drop entries already settled; keep the rest.
 //
+// Grid passes stage what they append in shared memory (SpStage).
+//
 // The next bucket's end follows the smallest pending far distance
 // (kept in shared memory per block, one global atomic per block and pass),
 // so empty buckets cost nothing.
@@ -40,8 +42,11 @@ namespace ghb {
 // warp; longer ones are cut into kSpChunk-entry chunks that a CHUNK pass, in
 // the same round, spreads over every warp (a warp walking a few 1,024-entry
 // rows while the rest of the grid waits at the barrier was the bottleneck).
+// Chunks are one step of a warp, kSpBatch x 32 entries: RMAT-16 0.58 ms with
+// 256 and 0.54 with 128, RMAT-18 on the caller's ids 0.84 and 0.80, uniform
+// graphs alike; 512 costs RMAT-20 raw 1.42 -> 1.70.
 constexpr int32_t kSpDirect = 64;
-constexpr int32_t kSpChunk = 256;
+constexpr int32_t kSpChunk = 128;
 constexpr int kSsspThreads = 512;
 // Passes over small queues run on block 0 alone (see sssp_persistent_kernel):
 // its queues' first kSoloQueue entries lie in shared memory, and it hands back
@@ -49,9 +54,10 @@ constexpr int kSsspThreads = 512;
 constexpr int32_t kSoloQueue = 2048;
 constexpr int32_t kSoloChunks = 32;
 // A queue is small up to kSoloEntries entries of mean degree.  1501 x 1999
-// grid: 30.8 ms with 3072, 35.8 with 6144 and 40.3 with 12288 (one block then
-// takes several turns of 512 rows per pass), 59.7 with every pass on the grid
-// and its decision read back through L2 (300 x 300: 3.3 ms against 9.0).
+// grid, before the staging below (32.4 ms with it): 30.8 ms with 3072, 35.8
+// with 6144 and 40.3 with 12288 (one block then takes several turns of 512
+// rows per pass), 59.7 with every pass on the grid and its decision read back
+// through L2 (300 x 300: 3.3 ms against 9.0).
 constexpr int64_t kSoloEntries = 3072;
 constexpr int kSoloTurns = 1 << 14;
 constexpr unsigned long long kSsspTimeBudgetNs = 120ull * 1000000000ull;  // two minutes
@@ -63,16 +69,16 @@ enum SsspMode : int32_t { kLight = 0, kHeavy = 1, kSplit = 2, kDone = 3, kChunk 
 // slot (p + 1) % 3 during pass p (all blocks read it last before the barrier
 // of pass p - 1).
 struct SpSlot {
-    int32_t q_tail;       // the next near queue
-    int32_t c_tail;       // chunks
-    int32_t r_add;        // additions to R
-    int32_t far_add;      // additions to the far list
-    unsigned long long fmin;  // smallest far distance added (bits)
-    unsigned long long examined;
-    int32_t stop;         // the time budget ran out
-    int32_t pad[23];
+    // A cache line for each: atomics on one line follow each other at about
+    // 2 ns, whichever of its words they take.
+    alignas(128) int32_t q_tail;   // the next near queue
+    alignas(128) int32_t c_tail;   // chunks
+    alignas(128) int32_t r_add;    // additions to R
+    alignas(128) int32_t far_add;  // additions to the far list
+    alignas(128) unsigned long long fmin;  // smallest far distance added (bits)
+    alignas(128) unsigned long long examined;
+    int32_t stop;                  // the time budget ran out
 };
-static_assert(sizeof(SpSlot) == 128, "a slot is one cache line");
 
 // Where the traversal stands: every block holds it in shared memory and
 // derives the next pass from it and the slot just filled, so no block waits
@@ -139,6 +145,24 @@ struct SpQueue {
     }
 };
 
+// What a warp has yet to append in a grid pass, by kind: it writes kSpStage at
+// a time behind one atomic on the list's counter, and the block's warps the
+// rest behind one at the end of the pass.  With an atomic per step of 128
+// entries relaxed and one per long row, the counters' cache line set the
+// pace, at 2 ns an atomic: a light pass over 690,000 rows of RMAT-22 took
+// 450 us and takes 130, its long rows' 23 M entries 517 and 210, a heavy
+// pass of 80 M entries 1,000 and 530.  One source on RMAT-22, resident, 6.1 ->
+// 3.0 ms, on the caller's ids 13.2 -> 4.5; RMAT-20 of degree 8 2.7 -> 1.9 and
+// 2.8 -> 1.3; uniform, 2^20 vertices of degree 16, 1.11 -> 0.77.  Grids, whose
+// passes are mostly solo, give 4 % for the longer code.
+enum SpKind : int { kNear = 0, kFar = 1, kSettled = 2, kSpKinds = 3 };
+constexpr int kSpStage = 128;
+constexpr int kSpWarps = kSsspThreads / 32;
+struct SpStage {
+    int32_t* buf;  // the warp's kSpKinds x kSpStage words; nullptr: append at once (solo passes)
+    int32_t n[kSpKinds];
+};
+
 struct SpCtx {
     const int32_t* __restrict__ rp;
     const int32_t* __restrict__ le;  // light ends (nullptr: no light/heavy split)
@@ -170,6 +194,68 @@ struct SpFound {
     unsigned long long fmin = ~0ull;
 };
 
+template <int KIND>
+__device__ __forceinline__ int32_t* sp_tail(const SpCtx& c) {
+    return KIND == kNear ? &c.slot->q_tail : KIND == kFar ? &c.slot->far_add : &c.slot->r_add;
+}
+template <int KIND>
+__device__ __forceinline__ int32_t sp_base(const SpCtx& c) {
+    return KIND == kNear ? c.q_base : KIND == kFar ? c.far_base : c.r_base;
+}
+template <int KIND>
+__device__ __forceinline__ int32_t* sp_list(const SpCtx& c) {
+    return KIND == kNear ? c.q_next.mem : KIND == kFar ? c.far_cur : c.R;
+}
+
+// The warp's staged vertices of one kind, to their list from position at.
+template <int KIND>
+__device__ __forceinline__ void sp_write(const SpCtx& c, SpStage& g, int32_t at) {
+    for (int32_t i = lane_id(); i < g.n[KIND]; i += 32) sp_list<KIND>(c)[at + i] = g.buf[KIND * kSpStage + i];
+}
+
+// Append v[q] of the lanes in m[q]; every lane of the warp calls it.
+template <int KIND, int Q>
+__device__ __forceinline__ void sp_append(const SpCtx& c, SpStage& g, const unsigned* m, const int32_t* v) {
+    int32_t total = 0;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) total += __popc(m[q]);
+    if (total == 0) return;
+    const int lane = lane_id();
+    const unsigned below = (1u << lane) - 1u;
+    int32_t at;
+    if (g.buf) {
+        static_assert(Q * 32 <= kSpStage, "a step's entries fit an empty buffer");
+        if (g.n[KIND] + total > kSpStage) {
+            int32_t to = 0;
+            if (lane == 0) to = sp_base<KIND>(c) + atomicAdd(sp_tail<KIND>(c), g.n[KIND]);
+            __syncwarp();
+            sp_write<KIND>(c, g, __shfl_sync(0xffffffffu, to, 0));
+            __syncwarp();
+            g.n[KIND] = 0;
+        }
+        at = g.n[KIND];
+        g.n[KIND] += total;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            if ((m[q] >> lane) & 1u) g.buf[KIND * kSpStage + at + __popc(m[q] & below)] = v[q];
+            at += __popc(m[q]);
+        }
+        return;
+    }
+    at = 0;
+    if (lane == 0) at = sp_base<KIND>(c) + atomicAdd(sp_tail<KIND>(c), total);
+    at = __shfl_sync(0xffffffffu, at, 0);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        if ((m[q] >> lane) & 1u) {
+            const int32_t i = at + __popc(m[q] & below);
+            if (KIND == kNear) c.q_next.put(i, v[q]);
+            else sp_list<KIND>(c)[i] = v[q];
+        }
+        at += __popc(m[q]);
+    }
+}
+
 // Relax entries j[q] (those with ok[q]) of rows whose source distances are
 // du[q]; every lane of the warp calls it.  Each step's accesses are issued for
 // all kSpBatch entries before any answer is used: a small pass is a chain of
@@ -180,7 +266,7 @@ struct SpFound {
 // round the entry is spare; one per vertex and round at most, so the queues
 // hold.)
 __device__ __forceinline__ void sp_relax_batch(const SpCtx& c, const double* du, const int32_t* j, const bool* ok,
-                                               SpFound& found) {
+                                               SpFound& found, SpStage& g) {
     int32_t v[kSpBatch];
     double w[kSpBatch], cur[kSpBatch];
 #pragma unroll
@@ -218,6 +304,11 @@ __device__ __forceinline__ void sp_relax_batch(const SpCtx& c, const double* du,
         nfar += __popc(far_m[q]);
     }
     if (nnear + nfar == 0) return;
+    if (g.buf) {
+        sp_append<kNear, kSpBatch>(c, g, near_m, v);
+        sp_append<kFar, kSpBatch>(c, g, far_m, v);
+        return;
+    }
     const int lane = lane_id();
     int32_t base = 0;
     if (lane == 0 && nnear) base = c.q_base + atomicAdd(&c.slot->q_tail, nnear);
@@ -234,7 +325,8 @@ __device__ __forceinline__ void sp_relax_batch(const SpCtx& c, const double* du,
 }
 
 // Relax [jb, je) of one row (distance du) with the whole warp.
-__device__ __forceinline__ void sp_warp_range(const SpCtx& c, double du, int32_t jb, int32_t je, SpFound& found) {
+__device__ __forceinline__ void sp_warp_range(const SpCtx& c, double du, int32_t jb, int32_t je, SpFound& found,
+                                              SpStage& g) {
     for (int64_t j0 = jb; j0 < je; j0 += 32 * kSpBatch) {
         int32_t jj[kSpBatch];
         bool ok[kSpBatch];
@@ -246,7 +338,7 @@ __device__ __forceinline__ void sp_warp_range(const SpCtx& c, double du, int32_t
             jj[q] = (int32_t)j;
             dd[q] = du;
         }
-        sp_relax_batch(c, dd, jj, ok, found);
+        sp_relax_batch(c, dd, jj, ok, found, g);
     }
 }
 
@@ -254,43 +346,67 @@ __device__ __forceinline__ void sp_warp_range(const SpCtx& c, double du, int32_t
 // longer than kSpDirect are appended, whole, to the chunk list of the CHUNK
 // pass that follows.
 __device__ __forceinline__ void sp_rows(const SpCtx& c, int32_t u, int32_t b, int32_t e, double du,
-                                        SpFound& found) {
+                                        SpFound& found, SpStage& g) {
     const int lane = lane_id();
-    if (e - b > kSpDirect) {
-        const int32_t nch = (e - b + kSpChunk - 1) / kSpChunk;
-        const int32_t pos = atomicAdd(&c.slot->c_tail, nch);
-        for (int32_t k = 0; k < nch; ++k) {
-            const int32_t cb = b + k * kSpChunk;
-            c.chunks[pos + k] = make_int4(u, cb, min(e, cb + kSpChunk), 0);
-        }
-        e = b;
-    }
-    // Rows of 32 entries or more: the whole warp, one row at a time.
-    unsigned med = __ballot_sync(0xffffffffu, e - b >= 32);
-    while (med) {
-        const int leader = __ffs(med) - 1;
-        med &= med - 1;
-        const int32_t lb = __shfl_sync(0xffffffffu, b, leader);
-        const int32_t lend = __shfl_sync(0xffffffffu, e, leader);
-        const double ld = __shfl_sync(0xffffffffu, du, leader);
-        sp_warp_range(c, ld, lb, lend, found);
-    }
-    if (e - b >= 32) e = b;
-    const int32_t d = e - b;
-    // Rows of a mesh: each lane its own, without the scan below.
-    if (__reduce_max_sync(0xffffffffu, (unsigned)d) <= (unsigned)kSpBatch) {
+    // Rows of a mesh: each lane its own, without votes and the scan below.
+    const int32_t longest = (int32_t)__reduce_max_sync(0xffffffffu, (unsigned)(e - b));
+    if (longest <= kSpBatch) {
         int32_t jj[kSpBatch];
         bool ok[kSpBatch];
         double dd[kSpBatch];
 #pragma unroll
         for (int q = 0; q < kSpBatch; ++q) {
             jj[q] = b + q;
-            ok[q] = q < d;
+            ok[q] = q < e - b;
             dd[q] = du;
         }
-        sp_relax_batch(c, dd, jj, ok, found);
+        sp_relax_batch(c, dd, jj, ok, found, g);
         return;
     }
+    if (longest > kSpDirect) {
+        // One atomic for the warp's long rows; the first kOwn chunks of a row
+        // are written by its lane, further ones by the warp.
+        constexpr int32_t kOwn = 4;
+        const int32_t nch = e - b > kSpDirect ? (e - b + kSpChunk - 1) / kSpChunk : 0;
+        int32_t incl = nch;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += x;
+        }
+        int32_t pos = 0;
+        if (lane == 31) pos = atomicAdd(&c.slot->c_tail, incl);
+        pos = __shfl_sync(0xffffffffu, pos, 31) + incl - nch;
+        for (int32_t k = 0; k < min(nch, kOwn); ++k) {
+            const int32_t cb = b + k * kSpChunk;
+            c.chunks[pos + k] = make_int4(u, cb, min(e, cb + kSpChunk), 0);
+        }
+        unsigned many = __ballot_sync(0xffffffffu, nch > kOwn);
+        while (many) {
+            const int leader = __ffs(many) - 1;
+            many &= many - 1;
+            const int32_t lu = __shfl_sync(0xffffffffu, u, leader), lb = __shfl_sync(0xffffffffu, b, leader);
+            const int32_t lend = __shfl_sync(0xffffffffu, e, leader), lpos = __shfl_sync(0xffffffffu, pos, leader);
+            const int32_t ln = __shfl_sync(0xffffffffu, nch, leader);
+            for (int32_t k = kOwn + lane; k < ln; k += 32) {
+                const int32_t cb = lb + k * kSpChunk;
+                c.chunks[lpos + k] = make_int4(lu, cb, min(lend, cb + kSpChunk), 0);
+            }
+        }
+        if (nch) e = b;
+    }
+    // Rows of 32 entries or more: the whole warp, one row at a time.
+    unsigned med = longest >= 32 ? __ballot_sync(0xffffffffu, e - b >= 32) : 0u;
+    while (med) {
+        const int leader = __ffs(med) - 1;
+        med &= med - 1;
+        const int32_t lb = __shfl_sync(0xffffffffu, b, leader);
+        const int32_t lend = __shfl_sync(0xffffffffu, e, leader);
+        const double ld = __shfl_sync(0xffffffffu, du, leader);
+        sp_warp_range(c, ld, lb, lend, found, g);
+    }
+    if (e - b >= 32) e = b;
+    const int32_t d = e - b;
     // Shorter rows: gathered warp-wide over a scan of their lengths.
     int32_t incl = d;
 #pragma unroll
@@ -320,7 +436,7 @@ __device__ __forceinline__ void sp_rows(const SpCtx& c, int32_t u, int32_t b, in
             ok[q] = k < total;
             jj[q] = ob + (k - oe);
         }
-        sp_relax_batch(c, dd, jj, ok, found);
+        sp_relax_batch(c, dd, jj, ok, found, g);
     }
 }
 
@@ -439,7 +555,8 @@ __device__ __forceinline__ void sp_total(const SpFound& found, unsigned long lon
 
 // One pass's share of warp `warp` of `nwarps` (thread `tid` of `nt`).
 __device__ __forceinline__ void sp_pass(const SpState& s, SpCtx& c, const SpQueue& q_cur, int32_t* fa, int32_t* fb,
-                                        int64_t tid, int64_t nt, SpFound& found) {
+                                        int64_t tid, int64_t nt, SpFound& found,
+                                        SpStage& g) {
     const int lane = lane_id();
     const int64_t warp = tid >> 5, nwarps = nt >> 5;
     const bool split = c.le != nullptr;
@@ -448,24 +565,29 @@ __device__ __forceinline__ void sp_pass(const SpState& s, SpCtx& c, const SpQueu
         for (int64_t i = warp; i < s.nc; i += nwarps) {
             const int4 ch = __ldcg(c.chunks + i);
             const double du = sp_dist(c.dist, ch.x);
-            sp_warp_range(c, du, ch.y, ch.z, found);
+            sp_warp_range(c, du, ch.y, ch.z, found, g);
         }
     } else if (s.mode == kSplit) {
         const int32_t* far = s.fsel ? fa : fb;
         const double old_thr = s.thr, nthr = s.new_thr;
-        for (int64_t i = tid; i < s.nq; i += nt) {
-            const int32_t v = __ldcg(far + i);
-            const double d = sp_dist(c.dist, v);
-            if (d < old_thr) continue;  // settled in an earlier bucket
-            if (d < nthr) {
-                if (atomicExch(c.near_stamp + v, c.round) != c.round)
-                    c.q_next.put(c.q_base + warp_append_active(&c.slot->q_tail), v);
-            } else {
-                if (atomicExch(c.far_stamp + v, ~c.phase) != ~c.phase)
-                    c.far_cur[c.far_base + warp_append_active(&c.slot->far_add)] = v;
-                const unsigned long long db = (unsigned long long)__double_as_longlong(d);
-                if (db < found.fmin) found.fmin = db;
+        for (int64_t i = tid; i - lane < s.nq; i += nt) {
+            int32_t v = 0;
+            bool near = false, keep = false;
+            if (i < s.nq) {
+                v = __ldcg(far + i);
+                const double d = sp_dist(c.dist, v);
+                // Below old_thr it was settled in an earlier bucket.
+                if (d >= old_thr && d < nthr) {
+                    near = atomicExch(c.near_stamp + v, c.round) != c.round;
+                } else if (d >= old_thr) {
+                    keep = atomicExch(c.far_stamp + v, ~c.phase) != ~c.phase;
+                    const unsigned long long db = (unsigned long long)__double_as_longlong(d);
+                    if (db < found.fmin) found.fmin = db;
+                }
             }
+            const unsigned near_m = __ballot_sync(0xffffffffu, near), keep_m = __ballot_sync(0xffffffffu, keep);
+            sp_append<kNear, 1>(c, g, &near_m, &v);
+            sp_append<kFar, 1>(c, g, &keep_m, &v);
         }
     } else {
         // Queue rows, 32 per warp; on small queues fewer, so that their rows
@@ -491,10 +613,10 @@ __device__ __forceinline__ void sp_pass(const SpState& s, SpCtx& c, const SpQueu
                     du = sp_dist(c.dist, u);
                 }
             }
-            sp_rows(c, u, b, e, du, found);
+            sp_rows(c, u, b, e, du, found, g);
             if (split && s.mode == kLight) {
-                const int32_t at = warp_append(&c.slot->r_add, settled);
-                if (settled) c.R[c.r_base + at] = u;
+                const unsigned settled_m = __ballot_sync(0xffffffffu, settled);
+                sp_append<kSettled, 1>(c, g, &settled_m, &u);
             }
         }
     }
@@ -512,7 +634,12 @@ __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent_kernel(
     __shared__ SpState s;
     __shared__ SpSlot own;  // the slot of a solo pass
     __shared__ unsigned long long s_fmin, s_exam, s_t0;
-    __shared__ int32_t s_fast[2][kSoloQueue];
+    // Solo runs: the two near queues' first entries.  Grid passes: the warps'
+    // staged vertices, and how many are left at the end, then where they go.
+    __shared__ int32_t s_lists[kSpWarps * kSpKinds * kSpStage];
+    static_assert(kSpWarps * kSpKinds * kSpStage >= 2 * kSoloQueue, "the solo queues fit");
+    auto fast = [&](int32_t sel) { return s_lists + sel * kSoloQueue; };
+    __shared__ int32_t s_left[kSpKinds][kSpWarps];
     const unsigned long long limit_ns = st->bar_limit_ns;
     const unsigned extra = st->bar_extra;
 
@@ -551,7 +678,7 @@ __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent_kernel(
     unsigned turn = 0;  // the grid's passes: which slot is filled
     while (s.mode != kDone) {
         auto context = [&](int32_t cap) {
-            c.q_next = SpQueue{s_fast[s.qsel ^ 1], s.qsel ? qa : qb, cap};
+            c.q_next = SpQueue{fast(s.qsel ^ 1), s.qsel ? qa : qb, cap};
             c.far_cur = s.fsel ? fb : fa;
             c.thr = s.thr;
             c.round = s.round;
@@ -569,12 +696,12 @@ __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent_kernel(
                 // The queue's first entries move to shared memory for the run.
                 const int32_t held = s.mode == kLight ? min(s.nq, kSoloQueue) : 0;
                 for (int32_t i = threadIdx.x; i < held; i += blockDim.x)
-                    s_fast[s.qsel][i] = __ldcg((s.qsel ? qb : qa) + i);
+                    fast(s.qsel)[i] = __ldcg((s.qsel ? qb : qa) + i);
                 // Entries that an unfinished round (its chunks come next) has
                 // queued move as well.
                 const int32_t held_next = min(s.q_next, kSoloQueue);
                 for (int32_t i = threadIdx.x; i < held_next; i += blockDim.x)
-                    s_fast[s.qsel ^ 1][i] = __ldcg((s.qsel ? qa : qb) + i);
+                    fast(s.qsel ^ 1)[i] = __ldcg((s.qsel ? qa : qb) + i);
                 const unsigned long long t_run = global_timer_ns();
                 if (threadIdx.x == 0) {
                     own.q_tail = own.c_tail = own.r_add = own.far_add = own.stop = 0;
@@ -585,9 +712,10 @@ __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent_kernel(
                 c.slot = &own;
                 for (int turns = 0; s.solo && turns < kSoloTurns; ++turns) {
                     context(kSoloQueue);
-                    const SpQueue q_cur{s_fast[s.qsel], s.qsel ? qb : qa, kSoloQueue};
+                    const SpQueue q_cur{fast(s.qsel), s.qsel ? qb : qa, kSoloQueue};
                     SpFound found;
-                    sp_pass(s, c, q_cur, fa, fb, threadIdx.x, blockDim.x, found);
+                    SpStage stage{nullptr, {0, 0, 0}};
+                    sp_pass(s, c, q_cur, fa, fb, threadIdx.x, blockDim.x, found, stage);
                     sp_total(found, &own.examined, &own.fmin);
                     __syncthreads();
                     if (threadIdx.x == 0) {
@@ -607,10 +735,10 @@ __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent_kernel(
                 // and the one that an unfinished round fills.
                 const int32_t back = s.mode == kLight ? min(s.nq, kSoloQueue) : 0;
                 for (int32_t i = threadIdx.x; i < back; i += blockDim.x)
-                    (s.qsel ? qb : qa)[i] = s_fast[s.qsel][i];
+                    (s.qsel ? qb : qa)[i] = fast(s.qsel)[i];
                 const int32_t back_next = min(s.q_next, kSoloQueue);
                 for (int32_t i = threadIdx.x; i < back_next; i += blockDim.x)
-                    (s.qsel ? qa : qb)[i] = s_fast[s.qsel ^ 1][i];
+                    (s.qsel ? qa : qb)[i] = fast(s.qsel ^ 1)[i];
                 // One pass of the whole grid follows even where the next is
                 // small: the run above ended by its own limits then.
                 if (threadIdx.x == 0) {
@@ -630,11 +758,41 @@ __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent_kernel(
         c.slot = slot;
         const SpQueue q_cur{nullptr, s.qsel ? qb : qa, 0};
         SpFound found;
-        sp_pass(s, c, q_cur, fa, fb, gtid, gsize, found);
-        // Block totals, then the barrier.
+        const int wid = threadIdx.x >> 5, lane = lane_id();
+        SpStage stage{s_lists + wid * kSpKinds * kSpStage, {0, 0, 0}};
+        sp_pass(s, c, q_cur, fa, fb, gtid, gsize, found, stage);
+        // What the warps have left and the block's totals, then the barrier.
+        if (lane < kSpKinds) s_left[lane][wid] = lane == kNear ? stage.n[kNear] : lane == kFar ? stage.n[kFar] : stage.n[kSettled];
         sp_total(found, &s_exam, &s_fmin);
         __syncthreads();
-        if (threadIdx.x == 0) {
+        if (wid == 0) {
+            // Lane k takes kind k's places for the whole block.
+            int32_t excl[kSpKinds], take = 0;
+#pragma unroll
+            for (int k = 0; k < kSpKinds; ++k) {
+                const int32_t x = lane < kSpWarps ? s_left[k][lane] : 0;
+                int32_t incl = x;
+#pragma unroll
+                for (int o = 1; o < kSpWarps; o <<= 1) {
+                    const int32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += y;
+                }
+                excl[k] = incl - x;
+                const int32_t total = __shfl_sync(0xffffffffu, incl, kSpWarps - 1);
+                if (lane == k) take = total;
+            }
+            int32_t at = 0;
+            if (take) {
+                if (lane == kNear) at = sp_base<kNear>(c) + atomicAdd(sp_tail<kNear>(c), take);
+                else if (lane == kFar) at = sp_base<kFar>(c) + atomicAdd(sp_tail<kFar>(c), take);
+                else at = sp_base<kSettled>(c) + atomicAdd(sp_tail<kSettled>(c), take);
+            }
+#pragma unroll
+            for (int k = 0; k < kSpKinds; ++k) {
+                const int32_t to = __shfl_sync(0xffffffffu, at, k);
+                if (lane < kSpWarps) s_left[k][lane] = to + excl[k];
+            }
+        } else if (threadIdx.x == 32) {
             if (s_exam) atomicAdd(&slot->examined, s_exam);
             if (s_fmin != ~0ull) atomicMin(&slot->fmin, s_fmin);
             s_exam = 0;
@@ -647,14 +805,20 @@ __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent_kernel(
                 if (global_timer_ns() - s_t0 > kSsspTimeBudgetNs) slot->stop = 1;
             }
         }
+        __syncthreads();
+        sp_write<kNear>(c, stage, s_left[kNear][wid]);
+        sp_write<kFar>(c, stage, s_left[kFar][wid]);
+        sp_write<kSettled>(c, stage, s_left[kSettled][wid]);
         if (!sp_barrier(st, limit_ns, extra)) return;
         if (threadIdx.x == 0) {
             SpSlot f;
-            const int4 a = __ldcg(reinterpret_cast<const int4*>(slot));
-            const ulonglong2 b = __ldcg(reinterpret_cast<const ulonglong2*>(slot) + 1);
+            f.q_tail = __ldcg(&slot->q_tail);
+            f.c_tail = __ldcg(&slot->c_tail);
+            f.r_add = __ldcg(&slot->r_add);
+            f.far_add = __ldcg(&slot->far_add);
+            f.fmin = __ldcg(&slot->fmin);
+            f.examined = __ldcg(&slot->examined);
             f.stop = __ldcg(&slot->stop);
-            f.q_tail = a.x, f.c_tail = a.y, f.r_add = a.z, f.far_add = a.w;
-            f.fmin = b.x, f.examined = b.y;
             sp_decide(s, f);
         }
         ++turn;

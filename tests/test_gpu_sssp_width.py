@@ -1,5 +1,5 @@
 """The bucket width of a resident single-source call: half the weight rule's
-from 2^24 entries on unless the rows are sparse, and the distances that any
+from 2^26 entries on unless the rows are sparse, and the distances that any
 width gives."""
 import numpy as np
 import pytest
@@ -21,11 +21,11 @@ def build(kind, n, degree):
 
 
 @pytest.mark.parametrize("kind,n,degree,half", [
-    ("uniform", 1 << 20, 7, False),   # below 2^24 entries
-    ("uniform", 1 << 20, 9, True),    # above, 18 a vertex
-    ("uniform", 5 << 19, 4, True),    # 8 a vertex
-    ("uniform", 7 << 20, 2, False),   # above, 4 a vertex
-    ("grid", 2100, 0, False),         # above, 4 a vertex
+    ("uniform", 1 << 20, 9, False),
+    ("uniform", 1 << 21, 15, False),  # below 2^26 entries
+    ("uniform", 1 << 21, 17, True),   # above, 34 a vertex
+    ("uniform", 10 << 20, 4, True),   # 8 a vertex
+    ("grid", 4200, 0, False),         # above, 4 a vertex
 ])
 def test_default_width(kind, n, degree, half):
     import graphhet_b200 as G
