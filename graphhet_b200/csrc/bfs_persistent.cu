@@ -1190,6 +1190,12 @@ int bfs_persistent_run(ghb_workspace* ws, int32_t n, int32_t n_active, int64_t m
         pol = policy_device_params();
         if (!pol) policy = GHB_POLICY_HEURISTIC;
     }
+    // The start state (pageable source: staged by the call).
+    BfsRunState h0;
+    std::memset(static_cast<void*>(&h0), 0, sizeof(h0));
+    h0.bar_limit_ns = (unsigned long long)ws->tune.barrier_limit_us * 1000ull;
+    h0.bar_extra = (unsigned)ws->tune.barrier_extra;
+    GHB_CUDA_TRY(cudaMemcpyAsync(rs, &h0, sizeof(h0), cudaMemcpyHostToDevice, st));
     int64_t m_total = m;
     if (m < 0) {
         int32_t* hp = reinterpret_cast<int32_t*>(ws->host_pinned);
@@ -1197,12 +1203,6 @@ int bfs_persistent_run(ghb_workspace* ws, int32_t n, int32_t n_active, int64_t m
         GHB_CUDA_TRY(cudaStreamSynchronize(st));
         m_total = hp[0];
     }
-    // The start state (pageable source: staged by the call).
-    BfsRunState h0;
-    std::memset(static_cast<void*>(&h0), 0, sizeof(h0));
-    h0.bar_limit_ns = (unsigned long long)ws->tune.barrier_limit_us * 1000ull;
-    h0.bar_extra = (unsigned)ws->tune.barrier_extra;
-    GHB_CUDA_TRY(cudaMemcpyAsync(rs, &h0, sizeof(h0), cudaMemcpyHostToDevice, st));
     if (stats) GHB_CUDA_TRY(cudaEventRecord(ws->ev_start, st));
     // Meshes, road networks, paths: up to 4.5 entries per vertex.  (A random
     // graph with six has ten levels, and the larger kernel cost it 5 %.)

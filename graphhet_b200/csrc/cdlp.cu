@@ -422,15 +422,16 @@ __device__ __forceinline__ void cdlp_try_rows(const int4* __restrict__ rows, int
 // [first[c], first[c + 1]): an iteration of a small graph is bound by its
 // launches, and on a large one a class's last blocks overlap the next.
 // kModeMin: the first iteration over distinct labels (classes 0..6).
-// kModeTables: class 6 with its tables (classes 0..6).  kModeTry: classes 6..9
-// without tables,
-// which take the L1 that labels and bits are served from; a class of which
+// kModeTables: class 6 with its tables (classes 0..6).  kModeSmall: classes
+// 0..5 alone, whose few registers let a multiprocessor hold its 64 warps (a
+// uniform graph of 2^20 vertices of degree 22: 250 us an iteration together
+// with the next, 200 apart).  kModeTry: classes 6..9 without tables, which take the L1 that labels and bits are served from; a class of which
 // more than one row in kTryShare needed its table last time is left whole to
 // the kernels with tables (a row is read twice otherwise).  RMAT-22, ten
 // iterations: 13.0 ms with a table for every row, 9.1 with led rows done in the
 // table kernels, 7.4 with this pass (an iteration that few labels move in takes
 // 0.32 ms where it took 1.3).
-enum CdlpMode { kModeMin = 0, kModeTables = 1, kModeTry = 2 };
+enum CdlpMode { kModeMin = 0, kModeTables = 1, kModeTry = 2, kModeSmall = 3 };
 constexpr int32_t kTryShare = 8;
 struct CdlpLight {
     int32_t off[11];    // rows of class c: [off[c], off[c + 1])
@@ -443,10 +444,9 @@ __device__ __forceinline__ bool needs_tables(int32_t before, int32_t count) {
     return before > count / kTryShare;
 }
 template <int kMode>
-__global__ void __launch_bounds__(kCdlpThreads) cdlp_light_kernel(const int4* __restrict__ rows, CdlpLight q,
-                                                                  const int32_t* __restrict__ col,
-                                                                  const int32_t* __restrict__ lab,
-                                                                  int32_t* __restrict__ out, CdlpChanged chg) {
+__global__ void __launch_bounds__(kCdlpThreads, kMode == kModeSmall ? 8 : 5)
+    cdlp_light_kernel(const int4* __restrict__ rows, CdlpLight q, const int32_t* __restrict__ col,
+                      const int32_t* __restrict__ lab, int32_t* __restrict__ out, CdlpChanged chg) {
     constexpr bool M = kMode == kModeMin;
     // The block's class, by selects: indexing the plan would copy it to the
     // stack of every thread.
@@ -464,6 +464,11 @@ __global__ void __launch_bounds__(kCdlpThreads) cdlp_light_kernel(const int4* __
     const int block = (int)blockIdx.x - f0, nblocks = f1 - f0;
     const int32_t count = o1 - o0;
     rows += o0;
+    if constexpr (kMode == kModeTry) {
+        if (!needs_tables(q.before[c - 6], count))
+            cdlp_try_rows(rows, count, col, lab, out, chg, block, nblocks, q.todo + (o0 - q.off[6]), q.now + (c - 6));
+        return;
+    }
     switch (c) {
         case 0: cdlp_copy_rows(rows, count, lab, out, block, nblocks); break;
         case 1: cdlp_small_rows<2, M>(rows, count, col, lab, out, chg, block, nblocks); break;
@@ -472,11 +477,7 @@ __global__ void __launch_bounds__(kCdlpThreads) cdlp_light_kernel(const int4* __
         case 4: cdlp_small_rows<16, M>(rows, count, col, lab, out, chg, block, nblocks); break;
         case 5: cdlp_small_rows<32, M>(rows, count, col, lab, out, chg, block, nblocks); break;
         default:
-            if constexpr (kMode == kModeTry) {
-                if (!needs_tables(q.before[c - 6], count))
-                    cdlp_try_rows(rows, count, col, lab, out, chg, block, nblocks, q.todo + (o0 - q.off[6]),
-                                  q.now + (c - 6));
-            } else {
+            if constexpr (kMode == kModeMin || kMode == kModeTables) {
                 __shared__ int32_t keys[kCdlpThreads / 32][kWarpSlots];
                 __shared__ int32_t cnts[kCdlpThreads / 32][kWarpSlots];
                 cdlp_warp_rows<M>(rows, count, col, lab, out, chg, block, nblocks, keys[threadIdx.x >> 5],
@@ -1001,12 +1002,8 @@ int cdlp_run(ghb_workspace* ws, int32_t n, const int32_t* rp, const int32_t* col
         GHB_REQUIRE(acc <= pool_bound && nch <= chunk_bound, "CDLP table pool bound");
         GHB_CUDA_TRY(cudaMemcpyAsync(tab_off, toff.data(), sizeof(int64_t) * (nlong + 1), cudaMemcpyHostToDevice, st));
         GHB_CUDA_TRY(cudaMemcpyAsync(chunks, ch.data(), sizeof(int32_t) * ch.size(), cudaMemcpyHostToDevice, st));
-        GHB_CUDA_TRY(cudaMemsetAsync(occ, 0, sizeof(int32_t) * nlong, st));
-        GHB_CUDA_TRY(cudaMemsetAsync(done, 0, sizeof(int32_t) * nlong, st));
-        GHB_CUDA_TRY(cudaMemsetAsync(best, 0, sizeof(unsigned long long) * nlong, st));
-        GHB_CUDA_TRY(cudaMemsetAsync(held, 0, sizeof(int32_t) * nlong, st));
-        GHB_CUDA_TRY(cudaMemsetAsync(lead, 0, sizeof(int2) * nlong, st));
-        GHB_CUDA_TRY(cudaMemsetAsync(seen, 0, sizeof(int4) * nch, st));
+        // occ, done, best, held, lead and seen lie behind one another.
+        GHB_CUDA_TRY(cudaMemsetAsync(occ, 0, (size_t)(reinterpret_cast<char*>(seen + nch) - reinterpret_cast<char*>(occ)), st));
         GHB_TRY(launch(ws, cdlp_pool_clear_kernel, dim3(grid_for(nlong, 1, ws->num_sms * 8)), dim3(256), 0, long_rows,
                        nlong, pool, (const int64_t*)tab_off));
         GHB_CUDA_TRY(cudaStreamSynchronize(st));  // toff and ch are read by the copies above
@@ -1043,9 +1040,10 @@ int cdlp_run(ghb_workspace* ws, int32_t n, const int32_t* rp, const int32_t* col
     // more than they save.
     const bool large = n >= kCheckRows && iterations > 2;
     if (large) {
-        GHB_CUDA_TRY(cudaMemsetAsync(nchanged, 0, sizeof(int32_t) * (iterations + 1), st));
-        // Before the first iteration that counts: as if every row had needed its table.
-        GHB_CUDA_TRY(cudaMemsetAsync(ntodo, 0, sizeof(int32_t) * 4 * (iterations + 1), st));
+        // nchanged and ntodo lie behind one another.  Before the first iteration
+        // that counts: as if every row had needed its table.
+        GHB_CUDA_TRY(cudaMemsetAsync(nchanged, 0, (size_t)(reinterpret_cast<char*>(ntodo + 4 * ((size_t)iterations + 1)) -
+                                                           reinterpret_cast<char*>(nchanged)), st));
         GHB_CUDA_TRY(cudaMemsetAsync(ntodo + (first_min ? 4 : 0), 0x7f, sizeof(int32_t) * 4, st));
     }
     auto light_plan = [&](int from, int classes) {
@@ -1062,7 +1060,9 @@ int cdlp_run(ghb_workspace* ws, int32_t n, const int32_t* rp, const int32_t* col
     };
     // Rows without entries keep their labels: once both buffers hold them
     // (after two iterations) class 0 is left out.
-    const CdlpLight light = light_plan(0, 7), all_light = light_plan(0, 10), later = light_plan(1, large ? 10 : 7);
+    const int classes = large ? 6 : 7;
+    const CdlpLight first = light_plan(0, 7), light = light_plan(0, classes), later = light_plan(1, classes);
+    CdlpLight longer = light_plan(6, 10);
 
     // Iteration it reads cur and writes nxt.  kMin (first iteration over
     // distinct labels): each row's smallest label.
@@ -1071,21 +1071,22 @@ int cdlp_run(ghb_workspace* ws, int32_t n, const int32_t* rp, const int32_t* col
         const int4* R = rows;
         const dim3 block(kCdlpThreads);
         const bool tries = large && !M;
-        CdlpLight q = it >= 2 ? later : tries ? all_light : light;
+        const CdlpLight q = M ? first : it >= 2 ? later : light;
         // Class 6 + k: listed rows, their number last time and this time.
         auto list = [&](int k) {
             return tries ? CdlpTodo{todo + (off[6 + k] - off[6]), ntodo + 4 * it + k, ntodo + 4 * (it + 1) + k}
                          : CdlpTodo{nullptr, nullptr, nullptr};
         };
-        if (tries) {
-            q.todo = todo;
-            q.before = ntodo + 4 * it;
-            q.now = ntodo + 4 * (it + 1);
-        }
         const dim3 grid(q.first[10]);
         if (grid.x)
-            GHB_TRY(launch(ws, M ? cdlp_light_kernel<kModeMin> : tries ? cdlp_light_kernel<kModeTry> : cdlp_light_kernel<kModeTables>,
+            GHB_TRY(launch(ws, M ? cdlp_light_kernel<kModeMin> : tries ? cdlp_light_kernel<kModeSmall> : cdlp_light_kernel<kModeTables>,
                            grid, block, 0, R, q, col, cur, nxt, chg));
+        if (tries && longer.first[10]) {
+            longer.todo = todo;
+            longer.before = ntodo + 4 * it;
+            longer.now = ntodo + 4 * (it + 1);
+            GHB_TRY(launch(ws, cdlp_light_kernel<kModeTry>, dim3(longer.first[10]), block, 0, R, longer, col, cur, nxt, chg));
+        }
         if (tries && cls[6])
             GHB_TRY(launch(ws, cdlp_warp_kernel, dim3(grid_for((int64_t)cls[6] * 32, kCdlpThreads, ws->num_sms * 7)), block, 0,
                            R + off[6], cls[6], col, cur, nxt, list(0), chg));
@@ -1110,12 +1111,13 @@ int cdlp_run(ghb_workspace* ws, int32_t n, const int32_t* rp, const int32_t* col
     int32_t* cur = labels;
     int32_t* nxt = other;
     for (int it = 0; it < iterations; ++it) {
-        const CdlpChanged chg{large && it > 0 ? changed : nullptr, nchanged + (it > 0 ? it - 1 : 0), n / 16};  // the bits pay while few moved
+        // The bits pay while few labels moved: never behind the first iteration.
+        const CdlpChanged chg{large && it > 1 ? changed : nullptr, nchanged + (it > 0 ? it - 1 : 0), n / 16};
         if (it == 0 && first_min)
             GHB_TRY(iteration(std::true_type{}, it, cur, nxt, chg));
         else
             GHB_TRY(iteration(std::false_type{}, it, cur, nxt, chg));
-        if (large && it + 1 < iterations)
+        if (large && it > 0 && it + 1 < iterations)
             GHB_TRY(launch(ws, cdlp_changed_kernel, dim3(grid_for(n, kCdlpThreads, g)), dim3(kCdlpThreads), 0, n,
                            (const int32_t*)cur, (const int32_t*)nxt, changed, nchanged + it));
         std::swap(cur, nxt);

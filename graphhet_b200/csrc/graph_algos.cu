@@ -52,7 +52,8 @@ int tc_run(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int32_t* c
 int tc_run_cached(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int32_t* col, int64_t* counts64,
                   int32_t* counts32, int64_t* total, std::atomic<int32_t>* flags_cache, bool ranked);
 int pagerank_run(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* in_rp, const int32_t* in_col,
-                 const int32_t* out_rp, const ghb_pr_options* o, double* rank, int32_t* iters_run);
+                 const int32_t* out_rp, const int32_t* perm, const ghb_pr_options* o, double* rank,
+                 int32_t* iters_run);
 int msbfs_batch(ghb_workspace* ws, int32_t n, int32_t n_active, const int32_t* out_rp, const int32_t* out_col,
                 const int32_t* in_rp, const int32_t* in_col, const int32_t* srcs_dev, int32_t k,
                 const int32_t* perm, int32_t* depth, int64_t* levels_out, int64_t* examined_out);
@@ -359,10 +360,7 @@ int ghb_graph_pagerank(ghb_workspace* ws, const ghb_graph* g, const ghb_pr_optio
     GHB_REQUIRE(rank && options, "NULL argument");
     GHB_REQUIRE(options->iterations >= 0, "iterations < 0");
     GHB_REQUIRE(options->precision == GHB_PR_FP64 || options->precision == GHB_PR_FP32_KAHAN, "bad precision");
-    GHB_TRY(ws_reserve_stage(ws, sizeof(double) * (size_t)g->n));
-    double* rnew = static_cast<double*>(ws->stage);
-    GHB_TRY(pagerank_run(ws, g->n, g->m_in, g->in_rowptr, g->in_col, g->rowptr, options, rnew, iterations_run));
-    return map_back_f64(ws, g, rnew, rank);
+    return pagerank_run(ws, g->n, g->m_in, g->in_rowptr, g->in_col, g->rowptr, g->perm, options, rank, iterations_run);
 }
 
 int ghb_graph_cdlp(ghb_workspace* ws, const ghb_graph* g, int32_t iterations, int32_t* labels) {

@@ -215,13 +215,13 @@ __global__ void __launch_bounds__(kPrThreads) pr_reduce_kernel(const double* par
 constexpr int kPrPerLane = 8;
 constexpr int32_t kPrTile = 32 * kPrPerLane;
 
-// Non-empty rows in ascending order: row ids and their first entries.
+// Non-empty rows in ascending order: row ids and their first entries (begin[k]
+// = m behind the last; only the device knows how many rows there are).
 struct PrRows {
     const int32_t* __restrict__ id;     // id[i]
     const int32_t* __restrict__ begin;  // begin[i], begin[k] = m
     const int32_t* __restrict__ deg;    // out-degrees
-    const int32_t* __restrict__ tile;   // tile[t]: the row (index) that holds entry t * kPrTile
-    int32_t k;
+    const int32_t* __restrict__ tile;   // tile[t]: the row (index) that holds entry t * kPrTile; tile[tiles]: the last
     int32_t m;
     int32_t tiles;
 };
@@ -268,7 +268,10 @@ __global__ void __launch_bounds__(256) pr_row_lists_kernel(int32_t n, const int3
     }
 }
 
-__global__ void pr_tile_rows_kernel(int32_t k, const int32_t* __restrict__ begin, int32_t tiles, int32_t* tile) {
+__global__ void pr_tile_rows_kernel(const int32_t* __restrict__ rows, const int32_t* __restrict__ begin, int32_t tiles,
+                                    int32_t* tile) {
+    const int32_t k = *rows;
+    if (blockIdx.x == 0 && threadIdx.x == 0) tile[tiles] = k - 1;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < tiles; t += (int64_t)gridDim.x * blockDim.x) {
         int32_t lo = 0, hi = k - 1;  // the last row that begins at or before the entry
         while (lo < hi) {
@@ -324,7 +327,7 @@ __global__ void __launch_bounds__(kPrPersistThreads) pr_tile_kernel(
     if (warp < R.tiles) {
         load_cols(warp, ahead);
         ahead0 = R.tile[warp];
-        ahead1 = warp + 1 < R.tiles ? R.tile[warp + 1] : R.k - 1;
+        ahead1 = R.tile[warp + 1];
     }
     for (int64_t t = warp; t < R.tiles; t += nwarps) {
         const int64_t t0 = t * kPrTile, t1 = min(t0 + kPrTile, (int64_t)R.m);
@@ -350,7 +353,7 @@ __global__ void __launch_bounds__(kPrPersistThreads) pr_tile_kernel(
         if (t + nwarps < R.tiles) {
             load_cols(t + nwarps, ahead);
             ahead0 = R.tile[t + nwarps];
-            ahead1 = t + nwarps + 1 < R.tiles ? R.tile[t + nwarps + 1] : R.k - 1;
+            ahead1 = R.tile[t + nwarps + 1];
         }
         if (__shfl_sync(0xffffffffu, e, 0) >= t1) {  // one row
             KSum<T> acc;
@@ -428,7 +431,7 @@ __global__ void __launch_bounds__(kPrThreads) pr_finish_kernel(
         if (t < R.tiles) {
             // The tile's last row crosses its end when it holds the next tile's
             // first entry as well, and begins here unless it began before.
-            const int32_t i = t + 1 < R.tiles ? R.tile[t + 1] : R.k - 1;
+            const int32_t i = R.tile[t + 1];
             const int64_t b = R.begin[i], e = R.begin[i + 1];
             if (b >= t * kPrTile && b < (t + 1) * kPrTile && e > (t + 1) * kPrTile) {
                 row = R.id[i];
@@ -477,17 +480,25 @@ __global__ void __launch_bounds__(kPrThreads) pr_finish_kernel(
     pr_reduce(part_sink, part_l1, nparts, n, damping, sc, l1_hist, iter, track_l1);
 }
 
+// The ranks to the caller, through perm where the rows are in other ids.
 template <class T>
-__global__ void pr_to_f64_kernel(const T* src, double* dst, int32_t n) {
+__global__ void pr_to_f64_kernel(const T* __restrict__ src, const int32_t* __restrict__ perm, double* dst, int32_t n) {
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n;
          v += (int64_t)gridDim.x * blockDim.x)
-        dst[v] = (double)src[v];
+        dst[v] = (double)src[perm ? perm[v] : v];
 }
 
 template <class T>
 int pagerank_impl(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* in_rp, const int32_t* in_col,
-                  const int32_t* out_rp, const ghb_pr_options* o, double* rank_out, int32_t* iters_run, bool ranked) {
+                  const int32_t* out_rp, const ghb_pr_options* o, double* rank_out, int32_t* iters_run, const int32_t* perm) {
+    const bool ranked = perm != nullptr;
     cudaStream_t st = ws->stream;
+    int32_t* hp = reinterpret_cast<int32_t*>(ws->host_pinned);
+    if (m < 0) {
+        GHB_CUDA_TRY(cudaMemcpyAsync(hp, in_rp + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        GHB_CUDA_TRY(cudaStreamSynchronize(st));
+        m = hp[0];
+    }
     const Tuning& tu = ws->tune;
     const int pthreads = tu.pr_threads;
     const unsigned max_rows = ws->num_sms * tu.pr_blocks_per_sm;  // persistent blocks
@@ -498,17 +509,15 @@ int pagerank_impl(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* in_rp,
     // entries, FP64, ten iterations: 8.3 ms without a cache, 7.8 with 64 to 96 KB,
     // 8.4 with 112, 13.1 with 144), and where the first ids are not the hubs
     // nothing is gained from 32 KB on (9.7 ms with 0 or 32 KB, 10.8 with 64).
-    const int32_t cache_kb = ranked ? tu.pr_cache_kb : std::min(tu.pr_cache_kb, 32);
+    // Below 2^24 entries a block gathers too little for its fill (ten iterations
+    // with 16 and 80 KB: 2 M entries 306 and 332 us, 8 M 485 and 498; with 32 M
+    // 1,260 and 1,220).
+    const int32_t most_kb = m < (1 << 24) ? 16 : ranked ? tu.pr_cache_kb : 32;
+    const int32_t cache_kb = std::min(tu.pr_cache_kb, most_kb);
     const size_t cache_bytes = std::min((size_t)cache_kb * 1024,
                                         block_smem > tile_bytes + 1024 ? (block_smem - tile_bytes - 1024) & ~(size_t)255 : 0);
     const int32_t cache_elems = (int32_t)(cache_bytes / sizeof(T));
     const size_t smem = (size_t)((cache_elems + 3) & ~3) * sizeof(T) + tile_bytes;
-    int32_t* hp = reinterpret_cast<int32_t*>(ws->host_pinned);
-    if (m < 0) {
-        GHB_CUDA_TRY(cudaMemcpyAsync(hp, in_rp + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-        GHB_CUDA_TRY(cudaStreamSynchronize(st));
-        m = hp[0];
-    }
     const int32_t tiles = (int32_t)((m + kPrTile - 1) / kPrTile);
     const unsigned grid_rows = tiles ? grid_for((int64_t)tiles * 32, pthreads, max_rows) : 0;
     const unsigned grid_fin = grid_for(std::max<int64_t>(tiles, n / 8), kPrThreads, ws->num_sms * 8);
@@ -559,13 +568,11 @@ int pagerank_impl(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* in_rp,
     // The non-empty rows, the empty ones, and each tile's first row.
     GHB_TRY(launch(ws, pr_row_flags_kernel, dim3(grid_for(n, 256, g)), dim3(256), 0, n, in_rp, flag));
     GHB_TRY(scan_exclusive_i32(ws, flag, pos, n, bs));
-    GHB_CUDA_TRY(cudaMemcpyAsync(hp, pos + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     GHB_TRY(launch(ws, pr_row_lists_kernel, dim3(grid_for(n, 256, g)), dim3(256), 0, n, in_rp, (const int32_t*)pos,
                    (const int32_t*)outdeg, row_id, row_begin, row_deg, bare, bare_count));
-    GHB_CUDA_TRY(cudaStreamSynchronize(st));
-    const PrRows rows{row_id, row_begin, row_deg, tile, hp[0], (int32_t)m, tiles};
+    const PrRows rows{row_id, row_begin, row_deg, tile, (int32_t)m, tiles};
     if (tiles)
-        GHB_TRY(launch(ws, pr_tile_rows_kernel, dim3(grid_for(tiles, 256, g)), dim3(256), 0, rows.k,
+        GHB_TRY(launch(ws, pr_tile_rows_kernel, dim3(grid_for(tiles, 256, g)), dim3(256), 0, (const int32_t*)(pos + n),
                        (const int32_t*)row_begin, tiles, tile));
 
     T *r_cur = ra, *r_nxt = rb, *c_cur = ca, *c_nxt = cb;
@@ -592,7 +599,7 @@ int pagerank_impl(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* in_rp,
         }
     }
     GHB_TRY(launch(ws, pr_to_f64_kernel<T>, dim3(grid_for(n, 256, ws->num_sms * 8)), dim3(256), 0, (const T*)r_cur,
-                   rank_out, n));
+                   perm, rank_out, n));
     if (o->l1_history && it > 0) {
         GHB_CUDA_TRY(cudaMemcpyAsync(o->l1_history, hist, sizeof(double) * it, cudaMemcpyDeviceToHost, st));
         GHB_CUDA_TRY(cudaStreamSynchronize(st));
@@ -603,11 +610,14 @@ int pagerank_impl(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* in_rp,
 
 }  // namespace
 
+// Rows in the order of a degree ranking (perm[caller's id]; rank in the
+// caller's ids), m entries.
 int pagerank_run(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* in_rp, const int32_t* in_col,
-                 const int32_t* out_rp, const ghb_pr_options* o, double* rank, int32_t* iters_run) {
+                 const int32_t* out_rp, const int32_t* perm, const ghb_pr_options* o, double* rank,
+                 int32_t* iters_run) {
     if (o->precision == GHB_PR_FP64)
-        return pagerank_impl<double>(ws, n, m, in_rp, in_col, out_rp, o, rank, iters_run, true);
-    return pagerank_impl<float>(ws, n, m, in_rp, in_col, out_rp, o, rank, iters_run, true);
+        return pagerank_impl<double>(ws, n, m, in_rp, in_col, out_rp, o, rank, iters_run, perm);
+    return pagerank_impl<float>(ws, n, m, in_rp, in_col, out_rp, o, rank, iters_run, perm);
 }
 
 }  // namespace ghb
@@ -625,6 +635,6 @@ extern "C" int ghb_pagerank(ghb_workspace* ws, int32_t n, const int32_t* in_rowp
     GHB_REQUIRE(options->precision == GHB_PR_FP64 || options->precision == GHB_PR_FP32_KAHAN,
                 "bad precision");
     if (options->precision == GHB_PR_FP64)
-        return pagerank_impl<double>(ws, n, -1, in_rowptr, in_col, out_rowptr, options, rank, iterations_run, false);
-    return pagerank_impl<float>(ws, n, -1, in_rowptr, in_col, out_rowptr, options, rank, iterations_run, false);
+        return pagerank_impl<double>(ws, n, -1, in_rowptr, in_col, out_rowptr, options, rank, iterations_run, nullptr);
+    return pagerank_impl<float>(ws, n, -1, in_rowptr, in_col, out_rowptr, options, rank, iterations_run, nullptr);
 }

@@ -81,16 +81,23 @@ struct CheckVisitor {
     const int32_t* rowptr;
     const int32_t* col;
     int32_t* flags;
-    __device__ bool want_row(int32_t) const { return true; }
+    int32_t lengths;  // the length bits of the thread's rows (0 at the start)
+    __device__ bool want_row(int32_t u) {
+        const int32_t d = rowptr[u + 1] - rowptr[u];
+        if (d > 0) lengths |= tc_length_bit(d);
+        return true;
+    }
     __device__ void operator()(int32_t u, int32_t v, int32_t j) const {
         int32_t f = 0;
         if (u == v) f |= kTcFlagLoop;
         if (j + 1 < rowptr[u + 1] && col[j + 1] <= v) f |= kTcFlagUnsorted;
         if (!row_contains(col, rowptr[v], rowptr[v + 1], u)) f |= kTcFlagAsym;
-        if (j == rowptr[u]) f |= tc_length_bit(rowptr[u + 1] - j);
-        if (f & ~*(volatile const int32_t*)flags) atomicOr(flags, f);
+        if (f && (f & ~*(volatile const int32_t*)flags)) atomicOr(flags, f);
     }
-    __device__ void finish() const {}
+    __device__ void finish() const {
+        const int32_t f = (int32_t)__reduce_or_sync(0xffffffffu, (unsigned)lengths);
+        if (lane_id() == 0 && (f & ~*(volatile const int32_t*)flags)) atomicOr(flags, f);
+    }
 };
 
 __device__ __forceinline__ bool ranks_above(const int32_t* __restrict__ rowptr, int32_t u, int32_t v) {
