@@ -291,10 +291,11 @@ __device__ __forceinline__ double warp_total(KSum<T> acc) {
 }
 
 // Bound by the gathers: each takes a 32-byte sector of L2 or its own pass of
-// the L1 pipe.  12 M vertices, 160 M entries, FP64: 0.66 ms an iteration (240 G
+// the L1 pipe.  12 M vertices, 160 M entries, FP64: 0.61 ms an iteration (260 G
 // gathers/s), where a thread per short row and a warp per chunk of a longer one
-// took 0.35 + 0.49 ms; straight on the caller's ids ten iterations take 9.5 ms,
-// 19.1 before.
+// took 0.35 + 0.49 ms.  Tiles and entries are counted in 32 bits (there are
+// fewer than 2^31): in 64 the kernel spilled, 0.68 ms.  Ten iterations in all
+// 7.0 ms with 256 entries a tile, 7.1 with 224, 7.4 with 160 or 320 (spills).
 template <class T>
 __global__ void __launch_bounds__(kPrPersistThreads) pr_tile_kernel(
     PrRows R, int32_t n, const int32_t* __restrict__ in_col, const T* __restrict__ contrib_old, const T* rank_old,
@@ -307,8 +308,8 @@ __global__ void __launch_bounds__(kPrPersistThreads) pr_tile_kernel(
     const uint64_t pol_stream = policy_evict_first();
     const uint64_t pol_keep = policy_evict_last();
     const int lane = lane_id();
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int32_t warp = (int32_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    const int32_t nwarps = (int32_t)((gridDim.x * blockDim.x) >> 5);
     double sink = 0.0, l1 = 0.0;
     const double base = sc->base;
     auto finish = [&](int32_t row, int32_t d, double sum) {
@@ -316,11 +317,11 @@ __global__ void __launch_bounds__(kPrPersistThreads) pr_tile_kernel(
     };
     // A tile is a chain of columns, gathers and writes; the next tile's columns
     // and this tile's row data are loaded under the gathers.
-    auto load_cols = [&](int64_t t, int32_t (&u)[kPrPerLane]) {
-        const int64_t t0 = t * kPrTile;
+    auto load_cols = [&](int32_t t, int32_t (&u)[kPrPerLane]) {
+        const uint32_t t0 = (uint32_t)t * kPrTile;
 #pragma unroll
         for (int q = 0; q < kPrPerLane; ++q)
-            u[q] = t0 + q * 32 + lane < R.m ? ld_stream(in_col + t0 + q * 32 + lane, pol_stream) : -1;
+            u[q] = t0 + q * 32 + lane < (uint32_t)R.m ? ld_stream(in_col + t0 + q * 32 + lane, pol_stream) : -1;
     };
     int32_t ahead[kPrPerLane];
     int32_t ahead0 = 0, ahead1 = 0;
@@ -329,8 +330,8 @@ __global__ void __launch_bounds__(kPrPersistThreads) pr_tile_kernel(
         ahead0 = R.tile[warp];
         ahead1 = R.tile[warp + 1];
     }
-    for (int64_t t = warp; t < R.tiles; t += nwarps) {
-        const int64_t t0 = t * kPrTile, t1 = min(t0 + kPrTile, (int64_t)R.m);
+    for (int32_t t = warp; t < R.tiles; t += nwarps) {
+        const uint32_t t0 = (uint32_t)t * kPrTile, t1 = min(t0 + kPrTile, (uint32_t)R.m);
         T x[kPrPerLane];
         unsigned ok = 0;
 #pragma unroll
@@ -355,15 +356,15 @@ __global__ void __launch_bounds__(kPrPersistThreads) pr_tile_kernel(
             ahead0 = R.tile[t + nwarps];
             ahead1 = R.tile[t + nwarps + 1];
         }
-        if (__shfl_sync(0xffffffffu, e, 0) >= t1) {  // one row
+        if ((uint32_t)__shfl_sync(0xffffffffu, e, 0) >= t1) {  // one row
             KSum<T> acc;
 #pragma unroll
             for (int q = 0; q < kPrPerLane; ++q)
                 if ((ok >> q) & 1u) acc.add(x[q]);
             const double v = warp_total(acc);
             if (lane == 0) {
-                if (b < t0) head[t] = v;
-                else if (e > t1) tail[t] = v;
+                if ((uint32_t)b < t0) head[t] = v;
+                else if ((uint32_t)e > t1) tail[t] = v;
                 else finish(id, deg, v);
             }
             continue;
@@ -372,8 +373,8 @@ __global__ void __launch_bounds__(kPrPersistThreads) pr_tile_kernel(
         for (int q = 0; q < kPrPerLane; ++q) vals[q * 32 + lane] = x[q];
         __syncwarp();
         while (true) {
-            const int32_t s = (int32_t)(max((int64_t)b, t0) - t0);
-            const int32_t len = i <= i1 ? (int32_t)(min((int64_t)e, t1) - t0) - s : 0;  // 0 or less: the next tile's row
+            const int32_t s = (int32_t)(max((uint32_t)b, t0) - t0);
+            const int32_t len = i <= i1 ? (int32_t)(min((uint32_t)e, t1) - t0) - s : 0;  // 0 or less: the next tile's row
             double v = 0.0;
             if (len > 0 && len < 32) {
                 KSum<T> acc;
@@ -391,8 +392,8 @@ __global__ void __launch_bounds__(kPrPersistThreads) pr_tile_kernel(
                 if (lane == l) v = w;
             }
             if (len > 0) {
-                if (b < t0) head[t] = v;
-                else if (e > t1) tail[t] = v;
+                if ((uint32_t)b < t0) head[t] = v;
+                else if ((uint32_t)e > t1) tail[t] = v;
                 else finish(id, deg, v);
             }
             i += 32;
