@@ -46,11 +46,39 @@ constexpr int32_t kMsspChunk = 32;
 constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;  // +infinity
 
 struct MsspCounters {
-    int32_t queued;       // vertices queued for the next round
-    int32_t big;          // rows of the current round handed to the chunk kernel
-    unsigned long long pmin;     // smallest pending distance (bits) at or above hi
-    unsigned long long examined; // entries relaxed
+    // On lines of their own: atomics on one line follow each other at 2 ns.
+    alignas(128) int32_t queued;       // vertices queued for the next round
+    alignas(128) unsigned long long pmin;  // smallest pending distance (bits) at or above hi
+    alignas(128) int32_t big;          // rows of the current round handed to the chunk kernel
+    unsigned long long examined;       // entries relaxed
 };
+static_assert(sizeof(MsspCounters) <= 512, "two copies lie behind one another in the pinned words");
+
+// Vertices a warp has yet to queue: written kMsspStage at most at a time behind
+// one atomic on the queue's counter.
+constexpr int kMsspStage = 64;
+struct MsspStage {
+    int32_t* buf;  // kMsspStage words of the warp's
+    int32_t n = 0;
+};
+__device__ __forceinline__ void mssp_flush(MsspStage& g, int32_t* queue, MsspCounters* cnt) {
+    if (g.n == 0) return;
+    int32_t at = 0;
+    if (lane_id() == 0) at = atomicAdd(&cnt->queued, g.n);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    __syncwarp();
+    for (int32_t i = lane_id(); i < g.n; i += 32) queue[at + i] = g.buf[i];
+    __syncwarp();
+    g.n = 0;
+}
+// Every lane of the warp calls it.
+__device__ __forceinline__ void mssp_stage(MsspStage& g, bool want, int32_t u, int32_t* queue, MsspCounters* cnt) {
+    const unsigned m = __ballot_sync(0xffffffffu, want);
+    if (m == 0) return;
+    if (g.n + __popc(m) > kMsspStage) mssp_flush(g, queue, cnt);
+    if (want) g.buf[g.n + __popc(m & ((1u << lane_id()) - 1u))] = u;
+    g.n += __popc(m);
+}
 
 // Each phase is a __device__ body (grid-stride) with a thin kernel around
 // it: the host-driven pass launches the kernels, the whole-pass cooperative
@@ -71,7 +99,10 @@ __global__ void mssp_seed_kernel(const int32_t* __restrict__ srcs, int32_t k, in
 // Bucket start: act bits of the distances in [lo, hi), queue, pending min.
 __device__ __forceinline__ void mssp_scan_body(int32_t n_scan, int32_t ks, int32_t words, double lo, double hi,
                                                const unsigned long long* d, unsigned long long* act, int32_t* queue,
-                                               MsspCounters* cnt) {
+                                               MsspCounters* cnt, MsspStage& g) {
+    __shared__ unsigned long long s_pmin;
+    if (threadIdx.x == 0) s_pmin = kInfBits;
+    __syncthreads();
     const int lane = lane_id();
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -92,35 +123,38 @@ __device__ __forceinline__ void mssp_scan_body(int32_t n_scan, int32_t ks, int32
             if (lane == 0) act[v * words + w] = word;
             any |= word != 0;
         }
-        if (any && lane == 0) queue[atomicAdd(&cnt->queued, 1)] = (int32_t)v;
+        mssp_stage(g, any && lane == 0, (int32_t)v, queue, cnt);
     }
+    mssp_flush(g, queue, cnt);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) pmin = fmin(pmin, __shfl_xor_sync(0xffffffffu, pmin, o));
-    if (lane == 0 && pmin < INFINITY)
-        atomicMin(&cnt->pmin, (unsigned long long)__double_as_longlong(pmin));
+    if (lane == 0 && pmin < INFINITY) atomicMin(&s_pmin, (unsigned long long)__double_as_longlong(pmin));
+    __syncthreads();
+    if (threadIdx.x == 0 && s_pmin != kInfBits) atomicMin(&cnt->pmin, s_pmin);
 }
 __global__ void __launch_bounds__(256) mssp_scan_kernel(int32_t n_scan, int32_t ks, int32_t words, double lo,
                                                         double hi, const unsigned long long* d,
                                                         unsigned long long* act, int32_t* queue,
                                                         MsspCounters* cnt) {
-    mssp_scan_body(n_scan, ks, words, lo, hi, d, act, queue, cnt);
+    __shared__ int32_t s_stage[256 / 32][kMsspStage];
+    MsspStage g{s_stage[threadIdx.x >> 5]};
+    mssp_scan_body(n_scan, ks, words, lo, hi, d, act, queue, cnt, g);
 }
 
 // Queues the vertices u of the lanes with `want` for the next round (once each).
 __device__ __forceinline__ void mssp_queue(bool want, int32_t u, int32_t* inq_next, int32_t* queue_next,
-                                           MsspCounters* cnt) {
-    const bool first = want && atomicExch(inq_next + u, 1) == 0;
-    const int32_t at = warp_append(&cnt->queued, first);
-    if (first) queue_next[at] = u;
+                                           MsspCounters* cnt, MsspStage& g) {
+    mssp_stage(g, want && atomicExch(inq_next + u, 1) == 0, u, queue_next, cnt);
 }
 
 // Relax entries [eb, ee) of v's row for v's active sources.  A row is a chain
 // of round trips (column, distance, minimum, queue), so a warp issues those of
 // several entries together: the columns and weights of 32 entries in one load,
-// the distances of kFlight / groups entries at a time.  A distance read above
+// the distances of kMsspFlight / groups entries at a time.  A distance read above
 // the new one is lowered without waiting for the answer; whoever else lowers it
-// meanwhile marks the same target, so nothing is lost.
-constexpr int kMsspFlight = 8;  // distance loads in flight per lane
+// meanwhile marks the same target, so nothing is lost.  Targets are queued once
+// per 32 entries.
+constexpr int kMsspFlight = 4;  // distance loads in flight per lane
 struct MsspArrays {
     const int32_t* __restrict__ col;
     const double* __restrict__ wt;
@@ -135,7 +169,8 @@ struct MsspArrays {
 };
 // Lanes over sources: lane handles s = lane + 32 (g0 + t), t < GROUPS.
 template <int GROUPS>
-__device__ __forceinline__ void mssp_relax_wide(const MsspArrays& a, int32_t v, int32_t eb, int32_t ee, int g0) {
+__device__ __forceinline__ void mssp_relax_wide(const MsspArrays& a, int32_t v, int32_t eb, int32_t ee, int g0,
+                                                MsspStage& g) {
     constexpr int kB = kMsspFlight / GROUPS;  // entries per step
     const int lane = lane_id();
     double dv[GROUPS];
@@ -152,6 +187,7 @@ __device__ __forceinline__ void mssp_relax_wide(const MsspArrays& a, int32_t v, 
         const int32_t left = ee - j0 < 32 ? ee - j0 : 32;
         const int32_t uj = lane < left ? a.col[j0 + lane] : 0;
         const double wj = lane < left ? a.wt[j0 + lane] : 0.0;
+        unsigned hit = 0;  // entries with a target below hi
         for (int32_t k0 = 0; k0 < left; k0 += kB) {
             int32_t u[kB];
             double nd[kB][GROUPS], cur[kB][GROUPS];
@@ -167,7 +203,6 @@ __device__ __forceinline__ void mssp_relax_wide(const MsspArrays& a, int32_t v, 
                         cur[q][t] = __longlong_as_double((long long)__ldcg(a.d + (int64_t)u[q] * a.ks + lane + 32 * (g0 + t)));
                 }
             }
-            unsigned hit = 0;  // entries of the step with a target below hi
 #pragma unroll
             for (int q = 0; q < kB; ++q)
 #pragma unroll
@@ -181,20 +216,16 @@ __device__ __forceinline__ void mssp_relax_wide(const MsspArrays& a, int32_t v, 
                         // The group's 32 sources: half a word.
                         if (lane == 0)
                             atomicOr(reinterpret_cast<unsigned*>(a.act_next + (int64_t)u[q] * a.words) + g0 + t, m);
-                        hit |= 1u << q;
+                        hit |= 1u << (k0 + q);
                     }
                 }
-            if (hit) {
-                int32_t mine = 0;
-#pragma unroll
-                for (int q = 0; q < kB; ++q) mine = lane == q ? u[q] : mine;
-                mssp_queue((hit >> lane) & 1u, mine, a.inq_next, a.queue_next, a.cnt);
-            }
         }
+        if (hit) mssp_queue((hit >> lane) & 1u, uj, a.inq_next, a.queue_next, a.cnt, g);
     }
 }
 // Lanes over entries, the few active sources one after another.
-__device__ __forceinline__ void mssp_relax_narrow(const MsspArrays& a, int32_t v, int32_t eb, int32_t ee) {
+__device__ __forceinline__ void mssp_relax_narrow(const MsspArrays& a, int32_t v, int32_t eb, int32_t ee,
+                                                  MsspStage& g) {
     constexpr int kB = 4;
     const int lane = lane_id();
     for (int w = 0; w < a.words; ++w) {
@@ -229,13 +260,13 @@ __device__ __forceinline__ void mssp_relax_narrow(const MsspArrays& a, int32_t v
                 if (!__any_sync(0xffffffffu, near != 0)) continue;
 #pragma unroll
                 for (int q = 0; q < kB; ++q)
-                    mssp_queue((near >> q) & 1u, u[q], a.inq_next, a.queue_next, a.cnt);
+                    mssp_queue((near >> q) & 1u, u[q], a.inq_next, a.queue_next, a.cnt, g);
             }
         }
     }
 }
 __device__ __forceinline__ void mssp_relax_range(int32_t v, int32_t eb, int32_t ee, const MsspArrays& a,
-                                                 unsigned long long& examined) {
+                                                 unsigned long long& examined, MsspStage& stage) {
     int nact = 0;
     for (int w = 0; w < a.words; ++w) nact += __popcll(__ldcg(a.act_cur + (int64_t)v * a.words + w));
     if (nact >= 4) {
@@ -243,10 +274,10 @@ __device__ __forceinline__ void mssp_relax_range(int32_t v, int32_t eb, int32_t 
         // walk, and are few bytes beside the distances.
         const int groups = a.ks >> 5;
         int g = 0;
-        for (; g + 2 <= groups; g += 2) mssp_relax_wide<2>(a, v, eb, ee, g);
-        if (g < groups) mssp_relax_wide<1>(a, v, eb, ee, g);
+        for (; g + 2 <= groups; g += 2) mssp_relax_wide<2>(a, v, eb, ee, g, stage);
+        if (g < groups) mssp_relax_wide<1>(a, v, eb, ee, g, stage);
     } else {
-        mssp_relax_narrow(a, v, eb, ee);
+        mssp_relax_narrow(a, v, eb, ee, stage);
     }
     if (lane_id() == 0) examined += (unsigned long long)(ee - eb) * (unsigned long long)nact;
 }
@@ -265,6 +296,8 @@ __global__ void __launch_bounds__(256) mssp_relax_kernel(int32_t q, const int32_
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     unsigned long long examined = 0;
     const MsspArrays arrays{col, wt, d, act_cur, act_next, inq_next, queue_next, cnt, ks, words, hi};
+    __shared__ int32_t s_stage[256 / 32][kMsspStage];
+    MsspStage stage{s_stage[threadIdx.x >> 5]};
     for (int64_t i = warp; i < q; i += nwarps) {
         const int32_t v = queue[i];
         const int32_t eb = rp[v], ee = rp[v + 1];
@@ -272,8 +305,9 @@ __global__ void __launch_bounds__(256) mssp_relax_kernel(int32_t q, const int32_
             if (lane_id() == 0) big[atomicAdd(&cnt_cur->big, 1)] = v;
             continue;
         }
-        mssp_relax_range(v, eb, ee, arrays, examined);
+        mssp_relax_range(v, eb, ee, arrays, examined, stage);
     }
+    mssp_flush(stage, queue_next, cnt);
     if (lane_id() == 0 && examined) atomicAdd(&cnt->examined, examined);
 }
 
@@ -305,6 +339,8 @@ __global__ void __launch_bounds__(256) mssp_relax_big_kernel(const int32_t* __re
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     unsigned long long examined = 0;
     const MsspArrays arrays{col, wt, d, act_cur, act_next, inq_next, queue_next, cnt, ks, words, hi};
+    __shared__ int32_t s_stage[256 / 32][kMsspStage];
+    MsspStage stage{s_stage[threadIdx.x >> 5]};
     for (int64_t c = warp; c < total; c += nwarps) {
         int32_t lo = 0, hi_i = nb - 1;
         while (lo < hi_i) {
@@ -315,8 +351,9 @@ __global__ void __launch_bounds__(256) mssp_relax_big_kernel(const int32_t* __re
         const int32_t v = big[lo];
         const int32_t eb = rp[v] + (int32_t)(c - cpre[lo]) * kMsspChunk;
         const int32_t ee = min(rp[v + 1], eb + kMsspChunk);
-        mssp_relax_range(v, eb, ee, arrays, examined);
+        mssp_relax_range(v, eb, ee, arrays, examined, stage);
     }
+    mssp_flush(stage, queue_next, cnt);
     if (lane_id() == 0 && examined) atomicAdd(&cnt->examined, examined);
 }
 
@@ -366,10 +403,13 @@ __device__ __forceinline__ double mp_pmin(const MsspCounters* c) {
     return b == kInfBits ? INFINITY : __longlong_as_double((long long)b);
 }
 
-// Four blocks per SM (64 registers, a small spill): with eight distance loads
-// in flight per lane, 64 sources on RMAT-18 take 10.2 ms, against 11.0 at three
-// blocks, 10.4 at five and 11.6 at six; half the loads in flight take 10.8 ms.
-// The pass waits on its gathers and atomics.
+// Four blocks per SM (64 registers, a small spill) and four distance loads in
+// flight per lane.  64 sources, with places in the queue staged by the warp:
+// RMAT-18 with the hop pass 10.2 ms (no more with six in flight, 11.5 with eight or
+// with five blocks, 11.7 with three), uniform, 100 k vertices of degree 16,
+// 3.7; 32 sources on a 512 x 512 grid 29 ms.  Without the staging, an atomic on
+// one cache line for every vertex queued and every warp's sums in every phase,
+// 10.8, 4.8 and 43 ms.  What is left waits on gathers and minima.
 __global__ void __launch_bounds__(kMsspThreads, kMsspBlocks) mssp_pass_kernel(
     int32_t n, int32_t n_active, int32_t k, int32_t ks, int32_t words, const int32_t* __restrict__ rp,
     const int32_t* __restrict__ col, const double* __restrict__ wt, const int32_t* srcs, const int32_t* __restrict__ perm,
@@ -406,6 +446,9 @@ __global__ void __launch_bounds__(kMsspThreads, kMsspBlocks) mssp_pass_kernel(
 
     __shared__ int32_t s_st[4];
     __shared__ double s_lo;
+    __shared__ int32_t s_stage[kMsspThreads / 32][kMsspStage];
+    MsspStage stage{s_stage[threadIdx.x >> 5]};
+    unsigned long long examined = 0;
     while (true) {
         if (threadIdx.x == 0) {
             volatile MsspRunState* v = st;
@@ -428,9 +471,8 @@ __global__ void __launch_bounds__(kMsspThreads, kMsspBlocks) mssp_pass_kernel(
         MsspCounters* cn = cnt;  // the round being filled
         const double lo = s_lo, hi = lo + st->delta;
         const MsspArrays arrays{col, wt, d, act_cur, act_next, inq_next, q_next, cn, ks, words, hi};
-        unsigned long long examined = 0;
         if (phase == kMpScan) {
-            mssp_scan_body(n_active, ks, words, lo, hi, d, act_cur, q_cur, cn);
+            mssp_scan_body(n_active, ks, words, lo, hi, d, act_cur, q_cur, cn, stage);
         } else if (phase == kMpRelax) {
             for (int64_t i = warp; i < q; i += nwarps) {
                 const int32_t v = __ldcg(q_cur + i);
@@ -444,13 +486,15 @@ __global__ void __launch_bounds__(kMsspThreads, kMsspBlocks) mssp_pass_kernel(
                         chunks[pos + c] = make_int4(v, eb + c * kMsspChunk, min(ee, eb + (c + 1) * kMsspChunk), 0);
                     continue;
                 }
-                mssp_relax_range(v, eb, ee, arrays, examined);
+                mssp_relax_range(v, eb, ee, arrays, examined, stage);
             }
+            mssp_flush(stage, q_next, cn);
         } else if (phase == kMpChunks) {
             for (int64_t i = warp; i < nch; i += nwarps) {
                 const int4 ch = __ldcg(chunks + i);
-                mssp_relax_range(ch.x, ch.y, ch.z, arrays, examined);
+                mssp_relax_range(ch.x, ch.y, ch.z, arrays, examined, stage);
             }
+            mssp_flush(stage, q_next, cn);
         } else {  // kMpClear: the processed vertices' act words and queue flags
             for (int64_t i = gtid; i < q; i += gsize) {
                 const int32_t v = __ldcg(q_cur + i);
@@ -458,7 +502,6 @@ __global__ void __launch_bounds__(kMsspThreads, kMsspBlocks) mssp_pass_kernel(
                 inq_cur[v] = 0;
             }
         }
-        if (lane == 0 && examined) atomicAdd(&cn->examined, examined);
         const bool ok = grid_sync_leader(
             &st->bar_count, &st->bar_release, &st->status,
             [&]() {
@@ -476,7 +519,6 @@ __global__ void __launch_bounds__(kMsspThreads, kMsspBlocks) mssp_pass_kernel(
                     // After a scan or a clear: the queue just filled decides.
                     int32_t queued;
                     if (phase == kMpClear) {
-                        s->examined = v->examined + c->examined;
                         queued = c->queued;  // the next round's queue (q_next)
                         s->sel = v->sel ^ 1;
                     } else {
@@ -484,7 +526,6 @@ __global__ void __launch_bounds__(kMsspThreads, kMsspBlocks) mssp_pass_kernel(
                     }
                     const double pmin = mp_pmin(cnt);
                     c->queued = 0;
-                    c->examined = 0;
                     c->pmin = kInfBits;
                     if (queued > 0) {
                         s->q = queued;
@@ -514,6 +555,12 @@ __global__ void __launch_bounds__(kMsspThreads, kMsspBlocks) mssp_pass_kernel(
             bar_limit_ns, bar_extra);
         if (!ok) return;
     }
+    __shared__ unsigned long long s_examined;
+    if (threadIdx.x == 0) s_examined = 0;
+    __syncthreads();
+    if (lane == 0 && examined) atomicAdd(&s_examined, examined);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_examined) atomicAdd(&st->examined, s_examined);
     // ---- output in the caller's ids
     for (int64_t v = gtid; v < n; v += gsize) {
         const int64_t p = perm ? perm[v] : v;
@@ -695,7 +742,8 @@ int mssssp_pass(ghb_workspace* ws, int32_t n, int32_t n_active, const int32_t* r
         return GHB_OK;
     };
     auto reset = [&](MsspCounters* p) -> int {
-        const MsspCounters z{0, 0, kInfBits, 0ull};
+        MsspCounters z{};
+        z.pmin = kInfBits;
         std::memcpy(reinterpret_cast<char*>(ws->host_pinned) + 512, &z, sizeof(z));
         GHB_CUDA_TRY(cudaMemcpyAsync(p, reinterpret_cast<char*>(ws->host_pinned) + 512, sizeof(z),
                                      cudaMemcpyHostToDevice, st));

@@ -38,3 +38,28 @@ def test_groups(G, k, persistent):
         dist = rg.mssssp(sources, ws=ws)[0].cpu().numpy()
         for i in sorted({0, k // 3, k // 2, k - 1}):
             assert np.array_equal(dist[i], O.sssp(og, int(sources[i]))), (log2, i)
+
+
+@pytest.mark.parametrize("leaves", [63, 64, 65, 1000, 20000])
+@pytest.mark.parametrize("persistent", [0, 1])
+def test_queue(G, leaves, persistent):
+    """Rounds that queue around and well past a warp's buffer of 64 vertices:
+    stars whose leaves lead on to a second star."""
+    n = 2 * leaves + 10
+    hub = np.arange(3)
+    leaf = np.arange(10, 10 + leaves)
+    src = np.concatenate([np.repeat(hub, leaves), leaf, leaf])
+    dst = np.concatenate([np.tile(leaf, 3), leaf + leaves, np.full(leaves, 5)])
+    og = O.make_graph(n, src.astype(np.int32), dst.astype(np.int32), False, weight_mode=1, weight_seed=leaves)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    rg = G.ResidentGraph(G.CSRGraph(n=og.n, rowptr=t(og.rowptr), col=t(og.col), w=t(og.w), directed=False))
+    ws = G.Workspace()
+    G.tune_set("mssp_persistent", persistent, ws=ws)
+    sources = np.array([0, 1, 2, 5, 12, n - 1] * 6)[:33]
+    for log2 in (2, -4):
+        G.tune_set("mssp_width_log2", log2, ws=ws)
+        dist, st = rg.mssssp(sources, ws=ws)
+        assert st["edges_examined"] > 0
+        dist = dist.cpu().numpy()
+        for i in (0, 3, 4, 5, 32):
+            assert np.array_equal(dist[i], O.sssp(og, int(sources[i]))), (log2, i)
