@@ -78,39 +78,118 @@ __global__ void perm_from_keys_kernel(int32_t n, const uint64_t* __restrict__ ke
     }
 }
 
-// One key per entry: (new row << bits) | new col, value = entry index.  A
-// warp per row; rows of 64 or more entries read col with 16-byte loads (four
-// entries a lane) between a scalar head up to the first 4-aligned entry and
-// a scalar tail, when col starts on a 16-byte boundary.
-__global__ void relabel_keys_kernel(int32_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ col,
-                                    const int32_t* __restrict__ perm, int bits, uint64_t* keys, uint32_t* vals) {
+// One key per entry: (new row << bits) | new col, value = entry index.  A warp takes
+// 32 rows: those of 32 entries or more one after another, the others packed
+// over a scan of their lengths, four columns and their new ids in flight per
+// lane either way.  Rows of kRelabelLong entries or more are listed (longer_rows
+// [0] their number) for a block each.  Bound by the gathers of the new ids; with
+// a warp per row the longest row's chain of loads set the pace (RMAT-22: 1.85 ms;
+// 0.60 and 0.35 for the long rows).
+constexpr int32_t kRelabelLong = 2048;
+__global__ void __launch_bounds__(256) relabel_keys_kernel(int32_t n, const int32_t* __restrict__ rp,
+                                                           const int32_t* __restrict__ col,
+                                                           const int32_t* __restrict__ perm, int bits, uint64_t* keys,
+                                                           uint32_t* vals, int32_t* longer_rows) {
+    constexpr int kB = 4;
     const int lane = lane_id();
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const bool vec = ((uintptr_t)col & 15) == 0;
-    for (int64_t u = warp; u < n; u += nwarps) {
+    auto emit = [&](const int64_t (&j)[kB], const bool (&ok)[kB], const int32_t (&row)[kB]) {
+        int32_t c[kB];
+#pragma unroll
+        for (int q = 0; q < kB; ++q) c[q] = ok[q] ? col[j[q]] : 0;
+#pragma unroll
+        for (int q = 0; q < kB; ++q) c[q] = ok[q] ? perm[c[q]] : 0;
+#pragma unroll
+        for (int q = 0; q < kB; ++q)
+            if (ok[q]) {
+                keys[j[q]] = ((uint64_t)(uint32_t)row[q] << bits) | (uint64_t)(uint32_t)c[q];
+                if (vals) vals[j[q]] = (uint32_t)j[q];
+            }
+    };
+    for (int64_t base = warp * 32; base < n; base += nwarps * 32) {
+        const int64_t u = base + lane;
+        const int32_t b = u < n ? rp[u] : 0;
+        int32_t e = u < n ? rp[u + 1] : 0;
+        const int32_t nu = u < n ? perm[u] : 0;
+        unsigned longer = __ballot_sync(0xffffffffu, e - b >= 32);
+        while (longer) {
+            const int l = __ffs(longer) - 1;
+            longer &= longer - 1;
+            const int32_t lb = __shfl_sync(0xffffffffu, b, l), le = __shfl_sync(0xffffffffu, e, l);
+            const int32_t lu = __shfl_sync(0xffffffffu, nu, l);
+            if (le - lb >= kRelabelLong) {
+                if (lane == 0) longer_rows[1 + atomicAdd(longer_rows, 1)] = (int32_t)(base + l);
+                continue;
+            }
+            for (int64_t j0 = lb; j0 < le; j0 += 32 * kB) {
+                int64_t j[kB];
+                bool ok[kB];
+                int32_t row[kB];
+#pragma unroll
+                for (int q = 0; q < kB; ++q) {
+                    j[q] = j0 + 32 * q + lane;
+                    ok[q] = j[q] < le;
+                    row[q] = lu;
+                }
+                emit(j, ok, row);
+            }
+        }
+        if (e - b >= 32) e = b;
+        int32_t incl = e - b;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += x;
+        }
+        const int32_t excl = incl - (e - b), total = __shfl_sync(0xffffffffu, incl, 31);
+        for (int32_t k0 = 0; k0 < total; k0 += 32 * kB) {
+            int64_t j[kB];
+            bool ok[kB];
+            int32_t row[kB];
+#pragma unroll
+            for (int q = 0; q < kB; ++q) {
+                const int32_t k = k0 + 32 * q + lane;
+                int owner = 0;
+#pragma unroll
+                for (int s = 16; s >= 1; s >>= 1) {
+                    const int32_t at = __shfl_sync(0xffffffffu, excl, owner + s);
+                    if (at <= k) owner += s;
+                }
+                const int32_t ob = __shfl_sync(0xffffffffu, b, owner), oe = __shfl_sync(0xffffffffu, excl, owner);
+                row[q] = __shfl_sync(0xffffffffu, nu, owner);
+                ok[q] = k < total;
+                j[q] = (int64_t)ob + (k - oe);
+            }
+            emit(j, ok, row);
+        }
+    }
+}
+
+// The long rows, a block each.
+__global__ void __launch_bounds__(1024) relabel_long_kernel(const int32_t* __restrict__ rp,
+                                                            const int32_t* __restrict__ col,
+                                                            const int32_t* __restrict__ perm, int bits, uint64_t* keys,
+                                                            uint32_t* vals, const int32_t* __restrict__ longer_rows) {
+    constexpr int kB = 4;
+    const int32_t rows = longer_rows[0];
+    for (int32_t i = blockIdx.x; i < rows; i += gridDim.x) {
+        const int32_t u = longer_rows[1 + i];
+        const int64_t b = rp[u], e = rp[u + 1];
         const uint64_t nu = (uint64_t)(uint32_t)perm[u] << bits;
-        const int32_t b = rp[u], e = rp[u + 1];
-        int32_t j0 = b, j1 = b;  // [j0, j1): the 4-aligned body
-        if (vec && e - b >= 64) {
-            j0 = (b + 3) & ~3;
-            j1 = e & ~3;
-        }
-        for (int32_t j = j0 + 4 * lane; j < j1; j += 128) {
-            const int4 c = *reinterpret_cast<const int4*>(col + j);
-            keys[j] = nu | (uint64_t)(uint32_t)perm[c.x];
-            keys[j + 1] = nu | (uint64_t)(uint32_t)perm[c.y];
-            keys[j + 2] = nu | (uint64_t)(uint32_t)perm[c.z];
-            keys[j + 3] = nu | (uint64_t)(uint32_t)perm[c.w];
-            if (vals) *reinterpret_cast<uint4*>(vals + j) = make_uint4(j, j + 1, j + 2, j + 3);
-        }
-        // Head [b, j0) and tail [j1, e) (the whole row when no body).
-        const int32_t head = j0 - b;
-        const int32_t rest = head + (e - j1);
-        for (int32_t t = lane; t < rest; t += 32) {
-            const int32_t j = t < head ? b + t : j1 + (t - head);
-            keys[j] = nu | (uint64_t)(uint32_t)perm[col[j]];
-            if (vals) vals[j] = (uint32_t)j;
+        for (int64_t j0 = b + threadIdx.x; j0 < e; j0 += 1024 * kB) {
+            int32_t c[kB];
+#pragma unroll
+            for (int q = 0; q < kB; ++q) c[q] = j0 + 1024 * q < e ? col[j0 + 1024 * q] : 0;
+#pragma unroll
+            for (int q = 0; q < kB; ++q) c[q] = j0 + 1024 * q < e ? perm[c[q]] : 0;
+#pragma unroll
+            for (int q = 0; q < kB; ++q) {
+                const int64_t j = j0 + 1024 * q;
+                if (j >= e) break;
+                keys[j] = nu | (uint64_t)(uint32_t)c[q];
+                if (vals) vals[j] = (uint32_t)j;
+            }
         }
     }
 }
@@ -248,7 +327,15 @@ int relabel_csr(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* rp, cons
     Carver c(ws->scratch);
     carve(c, &k0, &k1, &v0, &v1, &tmp);
     const unsigned g = ws->num_sms * 8;
-    GHB_TRY(launch(ws, relabel_keys_kernel, dim3(g), dim3(256), 0, n, rp, col, perm, bits, k0, v0));
+    // The list of long rows (fewer than m / kRelabelLong + 1) lies where the sort
+    // writes later.
+    int32_t* longer_rows = reinterpret_cast<int32_t*>(k1);
+    GHB_CUDA_TRY(cudaMemsetAsync(longer_rows, 0, sizeof(int32_t), ws->stream));
+    GHB_TRY(launch(ws, relabel_keys_kernel, dim3(grid_for(n, 256, g)), dim3(256), 0, n, rp, col, perm, bits, k0, v0,
+                   longer_rows));
+    if (m >= kRelabelLong)
+        GHB_TRY(launch(ws, relabel_long_kernel, dim3(ws->num_sms * 2), dim3(1024), 0, rp, col, perm, bits, k0, v0,
+                       (const int32_t*)longer_rows));
     cub::DoubleBuffer<uint64_t> dk(k0, k1);
     cub::DoubleBuffer<uint32_t> dv(v0, v1);
     size_t tb = sort_tmp;
