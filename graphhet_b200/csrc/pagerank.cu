@@ -495,6 +495,14 @@ int pagerank_impl(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* in_rp,
     const bool ranked = perm != nullptr;
     cudaStream_t st = ws->stream;
     int32_t* hp = reinterpret_cast<int32_t*>(ws->host_pinned);
+    // Not to be recorded: a later call may move the scratch that a graph would
+    // replay on.
+    cudaStreamCaptureStatus recording;
+    GHB_CUDA_TRY(cudaStreamIsCapturing(st, &recording));
+    if (recording != cudaStreamCaptureStatusNone) {
+        set_error("PageRank: operation not permitted when the stream is capturing");
+        return GHB_ERR_CUDA;
+    }
     if (m < 0) {
         GHB_CUDA_TRY(cudaMemcpyAsync(hp, in_rp + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
         GHB_CUDA_TRY(cudaStreamSynchronize(st));
