@@ -50,3 +50,29 @@ def test_tiles(G, case):
         rank, ran, _ = run(iterations=60, tolerance=1e-10)
         assert ran < 60
         assert np.abs(rank.cpu().numpy() - O.pagerank(og, ran, 0.85)).sum() <= 1e-12
+
+
+def test_refuses_capture(G):
+    """A call on a capturing stream is refused, and the workspace stays usable."""
+    og = rows_graph([5, 300, 40], 2000, 4)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    rg = G.ResidentGraph(G.CSRGraph(n=og.n, rowptr=t(og.rowptr), col=t(og.col), w=None, directed=True,
+                                    in_rowptr=t(og.in_rowptr), in_col=t(og.in_col), in_w=None))
+    ws = G.Workspace()
+    first = G_rank(rg.pagerank(iterations=3, ws=ws))
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    out = torch.empty(og.n, dtype=torch.float64, device="cuda")
+    with torch.cuda.stream(side), torch.cuda.graph(graph, stream=side):
+        with pytest.raises(Exception, match="captur"):
+            rg.pagerank(iterations=3, out=out, ws=ws)
+        out.zero_()
+    torch.cuda.synchronize()
+    assert np.array_equal(G_rank(rg.pagerank(iterations=3, ws=ws)), first)
+    rg.close()
+
+
+def G_rank(result):
+    r = result[0] if isinstance(result, tuple) else result
+    return r.cpu().numpy()
