@@ -532,8 +532,9 @@ namespace ghb {
 // queue L%2 and appends to queue (L+1)%2; frontier counters are triple-
 // buffered (level L appends to slot (L+1)%3 and block 0 clears slot (L+2)%3,
 // which nobody reads or writes again before the next barrier), so one grid
-// barrier per level suffices.  After each barrier every block reads the same
-// settled counters and takes the same decision: continue, or stop when the
+// barrier per level suffices.  After each barrier every thread reads the same
+// settled counters, adds them to its own sum of the entries reached (nothing
+// that block 0 still writes) and takes the same decision: continue, or stop when the
 // frontier is empty, when its out-entries reach exit_edges, at max_depth, or
 // when the direction rule (frontier entries > unexplored entries / alpha)
 // asks for a bottom-up level.
@@ -549,6 +550,7 @@ __global__ void __launch_bounds__(1024) bfs_push_persistent_kernel(
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     int32_t level = start_level;
     int L = 0;  // levels done in this launch
+    unsigned long long m_r = 0;  // entries out of the vertices they reached
     while (true) {
         volatile int32_t* vtail = ps->tail;
         const int32_t n_f = vtail[L % 3];
@@ -617,14 +619,15 @@ __global__ void __launch_bounds__(1024) bfs_push_persistent_kernel(
         const int32_t nf_next = vtail[L % 3];
         const unsigned long long mf_next = ((volatile unsigned long long*)ps->mf)[L % 3];
         const unsigned int dmax_next = ((volatile unsigned int*)ps->dmax)[L % 3];
+        m_r += mf_next;
         if (blockIdx.x == 0 && threadIdx.x == 0) {
-            ps->m_r += mf_next;
+            ps->m_r = m_r;
             ps->reached += nf_next;
             ps->levels_done = L;
         }
         // Stop for an empty frontier, at max_depth, when the frontier is too
         // big for one launch, or when the direction rule asks for bottom-up.
-        const double m_u = (double)(m_total - m_r_start - (int64_t)ps->m_r);
+        const double m_u = (double)(m_total - m_r_start - (int64_t)m_r);
         // Rows are walked by one warp each here, so a frontier holding a row of
         // kBigList entries or more goes back to the balanced host-driven path.
         if (nf_next == 0 || (int64_t)mf_next >= exit_edges || level >= max_depth || dmax_next >= (unsigned)kBigList ||
