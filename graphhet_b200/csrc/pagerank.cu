@@ -150,6 +150,8 @@ __device__ __forceinline__ void block_partials(double sink, double l1, double* p
 // pr_blocks_per_sm per SM, 1024 x 1 by default), so each fills the cache once
 // per launch.
 constexpr int kPrPersistThreads = 1024;
+// The most that a block may ask for beside its static words.
+constexpr int kPrMaxSmem = 226 * 1024;
 
 template <class T>
 __device__ __forceinline__ int32_t fill_hub_cache(T* cache, const T* __restrict__ contrib_old, int32_t n,
@@ -568,7 +570,9 @@ int pagerank_impl(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* in_rp,
     carve(c);
 
     const double d = o->damping;
-    GHB_CUDA_TRY(cudaFuncSetAttribute(pr_tile_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // One limit for every call: it belongs to the process, and another thread's
+    // call on another graph may lie between this and the launches below.
+    GHB_CUDA_TRY(cudaFuncSetAttribute(pr_tile_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrMaxSmem));
     // ps, pl, sc, bare_count and done lie behind one another.
     GHB_CUDA_TRY(cudaMemsetAsync(ps, 0, (size_t)(reinterpret_cast<char*>(done + 1) - reinterpret_cast<char*>(ps)), st));
     GHB_TRY(launch(ws, pr_init_kernel<T>, dim3(grid_init), dim3(kPrThreads), 0, n, out_rp, outdeg, ra, ca, cb, ps));
