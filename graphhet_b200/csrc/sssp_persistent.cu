@@ -35,6 +35,7 @@
 
 #include "common.cuh"
 #include "graph.cuh"
+#include "row_math.cuh"
 
 namespace ghb {
 
@@ -367,7 +368,7 @@ __device__ __forceinline__ void sp_rows(const SpCtx& c, int32_t u, int32_t b, in
         // One atomic for the warp's long rows; the first kOwn chunks of a row
         // are written by its lane, further ones by the warp.
         constexpr int32_t kOwn = 4;
-        const int32_t nch = e - b > kSpDirect ? (e - b + kSpChunk - 1) / kSpChunk : 0;
+        const int32_t nch = e - b > kSpDirect ? chunk_count(e - b, kSpChunk) : 0;
         int32_t incl = nch;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -379,7 +380,7 @@ __device__ __forceinline__ void sp_rows(const SpCtx& c, int32_t u, int32_t b, in
         pos = __shfl_sync(0xffffffffu, pos, 31) + incl - nch;
         for (int32_t k = 0; k < min(nch, kOwn); ++k) {
             const int32_t cb = b + k * kSpChunk;
-            c.chunks[pos + k] = make_int4(u, cb, min(e, cb + kSpChunk), 0);
+            c.chunks[pos + k] = make_int4(u, cb, chunk_end(cb, kSpChunk, e), 0);
         }
         unsigned many = __ballot_sync(0xffffffffu, nch > kOwn);
         while (many) {
@@ -390,7 +391,7 @@ __device__ __forceinline__ void sp_rows(const SpCtx& c, int32_t u, int32_t b, in
             const int32_t ln = __shfl_sync(0xffffffffu, nch, leader);
             for (int32_t k = kOwn + lane; k < ln; k += 32) {
                 const int32_t cb = lb + k * kSpChunk;
-                c.chunks[lpos + k] = make_int4(lu, cb, min(lend, cb + kSpChunk), 0);
+                c.chunks[lpos + k] = make_int4(lu, cb, chunk_end(cb, kSpChunk, lend), 0);
             }
         }
         if (nch) e = b;
