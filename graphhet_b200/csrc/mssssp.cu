@@ -32,6 +32,7 @@
 
 #include "common.cuh"
 #include "graph.cuh"
+#include "row_math.cuh"
 #include "scan.cuh"
 
 namespace ghb {
@@ -183,8 +184,8 @@ __device__ __forceinline__ void mssp_relax_wide(const MsspArrays& a, int32_t v, 
         on |= live ? 1u << t : 0u;
     }
     if (!__any_sync(0xffffffffu, on != 0)) return;
-    for (int32_t j0 = eb; j0 < ee; j0 += 32) {
-        const int32_t left = ee - j0 < 32 ? ee - j0 : 32;
+    for (uint32_t j0 = (uint32_t)eb; j0 < (uint32_t)ee; j0 += 32) {  // passes 2^31 behind the last entries
+        const int32_t left = (uint32_t)ee - j0 < 32u ? (int32_t)((uint32_t)ee - j0) : 32;
         const int32_t uj = lane < left ? a.col[j0 + lane] : 0;
         const double wj = lane < left ? a.wt[j0 + lane] : 0.0;
         unsigned hit = 0;  // entries with a target below hi
@@ -317,7 +318,7 @@ __global__ void mssp_big_chunks_kernel(const int32_t* __restrict__ big, const Ms
     const int32_t nb = cnt_cur->big;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nb; i += (int64_t)gridDim.x * blockDim.x) {
         const int32_t v = big[i];
-        nch[i] = (rp[v + 1] - rp[v] + kMsspChunk - 1) / kMsspChunk;
+        nch[i] = chunk_count(rp[v + 1] - rp[v], kMsspChunk);
     }
 }
 
@@ -350,7 +351,7 @@ __global__ void __launch_bounds__(256) mssp_relax_big_kernel(const int32_t* __re
         }
         const int32_t v = big[lo];
         const int32_t eb = rp[v] + (int32_t)(c - cpre[lo]) * kMsspChunk;
-        const int32_t ee = min(rp[v + 1], eb + kMsspChunk);
+        const int32_t ee = chunk_end(eb, kMsspChunk, rp[v + 1]);
         mssp_relax_range(v, eb, ee, arrays, examined, stage);
     }
     mssp_flush(stage, queue_next, cnt);
@@ -478,12 +479,14 @@ __global__ void __launch_bounds__(kMsspThreads, kMsspBlocks) mssp_pass_kernel(
                 const int32_t v = __ldcg(q_cur + i);
                 const int32_t eb = rp[v], ee = rp[v + 1];
                 if (ee - eb > kMsspWarpRow) {
-                    const int32_t nc = (ee - eb + kMsspChunk - 1) / kMsspChunk;
+                    const int32_t nc = chunk_count(ee - eb, kMsspChunk);
                     int32_t pos = 0;
                     if (lane == 0) pos = atomicAdd(&st->c_tail, nc);
                     pos = __shfl_sync(0xffffffffu, pos, 0);
-                    for (int32_t c = lane; c < nc; c += 32)
-                        chunks[pos + c] = make_int4(v, eb + c * kMsspChunk, min(ee, eb + (c + 1) * kMsspChunk), 0);
+                    for (int32_t c = lane; c < nc; c += 32) {
+                        const int32_t cb = eb + c * kMsspChunk;
+                        chunks[pos + c] = make_int4(v, cb, chunk_end(cb, kMsspChunk, ee), 0);
+                    }
                     continue;
                 }
                 mssp_relax_range(v, eb, ee, arrays, examined, stage);

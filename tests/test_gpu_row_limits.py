@@ -42,3 +42,21 @@ def test_sssp(graph, delta):
     dist, st = G.sssp(g, 1, inf=float("inf"), delta=delta)
     assert np.array_equal(dist.cpu().numpy(), want)
     assert st["reached"] == ROW + 1
+
+
+@pytest.mark.parametrize("persistent", [0, 1])
+@pytest.mark.parametrize("k", [1, 40, 70])  # a lane per entry; per source, one group of 32 and two
+def test_multi_source(graph, persistent, k):
+    import ctypes
+    import graphhet_b200 as G
+    g, want = graph
+    ws = G.Workspace()
+    G.tune_set("mssp_persistent", persistent, ws=ws)
+    srcs = torch.ones(k, dtype=torch.int32, device="cuda")
+    dist = torch.empty(k, N, dtype=torch.float64, device="cuda")
+    st = G.TraversalStats()
+    rc = G.lib().ghb_mssssp(ws.handle, N, G._ptr(g.rowptr), G._ptr(g.col), G._ptr(g.w), G._ptr(srcs), k,
+                            float("inf"), G._ptr(dist), ctypes.byref(st))
+    assert rc == 0, G.lib().ghb_last_error()
+    assert (dist.cpu().numpy() == want).all()
+    ws.close()
