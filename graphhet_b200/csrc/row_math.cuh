@@ -23,4 +23,7 @@ GHB_HD int32_t chunk_end(int32_t at, int32_t size, int32_t end) {
     return e < (uint32_t)end ? (int32_t)e : end;
 }
 
+// Middle of positions lo <= hi (their sum passes 2^31 from 2^30 entries on).
+GHB_HD int32_t row_middle(int32_t lo, int32_t hi) { return lo + ((hi - lo) >> 1); }
+
 }  // namespace ghb

@@ -27,6 +27,7 @@
 #include "edge_walk.cuh"
 #include "graph.cuh"
 #include "policy.cuh"
+#include "row_math.cuh"
 
 namespace ghb {
 
@@ -310,7 +311,7 @@ __global__ void light_end_kernel(int32_t n, const int32_t* __restrict__ rp, cons
     for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
         int32_t lo = rp[u], hi = rp[u + 1];
         while (lo < hi) {
-            const int32_t mid = (lo + hi) >> 1;
+            const int32_t mid = row_middle(lo, hi);
             if (sw_w[mid] < delta) lo = mid + 1;
             else hi = mid;
         }

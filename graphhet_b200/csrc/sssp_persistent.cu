@@ -844,7 +844,7 @@ __global__ void sp_light_end_kernel(int32_t n, const int32_t* __restrict__ rp, c
     for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
         int32_t lo = rp[u], hi = rp[u + 1];
         while (lo < hi) {
-            const int32_t mid = (lo + hi) >> 1;
+            const int32_t mid = row_middle(lo, hi);
             if (sw_w[mid] < delta) lo = mid + 1;
             else hi = mid;
         }

@@ -22,6 +22,7 @@
 #include "common.cuh"
 #include "edge_walk.cuh"
 #include "graph.cuh"
+#include "row_math.cuh"
 #include "scan.cuh"
 
 namespace ghb {
@@ -49,7 +50,7 @@ __device__ __forceinline__ int32_t lower_bound_from(const int32_t* __restrict__ 
     b = lo + 1;
     e = step < e - lo ? lo + step : e;  // col[e] >= x, or e is the row end
     while (b < e) {
-        const int32_t mid = b + ((e - b) >> 1);
+        const int32_t mid = row_middle(b, e);
         if (col[mid] < x) b = mid + 1;
         else e = mid;
     }
@@ -59,7 +60,7 @@ __device__ __forceinline__ int32_t lower_bound_from(const int32_t* __restrict__ 
 // First position in [b, e) of a sorted row whose entry is > x (e if none).
 __device__ __forceinline__ int32_t upper_bound_pos(const int32_t* __restrict__ col, int32_t b, int32_t e, int32_t x) {
     while (b < e) {
-        const int32_t mid = b + ((e - b) >> 1);
+        const int32_t mid = row_middle(b, e);
         if (col[mid] <= x) b = mid + 1;
         else e = mid;
     }
@@ -68,7 +69,7 @@ __device__ __forceinline__ int32_t upper_bound_pos(const int32_t* __restrict__ c
 
 __device__ __forceinline__ bool row_contains(const int32_t* __restrict__ col, int32_t b, int32_t e, int32_t x) {
     while (b < e) {
-        const int32_t mid = (b + e) >> 1;
+        const int32_t mid = row_middle(b, e);
         const int32_t y = col[mid];
         if (y == x) return true;
         if (y < x) b = mid + 1;

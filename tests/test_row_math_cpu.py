@@ -1,4 +1,4 @@
-"""Chunk positions at the largest CSRs (2^31 - 1 entries), compiled for the
+"""Chunk positions and midpoints at the largest CSRs (2^31 - 1 entries), compiled for the
 host and compared with Python's integers."""
 import ctypes
 import os
@@ -11,6 +11,7 @@ SOURCE = """
 #include "row_math.cuh"
 extern "C" int32_t count(int32_t len, int32_t size) { return ghb::chunk_count(len, size); }
 extern "C" int32_t end(int32_t at, int32_t size, int32_t e) { return ghb::chunk_end(at, size, e); }
+extern "C" int32_t middle(int32_t lo, int32_t hi) { return ghb::row_middle(lo, hi); }
 """
 TOP = 2**31 - 1
 
@@ -31,3 +32,9 @@ def test_chunks_up_to_the_last_entry(host, size):
     for end in [1, size, size + 5, 2**30, TOP - size, TOP - 1, TOP]:
         for at in [max(0, end - k) for k in (1, 2, size - 1, size, size + 1, 3 * size)]:
             assert host.end(at, size, end) == min(end, at + size)
+
+
+def test_midpoints_past_2_30(host):
+    for hi in [0, 1, 7, 2**30, 2**30 + 1, TOP - 1, TOP]:
+        for lo in [0, hi // 2, max(0, hi - 9), max(0, hi - 1), hi]:
+            assert host.middle(lo, hi) == (lo + hi) // 2
