@@ -21,6 +21,7 @@ void clear_error();
     do {                                                                           \
         cudaError_t _e = (expr);                                                   \
         if (_e != cudaSuccess) {                                                   \
+            cudaGetLastError(); /* reported here, not by the next launch's check */ \
             ::ghb::set_error(std::string(#expr) + ": " + cudaGetErrorString(_e) +  \
                              " (" __FILE__ ":" + std::to_string(__LINE__) + ")");   \
             return _e == cudaErrorMemoryAllocation ? GHB_ERR_OUT_OF_MEMORY          \

@@ -1013,6 +1013,36 @@ int tc_oriented_core(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* row
     return GHB_OK;
 }
 
+int tc_run_cached(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int32_t* col, int64_t* counts64,
+                  int32_t* counts32, int64_t* total, std::atomic<int32_t>* flags_cache, bool ranked);
+
+// Raw rows through a copy relabelled by degree (in the workspace's stage); check:
+// the rows' flags.
+static int tc_by_ranks(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* rowptr, const int32_t* col,
+                       int64_t* counts64, int32_t* counts32, int64_t* total, int32_t check) {
+    int32_t *perm, *iperm, *rp, *rcol, *repeat, *nact;
+    int64_t* by_rank;
+    auto stage = [&](Carver& k) {
+        perm = k.take<int32_t>(n);
+        iperm = k.take<int32_t>(n);
+        rp = k.take<int32_t>((size_t)n + 1);
+        rcol = k.take<int32_t>(m);
+        repeat = k.take<int32_t>(1);
+        by_rank = k.take<int64_t>(n);
+    };
+    Carver need(nullptr);
+    stage(need);
+    GHB_TRY(ws_reserve_stage(ws, need.off));
+    Carver k(ws->stage);
+    stage(k);
+    GHB_TRY(rank_by_degree(ws, n, rowptr, nullptr, perm, iperm, &nact));
+    GHB_TRY(relabel_csr(ws, n, m, rowptr, col, nullptr, perm, rp, rcol, nullptr, repeat));
+    std::atomic<int32_t> known{check};
+    GHB_TRY(tc_run_cached(ws, n, rp, rcol, by_rank, nullptr, total, &known, true));
+    return launch(ws, tc_unrank_kernel, dim3(grid_for(n, 256, ws->num_sms * 8)), dim3(256), 0, n, (const int32_t*)perm,
+                  (const int64_t*)by_rank, counts64, counts32);
+}
+
 // flags_cache (may be NULL): the input check's flags for this CSR, -1 when
 // not yet known; a known value skips the check.  ranked: ids are ranks by
 // degree, hubs first (a resident graph's).
@@ -1044,14 +1074,17 @@ int tc_run_cached(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int
         bsums = c.take<int64_t>(scan_scratch_words(n));
         ocol = c.take<int32_t>(m > 0 ? m : 1);
     };
-    Carver sizing(nullptr);
-    carve(sizing);
-    GHB_TRY(ws_reserve(ws, sizing.off));
-    Carver c(ws->scratch);
-    carve(c);
-
-    GHB_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * n, st));
-    GHB_CUDA_TRY(cudaMemsetAsync(tot, 0, sizeof(unsigned long long), st));
+    auto reserve = [&]() -> int {
+        Carver sizing(nullptr);
+        carve(sizing);
+        GHB_TRY(ws_reserve(ws, sizing.off));
+        Carver c(ws->scratch);
+        carve(c);
+        GHB_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * n, st));
+        GHB_CUDA_TRY(cudaMemsetAsync(tot, 0, sizeof(unsigned long long), st));
+        return GHB_OK;
+    };
+    GHB_TRY(reserve());
     int32_t check = flags_cache ? flags_cache->load(std::memory_order_relaxed) : -1;
     if (check < 0) {
         GHB_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int32_t), st));
@@ -1070,28 +1103,17 @@ int tc_run_cached(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int
         // long rows the copy costs more than the count (an ER graph of as many
         // entries counts in 1.2 ms), and so it does on a small graph (RMAT,
         // 1,000 vertices: 0.18 ms against 0.31).
-        GHB_CUDA_TRY(cudaStreamSynchronize(st));
-        int32_t *perm, *iperm, *rp, *rcol, *repeat, *nact;
-        int64_t* by_rank;
-        auto stage = [&](Carver& k) {
-            perm = k.take<int32_t>(n);
-            iperm = k.take<int32_t>(n);
-            rp = k.take<int32_t>((size_t)n + 1);
-            rcol = k.take<int32_t>(m);
-            repeat = k.take<int32_t>(1);
-            by_rank = k.take<int64_t>(n);
-        };
-        Carver need(nullptr);
-        stage(need);
-        GHB_TRY(ws_reserve_stage(ws, need.off));
-        Carver k(ws->stage);
-        stage(k);
-        GHB_TRY(rank_by_degree(ws, n, rowptr, nullptr, perm, iperm, &nact));
-        GHB_TRY(relabel_csr(ws, n, m, rowptr, col, nullptr, perm, rp, rcol, nullptr, repeat));
-        std::atomic<int32_t> known{check};
-        GHB_TRY(tc_run_cached(ws, n, rp, rcol, by_rank, nullptr, total, &known, true));
-        return launch(ws, tc_unrank_kernel, dim3(grid_for(n, 256, ws->num_sms * 8)), dim3(256), 0, n, (const int32_t*)perm,
-                      (const int64_t*)by_rank, counts64, counts32);
+        const int done = tc_by_ranks(ws, n, m, rowptr, col, counts64, counts32, total, check);
+        if (done != GHB_ERR_OUT_OF_MEMORY) return done;
+        // The copy (20 bytes an entry) does not fit: its place is given back and
+        // the hash kernels count on the caller's ids, in a third of that.
+        if (ws->stage) {
+            GHB_CUDA_TRY(cudaStreamSynchronize(st));
+            GHB_CUDA_TRY(cudaFree(ws->stage));
+            ws->stage = nullptr;
+            ws->stage_cap = 0;
+        }
+        GHB_TRY(reserve());
     }
     if (oriented && ranked) {
         GHB_TRY(tc_count_ranked(ws, n, m, rowptr, col, cnt, wb, lists, rk, check));
