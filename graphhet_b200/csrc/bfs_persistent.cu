@@ -527,9 +527,13 @@ __device__ __noinline__ void level_eval(const float* pol, const float* feat, flo
     if (margin < band) policy_eval_block(pol, feat, h1, h2, logit);
 }
 
-// kSquad: with squad runs (graphs of low mean degree).  A variant of its own:
-// the runs' shared memory and registers cost a graph whose levels are few and
-// wide about a tenth (RMAT-24: 0.59 ms instead of 0.52).
+// kSquad: with squad runs (see bfs_squads).  A variant of its own: the runs'
+// shared memory and registers cost a graph whose levels are few and wide about
+// a tenth (RMAT-24: 0.59 ms instead of 0.52), and levels that the whole grid runs
+// as much (a 300 x 300 grid forced bottom-up: 3.7 ms instead of 3.3).  What only
+// the runs need is left out of the other by `if constexpr`: under plain conditions
+// on kSquad its levels took 0.3 us more each (1000 x 1000 grid, every level
+// top-down on the grid: 13.2 ms instead of 12.6).
 template <bool kSquad>
 __global__ void __launch_bounds__(512, 2) bfs_persistent_kernel(
     int32_t n, int32_t n_active, const int32_t* __restrict__ out_rp, const int32_t* __restrict__ out_col,
@@ -562,12 +566,10 @@ __global__ void __launch_bounds__(512, 2) bfs_persistent_kernel(
     // stays in L2, and no block pays to stage it in shared memory.
     const bool net = pol != nullptr;
     const bool can_pull = in_rp != nullptr;
-    // Small levels run on the squad where nothing asks for a level's timing,
-    // features or a given schedule.  They stay top-down whatever the direction
-    // rule says: so few entries cost less than a bottom-up level's barrier.
-    const bool squad_ok = kSquad && !trace && !net && (policy == GHB_POLICY_HEURISTIC || policy == GHB_POLICY_PUSH);
-    auto squad_fits = [&](int32_t rows, unsigned long long entries) {
-        return squad_ok && rows <= kSquadRows && entries <= kSquadEntries;
+    // A small frontier goes to the squad.  Its levels stay top-down whatever the
+    // direction rule says: so few entries cost less than a bottom-up level's barrier.
+    auto squad_fits = [](int32_t rows, unsigned long long entries) {
+        return rows <= kSquadRows && entries <= kSquadEntries;
     };
     SquadShared* s_squad = nullptr;
     SquadCtx* s_ctx = nullptr;
@@ -576,16 +578,16 @@ __global__ void __launch_bounds__(512, 2) bfs_persistent_kernel(
         __shared__ SquadCtx squad_ctx;
         s_squad = &squad_shared;
         s_ctx = &squad_ctx;
-    }
-    if (kSquad && threadIdx.x == 0) {
-        s_ctx->rp = out_rp;
-        s_ctx->col = out_col;
-        s_ctx->visited = visited;
-        s_ctx->depth = depth;
-        s_ctx->queue[0] = qa, s_ctx->queue[1] = qb, s_ctx->queue[2] = qc;
-        s_ctx->f[0] = f0, s_ctx->f[1] = f1, s_ctx->f[2] = f2;
-        s_ctx->st = st;
-        s_ctx->max_depth = max_depth;
+        if (threadIdx.x == 0) {
+            s_ctx->rp = out_rp;
+            s_ctx->col = out_col;
+            s_ctx->visited = visited;
+            s_ctx->depth = depth;
+            s_ctx->queue[0] = qa, s_ctx->queue[1] = qb, s_ctx->queue[2] = qc;
+            s_ctx->f[0] = f0, s_ctx->f[1] = f1, s_ctx->f[2] = f2;
+            s_ctx->st = st;
+            s_ctx->max_depth = max_depth;
+        }
     }
     // The first level's state, worked out by every block (s_pl: the state
     // payload each barrier hands on; see p_sync).
@@ -652,69 +654,71 @@ __global__ void __launch_bounds__(512, 2) bfs_persistent_kernel(
         const int32_t* q_clear = cslot == 0 ? qa : (cslot == 1 ? qb : qc);
         const int32_t clear_nf = last_nf;
         const bool clear_sparse = last_top && (int64_t)clear_nf * 4 < words;
-        if (kSquad && (pl & kPlSquad)) {
-            // ---- the squad runs this level and the small ones after it; the
-            // other blocks wait at the barrier below.
-            if ((int)blockIdx.x < kSquadBlocks) {
-                if (!bfs_squad_run(*s_ctx, *s_squad, L, n_f, clear_sparse ? clear_nf : 0, clear_sparse ? 0 : words))
-                    return;
-            }
-            // Whichever block closes the barrier sets the handed-back
-            // frontier's bits and decides by the rule of any level.
-            if (!p_sync(st, [&]() {
-                    const int32_t nf = vs->squad_queue, lev = vs->squad_level;
-                    const int fs = lev % 3;
-                    uint32_t* f_out = fs == 0 ? f0 : (fs == 1 ? f1 : f2);
-                    const int32_t* q_out = fs == 0 ? qa : (fs == 1 ? qb : qc);
-                    for (int32_t i = threadIdx.x; i < nf; i += blockDim.x) {
-                        const int32_t u = __ldcg(q_out + i);
-                        atomicOr(f_out + (u >> 5), 1u << (u & 31));
-                    }
-                    if (threadIdx.x == 0) {
-                        const unsigned long long mf = vs->squad_mf, mr = vs->squad_mr, m_r = vs->m_r + mr;
-                        // The run expanded its first frontier and all that it
-                        // reached but the last.
-                        const unsigned long long ex = vs->examined + vs->mf[slot] + mr - mf;
-                        const bool done = nf == 0 || lev >= max_depth;
-                        const double m_u = (double)(m_total - (long long)m_r);
-                        const bool again = !done && squad_fits(nf, mf);
-                        const int nd = policy != GHB_POLICY_PUSH && can_pull && !again && (double)mf > m_u / alpha &&
-                                               (double)mf > (double)m_total / gamma
-                                           ? 1
-                                           : 0;
-                        s_pl = p_payload(nf, done, nd, p_append(nd, 0, mf) != 0, true) | (again ? kPlSquad : 0ull);
-                        st->examined = ex;
-                        st->ex_prev = ex;
-                        st->m_r = m_r;
-                        st->reached = vs->reached + (long long)vs->squad_reached;
-                        st->levels = lev;
-                        st->level = lev;
-                        st->t_prev = global_timer_ns();
-                        st->dir = nd;
-                        st->append = p_append(nd, 0, mf);
-                        st->queue_ok = 1;
-                        st->done = done ? 1 : 0;
-                        for (int k = 0; k < 3; ++k) {
-                            st->nf[k] = 0;
-                            st->mf[k] = 0;
-                            st->d2[k] = 0;
-                            st->dmax[k] = 0;
-                            st->big[k] = 0;
-                            st->squad[k].word = 0;
+        if constexpr (kSquad) {
+            if (pl & kPlSquad) {
+                // ---- the squad runs this level and the small ones after it; the
+                // other blocks wait at the barrier below.
+                if ((int)blockIdx.x < kSquadBlocks) {
+                    if (!bfs_squad_run(*s_ctx, *s_squad, L, n_f, clear_sparse ? clear_nf : 0, clear_sparse ? 0 : words))
+                        return;
+                }
+                // Whichever block closes the barrier sets the handed-back
+                // frontier's bits and decides by the rule of any level.
+                if (!p_sync(st, [&]() {
+                        const int32_t nf = vs->squad_queue, lev = vs->squad_level;
+                        const int fs = lev % 3;
+                        uint32_t* f_out = fs == 0 ? f0 : (fs == 1 ? f1 : f2);
+                        const int32_t* q_out = fs == 0 ? qa : (fs == 1 ? qb : qc);
+                        for (int32_t i = threadIdx.x; i < nf; i += blockDim.x) {
+                            const int32_t u = __ldcg(q_out + i);
+                            atomicOr(f_out + (u >> 5), 1u << (u & 31));
                         }
-                        st->mf[fs] = mf;  // a run that follows starts from it
-                        st->squad_queue = 0;
-                        st->squad_mf = 0;
-                        st->squad_mr = 0;
-                        st->squad_reached = 0;
-                    }
-                }, &s_pl))
-                return;
-            if (s_pl & kPlDone) break;
-            L = vs->level - 1;  // the run's last level: its bits are cleared already
-            last_nf = 0;
-            last_top = true;
-            continue;
+                        if (threadIdx.x == 0) {
+                            const unsigned long long mf = vs->squad_mf, mr = vs->squad_mr, m_r = vs->m_r + mr;
+                            // The run expanded its first frontier and all that it
+                            // reached but the last.
+                            const unsigned long long ex = vs->examined + vs->mf[slot] + mr - mf;
+                            const bool done = nf == 0 || lev >= max_depth;
+                            const double m_u = (double)(m_total - (long long)m_r);
+                            const bool again = !done && squad_fits(nf, mf);
+                            const int nd = policy != GHB_POLICY_PUSH && can_pull && !again && (double)mf > m_u / alpha &&
+                                                   (double)mf > (double)m_total / gamma
+                                               ? 1
+                                               : 0;
+                            s_pl = p_payload(nf, done, nd, p_append(nd, 0, mf) != 0, true) | (again ? kPlSquad : 0ull);
+                            st->examined = ex;
+                            st->ex_prev = ex;
+                            st->m_r = m_r;
+                            st->reached = vs->reached + (long long)vs->squad_reached;
+                            st->levels = lev;
+                            st->level = lev;
+                            st->t_prev = global_timer_ns();
+                            st->dir = nd;
+                            st->append = p_append(nd, 0, mf);
+                            st->queue_ok = 1;
+                            st->done = done ? 1 : 0;
+                            for (int k = 0; k < 3; ++k) {
+                                st->nf[k] = 0;
+                                st->mf[k] = 0;
+                                st->d2[k] = 0;
+                                st->dmax[k] = 0;
+                                st->big[k] = 0;
+                                st->squad[k].word = 0;
+                            }
+                            st->mf[fs] = mf;  // a run that follows starts from it
+                            st->squad_queue = 0;
+                            st->squad_mf = 0;
+                            st->squad_mr = 0;
+                            st->squad_reached = 0;
+                        }
+                    }, &s_pl))
+                    return;
+                if (s_pl & kPlDone) break;
+                L = vs->level - 1;  // the run's last level: its bits are cleared already
+                last_nf = 0;
+                last_top = true;
+                continue;
+            }
         }
         last_nf = n_f;
         last_top = dir == 0;
@@ -824,9 +828,10 @@ __global__ void __launch_bounds__(512, 2) bfs_persistent_kernel(
                 // also clear this level's bits: a traversal that is still
                 // narrow after kSquadLevel levels repays the hand-over (about
                 // two levels' time each way).
-                if (kSquad && !done && L >= kSquadLevel && dir == 0 && append && squad_fits(nf_next, mf_next) &&
-                    ((int64_t)n_f * 4 < words ? n_f <= 4 * kSquadRows : words <= kSquadWords))
-                    s_pl |= kPlSquad;
+                if constexpr (kSquad)
+                    if (!done && L >= kSquadLevel && dir == 0 && append && squad_fits(nf_next, mf_next) &&
+                        ((int64_t)n_f * 4 < words ? n_f <= 4 * kSquadRows : words <= kSquadWords))
+                        s_pl |= kPlSquad;
                 st->nf[cslot] = 0;
                 st->mf[cslot] = 0;
                 st->d2[cslot] = 0;
@@ -1133,6 +1138,14 @@ bool bfs_persistent_available(ghb_workspace* ws, int* blocks) {
     return *blocks > 0;
 }
 
+// Which calls run small levels on the squad: those on meshes, road networks and
+// paths, up to 4.5 entries per vertex (a random graph with six has ten levels,
+// and the larger kernel cost it 5 %), when nothing asks for a level's timing, a
+// given schedule, bottom-up levels or the network's choice.
+static bool bfs_squads(int32_t n, int64_t m, int policy, bool traced) {
+    return 2 * m <= 9 * (int64_t)n && !traced && (policy == GHB_POLICY_HEURISTIC || policy == GHB_POLICY_PUSH);
+}
+
 // One cooperative launch for the whole traversal.  depth: per-vertex output
 // in the graph's ids; with perm, src is the caller's id and
 // depth_out[v] = depth[perm[v]] as well.  m: the entries where the caller
@@ -1204,11 +1217,9 @@ int bfs_persistent_run(ghb_workspace* ws, int32_t n, int32_t n_active, int64_t m
         GHB_CUDA_TRY(cudaStreamSynchronize(st));
         m_total = hp[0];
     }
+    const bool squads = bfs_squads(n, m_total, policy, tcap > 0);
     if (stats) GHB_CUDA_TRY(cudaEventRecord(ws->ev_start, st));
-    // Meshes, road networks, paths: up to 4.5 entries per vertex.  (A random
-    // graph with six has ten levels, and the larger kernel cost it 5 %.)
-    const bool low_degree = 2 * m_total <= 9 * (int64_t)n;
-    GHB_TRY(launch_coop(ws, low_degree ? bfs_persistent_kernel<true> : bfs_persistent_kernel<false>, dim3(blocks),
+    GHB_TRY(launch_coop(ws, squads ? bfs_persistent_kernel<true> : bfs_persistent_kernel<false>, dim3(blocks),
                         dim3(512), 0, n,
                         n_active, out_rp, out_col, in_rp, in_col, src, max_depth, depth, vis, f0, f1, f2, qa, qb, qc, big,
                         policy, alpha, beta, gamma, (float)ws->tune.pol_band, m_total,
