@@ -54,6 +54,9 @@ struct ghb_gpma {
     double* s_val = nullptr;
     int64_t s_col_cap = 0, s_val_cap = 0;
     bool s_ok = false, s_val_ok = false;
+    // What the program does with a version: exported, looked at in the snapshot
+    // (s_seen); s_both: both, the last version that was exported.
+    bool s_exported = false, s_seen = false, s_both = false;
     int64_t version = 0;
     int64_t stats[GHB_GPMA_STATS] = {};
     unsigned long long* moved = nullptr;  // device: rows moved to fresh slots
@@ -1352,6 +1355,8 @@ int snapshot(ghb_workspace* ws, ghb_gpma* g, bool weights) {
 void invalidate(ghb_gpma* g) {
     g->s_ok = false;
     g->s_val_ok = false;
+    if (g->s_exported) g->s_both = g->s_seen;
+    g->s_exported = g->s_seen = false;
     g->version++;
 }
 
@@ -1584,6 +1589,7 @@ int ghb_gpma_csr(ghb_workspace* ws, ghb_gpma* g, int32_t weights, const int32_t*
     GHB_REQUIRE(ws && g, "NULL workspace / graph");
     GHB_REQUIRE(rowptr && col, "NULL rowptr / col");
     GHB_TRY(snapshot(ws, g, weights != 0));
+    g->s_seen = true;
     *rowptr = g->s_rowptr;
     *col = g->s_col;
     if (w) *w = weights ? g->s_val : nullptr;
@@ -1594,8 +1600,13 @@ int ghb_gpma_export(ghb_workspace* ws, ghb_gpma* g, int32_t* rowptr, int32_t* co
     ws = ws_resolve(ws);
     GHB_REQUIRE(ws && g, "NULL workspace / graph");
     GHB_REQUIRE(rowptr && (g->m == 0 || col), "NULL rowptr / col");
-    // Straight into the caller's arrays unless a snapshot is there to copy.
-    if (!g->s_ok || (w && !g->s_val_ok)) return compact_rows(ws, g, rowptr, col, w);
+    // Straight into the caller's arrays, unless a snapshot is there to copy or the
+    // program also looks at the versions it exports: then the snapshot is made
+    // first and copied.  RMAT-21, after an update: straight 0.38 ms, and as much
+    // again for a look; through the snapshot 0.65, and nothing for a look.
+    g->s_exported = true;
+    if ((!g->s_ok || (w && !g->s_val_ok)) && !g->s_both) return compact_rows(ws, g, rowptr, col, w);
+    GHB_TRY(snapshot(ws, g, w != nullptr));
     GHB_CUDA_TRY(cudaMemcpyAsync(rowptr, g->s_rowptr, sizeof(int32_t) * ((size_t)g->n + 1),
                                  cudaMemcpyDeviceToDevice, ws->stream));
     if (g->m > 0) {
