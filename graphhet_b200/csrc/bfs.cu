@@ -32,10 +32,8 @@ bool bfs_use_persistent(ghb_workspace* ws, const ghb_bfs_options* opt) {
            opt->policy == GHB_POLICY_SCHEDULE || opt->policy == GHB_POLICY_LEARNED;
 }
 
-// n_active: vertices [n_active, n) have no entries at all (a relabelled
-// graph puts them last); bottom-up levels skip them.
 int bfs_run(ghb_workspace* ws, int32_t n, int32_t n_active, const int32_t* out_rowptr, const int32_t* out_col,
-            const int32_t* in_rowptr, const int32_t* in_col, int32_t src, int32_t max_depth,
+            const int32_t* in_rowptr, const int32_t* in_col, int32_t src, const int32_t* perm, int32_t max_depth,
             int32_t* depth, const ghb_bfs_options* opt, ghb_traversal_stats* stats) {
     GHB_REQUIRE(n >= 1, "n must be >= 1");
     GHB_REQUIRE(n_active >= 0 && n_active <= n, "n_active outside [0, n]");
@@ -74,14 +72,14 @@ int bfs_run(ghb_workspace* ws, int32_t n, int32_t n_active, const int32_t* out_r
     cudaStream_t st = ws->stream;
     // m (total CSR entries) and deg(src) from rowptr.
     int32_t* hp32 = reinterpret_cast<int32_t*>(ws->host_pinned);
-    GHB_CUDA_TRY(cudaMemcpyAsync(hp32, out_rowptr + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    GHB_CUDA_TRY(cudaMemcpyAsync(hp32 + 1, out_rowptr + src, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    GHB_TRY(launch(ws, bfs_init_kernel, dim3(grid_for(n, 256, ws->num_sms * 8)), dim3(256), 0, n,
-                   words, src, depth, B.visited, B.front_a, B.queue_a));
+    int32_t* start = reinterpret_cast<int32_t*>(ws->dev_small);
+    GHB_TRY(launch(ws, bfs_init_kernel, dim3(grid_for(n, 256, ws->num_sms * 8)), dim3(256), 0, n, words, src, perm,
+                   out_rowptr, depth, B.visited, B.front_a, B.queue_a, start));
+    GHB_CUDA_TRY(cudaMemcpyAsync(hp32, start, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     if (stats || opt->record_trace) GHB_CUDA_TRY(cudaEventRecord(ws->ev_start, st));
     GHB_CUDA_TRY(cudaStreamSynchronize(st));
     const int64_t m_total = hp32[0];
-    const int64_t deg_src = (int64_t)hp32[2] - hp32[1];
+    const int64_t deg_src = hp32[1];
 
     int64_t n_f = 1, m_f = deg_src, m_r = deg_src, examined = 0, reached = 1;
     double deg2_f = (double)deg_src * deg_src, degmax_f = (double)deg_src;
@@ -300,7 +298,7 @@ int ghb_bfs(ghb_workspace* ws, int32_t n, const int32_t* out_rowptr, const int32
         return bfs_persistent_run(ws, n, n, -1, out_rowptr, out_col, can_pull ? in_rowptr : nullptr,
                                   can_pull ? in_col : nullptr, src, max_depth, depth, nullptr, nullptr, options, stats);
     }
-    return bfs_run(ws, n, n, out_rowptr, out_col, in_rowptr, in_col, src, max_depth, depth, options,
+    return bfs_run(ws, n, n, out_rowptr, out_col, in_rowptr, in_col, src, nullptr, max_depth, depth, options,
                    stats);
 }
 
@@ -310,20 +308,31 @@ int ghb_bfs_pred(ghb_workspace* ws, int32_t n, const int32_t* out_rowptr, const 
                  ghb_traversal_stats* stats) {
     ws = ws_resolve(ws);
     GHB_REQUIRE(ws, "no workspace");
+    return bfs_pred_run(ws, n, out_rowptr, out_col, in_rowptr, in_col, src, nullptr, max_depth, depth, pred, options,
+                        stats);
+}
+
+}  // extern "C"
+
+namespace ghb {
+
+int bfs_pred_run(ghb_workspace* ws, int32_t n, const int32_t* out_rowptr, const int32_t* out_col,
+                 const int32_t* in_rowptr, const int32_t* in_col, int32_t src, const int32_t* perm, int32_t max_depth,
+                 int32_t* depth, int32_t* pred, const ghb_bfs_options* options, ghb_traversal_stats* stats) {
     GHB_REQUIRE(pred != nullptr, "NULL pred");
-    GHB_TRY(bfs_run(ws, n, n, out_rowptr, out_col, in_rowptr, in_col, src, max_depth, depth, options,
-                    stats));
+    GHB_TRY(bfs_run(ws, n, n, out_rowptr, out_col, in_rowptr, in_col, src, perm, max_depth, depth, options, stats));
     const unsigned gmax = ws->num_sms * 8;
     if (in_rowptr && in_col) {
         // Smallest-id parent: first entry of the (sorted) in-row one level up.
         return launch(ws, bfs_pred_pull_kernel, dim3(grid_for((int64_t)n * 32, 256, gmax)), dim3(256),
-                      0, n, in_rowptr, in_col, (const int32_t*)depth, src, pred);
+                      0, n, in_rowptr, in_col, (const int32_t*)depth, src, perm, pred);
     }
     GHB_TRY(launch(ws, fill_i32_kernel, dim3(grid_for(n, 256, gmax)), dim3(256), 0, pred, (int64_t)n,
                    (int32_t)0x7fffffff));
     GHB_TRY(launch(ws, bfs_pred_push_kernel, dim3(grid_for((int64_t)n * 32, 256, gmax)), dim3(256), 0,
                    n, out_rowptr, out_col, (const int32_t*)depth, pred));
-    return launch(ws, bfs_pred_finish_kernel, dim3(grid_for(n, 256, gmax)), dim3(256), 0, n, src, pred);
+    return launch(ws, bfs_pred_finish_kernel, dim3(grid_for(n, 256, gmax)), dim3(256), 0, n, src, perm,
+                  pred);
 }
 
-}  // extern "C"
+}  // namespace ghb

@@ -24,8 +24,10 @@ __global__ void fill_i32_kernel(int32_t* p, int64_t count, int32_t value) {
         p[i] = value;
 }
 
-__global__ void bfs_init_kernel(int32_t n, int64_t words, int32_t src, int32_t* depth,
-                                uint32_t* visited, uint32_t* front, int32_t* queue) {
+__global__ void bfs_init_kernel(int32_t n, int64_t words, int32_t src, const int32_t* __restrict__ perm,
+                                const int32_t* __restrict__ out_rp, int32_t* depth, uint32_t* visited,
+                                uint32_t* front, int32_t* queue, int32_t* start) {
+    if (perm) src = perm[src];
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     for (int64_t v = t0; v < n; v += stride) depth[v] = (v == src) ? 0 : kInfDepth;
@@ -34,7 +36,11 @@ __global__ void bfs_init_kernel(int32_t n, int64_t words, int32_t src, int32_t* 
         visited[w] = bit;
         front[w] = bit;
     }
-    if (t0 == 0) queue[0] = src;
+    if (t0 == 0) {
+        queue[0] = src;
+        start[0] = out_rp[n];
+        start[1] = out_rp[src + 1] - out_rp[src];
+    }
 }
 
 namespace {
@@ -415,7 +421,8 @@ __global__ void __launch_bounds__(256) bfs_queue_from_bitmap_kernel(int64_t word
 __global__ void bfs_pred_pull_kernel(int32_t n, const int32_t* __restrict__ in_rp,
                                      const int32_t* __restrict__ in_col,
                                      const int32_t* __restrict__ depth, int32_t src,
-                                     int32_t* __restrict__ pred) {
+                                     const int32_t* __restrict__ perm, int32_t* __restrict__ pred) {
+    if (perm) src = perm[src];
     const int lane = lane_id();
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -460,7 +467,8 @@ __global__ void bfs_pred_push_kernel(int32_t n, const int32_t* __restrict__ out_
     }
 }
 
-__global__ void bfs_pred_finish_kernel(int32_t n, int32_t src, int32_t* pred) {
+__global__ void bfs_pred_finish_kernel(int32_t n, int32_t src, const int32_t* __restrict__ perm, int32_t* pred) {
+    if (perm) src = perm[src];
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n;
          v += (int64_t)gridDim.x * blockDim.x)
         if (v == src || pred[v] == kInfDepth) pred[v] = -1;

@@ -58,8 +58,11 @@ struct BfsBuffers {
 
 __global__ void fill_i32_kernel(int32_t* p, int64_t count, int32_t value);
 
-__global__ void bfs_init_kernel(int32_t n, int64_t words, int32_t src, int32_t* depth,
-                                uint32_t* visited, uint32_t* front, int32_t* queue);
+// Set-up of a host-driven BFS; start gets the entries and the source's row
+// length.  (With perm, src is the caller's id here and in the kernels below.)
+__global__ void bfs_init_kernel(int32_t n, int64_t words, int32_t src, const int32_t* __restrict__ perm,
+                                const int32_t* __restrict__ out_rp, int32_t* depth, uint32_t* visited,
+                                uint32_t* front, int32_t* queue, int32_t* start);
 
 __global__ void bfs_pull_kernel(int32_t n, int64_t words, const int32_t* __restrict__ in_rp,
                                 const int32_t* __restrict__ in_col,
@@ -79,11 +82,11 @@ constexpr int64_t kAppendMaxEdges = 1 << 16;
 __global__ void bfs_pred_pull_kernel(int32_t n, const int32_t* __restrict__ in_rp,
                                      const int32_t* __restrict__ in_col,
                                      const int32_t* __restrict__ depth, int32_t src,
-                                     int32_t* __restrict__ pred);
+                                     const int32_t* __restrict__ perm, int32_t* __restrict__ pred);
 __global__ void bfs_pred_push_kernel(int32_t n, const int32_t* __restrict__ out_rp,
                                      const int32_t* __restrict__ out_col,
                                      const int32_t* __restrict__ depth, int32_t* pred);
-__global__ void bfs_pred_finish_kernel(int32_t n, int32_t src, int32_t* pred);
+__global__ void bfs_pred_finish_kernel(int32_t n, int32_t src, const int32_t* __restrict__ perm, int32_t* pred);
 
 // One top-down level: the queue kernel (short and medium lists), then the
 // long lists edge-parallel.
@@ -127,6 +130,16 @@ __global__ void bfs_push_persistent_kernel(const int32_t* __restrict__ rowptr, c
 __global__ void bfs_bitmap_from_queue_kernel(const int32_t* __restrict__ q, int32_t count, uint32_t* f);
 
 bool bfs_use_persistent(ghb_workspace* ws, const ghb_bfs_options* opt);
+// Levels driven by the host, and the tree behind them.  n_active: vertices
+// [n_active, n) have no entries at all (a relabelled graph puts them last);
+// bottom-up levels skip them.  With perm, src is the caller's id; depth and
+// pred are in the rows' ids.
+int bfs_run(ghb_workspace* ws, int32_t n, int32_t n_active, const int32_t* out_rowptr, const int32_t* out_col,
+            const int32_t* in_rowptr, const int32_t* in_col, int32_t src, const int32_t* perm, int32_t max_depth,
+            int32_t* depth, const ghb_bfs_options* opt, ghb_traversal_stats* stats);
+int bfs_pred_run(ghb_workspace* ws, int32_t n, const int32_t* out_rowptr, const int32_t* out_col,
+                 const int32_t* in_rowptr, const int32_t* in_col, int32_t src, const int32_t* perm, int32_t max_depth,
+                 int32_t* depth, int32_t* pred, const ghb_bfs_options* options, ghb_traversal_stats* stats);
 // m: entries, or -1 to read them from out_rp (one wait).  With perm, src is
 // the caller's id and depth_out is written in the caller's ids.
 int bfs_persistent_run(ghb_workspace* ws, int32_t n, int32_t n_active, int64_t m, const int32_t* out_rp,

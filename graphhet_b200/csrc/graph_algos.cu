@@ -10,14 +10,11 @@
 
 namespace ghb {
 
-int bfs_run(ghb_workspace* ws, int32_t n, int32_t n_active, const int32_t* out_rowptr, const int32_t* out_col,
-            const int32_t* in_rowptr, const int32_t* in_col, int32_t src, int32_t max_depth, int32_t* depth,
-            const ghb_bfs_options* opt, ghb_traversal_stats* stats);
 int sssp_run(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int32_t* col, const double* w, int32_t src,
              double inf, double* dist_out, const ghb_sssp_options* opt, ghb_traversal_stats* stats);
 int sssp_pred_run(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int32_t* col, const double* w,
-                  const int32_t* in_rp, const int32_t* in_col, const double* in_w, int32_t src, double inf,
-                  const double* dist, int32_t* pred);
+                  const int32_t* in_rp, const int32_t* in_col, const double* in_w, int32_t src, const int32_t* perm,
+                  double inf, const double* dist, int32_t* pred);
 int sssp_delta_run(ghb_workspace* ws, ghb_graph* g, int32_t src, double inf, double delta, double* dist_out,
                    double* out, ghb_traversal_stats* stats);
 int sssp_choose_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const double* w, int32_t src,
@@ -151,9 +148,8 @@ int ghb_graph_bfs(ghb_workspace* ws, const ghb_graph* g, int32_t src, int32_t ma
     if (bfs_use_persistent(ws, options))
         return bfs_persistent_run(ws, g->n, g->n_active, g->m, g->rowptr, g->col, g->in_rowptr, g->in_col, src,
                                   max_depth, dnew, g->perm, depth, options, stats);
-    GHB_TRY(map_source(ws, g, src, &src));
-    GHB_TRY(bfs_run(ws, g->n, g->n_active, g->rowptr, g->col, g->in_rowptr, g->in_col, src, max_depth, dnew, options,
-                    stats));
+    GHB_TRY(bfs_run(ws, g->n, g->n_active, g->rowptr, g->col, g->in_rowptr, g->in_col, src, g->perm, max_depth, dnew,
+                    options, stats));
     return map_back_i32(ws, g, dnew, depth);
 }
 
@@ -165,9 +161,8 @@ int ghb_graph_bfs_pred(ghb_workspace* ws, const ghb_graph* g, int32_t src, int32
     GHB_TRY(ws_reserve_stage(ws, 2 * sizeof(int32_t) * (size_t)g->n + 256));
     int32_t* dnew = static_cast<int32_t*>(ws->stage);
     int32_t* pnew = dnew + (((size_t)g->n + 63) & ~(size_t)63);
-    GHB_TRY(map_source(ws, g, src, &src));
-    GHB_TRY(ghb_bfs_pred(ws, g->n, g->rowptr, g->col, g->in_rowptr, g->in_col, src, max_depth, dnew, pnew, options,
-                         stats));
+    GHB_TRY(bfs_pred_run(ws, g->n, g->rowptr, g->col, g->in_rowptr, g->in_col, src, g->perm, max_depth, dnew, pnew,
+                         options, stats));
     GHB_TRY(map_back_i32(ws, g, dnew, depth));
     return launch(ws, pred_map_kernel, dim3(grid_for(g->n, 256, ws->num_sms * 8)), dim3(256), 0, g->n,
                   (const int32_t*)g->perm, (const int32_t*)g->iperm, (const int32_t*)pnew, pred);
@@ -331,8 +326,8 @@ int ghb_graph_sssp_pred(ghb_workspace* ws, const ghb_graph* g, int32_t src, doub
     double* dnew = static_cast<double*>(ws->stage);
     int32_t* pnew = reinterpret_cast<int32_t*>(dnew + (((size_t)g->n + 63) & ~(size_t)63));
     GHB_TRY(graph_sssp_dispatch(ws, g, src, inf, dnew, dist, options, stats));
-    GHB_TRY(map_source(ws, g, src, &src));
-    GHB_TRY(sssp_pred_run(ws, g->n, g->rowptr, g->col, g->w, g->in_rowptr, g->in_col, g->in_w, src, inf, dnew, pnew));
+    GHB_TRY(sssp_pred_run(ws, g->n, g->rowptr, g->col, g->w, g->in_rowptr, g->in_col, g->in_w, src, g->perm, inf,
+                          dnew, pnew));
     return launch(ws, pred_map_kernel, dim3(grid_for(g->n, 256, ws->num_sms * 8)), dim3(256), 0, g->n,
                   (const int32_t*)g->perm, (const int32_t*)g->iperm, (const int32_t*)pnew, pred);
 }

@@ -206,9 +206,11 @@ __global__ void sssp_stats_kernel(int32_t n, const int32_t* __restrict__ rp, con
 
 // Predecessors after the distances are final: the smallest-id u in v's
 // in-row with dist[u] + w(u, v) == dist[v] exactly.
-__global__ void sssp_pred_pull_kernel(int32_t n, int32_t src, const int32_t* __restrict__ in_rp,
-                                      const int32_t* __restrict__ in_col, const double* __restrict__ in_w,
-                                      const double* __restrict__ dist, double inf, int32_t* __restrict__ pred) {
+__global__ void sssp_pred_pull_kernel(int32_t n, int32_t src, const int32_t* __restrict__ perm,
+                                      const int32_t* __restrict__ in_rp, const int32_t* __restrict__ in_col,
+                                      const double* __restrict__ in_w, const double* __restrict__ dist, double inf,
+                                      int32_t* __restrict__ pred) {
+    if (perm) src = perm[src];
     const int lane = lane_id();
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -253,7 +255,8 @@ __global__ void sssp_pred_push_kernel(int32_t n, const int32_t* __restrict__ rp,
     }
 }
 
-__global__ void sssp_pred_finish_kernel(int32_t n, int32_t src, int32_t* pred) {
+__global__ void sssp_pred_finish_kernel(int32_t n, int32_t src, const int32_t* __restrict__ perm, int32_t* pred) {
+    if (perm) src = perm[src];
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n;
          v += (int64_t)gridDim.x * blockDim.x)
         if (v == src || pred[v] == 0x7fffffff) pred[v] = -1;
@@ -793,18 +796,19 @@ int sssp_delta_run(ghb_workspace* ws, ghb_graph* g, int32_t src, double inf, dou
     return map_back_f64(ws, g, dist_out, out);
 }
 
+// Distances and trees in the rows' ids; with perm, src is the caller's id.
 int sssp_pred_run(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int32_t* col, const double* w,
-                  const int32_t* in_rp, const int32_t* in_col, const double* in_w, int32_t src, double inf,
-                  const double* dist, int32_t* pred) {
+                  const int32_t* in_rp, const int32_t* in_col, const double* in_w, int32_t src, const int32_t* perm,
+                  double inf, const double* dist, int32_t* pred) {
     const unsigned g = ws->num_sms * 8;
     if (in_rp && in_w) {
         return launch(ws, sssp_pred_pull_kernel, dim3(grid_for((int64_t)n * 32, 256, g)), dim3(256), 0, n, src,
-                      in_rp, in_col, in_w, dist, inf, pred);
+                      perm, in_rp, in_col, in_w, dist, inf, pred);
     }
     GHB_TRY(launch(ws, fill_i32, dim3(grid_for(n, 256, g)), dim3(256), 0, pred, (int64_t)n, (int32_t)0x7fffffff));
     GHB_TRY(launch(ws, sssp_pred_push_kernel, dim3(grid_for((int64_t)n * 32, 256, g)), dim3(256), 0, n, rowptr, col,
                    w, dist, inf, pred));
-    return launch(ws, sssp_pred_finish_kernel, dim3(grid_for(n, 256, g)), dim3(256), 0, n, src, pred);
+    return launch(ws, sssp_pred_finish_kernel, dim3(grid_for(n, 256, g)), dim3(256), 0, n, src, perm, pred);
 }
 
 }  // namespace ghb
@@ -827,7 +831,7 @@ int ghb_sssp_pred(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int
     GHB_REQUIRE(ws, "no workspace");
     GHB_REQUIRE(pred, "NULL pred");
     GHB_TRY(sssp_run(ws, n, rowptr, col, w, src, inf, dist, options, stats));
-    return sssp_pred_run(ws, n, rowptr, col, w, in_rowptr, in_col, in_w, src, inf, dist, pred);
+    return sssp_pred_run(ws, n, rowptr, col, w, in_rowptr, in_col, in_w, src, nullptr, inf, dist, pred);
 }
 
 }  // extern "C"
