@@ -1,6 +1,6 @@
 """Autotuner for libghb's launch shapes and thresholds (the workspace
-tunables of ghb_tune_set): PageRank's hub-cache size, persistent block shape
-and row split, and the multi-source BFS's block-row threshold and direction
+tunables of ghb_tune_set): PageRank's hub-cache size and persistent block
+shape, and the multi-source BFS's block-row threshold and direction
 switch.  None of them changes a result (PageRank stays within its 1e-6 bar,
 every depth stays bit-exact; `tune` checks both), only the time.
 
@@ -8,8 +8,9 @@ The search is coordinate descent over a small grid per parameter, starting
 from the current values: each candidate is timed with CUDA events (median of
 `reps` calls after one warm-up call) on the caller's graph, the best value of
 one parameter is kept before the next is tried, and the sweep runs twice.
-Infeasible shapes (more than 2,048 threads or 224 KB of shared memory per SM)
-are skipped.  `save` / `load` keep the chosen values as JSON.
+Infeasible shapes (more than 2,048 threads or 227 KB of shared memory per SM)
+are skipped, and so are values that come to a launch already timed.  `save` /
+`load` keep the chosen values as JSON.
 """
 from __future__ import annotations
 
@@ -19,7 +20,7 @@ from typing import Callable, Dict, List, Optional, Sequence, Tuple
 
 SPACES: Dict[str, Dict[str, List[int]]] = {
     "pagerank": {
-        "pr_cache_kb": [0, 32, 64, 80, 96, 112],
+        "pr_cache_kb": [0, 16, 32, 64, 80, 96, 112],
         "pr_threads": [256, 512, 1024],
         "pr_blocks_per_sm": [1, 2, 4],
     },
@@ -30,10 +31,28 @@ SPACES: Dict[str, Dict[str, List[int]]] = {
 }
 
 
-def feasible(cfg: Dict[str, int]) -> bool:
+def _cache_room(cfg: Dict[str, int], value_bytes: int) -> int:
+    """Bytes that PageRank's blocks can give the hub cache: their share of the
+    227 KB of shared memory without the warps' tiles (256 values each)."""
+    blocks = cfg.get("pr_blocks_per_sm", 1)
+    block = 227 * 1024 // blocks - (1024 if blocks > 1 else 0)
+    tiles = cfg.get("pr_threads", 1024) // 32 * 256 * value_bytes
+    return (block - tiles - 1024) // 256 * 256 if block > tiles + 1024 else 0
+
+
+def launched(cfg: Dict[str, int], entries: int, value_bytes: int = 4) -> Dict[str, int]:
+    """`cfg` with the hub cache (bytes, under "pr_cache_kb") that a PageRank call
+    on a resident graph of so many entries gets."""
+    if "pr_cache_kb" not in cfg:
+        return dict(cfg)
+    kb = cfg["pr_cache_kb"] if entries >= 1 << 24 else min(cfg["pr_cache_kb"], 16)
+    return dict(cfg, pr_cache_kb=min(kb * 1024, _cache_room(cfg, value_bytes)))
+
+
+def feasible(cfg: Dict[str, int], value_bytes: int = 4) -> bool:
+    """Whether the blocks fit a multiprocessor with the cache that is asked for."""
     threads = cfg.get("pr_threads", 1024) * cfg.get("pr_blocks_per_sm", 1)
-    smem = cfg.get("pr_cache_kb", 192) * cfg.get("pr_blocks_per_sm", 1)
-    return threads <= 2048 and smem <= 224
+    return threads <= 2048 and cfg.get("pr_cache_kb", 80) * 1024 <= _cache_room(cfg, value_bytes)
 
 
 def _timer(fn: Callable[[], object], reps: int) -> float:
@@ -101,15 +120,18 @@ def tune(rg, algo: str, sources: Sequence[int] = (), iterations: int = 10, reps:
             raise RuntimeError("tunable changed the result: %r" % c)
         return ms
 
+    shape = lambda c: tuple(sorted(launched(c, rg.m).items()))
     best_ms = measure(cfg)
+    timed = {shape(cfg)}
     for _ in range(rounds):
         for k, values in space.items():
             for v in values:
                 if v == cfg[k]:
                     continue
                 trial = dict(cfg, **{k: v})
-                if not feasible(trial):
+                if not feasible(trial) or shape(trial) in timed:
                     continue
+                timed.add(shape(trial))
                 ms = measure(trial)
                 if ms < best_ms:
                     best_ms, cfg = ms, trial
