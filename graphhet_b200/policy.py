@@ -446,12 +446,21 @@ def ms_install(path: str = MS_WEIGHTS_PATH) -> np.ndarray:
 
 
 # ------------------------------------------------------------- evaluation
+def as_schedule(trace: np.ndarray) -> List[int]:
+    """The decisions of a traced BFS as a schedule: a level's direction and, top
+    down, the form of its output."""
+    return [PULL if r[T_DIR] == 1 else (PUSH_BITMAP if r[T_FMT] == 1 else PUSH_QUEUE) for r in trace]
+
+
 def regret(rg, sources: Sequence[int], repeats: int = 3) -> Dict[str, float]:
     """Measured regret of the heuristic and the learned policy against the
     per-level oracle schedule on `rg` (needs an installed network): each
     policy's persistent BFS time over the sources (median of `repeats`) ÷ the
     oracle schedule's time, minus one.  Also the oracle's own estimate from
-    the cost table."""
+    the cost table.  All of them run their levels on the whole grid, so the
+    ratios are the decisions' own: on a graph of at most 4.5 entries per vertex
+    a call by the rule runs small levels on a few blocks, so there the rule's
+    decisions are replayed as a schedule; ms["rule_call"] is the call itself."""
     import graphhet_b200 as G
 
     def timed(src, **kw):
@@ -461,7 +470,14 @@ def regret(rg, sources: Sequence[int], repeats: int = 3) -> Dict[str, float]:
             ts.append(st["device_ms"])
         return float(np.median(ts)), st
 
-    tot = dict(heuristic=0.0, learned=0.0, oracle=0.0, beamer14=0.0, table=0.0)
+    def rule(src, **kw):
+        ms, st = timed(src, policy=G.POLICY_HEURISTIC, **kw)
+        if 2 * rg.m > 9 * rg.n:
+            return ms, ms
+        tr = rg.bfs(src, policy=G.POLICY_HEURISTIC, trace_cap=max(1, st["levels"]), **kw)[2]
+        return timed(src, policy=G.POLICY_SCHEDULE, schedule=as_schedule(tr))[0], ms
+
+    tot = dict(heuristic=0.0, learned=0.0, oracle=0.0, beamer14=0.0, table=0.0, rule_call=0.0)
     for s in sources:
         rg.bfs(s)
         r = replay_costs(rg, s)
@@ -470,9 +486,11 @@ def regret(rg, sources: Sequence[int], repeats: int = 3) -> Dict[str, float]:
         sched, cost, total = oracle_schedule(r["t_queue"], r["t_bitmap"], r["t_comp"], r["t_pull"])
         tot["table"] += total
         tot["oracle"] += timed(s, policy=G.POLICY_SCHEDULE, schedule=sched)[0]
-        tot["heuristic"] += timed(s, policy=G.POLICY_HEURISTIC)[0]
+        ms, call = rule(s)
+        tot["heuristic"] += ms
+        tot["rule_call"] += call
         # The classic rule: alpha 14, beta 24, no frontier guard.
-        tot["beamer14"] += timed(s, policy=G.POLICY_HEURISTIC, alpha=14.0, beta=24.0, gamma=1e30)[0]
+        tot["beamer14"] += rule(s, alpha=14.0, beta=24.0, gamma=1e30)[0]
         tot["learned"] += timed(s, policy=G.POLICY_LEARNED)[0]
     o = tot["oracle"]
     return dict(ms=tot, regret_heuristic=tot["heuristic"] / o - 1.0, regret_learned=tot["learned"] / o - 1.0,

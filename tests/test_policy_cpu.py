@@ -153,3 +153,10 @@ def test_shipped_ms_model_has_nine_finite_weights():
     z = np.load(P.MS_WEIGHTS_PATH)
     wts = z["weights"]
     assert wts.shape == (P.MS_FEATURES + 1,) and np.all(np.isfinite(wts))
+
+
+def test_a_trace_as_a_schedule():
+    tr = np.full((4, 24), -1.0, np.float32)
+    tr[:, P.T_DIR] = [0, 0, 1, 0]
+    tr[:, P.T_FMT] = [0, 1, -1, 0]
+    assert P.as_schedule(tr) == [P.PUSH_QUEUE, P.PUSH_BITMAP, P.PULL, P.PUSH_QUEUE]
