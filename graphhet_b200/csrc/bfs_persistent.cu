@@ -1197,11 +1197,11 @@ int bfs_persistent_run(ghb_workspace* ws, int32_t n, int32_t n_active, int64_t m
         sched_len = std::min<int32_t>(opt->schedule_len, 4096);
         GHB_CUDA_TRY(cudaMemcpyAsync(sched, opt->schedule, sched_len, cudaMemcpyHostToDevice, st));
     }
-    // The learned policy runs in the kernel when a network is installed;
-    // otherwise GHB_POLICY_LEARNED falls back to the heuristic.
+    // The learned policy runs in the kernel when a network is installed and has
+    // levels to decide; otherwise GHB_POLICY_LEARNED is the heuristic.
     const float* pol = nullptr;
     if (policy == GHB_POLICY_LEARNED) {
-        pol = policy_device_params();
+        if (ws->tune.pol_band > 0) pol = policy_device_params();
         if (!pol) policy = GHB_POLICY_HEURISTIC;
     }
     // The start state (pageable source: staged by the call).

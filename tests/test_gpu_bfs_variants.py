@@ -44,6 +44,11 @@ def test_variant(kind):
     try:
         depth, squad = variant(lambda: rg.bfs(7, policy=G.POLICY_LEARNED))
         assert not squad and torch.equal(depth, want)
+        ws = G.Workspace()  # a network with no level to decide is the rule
+        G.tune_set("pol_band", 0, ws=ws)
+        depth, squad = variant(lambda: rg.bfs(7, policy=G.POLICY_LEARNED, ws=ws))
+        assert squad == low and torch.equal(depth, want)
+        ws.close()
     finally:
         G.policy_load(None, None)
     rg.close()
