@@ -135,25 +135,40 @@ __global__ void sssp_split_kernel(const int32_t* __restrict__ far, int32_t far_c
         atomicMin(reinterpret_cast<unsigned long long*>(min_far), (unsigned long long)__double_as_longlong(mn));
 }
 
-// About a million of the weights: out[0] their sum, out[1] their number,
-// out[2] the entries.
+// About a million of the weights, and the rows' entries.  (Zeroed before.)
+struct WeightSample {
+    double sum, count, square;       // square: the sum of the squares
+    unsigned long long not_least;    // the smallest weight's bits, inverted
+    double entries, first_row;       // of all rows, of the first
+};
 __global__ void mean_weight_kernel(int32_t n, const int32_t* __restrict__ rowptr, const double* __restrict__ w,
-                                   double* out) {
+                                   WeightSample* out) {
     const int64_t m = rowptr[n];
     const int64_t stride = m >= (1 << 20) ? m / (1 << 20) : 1;
-    double s = 0.0;
+    double s = 0.0, q = 0.0;
+    unsigned long long least = 0;
     int64_t c = 0;
-    if (blockIdx.x == 0 && threadIdx.x == 0) out[2] = (double)m;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        out->entries = (double)m;
+        out->first_row = (double)(rowptr[1] - rowptr[0]);
+    }
     for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * stride; i < m;
          i += (int64_t)gridDim.x * blockDim.x * stride) {
-        s += w[i];
+        const double x = w[i];
+        s += x;
+        q += x * x;
+        least = max(least, ~(unsigned long long)__double_as_longlong(x));
         ++c;
     }
     s = warp_sum(s);
-    double cd = warp_sum((double)c);
+    q = warp_sum(q);
+    least = warp_max(least);
+    const double cd = warp_sum((double)c);
     if (lane_id() == 0) {
-        atomicAdd(out, s);
-        atomicAdd(out + 1, cd);
+        atomicAdd(&out->sum, s);
+        atomicAdd(&out->square, q);
+        atomicAdd(&out->count, cd);
+        atomicMax(&out->not_least, least);
     }
 }
 
@@ -343,27 +358,33 @@ __global__ void fill_i32(int32_t* p, int64_t count, int32_t value) {
 // weight times 32 over the mean degree (wider buckets on sparse graphs,
 // where rounds are latency-bound).  The policy network's bins and the
 // multi-source pass scale this width.
-// *entries: the rows' entries.
-int sssp_pick_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const double* w, double* delta,
-                    int64_t* entries) {
+static int sssp_sample(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const double* w, double* delta,
+                       WeightSample* sample) {
     cudaStream_t st = ws->stream;
-    double* acc = reinterpret_cast<double*>(ws->dev_small);
-    GHB_CUDA_TRY(cudaMemsetAsync(acc, 0, 3 * sizeof(double), st));
+    WeightSample* acc = reinterpret_cast<WeightSample*>(ws->dev_small);
+    GHB_CUDA_TRY(cudaMemsetAsync(acc, 0, sizeof(WeightSample), st));
     GHB_TRY(launch(ws, mean_weight_kernel, dim3(64), dim3(256), 0, n, rowptr, w, acc));
-    GHB_CUDA_TRY(cudaMemcpyAsync(ws->host_pinned, acc, 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
+    GHB_CUDA_TRY(cudaMemcpyAsync(ws->host_pinned, acc, sizeof(WeightSample), cudaMemcpyDeviceToHost, st));
     GHB_CUDA_TRY(cudaStreamSynchronize(st));
-    const double* h = reinterpret_cast<const double*>(ws->host_pinned);
-    const int64_t m = (int64_t)h[2];
-    *entries = m;
-    if (m == 0) {
+    std::memcpy(sample, ws->host_pinned, sizeof(WeightSample));
+    if (sample->entries == 0) {
         *delta = 1.0;
         return GHB_OK;
     }
-    const double mean_w = h[1] > 0 ? h[0] / h[1] : 1.0;
-    const double mean_d = (double)m / (double)n;
+    const double mean_w = sample->count > 0 ? sample->sum / sample->count : 1.0;
+    const double mean_d = sample->entries / (double)n;
     double d = mean_w * 32.0 / std::max(1.0, mean_d);
     if (!(d > 0)) d = 1.0;
     *delta = d;
+    return GHB_OK;
+}
+
+// *entries: the rows' entries.
+int sssp_pick_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const double* w, double* delta,
+                    int64_t* entries) {
+    WeightSample sample;
+    GHB_TRY(sssp_sample(ws, n, rowptr, w, delta, &sample));
+    *entries = (int64_t)sample.entries;
     return GHB_OK;
 }
 
@@ -372,14 +393,35 @@ int sssp_pick_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const d
 // its grid barriers whatever the graph, the entries it saves grow with the
 // graph.  With the light/heavy split (light_m entries, 0 without it), where
 // a settled vertex's heavy entries are read once however narrow the bucket,
-// half the width pays on large graphs: RMAT-22 4.2 ms with the whole width and
-// 3.1 with half, from two other sources 5.3 and 4.1, 6.0 and 3.5.  At 2^20
-// vertices of degree 10 the two meet (uniform: 0.94, 0.95 ms).  In between
-// (RMAT-21 3.1 and 2.4) the whole width stays: there the policy network is
-// measured against it.  Sparse graphs keep it too: a 1501 x 1999 grid takes
-// 37 ms with it and 43 with half.
-static double sssp_default_share(int32_t n, int64_t light_m) {
-    return light_m >= (1ll << 26) && light_m >= 6ll * n ? 0.5 : 1.0;
+// half the width pays on large graphs: RMAT-22 15.9 ms with the whole width and
+// 12.1 with half (three sources), RMAT-24 62 and 44; uniform, 2^22 vertices, 18
+// and 32 entries each, 8.6 and 8.1, 7.5 and 6.9.  At 2^20 vertices of degree 10 the
+// two meet (uniform: 0.94, 0.95 ms).  In between (RMAT-21 8.9 and 6.4) the whole
+// width stays: there the policy network is measured against it.  Sparse
+// graphs keep it too: a 1501 x 1999 grid takes 28 ms a source with it and 33 with half.
+//
+// The weights decide as well (all with 2^26 entries or more, whole and half):
+//  * none near zero: few entries are light in half a width.  U(0, 1) + 0.1 on uniform
+//    rows 6.9 and 6.8, + 0.25 6.1 and 6.4, + 0.5 5.5 and 6.3, + 1 5.1 and 6.3; on
+//    RMAT-22 Pareto weights from 1 on 8.2 and 9.2.
+//  * a few that make up most of the sum, on rows with hubs: their mean is far above
+//    what the hubs' short paths use.  RMAT-22, squares' mean over the mean's
+//    square 2.0 (exponential): 24.1 and 20.4; 6: 38.9 and 37.9; 20: 52.7 and 53.7; 65,
+//    from 0.001 on: 20.4 and 27.7.  Without hubs half is ahead (Pareto 20.1 and 15.5).
+//  * even ones on uniform rows of 9 to 16 entries: a bucket then holds about one
+//    weight.  2^23 vertices of 10 16.8 and 18.4, of 12 18.4 and 19.4, 5 * 2^20 of 14 9.6
+//    and 10.4; of 8 21.4 and 21.6, of 24 7.4 and 6.5.  With exponential weights
+//    half is twice as fast there (39.9 and 20.2).
+static double sssp_default_share(int32_t n, int64_t light_m, const WeightSample& w) {
+    if (light_m < (1ll << 26) || light_m < 6ll * n) return 1.0;
+    const unsigned long long bits = ~w.not_least;
+    double least;
+    std::memcpy(&least, &bits, sizeof(least));
+    const double mean = w.sum / w.count, spread = w.square / w.count / (mean * mean);
+    if (!(least <= 0.1 * mean)) return 1.0;
+    const bool hubs = w.first_row * n >= 32.0 * (double)light_m;
+    if (hubs) return spread <= 10.0 ? 0.5 : 1.0;
+    return spread >= 1.6 || light_m < 9ll * n || light_m >= 16ll * n ? 0.5 : 1.0;
 }
 
 // The width for one SSSP call: the caller's, else the weight rule's share
@@ -398,10 +440,12 @@ int sssp_choose_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const
         *delta = opt->delta;
         return GHB_OK;
     }
-    GHB_TRY(sssp_pick_delta(ws, n, rowptr, w, delta, entries));
+    WeightSample sample;
+    GHB_TRY(sssp_sample(ws, n, rowptr, w, delta, &sample));
+    *entries = (int64_t)sample.entries;
     const bool learned = opt && opt->policy == GHB_POLICY_LEARNED;
     const bool tracing = opt && opt->record_trace && opt->trace && opt->trace_cap > 0;
-    const double share = sssp_default_share(n, light_m);
+    const double share = sssp_default_share(n, light_m, sample);
     if (!learned && !tracing) {
         *delta *= share;
         return GHB_OK;
