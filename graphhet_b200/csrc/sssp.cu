@@ -393,34 +393,40 @@ int sssp_pick_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const d
 // its grid barriers whatever the graph, the entries it saves grow with the
 // graph.  With the light/heavy split (light_m entries, 0 without it), where
 // a settled vertex's heavy entries are read once however narrow the bucket,
-// half the width pays on large graphs: RMAT-22 15.9 ms with the whole width and
-// 12.1 with half (three sources), RMAT-24 62 and 44; uniform, 2^22 vertices, 18
-// and 32 entries each, 8.6 and 8.1, 7.5 and 6.9.  At 2^20 vertices of degree 10 the
-// two meet (uniform: 0.94, 0.95 ms).  In between (RMAT-21 8.9 and 6.4) the whole
-// width stays: there the policy network is measured against it.  Sparse
-// graphs keep it too: a 1501 x 1999 grid takes 28 ms a source with it and 33 with half.
+// half the width pays (whole and half, ms for three or four sources):
+//  * with hubs, whose rows are read again whenever their distance falls (the first
+//    row, the highest-ranked vertex's, holds 32 times the mean or more), from 2^23
+//    entries on: RMAT-19 3.3 and 2.7, RMAT-20 5.0 and 4.4, RMAT-21 8.9 and 6.4, RMAT-22
+//    15.9 and 12.1, RMAT-24 62 and 44; RMAT-21 with a = 0.35 (first row 245 times the
+//    mean) 11.0 and 7.6, power law of 2^20 vertices 8.2 and 6.1.  Below, RMAT-18 2.33
+//    and 2.22 but 1.93 and 2.07 with weights 1 to 100, RMAT-17 2.30 and 2.27.
+//  * without, from 2^26 on: uniform, 2^22 vertices, 18 and 32 entries each, 8.6 and 8.1,
+//    7.5 and 6.9.  Below, 2^20 vertices of 32 3.3 and 3.1, of 16 2.0 and 1.9, of 10 1.9
+//    and 1.8; 2^18 of 32 1.56 and 1.58.
+// Large graphs with hubs would take a quarter (RMAT-22 10.1), as the network's
+// widths do; the rule has the one step.  Sparse graphs keep the whole: a 1501 x
+// 1999 grid takes 28 ms a source with it and 33 with half.
 //
-// The weights decide as well (all with 2^26 entries or more, whole and half):
+// The weights decide as well (with 2^26 entries or more unless said):
 //  * none near zero: few entries are light in half a width.  U(0, 1) + 0.1 on uniform
 //    rows 6.9 and 6.8, + 0.25 6.1 and 6.4, + 0.5 5.5 and 6.3, + 1 5.1 and 6.3; on
 //    RMAT-22 Pareto weights from 1 on 8.2 and 9.2.
-//  * a few that make up most of the sum, on rows with hubs: their mean is far above
-//    what the hubs' short paths use.  RMAT-22, squares' mean over the mean's
-//    square 2.0 (exponential): 24.1 and 20.4; 6: 38.9 and 37.9; 20: 52.7 and 53.7; 65,
-//    from 0.001 on: 20.4 and 27.7.  Without hubs half is ahead (Pareto 20.1 and 15.5).
-//  * even ones on uniform rows of 9 to 16 entries: a bucket then holds about one
-//    weight.  2^23 vertices of 10 16.8 and 18.4, of 12 18.4 and 19.4, 5 * 2^20 of 14 9.6
+//  * a few that make up most of the sum, on rows with hubs: RMAT-22, squares' mean
+//    over the mean's square 2.0 (exponential): 24.1 and 20.4; 6: 38.9 and 37.9; 20: 52.7 and 53.7; 65,
+//    from 0.001 on: 20.4 and 27.7; RMAT-19, 2.0: 5.6 and 5.4; 2.8: 9.1 and 9.2; 3.4: 7.5
+//    and 7.8.  Without hubs half is ahead (Pareto 20.1 and 15.5).
+//  * even ones on uniform rows of 9 to 16 entries: 2^23 vertices of 10 16.8 and 18.4, of 12 18.4 and 19.4, 5 * 2^20 of 14 9.6
 //    and 10.4; of 8 21.4 and 21.6, of 24 7.4 and 6.5.  With exponential weights
 //    half is twice as fast there (39.9 and 20.2).
 static double sssp_default_share(int32_t n, int64_t light_m, const WeightSample& w) {
-    if (light_m < (1ll << 26) || light_m < 6ll * n) return 1.0;
+    const bool hubs = w.first_row * n >= 32.0 * (double)light_m, large = light_m >= (1ll << 26);
+    if (light_m < 6ll * n || !(large || (hubs && light_m >= (1ll << 23)))) return 1.0;
     const unsigned long long bits = ~w.not_least;
     double least;
     std::memcpy(&least, &bits, sizeof(least));
     const double mean = w.sum / w.count, spread = w.square / w.count / (mean * mean);
     if (!(least <= 0.1 * mean)) return 1.0;
-    const bool hubs = w.first_row * n >= 32.0 * (double)light_m;
-    if (hubs) return spread <= 10.0 ? 0.5 : 1.0;
+    if (hubs) return spread <= (large ? 10.0 : 2.1) ? 0.5 : 1.0;
     return spread >= 1.6 || light_m < 9ll * n || light_m >= 16ll * n ? 0.5 : 1.0;
 }
 
