@@ -427,7 +427,6 @@ __device__ __noinline__ bool bfs_squad_run(const SquadCtx& c, SquadShared& sh, i
     }
     __syncthreads();
     const unsigned long long limit = st->bar_limit_ns, t_run = global_timer_ns();
-    const int look_mask = solo_look_mask(limit);
     unsigned long long mr = 0, got = 0, last_mf = 0;  // thread 0: this block's totals
     int32_t count = i1 - i0;
     int par = 0;
@@ -453,7 +452,7 @@ __device__ __noinline__ bool bfs_squad_run(const SquadCtx& c, SquadShared& sh, i
             // One block asks for the end when its share is lopsided, the
             // first also in time for the other blocks' wait, which is bounded.
             const bool end = count > kSquadLean ||
-                             (me == 0 && (lev & look_mask) == look_mask && global_timer_ns() - t_run > limit / 8);
+                             (me == 0 && solo_look(lev, limit) && global_timer_ns() - t_run > limit / 8);
             unsigned long long* word = &st->squad[lev % 3].word;
             const unsigned long long mine = kSqArrive + kSqNf * (unsigned)min(count, (int32_t)kSqMfCap) +
                                             kSqMf * min(last_mf, kSqMfCap) + (end ? kSqEnd : 0ull);

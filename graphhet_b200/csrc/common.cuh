@@ -272,10 +272,12 @@ __device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned* gen, int
 
 // Some blocks run small passes of a few microseconds each while the others wait
 // at a barrier that gives up after limit_ns; they look at the clock after every
-// pass whose number has these bits set, and hand back an eighth of the limit
-// after they began.  Sixteen passes are a large part of a short limit (at 100 us
-// the barrier of SSSP on a mesh gave up), so there they look after each.
-__device__ __forceinline__ int solo_look_mask(unsigned long long limit_ns) { return limit_ns < 16000000ull ? 0 : 15; }
+// sixteenth pass and hand back an eighth of the limit after they began.  Sixteen
+// passes are a large part of a short limit (at 100 us the barrier of SSSP on a mesh
+// gave up), so there they look after each.
+__device__ __forceinline__ bool solo_look(int pass, unsigned long long limit_ns) {
+    return (pass & 15) == 15 || limit_ns < 16000000ull;
+}
 
 // Grid barrier with leader work, for cooperatively launched kernels.
 // *count (arrivals) and *release (epochs) must sit on different cache lines

@@ -704,7 +704,6 @@ __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent_kernel(
                 for (int32_t i = threadIdx.x; i < held_next; i += blockDim.x)
                     fast(s.qsel ^ 1)[i] = __ldcg((s.qsel ? qa : qb) + i);
                 const unsigned long long t_run = global_timer_ns();
-                const int look_mask = solo_look_mask(limit_ns);
                 if (threadIdx.x == 0) {
                     own.q_tail = own.c_tail = own.r_add = own.far_add = own.stop = 0;
                     own.fmin = ~0ull;
@@ -721,7 +720,7 @@ __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent_kernel(
                     sp_total(found, &own.examined, &own.fmin);
                     __syncthreads();
                     if (threadIdx.x == 0) {
-                        const bool look = (turns & look_mask) == look_mask;
+                        const bool look = solo_look(turns, limit_ns);
                         const unsigned long long now = look ? global_timer_ns() : 0;
                         own.stop = look && now - s_t0 > kSsspTimeBudgetNs;
                         sp_decide(s, own);
