@@ -57,12 +57,12 @@ enum DeviceStatus : int32_t {
     kDevOverflow = 2,
 };
 
-// Launch shapes and thresholds, per workspace.  The defaults are the
-// autotuner's choices on B200 (graphhet_b200/autotune.py on RMAT scale 24
-// for PageRank, scales 22 and 24 for the multi-source BFS); ghb_tune_set
+// Launch shapes and thresholds, per workspace.  The defaults of the multi-source
+// BFS are the autotuner's choices on B200 (graphhet_b200/autotune.py on RMAT
+// scales 22 and 24), PageRank's are measured beside its kernels; ghb_tune_set
 // changes them for other graphs.
 struct Tuning {
-    int32_t pr_cache_kb = 80;     // PageRank hub cache: shared memory per block (KB)
+    int32_t pr_cache_kb = 80;      // PageRank hub cache: shared memory per block (KB), at most (see pagerank_impl)
     int32_t pr_threads = 1024;     // threads of the persistent PageRank blocks
     int32_t pr_blocks_per_sm = 1;  // persistent PageRank blocks per SM
     int32_t pr_short = 64;         // accepted, without effect: every warp takes a tile of entries

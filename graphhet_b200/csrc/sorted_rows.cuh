@@ -28,8 +28,9 @@ __device__ __forceinline__ void fill_rows(RowGaps& g, int32_t* rowptr, int64_t r
     }
     for (int64_t r = r0; r <= r1; ++r) rowptr[r] = at;
 }
-// Every thread of the block, after a barrier that follows its fill_rows calls;
-// leaves the list empty after the next barrier.
+// Every thread of the block, once, after a barrier that follows its fill_rows
+// calls.  The list is not emptied: a kernel that fills twice sets count to zero
+// between two barriers.
 __device__ __forceinline__ void fill_long_rows(RowGaps& g, int32_t* rowptr) {
     const int n = min(g.count, RowGaps::kCap);
     for (int i = 0; i < n; ++i)

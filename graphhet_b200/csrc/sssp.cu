@@ -404,8 +404,8 @@ int sssp_pick_delta(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const d
 //    7.5 and 6.9.  Below, 2^20 vertices of 32 3.3 and 3.1, of 16 2.0 and 1.9, of 10 1.9
 //    and 1.8; 2^18 of 32 1.56 and 1.58.
 // Large graphs with hubs would take a quarter (RMAT-22 10.1), as the network's
-// widths do; the rule has the one step.  Sparse graphs keep the whole: a 1501 x
-// 1999 grid takes 28 ms a source with it and 33 with half.
+// widths do; the rule has the one step.  Sparse graphs keep the whole: a handle of
+// a 1501 x 1999 grid takes 28 ms a source with it and 33 with half.
 //
 // The weights decide as well (with 2^26 entries or more unless said):
 //  * none near zero: few entries are light in half a width.  U(0, 1) + 0.1 on uniform

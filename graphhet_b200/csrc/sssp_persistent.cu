@@ -55,10 +55,10 @@ constexpr int kSsspThreads = 512;
 constexpr int32_t kSoloQueue = 2048;
 constexpr int32_t kSoloChunks = 32;
 // A queue is small up to kSoloEntries entries of mean degree.  1501 x 1999
-// grid, before the staging below (32.4 ms with it): 30.8 ms with 3072, 35.8
-// with 6144 and 40.3 with 12288 (one block then takes several turns of 512
-// rows per pass), 59.7 with every pass on the grid and its decision read back
-// through L2 (300 x 300: 3.3 ms against 9.0).
+// grid, the caller's rows from a corner, before the staging below (33 ms with
+// it): 30.8 ms with 3072, 35.8 with 6144 and 40.3 with 12288 (one block then takes
+// several turns of 512 rows per pass), 59.7 with every pass on the grid and its
+// decision read back through L2 (300 x 300: 3.3 ms against 9.0).
 constexpr int64_t kSoloEntries = 3072;
 constexpr int kSoloTurns = 1 << 14;
 constexpr unsigned long long kSsspTimeBudgetNs = 120ull * 1000000000ull;  // two minutes

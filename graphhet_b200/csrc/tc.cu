@@ -14,8 +14,14 @@
 // each of its three vertices; the reference's count is 6x that (each
 // triangle is met from its 6 ordered edges), and its int32 wraps.
 //
-// Any other input takes the generic path: the reference's merge over every
-// entry, kept for exact parity on directed or unusual inputs.
+// On rows in rank order (a resident graph's, or a copy relabelled for the call)
+// the triangles that hold one of the 4,096 highest-ranked vertices are counted
+// through bitmaps of hub neighbours first, and the hash kernels take the rest.
+//
+// Directed rows and rows with loops that are strictly increasing go through the
+// hash kernels as they are, an entry counting as one pair, as in the reference.
+// Unsorted rows, and short directed ones, take the reference's merge over every
+// entry.
 #include <algorithm>
 #include <atomic>
 
@@ -592,7 +598,7 @@ constexpr int32_t kTcBitMin = 32;        // hub neighbours from which a vertex h
 constexpr int32_t kTcHubDirect = 8;      // rows over this many entries are listed as items
 constexpr int32_t kTcHubSlice = 128;     // entries of N+(a) per item: counts fit eight bit slices
 constexpr int kTcHubThreads = 128;
-constexpr int kTcHubBlocks = 4;  // per SM: 120 registers a thread
+constexpr int kTcHubBlocks = 4;  // per SM: 128 registers a thread
 constexpr int kTcSlices = 8;
 
 // oe[u]: end of N+(u); he[u]: end of its hub part.

@@ -178,7 +178,10 @@ int ghb_csr_merge_in_out(ghb_workspace* ws, int32_t n, const int32_t* in_rowptr,
                          const int32_t* out_col, int32_t* all_rowptr, int32_t* all_col);
 
 /* ------------------------------------------------------------------- BFS */
-/* Direction policy per level. */
+/* Direction policy per level.  On graphs of at most 4.5 entries per vertex
+ * untraced calls by the rule (or top-down throughout) run small levels on a
+ * few blocks; schedules, the network, traces and bottom-up calls run every
+ * level on the whole grid.  The depths are the same. */
 #define GHB_POLICY_HEURISTIC 0 /* Beamer alpha/beta rule + frontier guard     */
 #define GHB_POLICY_LEARNED 1   /* the trained MLP (ghb_policy_*); falls back   */
 #define GHB_POLICY_PUSH 2      /* top-down every level                        */
@@ -513,7 +516,8 @@ int ghb_gpma_stats(const ghb_gpma* g, int64_t* stats /* GHB_GPMA_STATS */);
 int ghb_gpma_csr(ghb_workspace* ws, ghb_gpma* g, int32_t weights, const int32_t** rowptr,
                  const int32_t** col, const double** w);
 /* The compact CSR copied into caller buffers (rowptr n + 1, col / w m; w may
- * be NULL). */
+ * be NULL).  Written straight from the rows, without the snapshot behind
+ * ghb_gpma_csr, unless the program looks at the versions that it exports. */
 int ghb_gpma_export(ghb_workspace* ws, ghb_gpma* g, int32_t* rowptr, int32_t* col, double* w);
 /* Weight of each key, 0 when the entry is absent. */
 int ghb_gpma_find(ghb_workspace* ws, const ghb_gpma* g, const uint64_t* keys, int64_t count,
