@@ -272,12 +272,13 @@ __device__ __forceinline__ int32_t old_rank(const uint64_t* __restrict__ skey, c
     return j + (insX[lo] - insX[a]) - (delX[lo] - delX[a]);
 }
 
-// Entries [j0, j0 + len), len <= kBigChunk, of an existing row (slots from s) to
+// Entries [j0, j0 + len), len <= 32 kPer, of an existing row (slots from s) to
 // their ranks in the rebuilt one (from o, d2 entries; updates skey[a, z)), by a
 // warp: all loads issued together, then one search for the updates that fall
 // between the chunk's first and last column.  Most chunks hold none (100,000
 // updates meet one entry in 450 of the rows they touch): their entries keep
 // their order at one common offset.  Returns the ranks outside the row.
+template <int kPer>
 __device__ __forceinline__ unsigned scatter_old_chunk(const uint64_t* __restrict__ skey, const int8_t* __restrict__ typ,
                                                       const int32_t* __restrict__ insX, const int32_t* __restrict__ delX,
                                                       int32_t a, int32_t z, uint32_t r, const int32_t* __restrict__ col,
@@ -285,7 +286,6 @@ __device__ __forceinline__ unsigned scatter_old_chunk(const uint64_t* __restrict
                                                       int32_t* __restrict__ scol, double* __restrict__ sval, int64_t o,
                                                       int32_t d2) {
     const int lane = lane_id();
-    constexpr int kPer = kBigChunk / 32;
     int32_t c[kPer];
     double w[kPer];
 #pragma unroll
@@ -343,21 +343,26 @@ __device__ __forceinline__ int32_t new_rank(const int32_t* __restrict__ pos, con
 // go to `big` (with the chunk counts of their old and new entries in big_d /
 // big_d2, zero past the list) for the grid-wide kernels; big_flag[k] tells
 // them apart.
-__global__ void upd_rows_warp_kernel(const int32_t* __restrict__ row_id, const int32_t* __restrict__ row_first,
-                                     const int32_t* __restrict__ headX, const int32_t* __restrict__ scrX,
-                                     const int32_t* __restrict__ exX, const int64_t* __restrict__ relX,
-                                     const uint64_t* __restrict__ skey, const uint32_t* __restrict__ sidx,
-                                     const double* __restrict__ values, const int8_t* __restrict__ typ,
-                                     const int32_t* __restrict__ pos, const int32_t* __restrict__ insX,
-                                     const int32_t* __restrict__ delX, int64_t base, int64_t b,
-                                     int64_t* __restrict__ start, int32_t* __restrict__ deg,
-                                     int32_t* __restrict__ cap, int32_t* __restrict__ col, double* __restrict__ val,
-                                     int32_t* __restrict__ scol, double* __restrict__ sval,
-                                     int32_t* __restrict__ big, int32_t* __restrict__ big_tail,
-                                     int32_t* __restrict__ big_d, int32_t* __restrict__ big_d2,
-                                     int8_t* __restrict__ big_flag, int32_t row_warp_max,
-                                     const int64_t* __restrict__ dst_start, unsigned long long* __restrict__ moved,
-                                     unsigned long long* __restrict__ bad_rank) {
+// A row is a chain of loads and searches, so the warps in flight set the time:
+// 64 entries a step in 32 registers.  With 256 a step (59 registers, four blocks
+// per SM) a batch of 60,000 on a 700 x 700 grid took 79 us in it and takes 45, 100,000
+// RMAT updates on RMAT-21 85 and 71.
+__global__ void __launch_bounds__(256, 8)
+    upd_rows_warp_kernel(const int32_t* __restrict__ row_id, const int32_t* __restrict__ row_first,
+                         const int32_t* __restrict__ headX, const int32_t* __restrict__ scrX,
+                         const int32_t* __restrict__ exX, const int64_t* __restrict__ relX,
+                         const uint64_t* __restrict__ skey, const uint32_t* __restrict__ sidx,
+                         const double* __restrict__ values, const int8_t* __restrict__ typ,
+                         const int32_t* __restrict__ pos, const int32_t* __restrict__ insX,
+                         const int32_t* __restrict__ delX, int64_t base, int64_t b,
+                         int64_t* __restrict__ start, int32_t* __restrict__ deg,
+                         int32_t* __restrict__ cap, int32_t* __restrict__ col, double* __restrict__ val,
+                         int32_t* __restrict__ scol, double* __restrict__ sval,
+                         int32_t* __restrict__ big, int32_t* __restrict__ big_tail,
+                         int32_t* __restrict__ big_d, int32_t* __restrict__ big_d2,
+                         int8_t* __restrict__ big_flag, int32_t row_warp_max,
+                         const int64_t* __restrict__ dst_start, unsigned long long* __restrict__ moved,
+                         unsigned long long* __restrict__ bad_rank) {
     const int lane = lane_id();
     const int64_t K = headX[b];
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -381,9 +386,24 @@ __global__ void upd_rows_warp_kernel(const int32_t* __restrict__ row_id, const i
         const int64_t s = start[r];
         const int64_t o = dst_start ? dst_start[r] : (int64_t)scrX[k];
         unsigned long long bad = 0;
-        for (int32_t j0 = 0; j0 < d; j0 += kBigChunk)
-            bad += scatter_old_chunk(skey, typ, insX, delX, a, z, (uint32_t)r, col, val, s, j0, min(kBigChunk, d - j0),
-                                     scol, sval, o, d2);
+        if (d <= 32) {
+            // An entry a lane, its rank searched for among the row's updates at once:
+            // a short row that is in the batch holds one between its ends as a rule.
+            if (lane < d) {
+                const int32_t c = col[s + lane];
+                const int32_t rk = old_rank(skey, typ, insX, delX, a, a, z, (uint32_t)r, c, lane);
+                if (rk >= d2) {
+                    ++bad;
+                } else if (rk >= 0) {
+                    scol[o + rk] = c;
+                    sval[o + rk] = val[s + lane];
+                }
+            }
+        } else {
+            for (int32_t j0 = 0; j0 < d; j0 += 64)
+                bad += scatter_old_chunk<2>(skey, typ, insX, delX, a, z, (uint32_t)r, col, val, s, j0, min(64, d - j0),
+                                            scol, sval, o, d2);
+        }
         for (int32_t i = a + lane; i < z; i += 32) {
             if (typ[i] != kIns) continue;
             const int32_t rk = new_rank(pos, insX, delX, a, i);
@@ -492,8 +512,8 @@ __global__ void big_scatter_old_kernel(const int32_t* __restrict__ big, const in
         const int64_t s = start[r];
         const int64_t o = dst_start ? dst_start[r] : (int64_t)scrX[k];
         const int32_t j0 = (int32_t)(ch - bex[i]) * kBigChunk;
-        const unsigned bad = scatter_old_chunk(skey, typ, insX, delX, a, z, (uint32_t)r, col, val, s, j0,
-                                               min(kBigChunk, d - j0), scol, sval, o, d2);
+        const unsigned bad = scatter_old_chunk<kBigChunk / 32>(skey, typ, insX, delX, a, z, (uint32_t)r, col, val, s,
+                                                               j0, min(kBigChunk, d - j0), scol, sval, o, d2);
         if (bad) atomicAdd(bad_rank, (unsigned long long)bad);
     }
 }
