@@ -54,8 +54,8 @@ struct ghb_gpma {
     double* s_val = nullptr;
     int64_t s_col_cap = 0, s_val_cap = 0;
     bool s_ok = false, s_val_ok = false;
-    // What the program does with a version: exported, looked at in the snapshot
-    // (s_seen); s_both: both, the last version that was exported.
+    // What the program does with a version: exported, wanted in the snapshot
+    // (looked at, or exported again); s_both: both, the last version exported.
     bool s_exported = false, s_seen = false, s_both = false;
     int64_t version = 0;
     int64_t stats[GHB_GPMA_STATS] = {};
@@ -1621,9 +1621,12 @@ int ghb_gpma_export(ghb_workspace* ws, ghb_gpma* g, int32_t* rowptr, int32_t* co
     GHB_REQUIRE(ws && g, "NULL workspace / graph");
     GHB_REQUIRE(rowptr && (g->m == 0 || col), "NULL rowptr / col");
     // Straight into the caller's arrays, unless a snapshot is there to copy or the
-    // program also looks at the versions it exports: then the snapshot is made
-    // first and copied.  RMAT-21, after an update: straight 0.38 ms, and as much
-    // again for a look; through the snapshot 0.65, and nothing for a look.
+    // program also looks at the versions it exports, or exports them again: then
+    // the snapshot is made first and copied.  RMAT-21, after an update: straight
+    // 0.38 ms, and as much again for a look or another export; through the snapshot
+    // 0.65, nothing for a look and 0.27 for another export (2^10 vertices: straight
+    // 56 us, another export 34).
+    if (g->s_exported) g->s_both = g->s_seen = true;
     g->s_exported = true;
     if ((!g->s_ok || (w && !g->s_val_ok)) && !g->s_both) return compact_rows(ws, g, rowptr, col, w);
     GHB_TRY(snapshot(ws, g, w != nullptr));

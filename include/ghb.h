@@ -517,7 +517,8 @@ int ghb_gpma_csr(ghb_workspace* ws, ghb_gpma* g, int32_t weights, const int32_t*
                  const int32_t** col, const double** w);
 /* The compact CSR copied into caller buffers (rowptr n + 1, col / w m; w may
  * be NULL).  Written straight from the rows, without the snapshot behind
- * ghb_gpma_csr, unless the program looks at the versions that it exports. */
+ * ghb_gpma_csr, unless the program looks at the versions that it exports or
+ * exports them again. */
 int ghb_gpma_export(ghb_workspace* ws, ghb_gpma* g, int32_t* rowptr, int32_t* col, double* w);
 /* Weight of each key, 0 when the entry is absent. */
 int ghb_gpma_find(ghb_workspace* ws, const ghb_gpma* g, const uint64_t* keys, int64_t count,

@@ -1,6 +1,7 @@
 """What an export and a look at the snapshot launch after a change of the
-dynamic graph: a program that does both pays for the rows' compaction once a
-version, one that only exports never fills the snapshot."""
+dynamic graph: a program that does both, or exports a version again and again,
+pays for the rows' compaction once a version; one that exports each version
+once never fills the snapshot."""
 import pytest
 
 pytest.importorskip("torch")
@@ -54,3 +55,16 @@ def test_launches_by_use():
         check(ex)
         assert n == straight
     assert look() == straight
+    change(0)
+    assert export()[0] == straight  # that version was looked at: by way of the snapshot
+    for k in range(3):
+        change(k)
+        assert export()[0] == straight
+    assert export()[0] == straight  # a version exported again: the snapshot is made
+    for k in range(3):
+        n, ex = export()
+        assert n == 0
+        check(ex)
+    for k in range(3):  # and in the versions that follow with the first export
+        change(k)
+        assert export()[0] == straight and export()[0] == 0
