@@ -41,11 +41,13 @@ def _cache_room(cfg: Dict[str, int], value_bytes: int) -> int:
 
 
 def launched(cfg: Dict[str, int], entries: int, value_bytes: int = 4) -> Dict[str, int]:
-    """`cfg` with the hub cache (bytes, under "pr_cache_kb") that a PageRank call
-    on a resident graph of so many entries gets."""
+    """`cfg` with the hub cache (bytes, under "pr_cache_kb") and the threads that a
+    PageRank call on a resident graph of so many entries gets."""
     if "pr_cache_kb" not in cfg:
         return dict(cfg)
-    kb = cfg["pr_cache_kb"] if entries >= 1 << 24 else min(cfg["pr_cache_kb"], 16)
+    kb = min(cfg["pr_cache_kb"], 0 if entries < 1 << 20 else 16 if entries < 1 << 24 else 1 << 10)
+    threads = min(cfg.get("pr_threads", 1024), 256 if entries < 1 << 18 else 512 if entries < 1 << 20 else 1024)
+    cfg = dict(cfg, pr_threads=threads)
     return dict(cfg, pr_cache_kb=min(kb * 1024, _cache_room(cfg, value_bytes)))
 
 

@@ -512,7 +512,12 @@ int pagerank_impl(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* in_rp,
         m = hp[0];
     }
     const Tuning& tu = ws->tune;
-    const int pthreads = tu.pr_threads;
+    // A small graph's few tiles spread over more blocks, without a cache that each
+    // would have to fill.  An iteration with a look at the change, 1,024 threads and
+    // 16 KB against these: 120 k entries 42.4 and 36.5 us, 200 k 42.7 and 35.5, 430 k
+    // 42.0 and 36.5; 8 k without the look 14.5 and 12.5.  From 2^20 entries on wider
+    // blocks are as good or better (2.4 M 28.7, 30.8 with 512, 35.8 with 256).
+    const int pthreads = std::min(tu.pr_threads, m < (1 << 18) ? 256 : m < (1 << 20) ? 512 : kPrPersistThreads);
     const unsigned max_rows = ws->num_sms * tu.pr_blocks_per_sm;  // persistent blocks
     // Hub cache and the warps' tiles share a block's shared memory.
     const size_t tile_bytes = (size_t)(pthreads / 32) * kPrTile * sizeof(T);
@@ -521,10 +526,10 @@ int pagerank_impl(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* in_rp,
     // entries, FP64, ten iterations: 8.3 ms without a cache, 7.8 with 64 to 96 KB,
     // 8.4 with 112, 13.1 with 144), and where the first ids are not the hubs
     // nothing is gained from 32 KB on (9.7 ms with 0 or 32 KB, 10.8 with 64).
-    // Below 2^24 entries a block gathers too little for its fill (ten iterations
-    // with 16 and 80 KB: 2 M entries 306 and 332 us, 8 M 485 and 498; with 32 M
+    // Below 2^24 entries a block gathers too little for its fill (and below 2^20 for
+    // any; ten iterations with 16 and 80 KB: 2 M entries 306 and 332 us, 8 M 485 and 498; with 32 M
     // 1,260 and 1,220).
-    const int32_t most_kb = m < (1 << 24) ? 16 : ranked ? tu.pr_cache_kb : 32;
+    const int32_t most_kb = m < (1 << 20) ? 0 : m < (1 << 24) ? 16 : ranked ? tu.pr_cache_kb : 32;
     const int32_t cache_kb = std::min(tu.pr_cache_kb, most_kb);
     const size_t cache_bytes = std::min((size_t)cache_kb * 1024,
                                         block_smem > tile_bytes + 1024 ? (block_smem - tile_bytes - 1024) & ~(size_t)255 : 0);

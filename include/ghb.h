@@ -64,9 +64,9 @@ int ghb_workspace_counters(ghb_workspace* ws, int64_t* kernel_launches, int64_t*
 ghb_workspace* ghb_default_workspace(void);
 /* Launch shapes and thresholds of this workspace (no counterpart in the
  * reference): "pr_cache_kb" PageRank hub cache in shared memory (at
- * most: 32 on the caller's ids, 16 below 2^24 entries, and what the block
- * shape leaves room for), "pr_threads" and "pr_blocks_per_sm" its persistent
- * blocks, "pr_short" / "pr_chunk" accepted without effect, "ms_warp_rest" /
+ * most: 32 on the caller's ids, 16 below 2^24 entries, none below 2^20, and
+ * what the block shape leaves room for), "pr_threads" (at most: 512 below
+ * 2^20 entries, 256 below 2^18) and "pr_blocks_per_sm" its persistent blocks, "pr_short" / "pr_chunk" accepted without effect, "ms_warp_rest" /
  * "ms_pull_div" the multi-source BFS's block-row threshold and direction
  * switch, "pol_band" (0-64) the band, in log2
  * units around the direction rule's threshold, inside which the learned
