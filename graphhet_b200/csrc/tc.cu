@@ -15,7 +15,7 @@
 // triangle is met from its 6 ordered edges), and its int32 wraps.
 //
 // On rows in rank order (a resident graph's, or a copy relabelled for the call)
-// the triangles that hold one of the 4,096 highest-ranked vertices are counted
+// that have many probes per entry, the triangles that hold one of the 4,096 highest-ranked vertices are counted
 // through bitmaps of hub neighbours first, and the hash kernels take the rest.
 //
 // Directed rows and rows with loops that are strictly increasing go through the
@@ -39,6 +39,10 @@ constexpr int32_t kTcFlags = 7;
 // Above the flags, the lengths that the rows have: a bit per class of them, so
 // that a count launches only the kernels whose rows exist.
 constexpr int32_t kTcLen32 = 8, kTcLen128 = 16, kTcLen1024 = 32, kTcLen4096 = 64, kTcLenMore = 128;
+constexpr int32_t kTcLengths = kTcLen32 | kTcLen128 | kTcLen1024 | kTcLen4096 | kTcLenMore;
+// Above those, the hash kernels' probes per entry (tc_probes_kernel).
+constexpr int kTcProbesShift = 8;
+constexpr unsigned long long kTcProbesMost = 1 << 20;
 __device__ __forceinline__ int32_t tc_length_bit(int32_t d) {
     return d <= 32 ? kTcLen32 : d <= 128 ? kTcLen128 : d <= 1024 ? kTcLen1024 : d <= 4096 ? kTcLen4096 : kTcLenMore;
 }
@@ -110,6 +114,29 @@ struct CheckVisitor {
 __device__ __forceinline__ bool ranks_above(const int32_t* __restrict__ rowptr, int32_t u, int32_t v) {
     const int32_t du = rowptr[u + 1] - rowptr[u], dv = rowptr[v + 1] - rowptr[v];
     return dv > du || (dv == du && v > u);
+}
+
+// Probes that the hash kernels would make, per entry of the CSR: the sum over
+// a -> b of |N+(b)| is the sum over b of |N+(b)| (d(b) - |N+(b)|), which is d f (1 - f)
+// per entry that leads to b, f being the share of b's row that ranks above b.
+// A warp per sampled entry takes f from 32 entries of the row; kTcProbeSamples
+// of them came within 5 % of the true figure on 29 graphs of 1.3 to 500 probes
+// an entry.  The samples lie at fixed places, so a graph always has the same
+// figure.  sum: in sixteenths.
+constexpr int kTcProbeSamples = 4096;
+__global__ void __launch_bounds__(256) tc_probes_kernel(int64_t m, const int32_t* __restrict__ rowptr,
+                                                        const int32_t* __restrict__ col, unsigned long long* sum) {
+    const int lane = lane_id();
+    const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (i >= kTcProbeSamples) return;
+    const int32_t v = col[((uint64_t)(i * 2654435761u) * (uint64_t)m) >> 32];
+    const int32_t b = rowptr[v], d = rowptr[v + 1] - b;
+    const int32_t k = min(d, 32);
+    bool up = false;
+    if (lane < k) up = ranks_above(rowptr, v, col[b + (int32_t)((int64_t)lane * d / k)]);
+    const int32_t f = __popc(__ballot_sync(0xffffffffu, up));
+    if (lane == 0 && f > 0 && f < k)
+        atomicAdd(sum, (unsigned long long)((int64_t)d * (f * (k - f)) * 16 / (k * k)));
 }
 
 // Adds 1 per call to cnt[u], merged across lanes that share u.
@@ -591,6 +618,14 @@ int tc_count_oriented(ghb_workspace* ws, int32_t first, int32_t n, int64_t m, co
 // Triangles without a hub lie in the rows' tails [he, oe) and go to the hash
 // kernels.  b below kTcBitMin hub neighbours, or of an id past the bitmap
 // table, has its hub neighbours probed one by one in a's bitmap.
+//
+// From kTcHubProbes probes an entry on, that is: below, the rows are short or
+// hold few hubs, and the passes over hubs cost more than they save.  In a
+// resident graph, with and without bitmaps: uniform, 12M entries and 10 probes
+// an entry, 845 us and 551; RMAT-18 of flat degrees, 13 probes, 855 and 511;
+// communities of 95 vertices, 15, 976 and 719; power law of exponent 2.3, 17,
+// 617 and 1,324; uniform, 32 (4,000 vertices), 160 and 511.
+constexpr int32_t kTcHubProbes = 16;
 constexpr int32_t kTcHubs = 4096;
 constexpr int32_t kTcHubWords = kTcHubs / 32;
 constexpr int32_t kTcBitRows = 1 << 18;  // ids that may have a bitmap (512 bytes each, 128 MB)
@@ -870,6 +905,7 @@ __global__ void __launch_bounds__(kTcHubThreads, kTcHubBlocks) tc_hub_items_kern
 }
 
 constexpr int64_t kTcRankEntries = 1 << 20;  // entries from which raw rows may be relabelled for the count
+constexpr int32_t kTcRankProbes = 24;        // and probes per entry
 
 // Scratch of the rank-ordered path.
 struct TcRanked {
@@ -888,12 +924,15 @@ struct TcRanked {
 };
 
 // Triangles of a symmetric, loop-free CSR with strictly increasing rows whose
-// ids are ranks (hubs first), into cnt (zeroed by the caller).
+// ids are ranks (hubs first), into cnt (zeroed by the caller).  probes: the hash
+// kernels' per entry.
 int tc_count_ranked(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* rp, const int32_t* col,
-                    unsigned long long* cnt, const WalkBuffers& wb, int32_t* lists, const TcRanked& r, int32_t lengths) {
+                    unsigned long long* cnt, const WalkBuffers& wb, int32_t* lists, const TcRanked& r, int32_t lengths,
+                    int32_t probes) {
     GHB_TRY(launch(ws, tc_rank_ends_kernel, dim3(grid_for(n, 256, ws->num_sms * 8)), dim3(256), 0, n, rp, col, r.he,
                    r.oe));
-    if (!ws->tune.tc_hash) return tc_count_oriented(ws, 0, n, m, rp, (const int32_t*)r.oe, col, cnt, wb, lists, lengths);
+    if (!ws->tune.tc_hash || probes < kTcHubProbes)
+        return tc_count_oriented(ws, 0, n, m, rp, (const int32_t*)r.oe, col, cnt, wb, lists, lengths);
     GHB_CUDA_TRY(cudaMemsetAsync(r.tails, 0, 3 * sizeof(int32_t), ws->stream));
     GHB_TRY(launch(ws, tc_hub_bitmap_kernel, dim3(grid_for((int64_t)r.bit_rows * 32, 256, ws->num_sms * 8)), dim3(256),
                    0, r.bit_rows, rp, (const int32_t*)r.he, col, r.bits));
@@ -1023,7 +1062,7 @@ int tc_run_cached(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int
                   int32_t* counts32, int64_t* total, std::atomic<int32_t>* flags_cache, bool ranked);
 
 // Raw rows through a copy relabelled by degree (in the workspace's stage); check:
-// the rows' flags.
+// the rows' figures.
 static int tc_by_ranks(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* rowptr, const int32_t* col,
                        int64_t* counts64, int32_t* counts32, int64_t* total, int32_t check) {
     int32_t *perm, *iperm, *rp, *rcol, *repeat, *nact;
@@ -1049,7 +1088,7 @@ static int tc_by_ranks(ghb_workspace* ws, int32_t n, int64_t m, const int32_t* r
                   (const int64_t*)by_rank, counts64, counts32);
 }
 
-// flags_cache (may be NULL): the input check's flags for this CSR, -1 when
+// flags_cache (may be NULL): the input check's figures for this CSR, -1 when
 // not yet known; a known value skips the check.  ranked: ids are ranks by
 // degree, hubs first (a resident graph's).
 int tc_run_cached(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int32_t* col, int64_t* counts64,
@@ -1093,22 +1132,31 @@ int tc_run_cached(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int
     GHB_TRY(reserve());
     int32_t check = flags_cache ? flags_cache->load(std::memory_order_relaxed) : -1;
     if (check < 0) {
-        GHB_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int32_t), st));
+        unsigned long long* probes = reinterpret_cast<unsigned long long*>(flags + 2);
+        GHB_CUDA_TRY(cudaMemsetAsync(flags, 0, 4 * sizeof(int32_t), st));
+        // Where the count that follows may go by it.
+        if (ranked ? m > 0 : m >= kTcRankEntries)
+            GHB_TRY(launch(ws, tc_probes_kernel, dim3(kTcProbeSamples / 8), dim3(256), 0, m, rowptr, col, probes));
         GHB_TRY(walk(ws, rowptr, col, (const int32_t*)nullptr, (const int32_t*)nullptr, (int64_t)n, (int64_t)n, wb,
                      CheckVisitor{rowptr, col, flags}));
-        GHB_CUDA_TRY(cudaMemcpyAsync(hp, flags, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        GHB_CUDA_TRY(cudaMemcpyAsync(hp, flags, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
         GHB_CUDA_TRY(cudaStreamSynchronize(st));
-        check = hp[0];
+        const unsigned long long mean = *reinterpret_cast<const unsigned long long*>(hp + 2) / (16 * kTcProbeSamples);
+        check = hp[0] | (int32_t)(std::min(mean, kTcProbesMost) << kTcProbesShift);
         if (flags_cache) flags_cache->store(check, std::memory_order_relaxed);
     }
     const bool oriented = (check & kTcFlags) == 0;
-    if (oriented && !ranked && ws->tune.tc_hash && check >= kTcLen1024 && m >= kTcRankEntries) {
-        // Rows over 128 entries in a graph that is not small: ranks by degree,
-        // and the hub bitmaps, repay a relabelled copy of the rows (RMAT-19 on
-        // the caller's ids: 9.9 ms by the hash kernels, 3.7 this way).  Without
-        // long rows the copy costs more than the count (an ER graph of as many
-        // entries counts in 1.2 ms), and so it does on a small graph (RMAT,
-        // 1,000 vertices: 0.18 ms against 0.31).
+    const int32_t lengths = check & kTcLengths, probes = check >> kTcProbesShift;
+    if (oriented && !ranked && ws->tune.tc_hash && lengths >= kTcLen1024 && m >= kTcRankEntries &&
+        probes >= kTcRankProbes) {
+        // Ranks by degree, and the hub bitmaps, repay a relabelled copy of the
+        // rows (90 us per million entries) where the hash kernels have many probes
+        // per entry.  By the hash kernels and this way: uniform, 64 vertices of
+        // 30,000 a row, 21 probes, 1.11 ms and 1.33; RMAT-18 of flat degrees, 13,
+        // 1.13 and 1.90; power law of exponent 2.3, 17, 1.47 and 1.61; RMAT-17,
+        // 29, 1.60 and 1.47; RMAT-18 of 4 edges a vertex, 30, 1.25 and 1.01;
+        // RMAT-18, 87, 6.0 and 1.9; a clique of 2,000, 333, 26 and 5.5.  On a
+        // small graph it is slower at any (RMAT, 1,000 vertices: 0.18 and 0.31).
         const int done = tc_by_ranks(ws, n, m, rowptr, col, counts64, counts32, total, check);
         if (done != GHB_ERR_OUT_OF_MEMORY) return done;
         // The copy (20 bytes an entry) does not fit: its place is given back and
@@ -1122,7 +1170,7 @@ int tc_run_cached(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int
         GHB_TRY(reserve());
     }
     if (oriented && ranked) {
-        GHB_TRY(tc_count_ranked(ws, n, m, rowptr, col, cnt, wb, lists, rk, check));
+        GHB_TRY(tc_count_ranked(ws, n, m, rowptr, col, cnt, wb, lists, rk, lengths, probes));
     } else if (oriented) {
         GHB_CUDA_TRY(cudaMemsetAsync(keep, 0, sizeof(int32_t) * n, st));
         GHB_TRY(walk(ws, rowptr, col, (const int32_t*)nullptr, (const int32_t*)nullptr, (int64_t)n, (int64_t)n,
@@ -1130,14 +1178,14 @@ int tc_run_cached(ghb_workspace* ws, int32_t n, const int32_t* rowptr, const int
         GHB_TRY(scan_exclusive_i32(ws, keep, orp, n, bsums));
         GHB_TRY(orient_fill(ws, n, rowptr, col, orp, ocol, lists));
         GHB_TRY(tc_count_oriented(ws, 0, n, m, (const int32_t*)orp, (const int32_t*)orp + 1, (const int32_t*)ocol, cnt,
-                                  wb, lists, check));
-    } else if (!(check & kTcFlagUnsorted) && ws->tune.tc_hash && check >= kTcLen128) {
+                                  wb, lists, lengths));
+    } else if (!(check & kTcFlagUnsorted) && ws->tune.tc_hash && lengths >= kTcLen128) {
         // Directed rows, loops: on strictly increasing rows the reference's
         // merge is an intersection, which the hash kernels count for every
         // entry of the rows themselves (directed RMAT-19 in a resident graph:
         // 2.4 s by one lane's merge per entry, 59 ms by the kernels).  Rows of
         // up to 32 entries merge in fewer launches.
-        GHB_TRY(tc_count_oriented(ws, 0, n, m, rowptr, rowptr + 1, col, cnt, wb, lists, check));
+        GHB_TRY(tc_count_oriented(ws, 0, n, m, rowptr, rowptr + 1, col, cnt, wb, lists, lengths));
     } else {
         GHB_TRY(walk(ws, rowptr, col, (const int32_t*)nullptr, (const int32_t*)nullptr, (int64_t)n, (int64_t)n, wb,
                      MergeVisitor{rowptr, col, cnt}));
