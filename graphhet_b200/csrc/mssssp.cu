@@ -44,6 +44,15 @@ namespace {
 // to 1,024 entries on one warp, an entry at a time.
 constexpr int32_t kMsspWarpRow = 32;
 constexpr int32_t kMsspChunk = 32;
+// The pass in one launch cuts at twice that from 2^21 entries, and 2^18 per source
+// (a chunk takes longer with each): the warps have chunks enough, and half as
+// many cost less to list and to draw.  With 32 and 64: clique of 3,000, 9M entries,
+// 1 source, 1.01 ms and 0.81; uniform, 34M, 8 sources, 32 and 23; RMAT-18, 7.6M, 2,
+// 1.50 and 1.34; but RMAT-14, 0.4M, 16, 0.83 and 0.97, and RMAT-18, 64, 8.7 and 9.4.
+constexpr int64_t kMsspCutEntries = 1 << 21, kMsspCutPerSource = 1 << 18;
+inline int32_t mssp_row_cut(int64_t m, int32_t k) {
+    return m >= std::max(kMsspCutEntries, kMsspCutPerSource * k) ? 2 * kMsspChunk : kMsspChunk;
+}
 constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;  // +infinity
 
 struct MsspCounters {
@@ -415,8 +424,8 @@ __global__ void __launch_bounds__(kMsspThreads, kMsspBlocks) mssp_pass_kernel(
     int32_t n, int32_t n_active, int32_t k, int32_t ks, int32_t words, const int32_t* __restrict__ rp,
     const int32_t* __restrict__ col, const double* __restrict__ wt, const int32_t* srcs, const int32_t* __restrict__ perm,
     double inf, double* dist_out, unsigned long long* d, unsigned long long* act_a, unsigned long long* act_b,
-    int32_t* inq_a, int32_t* inq_b, int32_t* q_a, int32_t* q_b, int4* chunks, MsspCounters* cnt, MsspRunState* st,
-    unsigned long long bar_limit_ns, unsigned bar_extra) {
+    int32_t* inq_a, int32_t* inq_b, int32_t* q_a, int32_t* q_b, int4* chunks, int32_t cut, MsspCounters* cnt,
+    MsspRunState* st, unsigned long long bar_limit_ns, unsigned bar_extra) {
     const int64_t gtid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t gsize = (int64_t)gridDim.x * blockDim.x;
     const int64_t warp = gtid >> 5;
@@ -478,14 +487,14 @@ __global__ void __launch_bounds__(kMsspThreads, kMsspBlocks) mssp_pass_kernel(
             for (int64_t i = warp; i < q; i += nwarps) {
                 const int32_t v = __ldcg(q_cur + i);
                 const int32_t eb = rp[v], ee = rp[v + 1];
-                if (ee - eb > kMsspWarpRow) {
-                    const int32_t nc = chunk_count(ee - eb, kMsspChunk);
+                if (ee - eb > cut) {
+                    const int32_t nc = chunk_count(ee - eb, cut);
                     int32_t pos = 0;
                     if (lane == 0) pos = atomicAdd(&st->c_tail, nc);
                     pos = __shfl_sync(0xffffffffu, pos, 0);
                     for (int32_t c = lane; c < nc; c += 32) {
-                        const int32_t cb = eb + c * kMsspChunk;
-                        chunks[pos + c] = make_int4(v, cb, chunk_end(cb, kMsspChunk, ee), 0);
+                        const int32_t cb = eb + c * cut;
+                        chunks[pos + c] = make_int4(v, cb, chunk_end(cb, cut, ee), 0);
                     }
                     continue;
                 }
@@ -636,8 +645,9 @@ int mssssp_pass_one_launch(ghb_workspace* ws, int32_t n, int32_t n_active, int64
     cudaStream_t st = ws->stream;
     const int32_t ks = (k + 31) & ~31;
     const int32_t words = (ks + 63) / 64;
-    // Chunks of one round: rows over kMsspWarpRow entries, ceil(len / kMsspChunk) each.
-    const int64_t chunk_cap = m / kMsspChunk + m / kMsspWarpRow + 64;
+    // Chunks of one round: rows over `cut` entries, ceil(len / cut) each.
+    const int32_t cut = mssp_row_cut(m, k);
+    const int64_t chunk_cap = 2 * (m / cut) + 64;
     auto carve = [&](Carver& c, unsigned long long** d, unsigned long long** aa, unsigned long long** ab,
                      int32_t** ia, int32_t** ib, int32_t** qa, int32_t** qb, int4** ch, MsspCounters** cnt,
                      MsspRunState** rs) {
@@ -671,8 +681,8 @@ int mssssp_pass_one_launch(ghb_workspace* ws, int32_t n, int32_t n_active, int64
         GHB_CUDA_TRY(cudaMemcpyAsync(&rs->budget, &budget, sizeof(budget), cudaMemcpyHostToDevice, st));
     }
     GHB_TRY(launch_coop(ws, mssp_pass_kernel, dim3(blocks), dim3(kMsspThreads), (size_t)0, n, n_active, k, ks, words,
-                        rp, col, wt, srcs_dev, perm, inf, dist_out, d, act_a, act_b, inq_a, inq_b, q_a, q_b, ch, cnt,
-                        rs, (unsigned long long)ws->tune.barrier_limit_us * 1000ull,
+                        rp, col, wt, srcs_dev, perm, inf, dist_out, d, act_a, act_b, inq_a, inq_b, q_a, q_b, ch, cut,
+                        cnt, rs, (unsigned long long)ws->tune.barrier_limit_us * 1000ull,
                         (unsigned)ws->tune.barrier_extra));
     GHB_CUDA_TRY(cudaMemcpyAsync(ws->host_pinned, rs, sizeof(MsspRunState), cudaMemcpyDeviceToHost, st));
     GHB_CUDA_TRY(cudaStreamSynchronize(st));
