@@ -164,6 +164,7 @@ __device__ __forceinline__ void mssp_queue(bool want, int32_t u, int32_t* inq_ne
 // the new one is lowered without waiting for the answer; whoever else lowers it
 // meanwhile marks the same target, so nothing is lost.  Targets are queued once
 // per 32 entries.
+constexpr int kMsspFew = 4;     // active sources from which lanes go over them
 constexpr int kMsspFlight = 4;  // distance loads in flight per lane
 struct MsspArrays {
     const int32_t* __restrict__ col;
@@ -233,53 +234,58 @@ __device__ __forceinline__ void mssp_relax_wide(const MsspArrays& a, int32_t v, 
         if (hit) mssp_queue((hit >> lane) & 1u, uj, a.inq_next, a.queue_next, a.cnt, g);
     }
 }
-// Lanes over entries, the few active sources one after another.
-__device__ __forceinline__ void mssp_relax_narrow(const MsspArrays& a, int32_t v, int32_t eb, int32_t ee,
-                                                  MsspStage& g) {
+// Lanes over entries, the few active sources (bits of act word w) one after another.
+__device__ __forceinline__ void mssp_relax_word(const MsspArrays& a, int32_t v, int32_t eb, int32_t ee, int w,
+                                                unsigned long long bits, MsspStage& g) {
     constexpr int kB = 4;
     const int lane = lane_id();
-    for (int w = 0; w < a.words; ++w) {
-        unsigned long long bits = __ldcg(a.act_cur + (int64_t)v * a.words + w);
-        while (bits) {
-            const int b = __ffsll((long long)bits) - 1;
-            const int s = w * 64 + b;
-            bits &= bits - 1;
-            const double dv = __longlong_as_double((long long)__ldcg(a.d + (int64_t)v * a.ks + s));
-            for (int64_t j0 = eb; j0 < ee; j0 += 32 * kB) {
-                int32_t u[kB];
-                double nd[kB], cur[kB];
+    while (bits) {
+        const int b = __ffsll((long long)bits) - 1;
+        const int s = w * 64 + b;
+        bits &= bits - 1;
+        const double dv = __longlong_as_double((long long)__ldcg(a.d + (int64_t)v * a.ks + s));
+        for (int64_t j0 = eb; j0 < ee; j0 += 32 * kB) {
+            int32_t u[kB];
+            double nd[kB], cur[kB];
 #pragma unroll
-                for (int q = 0; q < kB; ++q) {
-                    const int64_t j = j0 + 32 * q + lane;
-                    u[q] = j < ee ? a.col[j] : -1;
-                    nd[q] = j < ee ? dv + a.wt[j] : 0.0;
-                }
-#pragma unroll
-                for (int q = 0; q < kB; ++q)
-                    cur[q] = u[q] >= 0 ? __longlong_as_double((long long)__ldcg(a.d + (int64_t)u[q] * a.ks + s)) : 0.0;
-                unsigned near = 0;
-#pragma unroll
-                for (int q = 0; q < kB; ++q)
-                    if (u[q] >= 0 && nd[q] < cur[q]) {
-                        atomicMin(a.d + (int64_t)u[q] * a.ks + s, (unsigned long long)__double_as_longlong(nd[q]));
-                        if (nd[q] < a.hi) {
-                            atomicOr(a.act_next + (int64_t)u[q] * a.words + w, 1ull << b);
-                            near |= 1u << q;
-                        }
-                    }
-                if (!__any_sync(0xffffffffu, near != 0)) continue;
-#pragma unroll
-                for (int q = 0; q < kB; ++q)
-                    mssp_queue((near >> q) & 1u, u[q], a.inq_next, a.queue_next, a.cnt, g);
+            for (int q = 0; q < kB; ++q) {
+                const int64_t j = j0 + 32 * q + lane;
+                u[q] = j < ee ? a.col[j] : -1;
+                nd[q] = j < ee ? dv + a.wt[j] : 0.0;
             }
+#pragma unroll
+            for (int q = 0; q < kB; ++q)
+                cur[q] = u[q] >= 0 ? __longlong_as_double((long long)__ldcg(a.d + (int64_t)u[q] * a.ks + s)) : 0.0;
+            unsigned near = 0;
+#pragma unroll
+            for (int q = 0; q < kB; ++q)
+                if (u[q] >= 0 && nd[q] < cur[q]) {
+                    atomicMin(a.d + (int64_t)u[q] * a.ks + s, (unsigned long long)__double_as_longlong(nd[q]));
+                    if (nd[q] < a.hi) {
+                        atomicOr(a.act_next + (int64_t)u[q] * a.words + w, 1ull << b);
+                        near |= 1u << q;
+                    }
+                }
+            if (!__any_sync(0xffffffffu, near != 0)) continue;
+#pragma unroll
+            for (int q = 0; q < kB; ++q)
+                mssp_queue((near >> q) & 1u, u[q], a.inq_next, a.queue_next, a.cnt, g);
         }
     }
 }
+// FEW: fewer than kMsspFew sources in all, so one act word that is read once.
+template <bool FEW>
 __device__ __forceinline__ void mssp_relax_range(int32_t v, int32_t eb, int32_t ee, const MsspArrays& a,
                                                  unsigned long long& examined, MsspStage& stage) {
+    if constexpr (FEW) {
+        const unsigned long long bits = __ldcg(a.act_cur + v);
+        mssp_relax_word(a, v, eb, ee, 0, bits, stage);
+        if (lane_id() == 0) examined += (unsigned long long)(ee - eb) * (unsigned long long)__popcll(bits);
+        return;
+    }
     int nact = 0;
     for (int w = 0; w < a.words; ++w) nact += __popcll(__ldcg(a.act_cur + (int64_t)v * a.words + w));
-    if (nact >= 4) {
+    if (nact >= kMsspFew) {
         // 64 sources at a time: the row's entries come from L1 after the first
         // walk, and are few bytes beside the distances.
         const int groups = a.ks >> 5;
@@ -287,7 +293,8 @@ __device__ __forceinline__ void mssp_relax_range(int32_t v, int32_t eb, int32_t 
         for (; g + 2 <= groups; g += 2) mssp_relax_wide<2>(a, v, eb, ee, g, stage);
         if (g < groups) mssp_relax_wide<1>(a, v, eb, ee, g, stage);
     } else {
-        mssp_relax_narrow(a, v, eb, ee, stage);
+        for (int w = 0; w < a.words; ++w)
+            mssp_relax_word(a, v, eb, ee, w, __ldcg(a.act_cur + (int64_t)v * a.words + w), stage);
     }
     if (lane_id() == 0) examined += (unsigned long long)(ee - eb) * (unsigned long long)nact;
 }
@@ -315,7 +322,7 @@ __global__ void __launch_bounds__(256) mssp_relax_kernel(int32_t q, const int32_
             if (lane_id() == 0) big[atomicAdd(&cnt_cur->big, 1)] = v;
             continue;
         }
-        mssp_relax_range(v, eb, ee, arrays, examined, stage);
+        mssp_relax_range<false>(v, eb, ee, arrays, examined, stage);
     }
     mssp_flush(stage, queue_next, cnt);
     if (lane_id() == 0 && examined) atomicAdd(&cnt->examined, examined);
@@ -361,7 +368,7 @@ __global__ void __launch_bounds__(256) mssp_relax_big_kernel(const int32_t* __re
         const int32_t v = big[lo];
         const int32_t eb = rp[v] + (int32_t)(c - cpre[lo]) * kMsspChunk;
         const int32_t ee = chunk_end(eb, kMsspChunk, rp[v + 1]);
-        mssp_relax_range(v, eb, ee, arrays, examined, stage);
+        mssp_relax_range<false>(v, eb, ee, arrays, examined, stage);
     }
     mssp_flush(stage, queue_next, cnt);
     if (lane_id() == 0 && examined) atomicAdd(&cnt->examined, examined);
@@ -420,6 +427,11 @@ __device__ __forceinline__ double mp_pmin(const MsspCounters* c) {
 // 3.7; 32 sources on a 512 x 512 grid 29 ms.  Without the staging, an atomic on
 // one cache line for every vertex queued and every warp's sums in every phase,
 // 10.8, 4.8 and 43 ms.  What is left waits on gathers and minima.
+// FEW, without the code for many active sources: no spill.  A star of 2^20
+// vertices, 1 source, 1.24 ms by the other kernel and 1.05 (1.15 without the bounds
+// of 32 vertices at a time), RMAT-20, 2 sources, 5.7 and 5.0, a 700 x 700 grid 21.7
+// and 21.3; five blocks per SM spill (grid 22.3), six and eight more.
+template <bool FEW>
 __global__ void __launch_bounds__(kMsspThreads, kMsspBlocks) mssp_pass_kernel(
     int32_t n, int32_t n_active, int32_t k, int32_t ks, int32_t words, const int32_t* __restrict__ rp,
     const int32_t* __restrict__ col, const double* __restrict__ wt, const int32_t* srcs, const int32_t* __restrict__ perm,
@@ -484,9 +496,31 @@ __global__ void __launch_bounds__(kMsspThreads, kMsspBlocks) mssp_pass_kernel(
         if (phase == kMpScan) {
             mssp_scan_body(n_active, ks, words, lo, hi, d, act_cur, q_cur, cn, stage);
         } else if (phase == kMpRelax) {
-            for (int64_t i = warp; i < q; i += nwarps) {
-                const int32_t v = __ldcg(q_cur + i);
-                const int32_t eb = rp[v], ee = rp[v + 1];
+            // Many vertices a warp: the bounds of 32 are loaded together, a round trip
+            // to the queue and one to the rows for all of them.
+            const bool ahead = FEW && q >= 4 * nwarps;
+            int32_t lv = 0, lb = 0, le = 0;
+            int at = 32;
+            for (int64_t i = warp; i < q; i += nwarps, ++at) {
+                int32_t v, eb, ee;
+                if (ahead) {
+                    if (at == 32) {
+                        at = 0;
+                        const int64_t j = i + lane * nwarps;
+                        if (j < q) {
+                            lv = __ldcg(q_cur + j);
+                            lb = rp[lv];
+                            le = rp[lv + 1];
+                        }
+                    }
+                    v = __shfl_sync(0xffffffffu, lv, at);
+                    eb = __shfl_sync(0xffffffffu, lb, at);
+                    ee = __shfl_sync(0xffffffffu, le, at);
+                } else {
+                    v = __ldcg(q_cur + i);
+                    eb = rp[v];
+                    ee = rp[v + 1];
+                }
                 if (ee - eb > cut) {
                     const int32_t nc = chunk_count(ee - eb, cut);
                     int32_t pos = 0;
@@ -498,13 +532,13 @@ __global__ void __launch_bounds__(kMsspThreads, kMsspBlocks) mssp_pass_kernel(
                     }
                     continue;
                 }
-                mssp_relax_range(v, eb, ee, arrays, examined, stage);
+                mssp_relax_range<FEW>(v, eb, ee, arrays, examined, stage);
             }
             mssp_flush(stage, q_next, cn);
         } else if (phase == kMpChunks) {
             for (int64_t i = warp; i < nch; i += nwarps) {
                 const int4 ch = __ldcg(chunks + i);
-                mssp_relax_range(ch.x, ch.y, ch.z, arrays, examined, stage);
+                mssp_relax_range<FEW>(ch.x, ch.y, ch.z, arrays, examined, stage);
             }
             mssp_flush(stage, q_next, cn);
         } else {  // kMpClear: the processed vertices' act words and queue flags
@@ -613,6 +647,7 @@ __global__ void mssp_sources_kernel(int32_t k, const int32_t* __restrict__ perm,
 
 }  // namespace
 
+template <bool FEW>
 static int mssp_pass_blocks(ghb_workspace* ws) {
     static int cached[64] = {0};
     const int dev = ws->device;
@@ -620,7 +655,7 @@ static int mssp_pass_blocks(ghb_workspace* ws) {
     if (!cached[dev]) {
         int coop = 0, per_sm = 0;
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-        if (coop && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mssp_pass_kernel, kMsspThreads, 0) ==
+        if (coop && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mssp_pass_kernel<FEW>, kMsspThreads, 0) ==
                         cudaSuccess)
             cached[dev] = std::max(0, std::min(per_sm, kMsspBlocks)) * ws->num_sms;
         if (!cached[dev]) cached[dev] = -1;
@@ -637,7 +672,8 @@ int mssssp_pass_one_launch(ghb_workspace* ws, int32_t n, int32_t n_active, int64
                            int64_t* examined_out) {
     GHB_REQUIRE(k >= 1 && k <= 256, "multi-source SSSP pass of 1..256 sources");
     GHB_REQUIRE(delta > 0 && std::isfinite(delta), "bucket width must be positive");
-    const int blocks = mssp_pass_blocks(ws);
+    const bool few = k < kMsspFew;
+    const int blocks = few ? mssp_pass_blocks<true>(ws) : mssp_pass_blocks<false>(ws);
     if (blocks <= 0) {
         set_error("cooperative launch unavailable");
         return GHB_ERR_UNSUPPORTED;
@@ -680,7 +716,7 @@ int mssssp_pass_one_launch(ghb_workspace* ws, int32_t n, int32_t n_active, int64
         GHB_CUDA_TRY(cudaMemcpyAsync(&rs->delta, &dl, sizeof(dl), cudaMemcpyHostToDevice, st));
         GHB_CUDA_TRY(cudaMemcpyAsync(&rs->budget, &budget, sizeof(budget), cudaMemcpyHostToDevice, st));
     }
-    GHB_TRY(launch_coop(ws, mssp_pass_kernel, dim3(blocks), dim3(kMsspThreads), (size_t)0, n, n_active, k, ks, words,
+    GHB_TRY(launch_coop(ws, few ? mssp_pass_kernel<true> : mssp_pass_kernel<false>, dim3(blocks), dim3(kMsspThreads), (size_t)0, n, n_active, k, ks, words,
                         rp, col, wt, srcs_dev, perm, inf, dist_out, d, act_a, act_b, inq_a, inq_b, q_a, q_b, ch, cut,
                         cnt, rs, (unsigned long long)ws->tune.barrier_limit_us * 1000ull,
                         (unsigned)ws->tune.barrier_extra));
@@ -838,7 +874,7 @@ int mssssp_run(ghb_workspace* ws, int32_t n, int32_t n_active, const int32_t* rp
     int32_t* sdev = static_cast<int32_t*>(ws->stage);
     if (stats) GHB_CUDA_TRY(cudaEventRecord(ws->ev_start, st));
     int64_t rounds = 0, examined = 0;
-    const bool one_launch = ws->tune.mssp_persistent && mssp_pass_blocks(ws) > 0;
+    const bool one_launch = ws->tune.mssp_persistent && mssp_pass_blocks<false>(ws) > 0;
     if (one_launch && m < 0) {
         int32_t* hp = reinterpret_cast<int32_t*>(ws->host_pinned);
         GHB_CUDA_TRY(cudaMemcpyAsync(hp, rp + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));

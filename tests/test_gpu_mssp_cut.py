@@ -43,3 +43,23 @@ def test_cut(graph, k):
             assert np.array_equal(dist[i], O.sssp(graph, int(sources[i]))), (log2, i)
     rg.close()
     ws.close()
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4])
+def test_wide_rounds_of_short_rows(k):
+    """Rounds of many vertices a warp (the bounds of 32 loaded together): stars
+    whose leaves, 200,000 of them or some tens of thousands, have one entry or two."""
+    import graphhet_b200 as G
+    rng = np.random.default_rng(k)
+    leaves, n = 200000, 200000 + 40
+    leaf = np.arange(40, n)
+    src = np.concatenate([rng.integers(0, 3, leaves), rng.integers(3, 40, leaves // 5)])
+    dst = np.concatenate([leaf, leaf[rng.permutation(leaves)[:leaves // 5]]])
+    og = O.make_graph(n, src.astype(np.int32), dst.astype(np.int32), False, weight_mode=1, weight_seed=k)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    rg = G.ResidentGraph(G.CSRGraph(n=og.n, rowptr=t(og.rowptr), col=t(og.col), w=t(og.w), directed=False))
+    sources = [0, 50000, 7, 1][:k]
+    dist = rg.mssssp(sources)[0].cpu().numpy()
+    for i in range(k):
+        assert np.array_equal(dist[i], O.sssp(og, sources[i])), i
+    rg.close()
